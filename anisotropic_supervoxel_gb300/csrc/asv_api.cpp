@@ -1300,7 +1300,7 @@ asv_status asv_jfa_pass_host(asv_ctx *ctx, int step, float ratio, const int32_t 
     size_t n = (size_t)s.nvox;
     int32_t *din = ctx->d.labA + s.vox_off, *dout = ctx->d.labB + s.vox_off;
     CK(cudaMemcpyAsync(din, in, 4 * n, cudaMemcpyHostToDevice, ctx->st));
-    asv_launch_jfa_single(ctx->d, din, dout, step, ratio, ctx->st);
+    asv_launch_jfa_single(ctx->d, din, s.nvox, s.Kp, dout, step, ratio, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout, 4 * n, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));

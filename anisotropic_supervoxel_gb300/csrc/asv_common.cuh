@@ -112,7 +112,7 @@ void asv_launch_draw(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa(const AsvDev &d, int pass, int grid_blocks, cudaStream_t st);
 void asv_launch_jfa_first_scatter(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa_second_scatter(const AsvDev &d, cudaStream_t st);
-void asv_launch_jfa_single(const AsvDev &d, const int32_t *in, int32_t *out, int step, float ratio,
+void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
                            cudaStream_t st);
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);

@@ -686,6 +686,18 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // the voxel through the shader's ordered scan of its 27 candidates instead,
 // so every label equals the shader's.
 //
+// The passes are bound by instruction issue, so the three steps before the
+// walk handle four entries (a quad) per thread and access: a quad is copied
+// by one 16-byte cp.async where the width allows it, numbered through a byte
+// map that itself says which labels have a number (three instructions per
+// entry where a claimed-bits test took about seventeen), and converted with
+// one 16-byte load and store.  Each thread numbers the quads it copied, so
+// no barrier stands between; with the slot slices worked out by every warp
+// and the byte map reset behind the walk, a sub-tile has three barriers
+// (six before).  A 1280x720x30 window of 20 iterations: 65.2 -> 52.9 ms, the
+// 320x240x85 clip 13.9 -> 12.1 ms.  Widths that are no multiple of four
+// copy their quads by four 4-byte cp.async.
+//
 // Footprint slices ("slots") of a sub-tile of n chain positions: slot 0 the
 // minus slice of position 0, slots 1..n the centre slices, slot n+1 the plus
 // slice of position n-1, and where a chain ends inside the sub-tile slot
@@ -699,10 +711,12 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 #define ASV_BITS_MAXT 32         // labels per sub-tile footprint (one 32-bit mask)
 #define ASV_BITS_MAXKP 8192      // segment seed counts up to this use the bit-set form
 #define ASV_BITS_TLCAP 256       // claimed labels remembered for the reset
-#define ASV_BITS_NONE 255        // table number of no label
+#define ASV_BITS_FREE 255        // map8: label without a number yet
+#define ASV_BITS_NOLABEL 254     // map8[ASV_BITS_MAXKP]: no label (shifts to no bit)
+#define ASV_BITS_OVER 253        // map8: a label past the 32nd (the sub-tile takes the list form)
 #define ASV_ACC_ROW 7            // words per entry of the sub-tile's centroid-sum table (odd: the
                                  // entries' rows start in different shared-memory banks)
-#define ASV_BITS_AREA 62464      // shared bytes of the largest sub-tiles (step 4, 16 positions; step 6, 12)
+#define ASV_BITS_AREA 62464      // shared bytes of the largest sub-tiles (step 4, 16 positions)
 #define ASV_JFA_AREA (ASV_BITS_AREA > ASV_JFA_LIST_BYTES ? ASV_BITS_AREA : ASV_JFA_LIST_BYTES)
 
 struct AsvBitsShared {
@@ -712,19 +726,27 @@ struct AsvBitsShared {
     int tlab[ASV_BITS_TLCAP];                   // label of each number
     int slotz[20];                              // slice of each footprint slot
     int tcount;
-    unsigned char map8[ASV_BITS_MAXKP];         // number of each claimed label
+    unsigned char map8[ASV_BITS_MAXKP + 4];     // number of each claimed label, ASV_BITS_FREE between
 };
 #define ASV_JFA_SMEM (ASV_JFA_AREA + (int)sizeof(AsvBitsShared))
 
+// The footprint of a slot is kept as rows of 16-byte groups of four entries
+// (quads): its left edge is rounded down to four columns, so that for widths
+// that are multiples of four a quad is one aligned 16-byte copy, and a thread
+// numbers and converts four entries per shared-memory access.
 template <int S> struct AsvBitsGeo {
-    static constexpr int FW = ASV_TILE_X + 2 * S;                     // footprint width and height
-    static constexpr int FP = FW * FW;                                // footprint entries per slot
-    // chain positions per sub-tile: deep where the footprint stays small
-    static constexpr int SUB = S <= 4 ? 16 : 12;
+    static constexpr int AL = (S + 3) & ~3;                           // columns kept left and right of the tile
+    static constexpr int FW = ASV_TILE_X + 2 * AL;                    // footprint width and height
+    static constexpr int FH = ASV_TILE_Y + 2 * S;
+    static constexpr int FP = FW * FH;                                // footprint entries per slot
+    static constexpr int QW = FW / 4, QPS = FP / 4;                   // quads per row and per slot
+    // chain positions per sub-tile: as many as the shared area holds, up to
+    // 16 (steps 5-6: 10)
+    static constexpr int SUB = S <= 4 ? 16 : 10;
     static constexpr int NSLOT = SUB + 4;
-    static constexpr int NCOL = (FP + ASV_JFA_THREADS - 1) / ASV_JFA_THREADS;
     static constexpr int FLAB_BYTES = NSLOT * FP * 4;
     static_assert(FLAB_BYTES + SUB * ASV_JFA_THREADS * 4 <= ASV_BITS_AREA, "bit-set sub-tile exceeds the shared area");
+    static_assert(NSLOT <= 20, "slotz");
 };
 
 // 4-byte asynchronous copy global -> shared (cp.async, completed by
@@ -734,9 +756,72 @@ __device__ __forceinline__ void asv_cp_async4(void *dst, const void *src)
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
+// 16-byte form: both addresses 16-byte aligned (through L2 only: a tile's
+// footprint is read once per SM)
+__device__ __forceinline__ void asv_cp_async16(void *dst, const void *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
 __device__ __forceinline__ void asv_cp_async_wait()
 {
     asm volatile("cp.async.commit_group;\ncp.async.wait_all;\n" ::: "memory");
+}
+
+// Copies the four entries of one volume row from column x (any, also outside
+// the row: clamp to edge) to four shared words.  vec: the row width is a
+// multiple of four, so a quad inside the row is 16-byte aligned (x is a
+// multiple of four, the volumes start on a 2048-voxel boundary).
+__device__ __forceinline__ void asv_copy_quad(void *dst, const int32_t *__restrict__ src, int row, int x, int W,
+                                              bool vec)
+{
+    char *q = (char *)dst;
+    if (x >= 0 && x + 3 < W) {
+        const int32_t *g = src + row + x;
+        if (vec) asv_cp_async16(q, g);
+        else {
+#pragma unroll
+            for (int i = 0; i < 4; i++) asv_cp_async4(q + 4 * i, g + i);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; i++) asv_cp_async4(q + 4 * i, src + row + min(max(x + i, 0), W - 1));
+    }
+}
+
+// index of a label in map8: labels lie in [-1, Kp), no label is the last entry
+__device__ __forceinline__ unsigned asv_bits_slot(int v) { return min((unsigned)v, (unsigned)ASV_BITS_MAXKP); }
+
+// 1 << n, 0 for n > 31 (PTX shl clamps the amount)
+__device__ __forceinline__ unsigned asv_bit(unsigned n)
+{
+    unsigned r;
+    asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(n));
+    return r;
+}
+
+// a label seen without a number: the thread that claims it gives it the next one
+__device__ __forceinline__ void asv_bits_claim(AsvBitsShared &b, unsigned v)
+{
+    const unsigned bit = 1u << (v & 31);
+    if (atomicOr(&b.claim[v >> 5], bit) & bit) return;
+    const int idx = atomicAdd(&b.tcount, 1);
+    if (idx < ASV_BITS_TLCAP) b.tlab[idx] = (int)v;
+    b.map8[v] = (unsigned char)(idx < ASV_BITS_MAXT ? idx : ASV_BITS_OVER);
+}
+
+// the labels and claims of a finished sub-tile: back to unnumbered
+__device__ __forceinline__ void asv_bits_reset(AsvBitsShared &b, int T)
+{
+    if (T <= ASV_BITS_TLCAP) {
+        for (int i = threadIdx.x; i < T; i += ASV_JFA_THREADS) {
+            b.claim[b.tlab[i] >> 5] = 0u;
+            b.map8[b.tlab[i]] = ASV_BITS_FREE;
+        }
+    } else {
+        for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 32; i += ASV_JFA_THREADS) b.claim[i] = 0u;
+        for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 4; i += ASV_JFA_THREADS) ((unsigned *)b.map8)[i] = 0xffffffffu;
+    }
 }
 
 // The shader's ordered scan of the 27 candidates (slices centre, minus,
@@ -803,68 +888,67 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     const int x = min(gx, W - 1), y = min(gy, H - 1);
     const int col = y * W + x;
 
-    // slices of the footprint slots
-    bool brk = false;
-    if (tid < n) {
-        int r, j, len;
-        asv_chain_pos(p0 + tid, D, S, r, j, len);
-        const int z = r + j * S;
-        b.slotz[1 + tid] = z;
-        if (tid == 0) b.slotz[0] = max(z - S, 0);
-        if (tid == n - 1) b.slotz[n + 1] = z + S < D ? z + S : D - 1;
-        brk = tid < n - 1 && z + S >= D;
+    // slices of the footprint slots: every warp works them out and writes
+    // the same values, so no barrier is needed before they are read; brk
+    // has a bit for each position but the last where a chain ends
+    unsigned brk;
+    {
+        bool end = false;
+        if (lane < n) {
+            int r, j, len;
+            asv_chain_pos(p0 + lane, D, S, r, j, len);
+            const int z = r + j * S;
+            b.slotz[1 + lane] = z;
+            if (lane == 0) b.slotz[0] = max(z - S, 0);
+            if (lane == n - 1) b.slotz[n + 1] = z + S < D ? z + S : D - 1;
+            end = lane < n - 1 && z + S >= D;
+        }
+        if (lane == 0) { b.slotz[n + 2] = 0; b.slotz[n + 3] = D - 1; }
+        brk = __ballot_sync(0xffffffffu, end);
+        __syncwarp();
     }
-    if (tid == 0) { b.slotz[n + 2] = 0; b.slotz[n + 3] = D - 1; }
-    const bool any_brk = __syncthreads_or(brk);
-    const int nf = any_brk ? n + 4 : n + 2;
+    const int nf = brk ? n + 4 : n + 2;
 
     // footprint labels (clamp-to-edge) and the voxels' LAB, copied
-    // asynchronously; each thread copies the same footprint columns of every slot
-    int coff[G::NCOL];
-#pragma unroll
-    for (int i = 0; i < G::NCOL; i++) {
-        const int e = tid + i * ASV_JFA_THREADS, fy = e / FW, fx = e - fy * FW;
-        coff[i] = min(max(ty0 - S + fy, 0), H - 1) * W + min(max(tx0 - S + fx, 0), W - 1);
-    }
-    for (int k = 0; k < nf; k++) {
-        const int32_t *src = in + b.slotz[k] * sl;
-#pragma unroll
-        for (int i = 0; i < G::NCOL; i++) {
-            const int e = tid + i * ASV_JFA_THREADS;
-            if (e < FP) asv_cp_async4(flab + k * FP + e, src + coff[i]);
+    // asynchronously a quad at a time
+    const bool vec = (W & 3) == 0;
+    const int items = nf * G::QPS;
+    {
+        int slot = tid / G::QPS, q = tid - slot * G::QPS;
+        for (int e = tid; e < items; e += ASV_JFA_THREADS) {
+            const int fy = q / G::QW, fx = q - fy * G::QW;
+            asv_copy_quad(flab + 4 * e, in, b.slotz[slot] * sl + min(max(ty0 - S + fy, 0), H - 1) * W,
+                          tx0 - G::AL + 4 * fx, W, vec);
+            q += ASV_JFA_THREADS % G::QPS;
+            slot += ASV_JFA_THREADS / G::QPS;
+            if (q >= G::QPS) { q -= G::QPS; slot++; }
         }
+        const int q4 = tid & 63, lyy = min(ty0 + (q4 >> 2), H - 1);
+        for (int j = tid >> 6; j < n; j += 4)
+            asv_copy_quad(labsh + j * ASV_JFA_THREADS + 4 * q4, (const int32_t *)lab, b.slotz[j + 1] * sl + lyy * W,
+                          tx0 + 4 * (q4 & 3), W, vec);
     }
-    for (int j = 0; j < n; j++) asv_cp_async4(labsh + j * ASV_JFA_THREADS + tid, lab + b.slotz[j + 1] * sl + col);
     asv_cp_async_wait();
-    __syncthreads();
 
-    // number the distinct labels (each thread its own entries)
-    for (int k = 0; k < nf; k++) {
-#pragma unroll
-        for (int i = 0; i < G::NCOL; i++) {
-            const int e = tid + i * ASV_JFA_THREADS;
-            int v = e < FP ? flab[k * FP + e] : -1;
-            if ((unsigned)v >= (unsigned)Kp) v = -1;
-            const int vp = __shfl_up_sync(0xffffffffu, v, 1);
-            if (v >= 0 && !(lane > 0 && vp == v)) {
-                const unsigned w = (unsigned)v >> 5, bit = 1u << (v & 31);
-                if (!(*(volatile unsigned *)&b.claim[w] & bit) && !(atomicOr(&b.claim[w], bit) & bit)) {
-                    const int idx = atomicAdd(&b.tcount, 1);
-                    if (idx < ASV_BITS_TLCAP) b.tlab[idx] = v;
-                    b.map8[v] = (unsigned char)(idx < ASV_BITS_MAXT ? idx : ASV_BITS_NONE);
-                }
-            }
+    // number the distinct labels, each thread those of the quads it copied
+    // (its own copies are complete, so no barrier comes first)
+    for (int e = tid; e < items; e += ASV_JFA_THREADS) {
+        const int4 v = *(const int4 *)(flab + 4 * e);
+        const unsigned i0 = asv_bits_slot(v.x), i1 = asv_bits_slot(v.y), i2 = asv_bits_slot(v.z),
+                       i3 = asv_bits_slot(v.w);
+        const volatile unsigned char *mp = b.map8;
+        const unsigned m0 = mp[i0], m1 = mp[i1], m2 = mp[i2], m3 = mp[i3];
+        if (max(max(m0, m1), max(m2, m3)) == ASV_BITS_FREE) {
+            if (m0 == ASV_BITS_FREE) asv_bits_claim(b, i0);
+            if (m1 == ASV_BITS_FREE && i1 != i0) asv_bits_claim(b, i1);
+            if (m2 == ASV_BITS_FREE && i2 != i1) asv_bits_claim(b, i2);
+            if (m3 == ASV_BITS_FREE && i3 != i2) asv_bits_claim(b, i3);
         }
     }
     __syncthreads();
     const int T = b.tcount;
-    // the claim bits go back to zero for the next sub-tile
-    if (T <= ASV_BITS_TLCAP) {
-        for (int i = tid; i < T; i += ASV_JFA_THREADS) b.claim[b.tlab[i] >> 5] = 0u;
-    } else {
-        for (int i = tid; i < ASV_BITS_MAXKP / 32; i += ASV_JFA_THREADS) b.claim[i] = 0u;
-    }
     if (T > ASV_BITS_MAXT) {
+        asv_bits_reset(b, T);
         __syncthreads();
         if (tid == 0) b.tcount = 0;
         __syncthreads();
@@ -873,23 +957,22 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     for (int i = tid; i < 3 * T; i += ASV_JFA_THREADS) b.tdat[i] = __ldg(tab + 3 * b.tlab[i / 3] + i % 3);
     if (SUMS)
         for (int i = tid; i < (ASV_BITS_MAXT + 1) * ASV_ACC_ROW; i += ASV_JFA_THREADS) b.acc[i] = 0u;
-    // every footprint entry becomes its label's bit (0: no label), in place:
-    // each thread converts the entries it copied
-    for (int k = 0; k < nf; k++) {
-#pragma unroll
-        for (int i = 0; i < G::NCOL; i++) {
-            const int e = tid + i * ASV_JFA_THREADS;
-            if (e < FP) {
-                int *q = flab + k * FP + e;
-                const int l = *q;
-                *q = (int)((unsigned)l < (unsigned)Kp ? 1u << b.map8[l] : 0u);
-            }
-        }
+    // every footprint entry becomes its label's bit (0: no label), in place
+    for (int e = tid; e < items; e += ASV_JFA_THREADS) {
+        int4 *q = (int4 *)(flab + 4 * e);
+        const int4 v = *q;
+        const unsigned m0 = b.map8[asv_bits_slot(v.x)], m1 = b.map8[asv_bits_slot(v.y)],
+                       m2 = b.map8[asv_bits_slot(v.z)], m3 = b.map8[asv_bits_slot(v.w)];
+        *q = make_int4((int)asv_bit(m0), (int)asv_bit(m1), (int)asv_bit(m2), (int)asv_bit(m3));
     }
     __syncthreads();
+    // the numbers are read no more: unnumbered again for the next sub-tile
+    // (which starts after the barrier at the end)
+    asv_bits_reset(b, T);
+    if (tid == 0) b.tcount = 0;
 
     // the chain walk of this thread's column
-    const unsigned *f0 = (const unsigned *)flab + ly * FW + lx;  // candidate (x - S, y - S) of slot 0
+    const unsigned *f0 = (const unsigned *)flab + ly * FW + lx + (G::AL - S);  // candidate (x - S, y - S) of slot 0
     auto smask = [&](int k) -> unsigned {                         // a slice's 9 candidates
         const unsigned *f = f0 + k * FP;
         unsigned m = 0;
@@ -900,9 +983,8 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         return m;
     };
     const float2 vxy = make_float2((float)x + 0.5f, (float)y + 0.5f);
-    const unsigned m_zero = any_brk ? smask(n + 2) : 0u, m_last = any_brk ? smask(n + 3) : 0u;
+    const unsigned m_zero = brk ? smask(n + 2) : 0u, m_last = brk ? smask(n + 3) : 0u;
     unsigned mm = smask(0), mc = smask(1);
-    int im = 0;
     // centroid sums (last pass of an iteration): the thread's current run of
     // equal labels along its column, flushed into the sub-tile's table when
     // the label changes and at the end; the table goes to the global sums
@@ -911,9 +993,9 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     unsigned run_n = 0u, run_z = 0u, run_l = 0u, run_a = 0u, run_b = 0u;
     for (int j = 0; j < n; j++) {
         const int z = b.slotz[j + 1];
-        const bool chain = z + S < D;                         // the plus slice is the next centre
-        const int ip = j == n - 1 ? n + 1 : (chain ? j + 2 : n + 3);
-        const unsigned mp = (j < n - 1 && !chain) ? m_last : smask(ip);
+        const bool end = (brk >> j) & 1u;                     // the chain ends here and another one starts
+        const int ip = end ? n + 3 : j + 2;                   // else the plus slice is the next slot
+        const unsigned mp = end ? m_last : smask(j + 2);
         const uchar4 c = labsh[j * ASV_JFA_THREADS + tid];
         const float2 vzl = make_float2((float)z + 0.5f, (float)c.x), vab = make_float2((float)c.y, (float)c.z);
         unsigned m = mm | mc | mp;
@@ -927,7 +1009,10 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
                                             ratio);
             if (da < best) { best = da; bt = ta; tie = false; } else if (da == best) tie = true;
         }
-        if (tie) bt = asv_bits_ordered<S>(f0 + (j + 1) * FP, f0 + im * FP, f0 + ip * FP, b, vxy, vzl, vab, ratio);
+        if (tie) {
+            const int im = j > 0 && ((brk >> (j - 1)) & 1u) ? n + 2 : j;   // slot of the minus slice
+            bt = asv_bits_ordered<S>(f0 + (j + 1) * FP, f0 + im * FP, f0 + ip * FP, b, vxy, vzl, vab, ratio);
+        }
         const int label = bt >= 0 ? b.tlab[bt] : -1;
         if (valid) out[z * sl + col] = label;
         if (SUMS && valid) {
@@ -942,8 +1027,8 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
             run_l += c.x; run_a += c.y; run_b += c.z;
         }
         if (j + 1 < n) {
-            if (chain) { mm = mc; mc = mp; im = j + 1; }
-            else { mm = m_zero; mc = smask(j + 2); im = n + 2; }
+            if (!end) { mm = mc; mc = mp; }
+            else { mm = m_zero; mc = smask(j + 2); }
         }
     }
     if (SUMS) {
@@ -970,7 +1055,6 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         }
     }
     __syncthreads();                                          // the footprint and table are reused
-    if (tid == 0) b.tcount = 0;
     return true;
 }
 
@@ -995,13 +1079,15 @@ __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int
     // outnumber the positions from step 3 on, where the list form is faster
     if (step <= ASV_BITS_MAXS && Kp <= ASV_BITS_MAXKP && n <= 32 * 4 && (zrun >= 8 || step <= 2)) {
         fail = 0u;
+        // (sub-tiles of equal depth: 30 positions are 15 + 15, not 16 + 14)
 #define ASV_BITS_CASE(S_)                                                                                    \
     case S_:                                                                                                 \
-        sub = AsvBitsGeo<S_>::SUB;                                                                           \
-        for (int q0 = 0; q0 < n; q0 += AsvBitsGeo<S_>::SUB)                                                  \
+        sub = (n + AsvBitsGeo<S_>::SUB - 1) / AsvBitsGeo<S_>::SUB;                                           \
+        sub = (n + sub - 1) / sub;                                                                           \
+        for (int q0 = 0, i = 0; q0 < n; q0 += sub, i++)                                                      \
             if (!asv_jfa_bits_sub<S_, SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, tx0, ty0, p0 + q0, \
-                                            min(AsvBitsGeo<S_>::SUB, n - q0), ratio, smem))                  \
-                fail |= 1u << (q0 / AsvBitsGeo<S_>::SUB);                                                  \
+                                            min(sub, n - q0), ratio, smem))                                  \
+                fail |= 1u << i;                                                                             \
         break;
         switch (step) {
             ASV_BITS_CASE(1) ASV_BITS_CASE(2) ASV_BITS_CASE(3) ASV_BITS_CASE(4) ASV_BITS_CASE(5) ASV_BITS_CASE(6)
@@ -1020,7 +1106,11 @@ __device__ __forceinline__ void asv_jfa_smem_init(unsigned char *smem)
 {
     AsvBitsShared &b = *(AsvBitsShared *)(smem + ASV_JFA_AREA);
     for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 32; i += blockDim.x) b.claim[i] = 0u;
-    if (threadIdx.x == 0) b.tcount = 0;
+    for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 4; i += blockDim.x) ((unsigned *)b.map8)[i] = 0xffffffffu;
+    if (threadIdx.x == 0) {
+        b.tcount = 0;
+        b.map8[ASV_BITS_MAXKP] = ASV_BITS_NOLABEL;
+    }
     __syncthreads();
 }
 
@@ -1205,6 +1295,13 @@ __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d)
                                                ((unsigned long long)rank << 16) | (unsigned long long)label;
                 atomicMin(d.jkeys + v, key);
             }
+}
+
+// a caller's labels outside [0, Kp) become -1, as the passes' own labels are
+__global__ void k_label_clean(int32_t *__restrict__ lbl, long long n, int Kp)
+{
+    const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (v < n && (unsigned)lbl[v] >= (unsigned)Kp) lbl[v] = -1;
 }
 
 // single-segment pass with explicit step and ratio (test entry point)
@@ -1676,10 +1773,11 @@ void asv_launch_jfa_second_scatter(const AsvDev &d, cudaStream_t st)
     k_jfa_second<true><<<blocks, 256, 0, st>>>(d);
 }
 
-void asv_launch_jfa_single(const AsvDev &d, const int32_t *in, int32_t *out, int step, float ratio,
+void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
                            cudaStream_t st)
 {
     asv_jfa_attributes();
+    k_label_clean<<<(unsigned)((nvox + 255) / 256), 256, 0, st>>>(in, nvox, Kp);
     k_jfa_single<<<asv_jfa_grid_blocks(d.total_tiles), 256, ASV_JFA_SMEM, st>>>(d, in, out, step, ratio);
 }
 
