@@ -448,7 +448,7 @@ __global__ void k_draw(AsvDev d)
 // ---------------------------------------------------------------------------
 #define ASV_JFA_THREADS 256
 #define ASV_SLICE_MAX 9
-typedef int asv_list_t;      // candidate-list entry in shared memory (ids < 32768)
+typedef unsigned short asv_list_t;   // candidate-list entry in shared memory (ids < 32768)
 
 // chain order of the D slices for `step`: position p -> residue r, index j
 // in the chain, chain length len (z = r + j * step)
@@ -481,7 +481,7 @@ __device__ __forceinline__ int asv_slice_list(const int32_t *__restrict__ in, in
 #pragma unroll
         for (int e = 0; e < k; e++) fresh = fresh && c[k] != c[e];
         if (fresh) {
-            lst[n * ASV_JFA_THREADS] = c[k];
+            lst[n * ASV_JFA_THREADS] = (asv_list_t)c[k];
             n++;
         }
     }
@@ -503,7 +503,7 @@ __device__ __forceinline__ int asv_merge_lists(const asv_list_t *__restrict__ A,
     for (int i = 0; i < n; i++) {
         const int l = i < nb ? B[i * ASV_JFA_THREADS] : C[(i - nb) * ASV_JFA_THREADS];
         if (l != h0 && l != h1 && l != h2 && l != h3 && l != r1 && l != r2) {
-            X[nx * ASV_JFA_THREADS] = l;
+            X[nx * ASV_JFA_THREADS] = (asv_list_t)l;
             nx++;
             r2 = r1; r1 = l;
         }
@@ -680,11 +680,11 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // list form) and turns every footprint entry into its label's bit.  A
 // voxel's candidate mask is the OR of the 9 bits of each of its three
 // slices (the plus slice's mask becomes the next position's centre mask);
-// the voxel evaluates the labels of its mask in any order and keeps the
-// least distance below 1e8.  An exact tie at the least distance between two
-// labels (about 30 per million voxel-passes on the benchmarked clips) sends
-// the voxel through the shader's ordered scan of its 27 candidates instead,
-// so every label equals the shader's.
+// a voxel with one candidate takes it, the others take the least score of
+// their mask's labels (below), and the few whose scores are too close to call
+// (1 or 2 in a thousand) the shader's own arithmetic: least distance below
+// 1e8, and where two labels tie exactly at it, the shader's ordered scan of
+// the voxel's 27 candidates.  So every label equals the shader's.
 //
 // The passes are bound by instruction issue, so the three steps before the
 // walk handle four entries (a quad) per thread and access: a quad is copied
@@ -694,9 +694,17 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // one 16-byte load and store.  Each thread numbers the quads it copied, so
 // no barrier stands between; with the slot slices worked out by every warp
 // and the byte map reset behind the walk, a sub-tile has three barriers
-// (six before).  A 1280x720x30 window of 20 iterations: 65.2 -> 52.9 ms, the
+// (six before).  A 1280x720x30 window of 20 iterations: 65.2 -> 53.8 ms, the
 // 320x240x85 clip 13.9 -> 12.1 ms.  Widths that are no multiple of four
-// copy their quads by four 4-byte cp.async.
+// copy their quads by four 4-byte cp.async.  A quad whose labels all have
+// numbers already is turned into bits at once.
+//
+// Scores instead of the shader's arithmetic took the evaluation from 44 to 28
+// instructions per candidate, and fewer registers: 64, so that with the LAB
+// values read straight from global memory (one position ahead) four blocks
+// fit an SM, three before.  Passes of a 1280x720x30 window (steps 6, 3, 2, 1,
+// 2, 1 + sums) 499, 479, 439, 409, 443, 509 -> 316, 342, 315, 298, 326,
+// 425 us; issue slots 63 -> 67 % used.
 //
 // Footprint slices ("slots") of a sub-tile of n chain positions: slot 0 the
 // minus slice of position 0, slots 1..n the centre slices, slot n+1 the plus
@@ -716,15 +724,21 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 #define ASV_BITS_OVER 253        // map8: a label past the 32nd (the sub-tile takes the list form)
 #define ASV_ACC_ROW 7            // words per entry of the sub-tile's centroid-sum table (odd: the
                                  // entries' rows start in different shared-memory banks)
-#define ASV_BITS_AREA 62464      // shared bytes of the largest sub-tiles (step 4, 16 positions)
+#define ASV_BITS_AREA 43264      // shared bytes of the largest sub-tiles (step 5, 9 positions): four blocks per SM
 #define ASV_JFA_AREA (ASV_BITS_AREA > ASV_JFA_LIST_BYTES ? ASV_BITS_AREA : ASV_JFA_LIST_BYTES)
 
+#define ASV_ECO_ROW 5            // float4 per label of the score table (3.5 used; the odd count
+                                 // spreads the rows of eight labels over all banks)
+
 struct AsvBitsShared {
-    float4 tdat[3 * ASV_BITS_MAXT];             // the table's seed rows (as jtab)
+    float4 eco[ASV_ECO_ROW * ASV_BITS_MAXT];    // score coefficients per table entry (asv_bits_coefs)
     unsigned acc[(ASV_BITS_MAXT + 1) * ASV_ACC_ROW];   // centroid sums of the sub-tile per table entry (+ label -1)
     unsigned claim[ASV_BITS_MAXKP / 32];        // labels numbered in this sub-tile (all zero between)
-    int tlab[ASV_BITS_TLCAP];                   // label of each number
-    int slotz[20];                              // slice of each footprint slot
+    int4 slot[20];                              // per footprint slot: offset of its slice, slice relative to the
+                                                // sub-tile's middle one (float bits), 2 z + 1 (positions' slots)
+    unsigned short tlab[ASV_BITS_TLCAP];        // label of each number
+    float magic[3];                             // 2^23 + the colour the scores are relative to
+    float margin[2];                            // scores' error margin: [0] + [1] |colour|^2; [0] infinite: no scores
     int tcount;
     unsigned char map8[ASV_BITS_MAXKP + 4];     // number of each claimed label, ASV_BITS_FREE between
 };
@@ -740,14 +754,27 @@ template <int S> struct AsvBitsGeo {
     static constexpr int FH = ASV_TILE_Y + 2 * S;
     static constexpr int FP = FW * FH;                                // footprint entries per slot
     static constexpr int QW = FW / 4, QPS = FP / 4;                   // quads per row and per slot
-    // chain positions per sub-tile: as many as the shared area holds, up to
-    // 16 (steps 5-6: 10)
-    static constexpr int SUB = S <= 4 ? 16 : 10;
+    // chain positions per sub-tile: as many as the shared area holds, up to 16
+    static constexpr int SUB = S <= 3 ? 16 : (S == 4 ? 14 : (S == 5 ? 9 : 8));
     static constexpr int NSLOT = SUB + 4;
     static constexpr int FLAB_BYTES = NSLOT * FP * 4;
-    static_assert(FLAB_BYTES + SUB * ASV_JFA_THREADS * 4 <= ASV_BITS_AREA, "bit-set sub-tile exceeds the shared area");
+    static_assert(FLAB_BYTES <= ASV_BITS_AREA, "bit-set sub-tile exceeds the shared area");
     static_assert(NSLOT <= 20, "slotz");
 };
+
+// Slice of chain position p of the D slices for step S (asv_chain_pos's z).
+// The quotients by the chain lengths go through FP32: numerators and
+// denominators are below 4097, so (p + 0.5) / d is at least 0.5 / 4096 of its
+// value away from an integer, far above the division's error.
+template <int S>
+__device__ __forceinline__ int asv_chain_z(int p, int D)
+{
+    const int q = D / S, m = D - q * S, big = m * (q + 1);
+    const bool lo = p < big || q == 0;
+    const int d = lo ? q + 1 : q, pp = lo ? p : p - big;
+    const int r = (int)__fdividef((float)pp + 0.5f, (float)d);
+    return (lo ? r : m + r) + (pp - r * d) * S;
+}
 
 // 4-byte asynchronous copy global -> shared (cp.async, completed by
 // asv_cp_async_wait)
@@ -801,12 +828,17 @@ __device__ __forceinline__ unsigned asv_bit(unsigned n)
 }
 
 // a label seen without a number: the thread that claims it gives it the next one
-__device__ __forceinline__ void asv_bits_claim(AsvBitsShared &b, unsigned v)
+// and starts the copy of its seed table row
+__device__ __forceinline__ void asv_bits_claim(AsvBitsShared &b, unsigned v, const float4 *__restrict__ tab)
 {
     const unsigned bit = 1u << (v & 31);
     if (atomicOr(&b.claim[v >> 5], bit) & bit) return;
     const int idx = atomicAdd(&b.tcount, 1);
-    if (idx < ASV_BITS_TLCAP) b.tlab[idx] = (int)v;
+    if (idx < ASV_BITS_TLCAP) b.tlab[idx] = (unsigned short)v;
+    if (idx < ASV_BITS_MAXT) {
+#pragma unroll
+        for (int k = 0; k < 3; k++) asv_cp_async16(b.eco + ASV_ECO_ROW * idx + k, tab + 3 * v + k);
+    }
     b.map8[v] = (unsigned char)(idx < ASV_BITS_MAXT ? idx : ASV_BITS_OVER);
 }
 
@@ -824,46 +856,149 @@ __device__ __forceinline__ void asv_bits_reset(AsvBitsShared &b, int T)
     }
 }
 
-// The shader's ordered scan of the 27 candidates (slices centre, minus,
+// ---------------------------------------------------------------------------
+// Scores.  Which label of a voxel's mask has the least distance is mostly
+// decided without the shader's arithmetic: the distance is a quadratic form
+// of the voxel's coordinates plus a colour term, so with the coordinates
+// (u, v, w) and the colour (l, a, b) taken relative to the sub-tile's middle,
+// distance - (l^2 + a^2 + b^2) is
+//   max(K0 + ku u + kv v + kw w + kuu u^2 + kvv v^2 + kww w^2 + kuv u v
+//       + kuw u w + kvw v w, c0) + cl l + ca a + cb b
+// (K0 and c0 hold the colour constant c0 = |seed colour|^2; the max is the
+// clamp of a negative form, flood.gs:90-93): fourteen coefficients per label,
+// ten fused multiply-adds and additions where the shader's order takes
+// twenty-one, nothing between them that must round apart.
+//
+// Both this score and the shader's rounded distance are off the exact value
+// by no more than a bound that follows from the operands' sizes.  With
+// e = 2^-24, A = ratio * sum |M_ij| |d_i| |d_j| over the sub-tile's extent and
+// C = |s|^2 + 2 sum |s_k| |c_k| for the relative colours s of the seed and c of
+// the voxel:
+//   shader's distance: 9 e A + 6 e distance (each term passes at most 9
+//     roundings, a colour term 6),
+//   score: 17 e A + 11 e C (coefficients up to 10 roundings, the sum 7).
+// So where the least score is below every other by more than
+//   72 e A + 32 e C + 16 e (sum of both distances)
+// (the larger label's bounds, twice, with room to spare) it is the strictly
+// least shader distance.  With S the largest relative seed colour component
+// of the table, q = |(l, a, b)|^2 and |l| + |a| + |b| <= q / 32 + 24, that is
+// at most margin[0] + margin[1] q + 16 e (both scores), where
+//   margin[0] = max over the labels of 72 e A + 32 e |s|^2, + 64 e S 24,
+//   margin[1] = 64 e S / 32 + 32 e.
+// Any closer voxel is evaluated in the shader's order (asv_bits_exact), so
+// the labels are the shader's in every case.  A label whose A or colour is
+// not finite or so large that a distance might reach 1e8 gives an infinite
+// margin: that sub-tile takes no scores.
+// ---------------------------------------------------------------------------
+#define ASV_EPS 5.9604645e-8f    // 2^-24
+
+// One warp, lane = table entry: replaces the entry's seed table row, which the
+// claiming thread copied to the entry's place, by its score coefficients
+// (ox, oy, oz: the sub-tile's middle, wmax: the largest |w| of its positions).
+__device__ __forceinline__ void asv_bits_coefs(AsvBitsShared &b, int T, float ox, float oy, float oz, float wmax,
+                                               float ratio)
+{
+    const int lane = threadIdx.x & 31;
+    const bool on = lane < T;
+    float4 *e = b.eco + ASV_ECO_ROW * lane;
+    float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
+    if (on) { r0 = e[0]; r1 = e[1]; r2 = e[2]; }
+    const float col[3] = { -r0.w, -r2.z, -r2.w };
+    float s[3], mid[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {                     // middle of the labels' colours
+        const int q = min(max(__float2int_rn(col[k]), 0), 255);
+        const int lo = __reduce_min_sync(FULL, on ? q : 255), hi = __reduce_max_sync(FULL, on ? q : 0);
+        mid[k] = (float)((lo + hi) >> 1);
+        s[k] = col[k] - mid[k];
+    }
+    const float su = -(r0.x + ox), sv = -(r0.y + oy), sw = -(r0.z + oz);
+    const float a00 = ratio * r1.x, a11 = ratio * r1.y, a02 = ratio * r1.z, a12 = ratio * r1.w;
+    const float a01 = ratio * r2.x, a22 = ratio * r2.y;
+    const float c0 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+    const float ku = -(2.0f * a00 * su + a01 * sv + a02 * sw);
+    const float kv = -(2.0f * a11 * sv + a01 * su + a12 * sw);
+    const float kw = -(2.0f * a22 * sw + a02 * su + a12 * sv);
+    const float k0 = a00 * su * su + a01 * su * sv + a02 * su * sw + a11 * sv * sv + a12 * sv * sw + a22 * sw * sw;
+    const float X = fabsf(su) + 8.0f, Y = fabsf(sv) + 8.0f, Z = fabsf(sw) + wmax;
+    const float A = fabsf(a00) * X * X + fabsf(a01) * X * Y + fabsf(a02) * X * Z + fabsf(a11) * Y * Y +
+                    fabsf(a12) * Y * Z + fabsf(a22) * Z * Z;
+    const float smax = fmaxf(fmaxf(fabsf(s[0]), fabsf(s[1])), fabsf(s[2]));
+    const bool ok = A < 1e7f && smax < 1000.0f && s[0] == s[0] && s[1] == s[1] && s[2] == s[2];   // false for NaN
+    const float mg = ok ? 72.0f * ASV_EPS * A + 32.0f * ASV_EPS * c0 + 1e-30f : __int_as_float(0x7f800000);
+    const unsigned top = __reduce_max_sync(FULL, on ? __float_as_uint(mg) : 0u);     // non-negative floats
+    const unsigned stop = __reduce_max_sync(FULL, on && ok ? __float_as_uint(smax) : 0u);
+    if (on) {
+        e[0] = make_float4(ku, kv, a00, a11);
+        e[1] = make_float4(a02, a12, a22, a01);
+        e[2] = make_float4(kw, k0 + c0, c0, -2.0f * s[0]);
+        *(float2 *)(e + 3) = make_float2(-2.0f * s[1], -2.0f * s[2]);
+    }
+    if (lane == 0) {
+        const float S = __uint_as_float(stop);
+        b.margin[0] = __uint_as_float(top) + 64.0f * 24.0f * ASV_EPS * S;
+        b.margin[1] = 2.0f * ASV_EPS * S + 32.0f * ASV_EPS;
+#pragma unroll
+        for (int k = 0; k < 3; k++) b.magic[k] = 8388608.0f + mid[k];
+    }
+}
+
+// The label of mask m for one voxel in the shader's own arithmetic: least
+// distance below 1e8 over the mask's labels in any order; where two tie at
+// it, the shader's ordered scan of the 27 candidates (slices centre, minus,
 // plus; rows y-S, y, y+S; columns x-S, x, x+S) over the footprint's label
-// bits, strict '<' from 1e8 (flood.gs:63, :95-99): the tie-break path.
+// bits, strict '<' from 1e8 (flood.gs:63, :95-99).  Returns the table entry
+// or -1.
 template <int S>
-__device__ __noinline__ int asv_bits_ordered(const unsigned *__restrict__ fc, const unsigned *__restrict__ fm,
-                                             const unsigned *__restrict__ fp, const AsvBitsShared &b,
-                                             float2 vxy, float2 vzl, float2 vab, float ratio)
+__device__ __noinline__ int asv_bits_exact(unsigned m, const unsigned *__restrict__ fc, const unsigned *__restrict__ fm,
+                                           const unsigned *__restrict__ fp, const AsvBitsShared &b,
+                                           const float4 *__restrict__ tab, int x, int y, int z, unsigned c, float ratio)
 {
     constexpr int FW = AsvBitsGeo<S>::FW;
+    const float2 vxy = make_float2((float)x + 0.5f, (float)y + 0.5f);
+    const float2 vzl = make_float2((float)z + 0.5f, (float)(c & 255u));
+    const float2 vab = make_float2((float)((c >> 8) & 255u), (float)((c >> 16) & 255u));
     float mind = 100000000.0f;
     int best = -1;
+    bool tie = false;
+    while (m) {
+        const int e = __ffs(m) - 1;
+        m &= m - 1;
+        const float dist = asv_jfa_dist(tab, b.tlab[e], vxy, vzl, vab, ratio);
+        if (dist < mind) { mind = dist; best = e; tie = false; } else if (dist == mind) tie = true;
+    }
+    if (!tie) return best;
+    mind = 100000000.0f;
+    best = -1;
     for (int k = 0; k < 3; k++) {
         const unsigned *f = k == 0 ? fc : (k == 1 ? fm : fp);
         for (int a = 0; a < 3; a++)
-            for (int c = 0; c < 3; c++) {
-                const unsigned bit = f[a * S * FW + c * S];
+            for (int o = 0; o < 3; o++) {
+                const unsigned bit = f[a * S * FW + o * S];
                 if (!bit) continue;
                 const int e = __ffs(bit) - 1;
-                const float dist = asv_jfa_dist_v(b.tdat[3 * e], b.tdat[3 * e + 1], b.tdat[3 * e + 2], vxy, vzl,
-                                                  vab, ratio);
+                const float dist = asv_jfa_dist(tab, b.tlab[e], vxy, vzl, vab, ratio);
                 if (dist < mind) { mind = dist; best = e; }
             }
     }
-    return best;                                              // table entry, or -1
+    return best;
 }
 
 // A thread's run of voxels with one label, added to its table entry's
 // centroid sums in shared memory: count n, sum of 2z+1 and of L, a, b; the
 // column's 2x+1 and 2y+1 times n.  Exact u32 sums (a sub-tile holds at most
 // 16 x 256 voxels of coordinates below 4096).
-__device__ __forceinline__ void asv_run_flush(unsigned *__restrict__ a, unsigned n, unsigned sz, unsigned sl,
-                                              unsigned sa, unsigned sb, int x, int y)
+__device__ __forceinline__ void asv_run_flush(unsigned *__restrict__ a, unsigned sz, unsigned la, unsigned bn, int x,
+                                              int y)
 {
+    const unsigned n = bn >> 16;
     atomicAdd(a + 0, n * (2u * (unsigned)x + 1u));
     atomicAdd(a + 1, n * (2u * (unsigned)y + 1u));
     atomicAdd(a + 2, sz);
     atomicAdd(a + 3, n);
-    atomicAdd(a + 4, sl);
-    atomicAdd(a + 5, sa);
-    atomicAdd(a + 6, sb);
+    atomicAdd(a + 4, la & 0xffffu);
+    atomicAdd(a + 5, la >> 16);
+    atomicAdd(a + 6, bn & 0xffffu);
 }
 
 // One sub-tile of n <= SUB chain positions from p0 in bit-set form; false
@@ -878,7 +1013,6 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     using G = AsvBitsGeo<S>;
     constexpr int FW = G::FW, FP = G::FP;
     int *flab = (int *)smem;                                   // labels, then their bits
-    uchar4 *labsh = (uchar4 *)(smem + G::FLAB_BYTES);
     AsvBitsShared &b = *(AsvBitsShared *)(smem + ASV_JFA_AREA);
     const int tid = threadIdx.x, lane = tid & 31;
     const int sl = W * H;
@@ -892,59 +1026,65 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     // the same values, so no barrier is needed before they are read; brk
     // has a bit for each position but the last where a chain ends
     unsigned brk;
+    int zc;                                                    // middle slice of the positions
+    float wmax;                                                // largest distance from it
     {
-        bool end = false;
-        if (lane < n) {
-            int r, j, len;
-            asv_chain_pos(p0 + lane, D, S, r, j, len);
-            const int z = r + j * S;
-            b.slotz[1 + lane] = z;
-            if (lane == 0) b.slotz[0] = max(z - S, 0);
-            if (lane == n - 1) b.slotz[n + 1] = z + S < D ? z + S : D - 1;
-            end = lane < n - 1 && z + S >= D;
+        const int z = lane < n ? asv_chain_z<S>(p0 + lane, D) : 0;
+        const bool end = lane < n - 1 && z + S >= D;
+        brk = __ballot_sync(FULL, end);
+        const int z0 = __reduce_min_sync(FULL, lane < n ? z : D), z1 = __reduce_max_sync(FULL, z);
+        zc = (z0 + z1) >> 1;
+        wmax = (float)(z1 - zc);                               // z1 - zc >= zc - z0
+        if (lane < n) b.slot[1 + lane] = make_int4(z * sl, __float_as_int((float)(z - zc)), 2 * z + 1, 0);
+        if (lane == 0) {
+            b.slot[0].x = max(z - S, 0) * sl;
+            b.slot[n + 2].x = 0;
+            b.slot[n + 3].x = (D - 1) * sl;
         }
-        if (lane == 0) { b.slotz[n + 2] = 0; b.slotz[n + 3] = D - 1; }
-        brk = __ballot_sync(0xffffffffu, end);
+        if (lane == n - 1) b.slot[n + 1].x = (z + S < D ? z + S : D - 1) * sl;
         __syncwarp();
     }
     const int nf = brk ? n + 4 : n + 2;
 
-    // footprint labels (clamp-to-edge) and the voxels' LAB, copied
-    // asynchronously a quad at a time
+    // footprint labels (clamp-to-edge), copied asynchronously a quad at a time
     const bool vec = (W & 3) == 0;
     const int items = nf * G::QPS;
     {
         int slot = tid / G::QPS, q = tid - slot * G::QPS;
         for (int e = tid; e < items; e += ASV_JFA_THREADS) {
             const int fy = q / G::QW, fx = q - fy * G::QW;
-            asv_copy_quad(flab + 4 * e, in, b.slotz[slot] * sl + min(max(ty0 - S + fy, 0), H - 1) * W,
+            asv_copy_quad(flab + 4 * e, in, b.slot[slot].x + min(max(ty0 - S + fy, 0), H - 1) * W,
                           tx0 - G::AL + 4 * fx, W, vec);
             q += ASV_JFA_THREADS % G::QPS;
             slot += ASV_JFA_THREADS / G::QPS;
             if (q >= G::QPS) { q -= G::QPS; slot++; }
         }
-        const int q4 = tid & 63, lyy = min(ty0 + (q4 >> 2), H - 1);
-        for (int j = tid >> 6; j < n; j += 4)
-            asv_copy_quad(labsh + j * ASV_JFA_THREADS + 4 * q4, (const int32_t *)lab, b.slotz[j + 1] * sl + lyy * W,
-                          tx0 + 4 * (q4 & 3), W, vec);
     }
     asv_cp_async_wait();
 
     // number the distinct labels, each thread those of the quads it copied
-    // (its own copies are complete, so no barrier comes first)
-    for (int e = tid; e < items; e += ASV_JFA_THREADS) {
-        const int4 v = *(const int4 *)(flab + 4 * e);
+    // (its own copies are complete, so no barrier comes first), and turn the
+    // quads' entries into their labels' bits in place (0: no label).  A quad
+    // with a label that had no number yet is turned after the barrier.
+    unsigned pend = 0u;
+    for (int e = tid, k = 0; e < items; e += ASV_JFA_THREADS, k++) {
+        int4 *q = (int4 *)(flab + 4 * e);
+        const int4 v = *q;
         const unsigned i0 = asv_bits_slot(v.x), i1 = asv_bits_slot(v.y), i2 = asv_bits_slot(v.z),
                        i3 = asv_bits_slot(v.w);
         const volatile unsigned char *mp = b.map8;
         const unsigned m0 = mp[i0], m1 = mp[i1], m2 = mp[i2], m3 = mp[i3];
         if (max(max(m0, m1), max(m2, m3)) == ASV_BITS_FREE) {
-            if (m0 == ASV_BITS_FREE) asv_bits_claim(b, i0);
-            if (m1 == ASV_BITS_FREE && i1 != i0) asv_bits_claim(b, i1);
-            if (m2 == ASV_BITS_FREE && i2 != i1) asv_bits_claim(b, i2);
-            if (m3 == ASV_BITS_FREE && i3 != i2) asv_bits_claim(b, i3);
+            if (m0 == ASV_BITS_FREE) asv_bits_claim(b, i0, tab);
+            if (m1 == ASV_BITS_FREE && i1 != i0) asv_bits_claim(b, i1, tab);
+            if (m2 == ASV_BITS_FREE && i2 != i1) asv_bits_claim(b, i2, tab);
+            if (m3 == ASV_BITS_FREE && i3 != i2) asv_bits_claim(b, i3, tab);
+            pend |= 1u << k;
+        } else {
+            *q = make_int4((int)asv_bit(m0), (int)asv_bit(m1), (int)asv_bit(m2), (int)asv_bit(m3));
         }
     }
+    asv_cp_async_wait();                                       // the claimed labels' rows
     __syncthreads();
     const int T = b.tcount;
     if (T > ASV_BITS_MAXT) {
@@ -954,17 +1094,17 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         __syncthreads();
         return false;
     }
-    for (int i = tid; i < 3 * T; i += ASV_JFA_THREADS) b.tdat[i] = __ldg(tab + 3 * b.tlab[i / 3] + i % 3);
     if (SUMS)
         for (int i = tid; i < (ASV_BITS_MAXT + 1) * ASV_ACC_ROW; i += ASV_JFA_THREADS) b.acc[i] = 0u;
-    // every footprint entry becomes its label's bit (0: no label), in place
-    for (int e = tid; e < items; e += ASV_JFA_THREADS) {
-        int4 *q = (int4 *)(flab + 4 * e);
+    while (pend) {
+        int4 *q = (int4 *)(flab + 4 * (tid + ASV_JFA_THREADS * (__ffs(pend) - 1)));
+        pend &= pend - 1;
         const int4 v = *q;
         const unsigned m0 = b.map8[asv_bits_slot(v.x)], m1 = b.map8[asv_bits_slot(v.y)],
                        m2 = b.map8[asv_bits_slot(v.z)], m3 = b.map8[asv_bits_slot(v.w)];
         *q = make_int4((int)asv_bit(m0), (int)asv_bit(m1), (int)asv_bit(m2), (int)asv_bit(m3));
     }
+    if (tid < 32) asv_bits_coefs(b, T, (float)(tx0 + 8), (float)(ty0 + 8), (float)zc + 0.5f, wmax, ratio);
     __syncthreads();
     // the numbers are read no more: unnumbered again for the next sub-tile
     // (which starts after the barrier at the end)
@@ -973,8 +1113,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
 
     // the chain walk of this thread's column
     const unsigned *f0 = (const unsigned *)flab + ly * FW + lx + (G::AL - S);  // candidate (x - S, y - S) of slot 0
-    auto smask = [&](int k) -> unsigned {                         // a slice's 9 candidates
-        const unsigned *f = f0 + k * FP;
+    auto smask = [&](const unsigned *f) -> unsigned {             // a slice's 9 candidates
         unsigned m = 0;
 #pragma unroll
         for (int a = 0; a < 3; a++)
@@ -982,62 +1121,89 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
             for (int c = 0; c < 3; c++) m |= f[a * S * FW + c * S];
         return m;
     };
-    const float2 vxy = make_float2((float)x + 0.5f, (float)y + 0.5f);
-    const unsigned m_zero = brk ? smask(n + 2) : 0u, m_last = brk ? smask(n + 3) : 0u;
-    unsigned mm = smask(0), mc = smask(1);
+    const float2 uv = make_float2((float)lx - 7.5f, (float)ly - 7.5f);
+    const float mg0 = b.margin[0], mg1 = b.margin[1];
+    const float mgl = b.magic[0], mga = b.magic[1], mgb = b.magic[2];
+    const bool fast = mg0 < 1e30f;
+    const unsigned m_zero = brk ? smask(f0 + (n + 2) * FP) : 0u, m_last = brk ? smask(f0 + (n + 3) * FP) : 0u;
+    unsigned mm = smask(f0), mc = smask(f0 + FP);
     // centroid sums (last pass of an iteration): the thread's current run of
     // equal labels along its column, flushed into the sub-tile's table when
     // the label changes and at the end; the table goes to the global sums
     // once per sub-tile (centroids.vs:19-54; label -1 counts in slot Kp)
     int run_e = -1;
-    unsigned run_n = 0u, run_z = 0u, run_l = 0u, run_a = 0u, run_b = 0u;
-    for (int j = 0; j < n; j++) {
-        const int z = b.slotz[j + 1];
-        const bool end = (brk >> j) & 1u;                     // the chain ends here and another one starts
-        const int ip = end ? n + 3 : j + 2;                   // else the plus slice is the next slot
-        const unsigned mp = end ? m_last : smask(j + 2);
-        const uchar4 c = labsh[j * ASV_JFA_THREADS + tid];
-        const float2 vzl = make_float2((float)z + 0.5f, (float)c.x), vab = make_float2((float)c.y, (float)c.z);
-        unsigned m = mm | mc | mp;
-        float best = 100000000.0f;
-        int bt = -1;
-        bool tie = false;
-        while (m) {
-            const int ta = __ffs(m) - 1;
-            m &= m - 1;
-            const float da = asv_jfa_dist_v(b.tdat[3 * ta], b.tdat[3 * ta + 1], b.tdat[3 * ta + 2], vxy, vzl, vab,
-                                            ratio);
-            if (da < best) { best = da; bt = ta; tie = false; } else if (da == best) tie = true;
+    unsigned run_z = 0u, run_la = 0u, run_bn = 0u;            // L | a << 16, b | count << 16 (16 x 255 < 2^16)
+    const unsigned *fn = f0 + 2 * FP;                         // the next slot
+    const unsigned *lab32 = (const unsigned *)lab;
+    unsigned ends = brk, c4n = __ldg(lab32 + (b.slot[1].x + col));
+    for (int j = 0; j < n; j++, fn += FP, ends >>= 1) {
+        const int4 at = b.slot[j + 1];
+        const unsigned c4 = c4n;
+        c4n = __ldg(lab32 + (b.slot[j + 2].x + col));         // the next position's (after the last one: unused)
+        const bool end = ends & 1u;                           // the chain ends here and another one starts:
+        const unsigned mx = smask(fn);                        // the next slot is its centre, else this one's plus
+        const unsigned m = mm | mc | (end ? m_last : mx);
+        int bt = 31 - __clz((int)m);                          // the only candidate, or -1
+        bool slow = !fast && m;
+        if (fast && (m & (m - 1))) {
+            const float w = __int_as_float(at.y);
+            const float2 ww = make_float2(w, w);
+            // bytes to floats: 2^23 + byte, minus 2^23 + the middle colour
+            const float fl = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7650)) - mgl;
+            const float fa = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7651)) - mga;
+            const float fb = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7652)) - mgb;
+            float best = 3e38f, sec = 3e38f;
+            unsigned rest = m;
+            do {
+                const int t = 31 - __clz((int)rest);
+                rest ^= 1u << t;
+                const float4 *e = b.eco + ASV_ECO_ROW * t;
+                const float4 e0 = e[0], e1 = e[1], e2 = e[2];
+                const float2 e3 = *(const float2 *)(e + 3);
+                float2 g = __ffma2_rn(make_float2(e0.z, e0.w), uv, make_float2(e0.x, e0.y));
+                g = __ffma2_rn(make_float2(e1.x, e1.y), ww, g);
+                g.x = __fmaf_rn(e1.w, uv.y, g.x);
+                float p = __fmaf_rn(__fmaf_rn(e1.z, w, e2.x), w, e2.y);
+                p = __fmaf_rn(g.x, uv.x, p);
+                p = fmaxf(__fmaf_rn(g.y, uv.y, p), e2.z);
+                p = __fmaf_rn(e2.w, fl, p);
+                p = __fmaf_rn(e3.x, fa, p);
+                p = __fmaf_rn(e3.y, fb, p);
+                sec = fminf(sec, fmaxf(best, p));
+                bt = p < best ? t : bt;
+                best = fminf(best, p);
+            } while (rest);
+            const float q = __fmaf_rn(fl, fl, __fmaf_rn(fa, fa, fb * fb));
+            slow = !(sec - best > __fmaf_rn(16.0f * ASV_EPS, sec + best, __fmaf_rn(mg1, q, mg0)));
         }
-        if (tie) {
-            const int im = j > 0 && ((brk >> (j - 1)) & 1u) ? n + 2 : j;   // slot of the minus slice
-            bt = asv_bits_ordered<S>(f0 + (j + 1) * FP, f0 + im * FP, f0 + ip * FP, b, vxy, vzl, vab, ratio);
+        if (slow) {
+            const unsigned *fm = j > 0 && ((brk >> (j - 1)) & 1u) ? f0 + (n + 2) * FP : fn - 2 * FP;   // minus slice
+            bt = asv_bits_exact<S>(m, fn - FP, fm, end ? f0 + (n + 3) * FP : fn, b, tab, x, y, at.z >> 1, c4, ratio);
         }
         const int label = bt >= 0 ? b.tlab[bt] : -1;
-        if (valid) out[z * sl + col] = label;
+        if (valid) out[at.x + col] = label;
         if (SUMS && valid) {
             const int e = bt >= 0 ? bt : ASV_BITS_MAXT;
             if (e != run_e) {
-                if (run_e >= 0) asv_run_flush(b.acc + ASV_ACC_ROW * run_e, run_n, run_z, run_l, run_a, run_b, x, y);
+                if (run_e >= 0) asv_run_flush(b.acc + ASV_ACC_ROW * run_e, run_z, run_la, run_bn, x, y);
                 run_e = e;
-                run_n = run_z = run_l = run_a = run_b = 0u;
+                run_z = run_la = run_bn = 0u;
             }
-            run_n++;
-            run_z += 2u * (unsigned)z + 1u;
-            run_l += c.x; run_a += c.y; run_b += c.z;
+            run_z += (unsigned)at.z;
+            run_la += __byte_perm(c4, 0u, 0x4140);
+            run_bn += __byte_perm(c4, 1u, 0x7472);            // bytes (b, 0, 1, 0)
         }
-        if (j + 1 < n) {
-            if (!end) { mm = mc; mc = mp; }
-            else { mm = m_zero; mc = smask(j + 2); }
-        }
+        mm = end ? m_zero : mc;
+        mc = mx;
     }
     if (SUMS) {
         // the runs left at the end, grouped by entry across the warp (every
         // lane of the block gets here; lanes without a run join with entry
         // -1, which adds nothing), so a warp adds each entry once
         const unsigned grp = __match_any_sync(0xffffffffu, run_e);
+        const unsigned run_n = run_bn >> 16;
         const unsigned q[7] = { run_n * (2u * (unsigned)x + 1u), run_n * (2u * (unsigned)y + 1u), run_z, run_n,
-                                run_l, run_a, run_b };
+                                run_la & 0xffffu, run_la >> 16, run_bn & 0xffffu };
         unsigned t[7];
 #pragma unroll
         for (int k = 0; k < 7; k++) t[k] = __reduce_add_sync(grp, q[k]);
@@ -1115,7 +1281,7 @@ __device__ __forceinline__ void asv_jfa_smem_init(unsigned char *smem)
 }
 
 // tile = ASV_TILE_X x ASV_TILE_Y columns x S.zrun chain positions
-__global__ void __launch_bounds__(ASV_JFA_THREADS, 3) k_jfa(AsvDev d, int pass,
+__global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
                                                          const int32_t *__restrict__ in,
                                                          int32_t *__restrict__ out)
 {
