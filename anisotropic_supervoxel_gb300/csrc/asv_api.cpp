@@ -344,21 +344,99 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
     return vox * per_vox + seeds * per_seed + cells * 4 + chunks * 4 + fixed + seg.size() * per_seg;
 }
 
-// JFA tile depth for a set of segments: the configured one, else the
-// deepest of 32/16/8 that still gives every resident block four tiles
-// (deeper runs share more slices; shallower ones balance the GPU), else 4.
+// A tile depth that cuts D positions evenly into as many tiles as z does
+static int even_depth(int D, int z)
+{
+    const int tiles = (D + z - 1) / z;
+    return (D + tiles - 1) / tiles;
+}
+
+// Chain positions that a sub-tile of a JFA pass's bit-set form may hold so
+// that its labels fit the 32 of its masks, 0: list form.  The footprint's box
+// (16 + 2 AL columns, AL the step rounded up to four, by 16 + 2 step rows by
+// (depth + 2) step slices) crosses about prod(1 + side / spacing) seeds'
+// cells; real ones are less regular, so up to 14 of the estimate are taken
+// without loss (measured at spacings 9 to 23: at spacing 18 and step 2 a loop
+// of six iterations took 4.81 ms with depth 8, estimate 10, 5.05 with 16,
+// estimate 15), and up to 24 at the least depth, which still beats the list
+// form there (spacing 9, step 1: 5.56 against 5.78 ms; step 2, estimate 28:
+// 5.67 against 5.63).
+static int label_depth(int D, double spacing, int step)
+{
+    const int al = (step + 3) & ~3;
+    const double xy = (1.0 + (16 + 2 * al) / spacing) * (1.0 + (16 + 2 * step) / spacing);
+    for (int c : { 16, 8, 4 }) {
+        const double labels = xy * (1.0 + std::min(D, (c + 2) * step) / spacing);
+        if (labels <= 14.0 || (c == 4 && labels <= 24.0)) return c;
+    }
+    return 0;
+}
+
+static double seed_spacing(long long nvox, int Kp) { return std::cbrt((double)nvox / std::max(Kp, 1)); }
+
+// SegDesc::depth of every pass.  The first gathering pass (the third) sees
+// labels around the seeds only and takes the deepest sub-tiles.  A tile is
+// cut evenly: 30 positions are 15 + 15, not 16 + 14.
+static void set_depths(SegDesc &s)
+{
+    const double spacing = seed_spacing(s.nvox, s.Kp);
+    for (int p = 0; p < s.npass; p++) {
+        const int step = s.steps[p];
+        const int cap = std::min(asv_jfa_max_depth(step), p == s.npass - 1 ? 15 : 16);   // 15: asv_run_words
+        int d = cap ? std::min(cap, p == 2 ? 16 : label_depth(s.D, spacing, step)) : 0;
+        if (d) {
+            const int z = std::min(s.zrun, s.D), parts = (z + d - 1) / d;
+            d = std::max((z + parts - 1) / parts, 4);
+        }
+        s.depth[p] = d;
+    }
+}
+
+// JFA tile depth for a set of segments: the configured one, else the one of
+// least estimated time.  A tile of z positions costs about z + 3 per sub-tile
+// (staging, numbering and barriers weigh like three positions).  The resident
+// blocks, four per SM, take the tiles in rounds; fewer tiles than that on an
+// SM run at 0.41, 0.69 and 0.85 of its full rate (one, two and three blocks),
+// which behind a full round costs a bit less, as the blocks do not end
+// together.  Fitted on clips of 160x120x40 to 1280x720x30 at every depth: the
+// choice is within 2 % of the best one, where the deepest of 32, 16 and 8 that
+// gave every block four tiles was up to 8 % off (320x240x85: depth 8 4.50 ms
+// for six iterations, 15 4.34; 641x360x30: depth 8 4.80, 15 4.46).
 static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
 {
     if (ctx->cfg.jfa_zrun > 0) return std::min(ctx->cfg.jfa_zrun, 256);
-    const long long want = 4LL * asv_jfa_resident_blocks();
-    for (int z : { 32, 16, 8 }) {
+    const int per_sm = 4;
+    const long long sms = std::max(1, asv_jfa_resident_blocks() / per_sm);
+    static const double rate[4] = { 1.0, 0.41, 0.69, 0.85 };
+    int best = 4;
+    double least = 0.0;
+    for (int z = 1; z <= 32; z++) {
         long long tiles = 0;
-        for (const SegHost &h : seg)
-            tiles += (long long)((h.W + ASV_TILE_X - 1) / ASV_TILE_X) * ((h.H + ASV_TILE_Y - 1) / ASV_TILE_Y)
-                     * ((h.D + z - 1) / z);
-        if (tiles >= want) return z;
+        double work = 0.0;
+        for (const SegHost &h : seg) {
+            const long long col = (long long)((h.W + ASV_TILE_X - 1) / ASV_TILE_X) * ((h.H + ASV_TILE_Y - 1) / ASV_TILE_Y);
+            const int ze = even_depth(h.D, z), nz = (h.D + ze - 1) / ze;
+            tiles += col * nz;
+            const double sp = seed_spacing((long long)h.W * h.H * h.D, h.Kp);
+            const int d1 = label_depth(h.D, sp, 1), d2 = label_depth(h.D, sp, 2), d = std::max((d1 + d2) / 2, 4);
+            work += (double)col * (h.D + 3.0 * nz * ((ze + d - 1) / d));
+        }
+        const long long m = (tiles + sms - 1) / sms, q = m / per_sm, k = m % per_sm;
+        double rounds = (double)(per_sm * q);
+        if (k) rounds += q ? 0.6 * k / rate[k] + 0.4 * k : k / rate[k];
+        const double cost = work / tiles * rounds;
+        if (least == 0.0 || cost < least) { best = z; least = cost; }
     }
-    return 4;
+    return best;
+}
+
+static void set_tiles(SegDesc &s)
+{
+    s.tiles_x = (s.W + ASV_TILE_X - 1) / ASV_TILE_X;
+    s.tiles_y = (s.H + ASV_TILE_Y - 1) / ASV_TILE_Y;
+    auto inv = [](int d) { return d == 1 ? 0u : (unsigned)(((1ull << 32) + d - 1) / d); };
+    s.inv_tiles_x = inv(s.tiles_x);
+    s.inv_tiles_y = inv(s.tiles_y);
 }
 
 // Allocates the packed device arrays for the segments in ctx->seg.
@@ -381,19 +459,19 @@ asv_status asv_build_layout(asv_ctx *ctx)
         s.seed_off = seeds;
         s.npass = h.npass;
         for (int p = 0; p < h.npass; p++) { s.steps[p] = h.steps[p]; s.ratio[p] = h.rmul[p] * h.ratio; }
-        s.tiles_x = (h.W + ASV_TILE_X - 1) / ASV_TILE_X;
-        s.tiles_y = (h.H + ASV_TILE_Y - 1) / ASV_TILE_Y;
-        s.zrun = zrun;
+        set_tiles(s);
+        s.zrun = even_depth(h.D, zrun);
         s.angle_filter = ctx->cfg.variant == ASV_VARIANT_PLAIN ? 1 : 0;
         s.wNum = h.g.wNum; s.hNum = h.g.hNum; s.dNum = h.g.dNum;
         s.cell_off = cells;
         s.final_buf = h.npass & 1;
+        set_depths(s);
         h.vox_off = vox; h.seed_off = seeds;
         tile_p[i] = tiles; chunk_p[i] = chunks; seed_p[i] = seeds;
         int nchunk = (int)((n + ASV_CHUNK - 1) / ASV_CHUNK);
         vox += (long long)nchunk * ASV_CHUNK;
         chunks += nchunk;
-        tiles += s.tiles_x * s.tiles_y * ((h.D + zrun - 1) / zrun);
+        tiles += s.tiles_x * s.tiles_y * ((h.D + s.zrun - 1) / s.zrun);
         seeds += ((h.Kp + 64 + 31) / 32) * 32;
         cells += h.W + h.H + h.D + 2 * h.g.wNum;
         ctx->maxpass = std::max(ctx->maxpass, h.npass);
@@ -485,6 +563,22 @@ static void do_first_init(asv_ctx *ctx)
     ctx->launches += 2;
 }
 
+// the step of pass p, and whether it forms the centroid sums, where both are
+// the same for every segment that runs the pass (k_jfa's variant for them
+// takes it), else 0
+static int pass_step(const asv_ctx *ctx, int p, int *sums)
+{
+    int step = 0;
+    for (const SegDesc &s : ctx->sd) {
+        if (p >= s.npass) continue;
+        const int last = p == s.npass - 1;
+        if (step && (s.steps[p] != step || last != *sums)) return 0;
+        step = s.steps[p];
+        *sums = last;
+    }
+    return step;
+}
+
 // the JFA ladder; the last pass of each segment also forms its centroid sums
 static void do_flood(asv_ctx *ctx, int evbase)
 {
@@ -498,7 +592,9 @@ static void do_flood(asv_ctx *ctx, int evbase)
             asv_launch_jfa_second_scatter(ctx->d, ctx->st);  // from the first pass's sparse labels
             ctx->launches += 2;
         } else {
-            asv_launch_jfa(ctx->d, p, ctx->jfa_blocks, ctx->st);
+            int sums = 0;
+            const int step = pass_step(ctx, p, &sums);
+            asv_launch_jfa(ctx->d, p, step, sums, ctx->jfa_blocks, ctx->st);
             ctx->launches++;
         }
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p + 1);
@@ -935,9 +1031,10 @@ static asv_status set_zrun(asv_ctx *ctx, int z)
     int tiles = 0;
     for (int i = 0; i < nseg; i++) {
         SegDesc &sd = ctx->sd[i];
-        sd.zrun = z;
+        sd.zrun = even_depth(sd.D, z);
+        set_depths(sd);
         tp[i] = tiles;
-        tiles += sd.tiles_x * sd.tiles_y * ((sd.D + z - 1) / z);
+        tiles += sd.tiles_x * sd.tiles_y * ((sd.D + sd.zrun - 1) / sd.zrun);
     }
     tp[nseg] = tiles;
     CK(cudaMemcpyAsync((void *)ctx->d.segs, ctx->sd.data(), sizeof(SegDesc) * nseg, cudaMemcpyHostToDevice,
@@ -1731,13 +1828,13 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
     sd.vox_off = 0; sd.nvox = (long long)WH * Db; sd.seed_off = 0;
     sd.npass = h.npass;
     for (int p = 0; p < h.npass; p++) { sd.steps[p] = h.steps[p]; sd.ratio[p] = h.rmul[p] * h.ratio; }
-    sd.tiles_x = (m.W + ASV_TILE_X - 1) / ASV_TILE_X;
-    sd.tiles_y = (m.H + ASV_TILE_Y - 1) / ASV_TILE_Y;
-    sd.zrun = pick_zrun(ctx, std::vector<SegHost>(1, h));
+    set_tiles(sd);
+    sd.zrun = even_depth(Db, pick_zrun(ctx, std::vector<SegHost>(1, h)));
     sd.angle_filter = 0;
     sd.wNum = h.g.wNum; sd.hNum = h.g.hNum; sd.dNum = h.g.dNum;
     sd.cell_off = 0;
     sd.final_buf = h.npass & 1;
+    set_depths(sd);
     sd.lab_from = (long long)z0 * WH;
     const int tiles = sd.tiles_x * sd.tiles_y * ((Db + sd.zrun - 1) / sd.zrun);
     const int chunks = (int)((sd.nvox + ASV_CHUNK - 1) / ASV_CHUNK);

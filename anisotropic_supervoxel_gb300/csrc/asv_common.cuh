@@ -15,6 +15,7 @@
 #define ASV_CHUNK 2048       // voxels per block in the per-voxel kernels
 #define ASV_TILE_X 16        // JFA tile: 16 x 16 columns x SegDesc::zrun chain positions
 #define ASV_TILE_Y 16        // (a warp covers 16 x 2 columns: fewer distinct candidates)
+#define ASV_BITS_MAXS 6      // largest step of a JFA pass's bit-set form
 #define ASV_RING 24          // 8 one-ring + 16 two-ring neighbours of the metric fallback
 #define ASV_POST_WORDS 16    // per-segment post-processing record
 
@@ -26,7 +27,9 @@ struct SegDesc {
     int npass;
     int steps[ASV_MAXP];
     float ratio[ASV_MAXP];   // ratio of each pass (base ratio x 1 or x 2)
+    int depth[ASV_MAXP];     // chain positions per sub-tile of each pass's bit-set form, 0: list form
     int tiles_x, tiles_y;
+    unsigned inv_tiles_x, inv_tiles_y;   // ceil(2^32 / tiles), 0 for one tile (asv_quotient)
     int zrun;                // JFA tile depth: chain positions per column and tile
     int angle_filter;        // plain reseed flow-angle filter
     int wNum, hNum, dNum;    // seed grid (density placement)
@@ -43,6 +46,13 @@ enum {
 };
 
 #ifdef __CUDACC__
+// n / d for n < 2^24, d <= 256, from inv = ceil(2^32 / d) (0 for d = 1): inv * d
+// exceeds 2^32 by less than d, so the product's error stays below 1 / d.
+__device__ __forceinline__ int asv_quotient(int n, unsigned inv)
+{
+    return inv ? (int)__umulhi((unsigned)n, inv) : n;
+}
+
 // Binary search: largest i in [0, n) with prefix[i] <= v.
 __device__ __forceinline__ int asv_find_seg(const int *__restrict__ prefix, int n, int v)
 {
@@ -109,7 +119,7 @@ void asv_launch_density(const AsvDev &d, cudaStream_t st);
 void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st);
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st);
 void asv_launch_draw(const AsvDev &d, cudaStream_t st);
-void asv_launch_jfa(const AsvDev &d, int pass, int grid_blocks, cudaStream_t st);
+void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_blocks, cudaStream_t st);
 void asv_launch_jfa_first_scatter(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa_second_scatter(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
@@ -120,3 +130,4 @@ void asv_launch_post(const AsvDev &d, cudaStream_t st);
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st);
 int asv_jfa_grid_blocks(int total_tiles);
 int asv_jfa_resident_blocks();
+int asv_jfa_max_depth(int step);   // chain positions a sub-tile of the step can hold

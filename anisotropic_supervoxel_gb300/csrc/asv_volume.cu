@@ -623,7 +623,7 @@ template <bool SUMS>
 __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int32_t *__restrict__ out,
                                             const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
                                             unsigned long long *__restrict__ sums, int slot0, int W, int H, int D,
-                                            int Kp, int x, int y, int p0, int zrun, int step,
+                                            int Kp, int x, int y, int p0, int n, int step,
                                             float ratio, asv_list_t *__restrict__ lists, bool valid)
 {
     const int sl = W * H;                       // segments hold < 2^31 voxels
@@ -635,7 +635,6 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
     int r, j, len;
     asv_chain_pos(p0, D, step, r, j, len);
     int z = r + j * step;
-    int n = min(zrun, D - p0);
     int sm = 0, sc = 1, sp = 2;                 // list rows of the minus / centre / plus slices
     int nm = asv_slice_list(in, max(z - step, 0) * sl, xs, ys, Kp, lists + sm * row);
     int nc = asv_slice_list(in, z * sl, xs, ys, Kp, lists + sc * row);
@@ -715,14 +714,13 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // and its plus slice the centre of the one after it.
 // ---------------------------------------------------------------------------
 #define ASV_JFA_LIST_BYTES (5 * ASV_SLICE_MAX * ASV_JFA_THREADS * (int)sizeof(asv_list_t))
-#define ASV_BITS_MAXS 6          // largest step taken in bit-set form
 #define ASV_BITS_MAXT 32         // labels per sub-tile footprint (one 32-bit mask)
 #define ASV_BITS_MAXKP 8192      // segment seed counts up to this use the bit-set form
 #define ASV_BITS_TLCAP 256       // claimed labels remembered for the reset
 #define ASV_BITS_FREE 255        // map8: label without a number yet
 #define ASV_BITS_NOLABEL 254     // map8[ASV_BITS_MAXKP]: no label (shifts to no bit)
 #define ASV_BITS_OVER 253        // map8: a label past the 32nd (the sub-tile takes the list form)
-#define ASV_ACC_ROW 7            // words per entry of the sub-tile's centroid-sum table (odd: the
+#define ASV_ACC_ROW 5            // words per entry of the sub-tile's centroid-sum table (odd: the
                                  // entries' rows start in different shared-memory banks)
 #define ASV_BITS_AREA 43264      // shared bytes of the largest sub-tiles (step 5, 9 positions): four blocks per SM
 #define ASV_JFA_AREA (ASV_BITS_AREA > ASV_JFA_LIST_BYTES ? ASV_BITS_AREA : ASV_JFA_LIST_BYTES)
@@ -985,20 +983,28 @@ __device__ __noinline__ int asv_bits_exact(unsigned m, const unsigned *__restric
 }
 
 // A thread's run of voxels with one label, added to its table entry's
-// centroid sums in shared memory: count n, sum of 2z+1 and of L, a, b; the
-// column's 2x+1 and 2y+1 times n.  Exact u32 sums (a sub-tile holds at most
-// 16 x 256 voxels of coordinates below 4096).
-__device__ __forceinline__ void asv_run_flush(unsigned *__restrict__ a, unsigned sz, unsigned la, unsigned bn, int x,
-                                              int y)
+// centroid sums in shared memory.  A run is its sum of 2 z + 1, its sums of
+// L | a << 16 and its sums of b | count << 16; an entry has five words:
+// sums of the columns x | y << 16 within the tile, of count << 20 | L, of
+// 2 z + 1, of a and of b.  All exact: a summing sub-tile has at most 15 x 256
+// = 3840 voxels, so the columns stay below 3840 * 15 < 2^16, L below 3840 *
+// 255 < 2^20 and the count below 2^12.  (With seven words, one sum each, the
+// summing pass of a 1280x720x30 window took 425 us.)
+__device__ __forceinline__ void asv_run_words(unsigned w[ASV_ACC_ROW], unsigned z, unsigned la, unsigned bn, unsigned xy)
 {
-    const unsigned n = bn >> 16;
-    atomicAdd(a + 0, n * (2u * (unsigned)x + 1u));
-    atomicAdd(a + 1, n * (2u * (unsigned)y + 1u));
-    atomicAdd(a + 2, sz);
-    atomicAdd(a + 3, n);
-    atomicAdd(a + 4, la & 0xffffu);
-    atomicAdd(a + 5, la >> 16);
-    atomicAdd(a + 6, bn & 0xffffu);
+    w[0] = (bn >> 16) * xy;
+    w[1] = ((bn & 0xffff0000u) << 4) | (la & 0xffffu);
+    w[2] = z;
+    w[3] = la >> 16;
+    w[4] = bn & 0xffffu;
+}
+
+__device__ __forceinline__ void asv_run_flush(unsigned *__restrict__ a, unsigned z, unsigned la, unsigned bn, unsigned xy)
+{
+    unsigned w[ASV_ACC_ROW];
+    asv_run_words(w, z, la, bn, xy);
+#pragma unroll
+    for (int k = 0; k < ASV_ACC_ROW; k++) atomicAdd(a + k, w[k]);
 }
 
 // One sub-tile of n <= SUB chain positions from p0 in bit-set form; false
@@ -1132,6 +1138,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     // the label changes and at the end; the table goes to the global sums
     // once per sub-tile (centroids.vs:19-54; label -1 counts in slot Kp)
     int run_e = -1;
+    const unsigned lxy = (unsigned)lx | ((unsigned)ly << 16);
     unsigned run_z = 0u, run_la = 0u, run_bn = 0u;            // L | a << 16, b | count << 16 (16 x 255 < 2^16)
     const unsigned *fn = f0 + 2 * FP;                         // the next slot
     const unsigned *lab32 = (const unsigned *)lab;
@@ -1185,7 +1192,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         if (SUMS && valid) {
             const int e = bt >= 0 ? bt : ASV_BITS_MAXT;
             if (e != run_e) {
-                if (run_e >= 0) asv_run_flush(b.acc + ASV_ACC_ROW * run_e, run_z, run_la, run_bn, x, y);
+                if (run_e >= 0) asv_run_flush(b.acc + ASV_ACC_ROW * run_e, run_z, run_la, run_bn, lxy);
                 run_e = e;
                 run_z = run_la = run_bn = 0u;
             }
@@ -1201,70 +1208,96 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         // lane of the block gets here; lanes without a run join with entry
         // -1, which adds nothing), so a warp adds each entry once
         const unsigned grp = __match_any_sync(0xffffffffu, run_e);
-        const unsigned run_n = run_bn >> 16;
-        const unsigned q[7] = { run_n * (2u * (unsigned)x + 1u), run_n * (2u * (unsigned)y + 1u), run_z, run_n,
-                                run_la & 0xffffu, run_la >> 16, run_bn & 0xffffu };
-        unsigned t[7];
+        unsigned w[ASV_ACC_ROW];
+        asv_run_words(w, run_z, run_la, run_bn, lxy);
 #pragma unroll
-        for (int k = 0; k < 7; k++) t[k] = __reduce_add_sync(grp, q[k]);
+        for (int k = 0; k < ASV_ACC_ROW; k++) w[k] = __reduce_add_sync(grp, w[k]);
         if (run_e >= 0 && lane == __ffs(grp) - 1) {
 #pragma unroll
-            for (int k = 0; k < 7; k++) atomicAdd(b.acc + ASV_ACC_ROW * run_e + k, t[k]);
+            for (int k = 0; k < ASV_ACC_ROW; k++) atomicAdd(b.acc + ASV_ACC_ROW * run_e + k, w[k]);
         }
         __syncthreads();
-        for (int i = tid; i < (T + 1) * 7; i += ASV_JFA_THREADS) {
-            const int e = i / 7, k = i - e * 7;
+        for (int i = tid; i < (T + 1) * 8; i += ASV_JFA_THREADS) {
+            const int e = i >> 3, k = i & 7;
             const int ent = e < T ? e : ASV_BITS_MAXT;           // the -1 entry after the T labels
-            const unsigned v = b.acc[ASV_ACC_ROW * ent + k];
-            if (v) atomicAdd(sums + 8ull * (slot0 + (ent < ASV_BITS_MAXT ? b.tlab[ent] : Kp)) + k,
-                             (unsigned long long)v);
+            const unsigned *a = b.acc + ASV_ACC_ROW * ent;
+            const unsigned cnt = a[1] >> 20;
+            if (k == 7 || !cnt) continue;
+            unsigned v;                                          // 2 x + 1 = 2 (tx0 + column) + 1
+            if (k == 0) v = 2u * (a[0] & 0xffffu) + cnt * (2u * (unsigned)tx0 + 1u);
+            else if (k == 1) v = 2u * (a[0] >> 16) + cnt * (2u * (unsigned)ty0 + 1u);
+            else if (k == 3) v = cnt;
+            else if (k == 4) v = a[1] & 0xfffffu;
+            else v = a[k == 2 ? 2 : k - 2];
+            atomicAdd(sums + 8ull * (slot0 + (ent < ASV_BITS_MAXT ? b.tlab[ent] : Kp)) + k, (unsigned long long)v);
         }
     }
     __syncthreads();                                          // the footprint and table are reused
     return true;
 }
 
+// Variants of k_jfa: ST is the step of the pass (1 to 6), ASV_JFA_LIST for the
+// larger ones (list form only) or 0 for segments of different steps; SUMS 0
+// or 1, or 2 where the pass is the last one of some segments only.  A variant
+// holds just the code of its pass: against the one kernel for all (now <0,
+// 2>), which keeps the registers of the worst of them, the 240x160x30 clip
+// with its full ladder took 3.96 instead of 4.39 ms, the 640x480x60 one 16.1
+// instead of 16.7.
+#define ASV_JFA_LIST 7
 // one tile of a pass: bit-set form by sub-tiles where it applies, else (or
 // for a sub-tile whose footprint holds too many labels) the list form
-template <bool SUMS>
+template <int ST, bool SUMS>
 __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int32_t *__restrict__ out,
                                              const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
                                              unsigned long long *__restrict__ sums, int slot0, int W, int H, int D,
-                                             int Kp, int tx0, int ty0, int p0, int zrun, int step, float ratio,
-                                             unsigned char *smem)
+                                             int Kp, int tx0, int ty0, int p0, int zrun, int depth, int step,
+                                             float ratio, unsigned char *smem)
 {
     const int n = min(zrun, D - p0);
     const int lx = threadIdx.x % ASV_TILE_X, ly = threadIdx.x / ASV_TILE_X;
     const int gx = tx0 + lx, gy = ty0 + ly;
     const bool valid = gx < W && gy < H;                       // block-uniform loop: every lane runs the tile
-    // sub-tiles the bit-set form leaves (a bit per sub-tile of `sub` positions)
-    // go through one inlined copy of the list form
-    unsigned fail = 1u;
-    int sub = n;
-    // <= 32 sub-tiles of >= 4; with tiles of 4 positions the footprint slots
-    // outnumber the positions from step 3 on, where the list form is faster
-    if (step <= ASV_BITS_MAXS && Kp <= ASV_BITS_MAXKP && n <= 32 * 4 && (zrun >= 8 || step <= 2)) {
-        fail = 0u;
-        // (sub-tiles of equal depth: 30 positions are 15 + 15, not 16 + 14)
+    // `todo` has a bit for each position of the tile (32 at a time).  A round
+    // cuts the positions to do in sub-tiles of `cap`; the sub-tiles whose
+    // labels do not fit go to the next round, half as deep, and below four
+    // positions to one inlined copy of the list form.
+    for (int c0 = 0; c0 < n; c0 += 32) {
+        const int nc = min(n - c0, 32), pc = p0 + c0;
+        unsigned todo = 0xffffffffu >> (32 - nc);
+        int cap = SUMS ? min(depth, 15) : depth;               // 15: asv_run_words
+        if (Kp > ASV_BITS_MAXKP) cap = 0;
 #define ASV_BITS_CASE(S_)                                                                                    \
     case S_:                                                                                                 \
-        sub = (n + AsvBitsGeo<S_>::SUB - 1) / AsvBitsGeo<S_>::SUB;                                           \
-        sub = (n + sub - 1) / sub;                                                                           \
-        for (int q0 = 0, i = 0; q0 < n; q0 += sub, i++)                                                      \
-            if (!asv_jfa_bits_sub<S_, SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, tx0, ty0, p0 + q0, \
-                                            min(sub, n - q0), ratio, smem))                                  \
-                fail |= 1u << i;                                                                             \
+        cap = min(cap, AsvBitsGeo<S_>::SUB);                                                                 \
+        do {                                                                                                 \
+            const int q = __ffs(todo) - 1;                                                                   \
+            const unsigned past = ~(todo >> q);                                                              \
+            const int m = min(cap, past ? __ffs(past) - 1 : 32);                                             \
+            const unsigned bits = (0xffffffffu >> (32 - m)) << q;                                            \
+            todo &= ~bits;                                                                                   \
+            if (!asv_jfa_bits_sub<S_, SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, tx0, ty0, pc + q,   \
+                                            m, ratio, smem))                                                 \
+                fail |= bits;                                                                                \
+        } while (todo);                                                                                      \
         break;
-        switch (step) {
-            ASV_BITS_CASE(1) ASV_BITS_CASE(2) ASV_BITS_CASE(3) ASV_BITS_CASE(4) ASV_BITS_CASE(5) ASV_BITS_CASE(6)
+        while (ST != ASV_JFA_LIST && cap >= 4 && todo) {
+            unsigned fail = 0u;
+            switch (ST ? ST : step) {
+                ASV_BITS_CASE(1) ASV_BITS_CASE(2) ASV_BITS_CASE(3) ASV_BITS_CASE(4) ASV_BITS_CASE(5) ASV_BITS_CASE(6)
+            }
+            todo = fail;
+            cap = (cap + 1) >> 1;
         }
 #undef ASV_BITS_CASE
-    }
-    for (int i = 0; fail; i++, fail >>= 1) {
-        if (!(fail & 1u)) continue;
-        asv_jfa_run<SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, min(gx, W - 1), min(gy, H - 1), p0 + i * sub,
-                          min(sub, n - i * sub), step, ratio, (asv_list_t *)smem + threadIdx.x, valid);
-        __syncthreads();                                       // the list rows alias the footprint
+        while (todo) {                                         // runs of positions left
+            const int q = __ffs(todo) - 1;
+            const unsigned past = ~(todo >> q);
+            const int m = past ? __ffs(past) - 1 : 32;
+            todo &= ~((0xffffffffu >> (32 - m)) << q);
+            asv_jfa_run<SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, min(gx, W - 1), min(gy, H - 1), pc + q, m,
+                              step, ratio, (asv_list_t *)smem + threadIdx.x, valid);
+            __syncthreads();                                   // the list rows alias the footprint
+        }
     }
 }
 
@@ -1281,27 +1314,28 @@ __device__ __forceinline__ void asv_jfa_smem_init(unsigned char *smem)
 }
 
 // tile = ASV_TILE_X x ASV_TILE_Y columns x S.zrun chain positions
+template <int ST, int SUMS>
 __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
                                                          const int32_t *__restrict__ in,
                                                          int32_t *__restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char asv_jfa_smem[];
-    asv_jfa_smem_init(asv_jfa_smem);
+    if (ST != ASV_JFA_LIST) asv_jfa_smem_init(asv_jfa_smem);
     for (int t = blockIdx.x; t < d.total_tiles; t += gridDim.x) {
         const int si = asv_find_seg(d.tile_prefix, d.nseg, t);
         const SegDesc &S = d.segs[si];
         if (pass >= S.npass) continue;
         const int lt = t - d.tile_prefix[si];
-        const int tx = lt % S.tiles_x, rest = lt / S.tiles_x;
-        const int ty = rest % S.tiles_y, p0 = (rest / S.tiles_y) * S.zrun;
-        if (pass == S.npass - 1)                   // the iteration's labels: sum them
-            asv_jfa_tile<true>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
+        const int rest = asv_quotient(lt, S.inv_tiles_x), tx = lt - rest * S.tiles_x;
+        const int tz = asv_quotient(rest, S.inv_tiles_y), ty = rest - tz * S.tiles_y, p0 = tz * S.zrun;
+        if (SUMS == 1 || (SUMS == 2 && pass == S.npass - 1))   // the iteration's labels: sum them
+            asv_jfa_tile<ST, true>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
                                d.sums, S.seed_off, S.W, S.H, S.D, S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0,
-                               S.zrun, S.steps[pass], S.ratio[pass], asv_jfa_smem);
+                               S.zrun, S.depth[pass], S.steps[pass], S.ratio[pass], asv_jfa_smem);
         else
-            asv_jfa_tile<false>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
+            asv_jfa_tile<ST, false>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
                                 nullptr, 0, S.W, S.H, S.D, S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0,
-                                S.zrun, S.steps[pass], S.ratio[pass], asv_jfa_smem);
+                                S.zrun, S.depth[pass], S.steps[pass], S.ratio[pass], asv_jfa_smem);
     }
 }
 
@@ -1483,8 +1517,9 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS) k_jfa_single(AsvDev d, const 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx = t % S.tiles_x, rest = t / S.tiles_x;
         const int ty = rest % S.tiles_y, p0 = (rest / S.tiles_y) * S.zrun;
-        asv_jfa_tile<false>(in, out, d.lab + S.vox_off, d.jtab + 3 * S.seed_off, nullptr, 0, S.W, S.H, S.D,
-                            S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0, S.zrun, step, ratio, asv_jfa_smem);
+        asv_jfa_tile<0, false>(in, out, d.lab + S.vox_off, d.jtab + 3 * S.seed_off, nullptr, 0, S.W, S.H, S.D,
+                            S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0, S.zrun, step <= ASV_BITS_MAXS ? 16 : 0, step, ratio,
+                            asv_jfa_smem);
     }
 }
 
@@ -1875,6 +1910,19 @@ void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st)
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st) { k_first_init<<<seed_blocks(d), 128, 0, st>>>(d); }
 void asv_launch_draw(const AsvDev &d, cudaStream_t st) { k_draw<<<seed_blocks(d), 128, 0, st>>>(d); }
 
+typedef void (*AsvJfaKernel)(AsvDev, int, const int32_t *, int32_t *);
+
+// k_jfa's variant for a pass of this step (0: segments of different steps, or
+// of different ladders' lengths at a last pass)
+static AsvJfaKernel asv_jfa_variant(int step, int sums)
+{
+    static const AsvJfaKernel k[ASV_JFA_LIST + 1][2] = {
+        { k_jfa<0, 2>, k_jfa<0, 2> }, { k_jfa<1, 0>, k_jfa<1, 1> }, { k_jfa<2, 0>, k_jfa<2, 1> },
+        { k_jfa<3, 0>, k_jfa<3, 1> }, { k_jfa<4, 0>, k_jfa<4, 1> }, { k_jfa<5, 0>, k_jfa<5, 1> },
+        { k_jfa<6, 0>, k_jfa<6, 1> }, { k_jfa<ASV_JFA_LIST, 0>, k_jfa<ASV_JFA_LIST, 1> } };
+    return k[step < ASV_JFA_LIST ? step : ASV_JFA_LIST][sums];
+}
+
 // k_jfa's dynamic shared memory (list rows or bit-set footprint, and the
 // bit-set table) exceeds the 48 KiB default: raised once per device
 static void asv_jfa_attributes()
@@ -1885,7 +1933,10 @@ static void asv_jfa_attributes()
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return;
-    cudaFuncSetAttribute(k_jfa, cudaFuncAttributeMaxDynamicSharedMemorySize, ASV_JFA_SMEM);
+    for (int st = 0; st < ASV_JFA_LIST; st++)
+        for (int sums = 0; sums < 2; sums++)
+            cudaFuncSetAttribute((const void *)asv_jfa_variant(st, sums), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 ASV_JFA_SMEM);
     cudaFuncSetAttribute(k_jfa_single, cudaFuncAttributeMaxDynamicSharedMemorySize, ASV_JFA_SMEM);
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
@@ -1899,11 +1950,18 @@ int asv_jfa_resident_blocks()
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         asv_jfa_attributes();
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_jfa, ASV_JFA_THREADS, ASV_JFA_SMEM);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_jfa<0, 2>, ASV_JFA_THREADS, ASV_JFA_SMEM);
         const int b = sms * (per > 0 ? per : 1);
         return b > 0 ? b : 1024;
     }();
     return blocks;
+}
+
+int asv_jfa_max_depth(int step)
+{
+    static const int sub[ASV_BITS_MAXS + 1] = { 0, AsvBitsGeo<1>::SUB, AsvBitsGeo<2>::SUB, AsvBitsGeo<3>::SUB,
+                                                AsvBitsGeo<4>::SUB, AsvBitsGeo<5>::SUB, AsvBitsGeo<6>::SUB };
+    return step >= 1 && step <= ASV_BITS_MAXS ? sub[step] : 0;
 }
 
 int asv_jfa_grid_blocks(int total_tiles)
@@ -1912,12 +1970,13 @@ int asv_jfa_grid_blocks(int total_tiles)
     return total_tiles < blocks ? total_tiles : blocks;
 }
 
-void asv_launch_jfa(const AsvDev &d, int pass, int grid_blocks, cudaStream_t st)
+void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_blocks, cudaStream_t st)
 {
     const int32_t *in = (pass & 1) ? d.labB : d.labA;
     int32_t *out = (pass & 1) ? d.labA : d.labB;
     asv_jfa_attributes();
-    k_jfa<<<grid_blocks, 256, ASV_JFA_SMEM, st>>>(d, pass, in, out);
+    asv_jfa_variant(step, sums)<<<grid_blocks, ASV_JFA_THREADS, step < ASV_JFA_LIST ? ASV_JFA_SMEM : ASV_JFA_LIST_BYTES,
+                                  st>>>(d, pass, in, out);
 }
 
 void asv_launch_jfa_first_scatter(const AsvDev &d, cudaStream_t st)
