@@ -153,6 +153,11 @@ struct asv_ctx {
     bool have_rgb = false, have_flow = false, have_pos0 = false, have_M0 = false, have_lab = false;
     bool seeded = false, ran = false;
     bool drawn = false;          // labA holds a fresh seed draw: the first pass may scatter
+    bool undraw = false;         // ... and nothing else: the second pass may take the seeds out instead of a fill
+    // fills of the label volumes run beside the (latency-bound) metric solves
+    // of the next seeds, on a stream of their own between two events
+    cudaStream_t side = nullptr;
+    cudaEvent_t side_ev[2] = { nullptr, nullptr };
     int post_host[ASV_POST_WORDS];
     // graph
     cudaGraphExec_t gexec = nullptr;
@@ -275,7 +280,7 @@ static void free_layout(asv_ctx *ctx)
     ctx->bytes = 0;
     ctx->d = AsvDev{};
     ctx->have_rgb = ctx->have_flow = ctx->have_pos0 = ctx->have_M0 = ctx->have_lab = false;
-    ctx->seeded = ctx->ran = ctx->drawn = false;
+    ctx->seeded = ctx->ran = ctx->drawn = ctx->undraw = false;
     ctx->sm.on = false;
 }
 
@@ -336,8 +341,8 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
     // rgb 3 + lab 4 + fwd/bwd 16 + two label buffers 8 + first-pass keys 8
     size_t per_vox = 3 + 4 + 8 + 8 + 4 + 4 + 8;
     // float4 pos0/pos/slab/grid, 8-float M0/M/Mself/Mmemo, jtab 3 float4, 8 u64
-    // sums, int neg/mkey/rank, u64 dacc, the metric ring
-    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 3 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 8;
+    // sums, int neg/mkey/rank/neglist, u64 dacc, the metric ring
+    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 4 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 8;
     // each of the ~30 allocations rounds up to 256 bytes
     size_t fixed = 32 * 256 + 256 * 4 + 16;
     size_t per_seg = sizeof(SegDesc) + 3 * 4 + ASV_POST_WORDS * 4;
@@ -500,6 +505,8 @@ asv_status asv_build_layout(asv_ctx *ctx)
     AL(d.Mself, (size_t)seeds * 8); AL(d.neg, seeds);
     AL(d.Mmemo, (size_t)seeds * 8); AL(d.mkey, seeds);
     AL(d.Mring, (size_t)seeds * ASV_RING * 8); AL(d.ringok, (size_t)seeds * ASV_RING);
+    AL(d.neglist, seeds); AL(d.negcount, 1);
+    CK(cudaMemsetAsync(d.negcount, 0, sizeof(int), ctx->st));
     AL(d.grid, seeds);
     AL(d.dacc, seeds);
     AL(d.cells, std::max(cells, 1));
@@ -559,7 +566,7 @@ static void do_first_init(asv_ctx *ctx)
     asv_launch_first_init(ctx->d, ctx->st);
     cudaMemsetAsync(ctx->d.labA, 0xff, sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK, ctx->st);
     asv_launch_draw(ctx->d, ctx->st);
-    ctx->drawn = true;
+    ctx->drawn = ctx->undraw = true;
     ctx->launches += 2;
 }
 
@@ -580,16 +587,19 @@ static int pass_step(const asv_ctx *ctx, int p, int *sums)
 }
 
 // the JFA ladder; the last pass of each segment also forms its centroid sums
-static void do_flood(asv_ctx *ctx, int evbase)
+// (prepared: the next seeds left labB at -1, the sums at zero and the first
+// pass's list empty)
+static void do_flood(asv_ctx *ctx, int evbase, bool prepared)
 {
-    cudaMemsetAsync(ctx->d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)ctx->d.total_seeds, ctx->st);
+    if (!prepared)
+        cudaMemsetAsync(ctx->d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)ctx->d.total_seeds, ctx->st);
     for (int p = 0; p < ctx->maxpass; p++) {
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p);
         if (p == 0 && ctx->drawn) {
-            asv_launch_jfa_first_scatter(ctx->d, ctx->st);   // step 1 from the drawn seeds
-            ctx->launches += 2;
+            asv_launch_jfa_first(ctx->d, prepared, !ctx->undraw, ctx->st);   // step 1 from the drawn seeds
+            ctx->launches++;
         } else if (p == 1 && ctx->drawn) {
-            asv_launch_jfa_second_scatter(ctx->d, ctx->st);  // from the first pass's sparse labels
+            asv_launch_jfa_second_scatter(ctx->d, ctx->undraw, ctx->st);   // from the first pass's sparse labels
             ctx->launches += 2;
         } else {
             int sums = 0;
@@ -599,7 +609,7 @@ static void do_flood(asv_ctx *ctx, int evbase)
         }
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p + 1);
     }
-    ctx->drawn = false;
+    ctx->drawn = ctx->undraw = false;
 }
 
 // the reseed of centroids_next_seeds (the sums came with the flood)
@@ -616,17 +626,26 @@ static void do_sums_from_labels(asv_ctx *ctx)
     ctx->launches++;
 }
 
-static void do_next_seeds(asv_ctx *ctx)
+// The metric at the new seed positions and the redraw.  loop: inside the
+// Lloyd loop, where the positions are formed here too (k_finalize otherwise)
+// and the next flood finds labB filled, the sums zeroed and its list empty.
+static void do_next_seeds(asv_ctx *ctx, bool loop)
 {
-    asv_launch_metric(ctx->d, 1, ctx->st);
-    cudaMemsetAsync(ctx->d.labA, 0xff, sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK, ctx->st);
-    asv_launch_draw(ctx->d, ctx->st);
-    ctx->drawn = true;
-    ctx->launches += 6;       // five metric kernels + the seed draw
+    const size_t bytes = sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK;
+    cudaEventRecord(ctx->side_ev[0], ctx->st);
+    cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0);
+    cudaMemsetAsync(ctx->d.labA, 0xff, bytes, ctx->side);
+    if (loop) cudaMemsetAsync(ctx->d.labB, 0xff, bytes, ctx->side);
+    cudaEventRecord(ctx->side_ev[1], ctx->side);
+    asv_launch_next_seeds(ctx->d, loop, loop, ctx->st,
+                          [](void *c) { cudaStreamWaitEvent(((asv_ctx *)c)->st, ((asv_ctx *)c)->side_ev[1], 0); }, ctx);
+    ctx->drawn = ctx->undraw = true;
+    ctx->launches += 3;       // two metric kernels, the combination with the draw
 }
 
 static void do_post(asv_ctx *ctx)
 {
+    ctx->undraw = false;      // one of the label volumes takes the result
     asv_launch_post(ctx->d, ctx->st);
     ctx->launches += 4;
 }
@@ -638,9 +657,8 @@ static void enqueue_lloyd(asv_ctx *ctx, bool instrument)
     const int per_it = 2 * ctx->maxpass;
     do_first_init(ctx);
     for (int it = 1; it <= I; it++) {
-        if (it > 1) do_next_seeds(ctx);
-        do_flood(ctx, instrument ? (it - 1) * per_it : -1);
-        do_centroids(ctx, it != I);
+        if (it > 1) do_next_seeds(ctx, true);
+        do_flood(ctx, instrument ? (it - 1) * per_it : -1, it > 1);
     }
     do_post(ctx);
 }
@@ -735,6 +753,9 @@ asv_status asv_create(const asv_config *cfg, asv_ctx **out)
         if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return ASV_ERR_CUDA; }
         ctx->own_st = true;
     }
+    bool ok = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t &e : ctx->side_ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (!ok) { asv_destroy(ctx); cudaGetLastError(); return ASV_ERR_CUDA; }
     *out = ctx;
     return ASV_OK;
 }
@@ -751,6 +772,8 @@ asv_status asv_destroy(asv_ctx *ctx)
     for (auto e : ctx->ev) cudaEventDestroy(e);
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     for (auto e : ctx->sev) if (e) cudaEventDestroy(e);
+    for (auto e : ctx->side_ev) if (e) cudaEventDestroy(e);
+    if (ctx->side) cudaStreamDestroy(ctx->side);
     if (ctx->cp) {
         cudaStreamDestroy(ctx->cp);
         for (int k = 0; k < 2; k++) { cudaEventDestroy(ctx->fed_ev[k]); cudaEventDestroy(ctx->used_ev[k]); }
@@ -929,7 +952,7 @@ asv_status asv_flood(asv_ctx *ctx, int lloyd_iter)
     if (!ctx) return ASV_ERR_BAD_ARG;
     (void)lloyd_iter;
     if (!ctx->seeded) return fail(ctx, ASV_ERR_STATE, "no seeds drawn: call asv_ld_first_init first");
-    do_flood(ctx, -1);
+    do_flood(ctx, -1, false);
     CK(cudaGetLastError());
     return ASV_OK;
 }
@@ -948,7 +971,7 @@ asv_status asv_ld_next_seeds_matrix(asv_ctx *ctx, int lloyd_iter)
     if (!ctx) return ASV_ERR_BAD_ARG;
     (void)lloyd_iter;
     if (!ctx->seeded) return fail(ctx, ASV_ERR_STATE, "no seeds drawn: call asv_ld_first_init first");
-    do_next_seeds(ctx);
+    do_next_seeds(ctx, false);
     CK(cudaGetLastError());
     return ASV_OK;
 }
@@ -1329,6 +1352,7 @@ asv_status asv_set_seeds(asv_ctx *ctx, const float *in, int Kp)
     CK(cudaMemcpyAsync(ctx->d.M + 8 * (size_t)off, m.data(), sizeof(float) * 8 * Kp, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemsetAsync(ctx->d.mkey + off, 0xff, sizeof(int) * Kp, ctx->st));   // drop the reseed memo
     asv_launch_draw(ctx->d, ctx->st);   // packs the JFA table (the label write is ignored here)
+    ctx->undraw = false;                // (but the seeds drawn before may stand elsewhere)
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->st));
     ctx->seeded = true;
@@ -1377,6 +1401,7 @@ asv_status asv_check_dead_seeds_host(asv_ctx *ctx, const int32_t *raw_in, int32_
     const SegDesc &s = ctx->sd[0];
     for (long long v = 0; v < s.nvox; v++)
         if (raw_in[v] < -1 || raw_in[v] >= s.Kp) return fail(ctx, ASV_ERR_BAD_ARG, "label outside [-1, Kp)");
+    ctx->undraw = false;
     int32_t *fin = (s.final_buf ? ctx->d.labB : ctx->d.labA) + s.vox_off;
     CK(cudaMemcpyAsync(fin, raw_in, 4 * (size_t)s.nvox, cudaMemcpyHostToDevice, ctx->st));
     do_sums_from_labels(ctx);
@@ -1395,6 +1420,7 @@ asv_status asv_jfa_pass_host(asv_ctx *ctx, int step, float ratio, const int32_t 
         return fail(ctx, ASV_ERR_STATE, "need a clip, its LAB volume and a seed table");
     const SegDesc &s = ctx->sd[0];
     size_t n = (size_t)s.nvox;
+    ctx->undraw = false;
     int32_t *din = ctx->d.labA + s.vox_off, *dout = ctx->d.labB + s.vox_off;
     CK(cudaMemcpyAsync(din, in, 4 * n, cudaMemcpyHostToDevice, ctx->st));
     asv_launch_jfa_single(ctx->d, din, s.nvox, s.Kp, dout, step, ratio, ctx->st);
@@ -1879,7 +1905,7 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
     // seed_matrix, RGB2LAB (above), Lloyd loop, check_dead_seeds (Render.cpp:470-512)
     ctx->launches = 4;                                           // LAB, density (2), seed composition
     asv_launch_metric(d, 0, st);
-    ctx->launches += 5;
+    ctx->launches += 3;
     if (ctx->cfg.use_graph && !ctx->cfg.instrument) {
         const bool same = ctx->sgexec && std::memcmp(&ctx->skey, &d, sizeof(AsvDev)) == 0 &&
                           ctx->skey_blocks == ctx->jfa_blocks && ctx->skey_passes == ctx->maxpass &&

@@ -100,6 +100,7 @@ struct AsvDev {
     float *Mself; int *neg;      // metric scratch
     float *Mmemo; int *mkey;     // reseed memo: metric of the voxel key of the last solve
     float *Mring; int *ringok;
+    int *neglist, *negcount;     // seeds whose own metric is not PSD (empty between solves)
     float4 *grid;                // grid seeds
     unsigned long long *dacc;    // density accumulators (2^-24 units)
     int *cells;                  // cell tables
@@ -120,14 +121,16 @@ void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st);
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st);
 void asv_launch_draw(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_blocks, cudaStream_t st);
-void asv_launch_jfa_first_scatter(const AsvDev &d, cudaStream_t st);
-void asv_launch_jfa_second_scatter(const AsvDev &d, cudaStream_t st);
+void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t st);
+void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st);
 void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
                            cudaStream_t st);
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);
 void asv_launch_post(const AsvDev &d, cudaStream_t st);
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st);
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st, void (*before_draw)(void *),
+                           void *arg);
 int asv_jfa_grid_blocks(int total_tiles);
 int asv_jfa_resident_blocks();
 int asv_jfa_max_depth(int step);   // chain positions a sub-tile of the step can hold

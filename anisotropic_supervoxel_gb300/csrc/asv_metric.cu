@@ -16,14 +16,19 @@
 // One warp per solve: lane i holds row i of the system; column dot products
 // are butterfly sums over the lanes (asv_lane_sum), which leave the same bits
 // on every lane, so all lanes apply the same rotations.
-// Launches: k_metric_self (a warp per seed), k_metric_psd (a thread per
-// solve: the FP64 PSD tests), k_metric_ring (a warp per seed and neighbour,
-// only for non-PSD seeds), k_metric_psd again, k_metric_combine (a thread per
-// seed).  A reseed solve is skipped when the seed's voxel is the one of its
+// Launches: k_metric_self (a warp per seed: in a reseed first the seed's new
+// position, then its solve and PSD test; the non-PSD seeds are listed),
+// k_metric_ring (a warp per listed seed and neighbour) and k_metric_combine (a
+// thread per seed: the fallbacks, and the seed's draw where the next flood
+// follows).  A reseed solve is skipped when the seed's voxel is the one of its
 // previous reseed solve in this Lloyd run: the metric is a function of that
 // voxel and the flow only, so the stored result is the solve's result.
+// The chain is latency-bound (a few warps per SM, at most some sixty rotations
+// one after another), so its launches count: seven kernels before, with the
+// position, the PSD tests (twice) and the draw on their own and a ring warp
+// for every seed, took about 80 us of a Lloyd iteration on the 320x240x85 clip.
 // Compiled with -fmad=false.
-#include "asv_common.cuh"
+#include "asv_seed.cuh"
 
 #include <float.h>
 
@@ -41,6 +46,19 @@ __device__ __forceinline__ float asv_lane_sum(float v)
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) v = v + __shfl_xor_sync(FULL, v, off);
     return v;
+}
+
+// |ga| <= FLT_EPSILON * sqrtf(q), the rotation test, mostly without the square
+// root, which would stand in the chain of every pair: away from the boundary
+// (FLT_EPSILON^2 = 2^-46, all roundings below 2^-21) the squares decide
+__device__ __forceinline__ bool asv_orthogonal(float ga, float q)
+{
+    const float g2 = ga * ga, lim = q * 0x1p-46f;
+    if (q > 1e-20f && q < 1e30f) {
+        if (g2 > lim * (1.0f + 0x1p-18f)) return false;
+        if (g2 < lim * (1.0f - 0x1p-18f)) return true;
+    }
+    return fabsf(ga) <= FLT_EPSILON * sqrtf(q);
 }
 
 // min-norm least squares in FP32; u = this lane's row (zero beyond m),
@@ -61,7 +79,7 @@ __device__ void asv_lsq_minnorm_warp(int m, float u[6], float bl, float x[6])
                 const float be = asv_lane_sum(u[q] * u[q]);
                 const float ga = asv_lane_sum(u[p] * u[q]);
                 if (ga == 0.0f) continue;
-                if (fabsf(ga) <= FLT_EPSILON * sqrtf(al * be)) continue;
+                if (asv_orthogonal(ga, al * be)) continue;
                 float zeta = (be - al) / (2.0f * ga);
                 float t = 1.0f / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
                 if (zeta < 0.0f) t = -t;
@@ -188,6 +206,28 @@ __device__ int asv_m6_negative(const float M[6])
     return 0;
 }
 
+// The same, decided in FP32 where the minors are clear of their rounding
+// (a two-by-two minor is off by at most 2^-22 of its terms, the determinant by
+// 2^-20 of its terms' sum), as they are for nearly every flow: the FP64 test
+// of one matrix takes longer than its solve's last sweep.
+__device__ int asv_m6_negative_quick(const float M[6])
+{
+    const float a = M[0], b = M[1], c = M[2], d = M[3], e = M[4], f = M[5];
+    const float ad = a * d, bb = b * b, af = a * f, cc = c * c, df = d * f, ee = e * e;
+    const float t1 = ad * f, t2 = 2.0f * b * c * e, t3 = a * ee, t4 = d * cc, t5 = f * bb;
+    const float sum = fabsf(t1) + fabsf(t2) + fabsf(t3) + fabsf(t4) + fabsf(t5);
+    const float least = fminf(fminf(ad + bb, af + cc), fminf(df + ee, sum));
+    const float most = fmaxf(fmaxf(fmaxf(a, d), f), fmaxf(fmaxf(fabsf(b), fabsf(c)), fabsf(e)));
+    // (the ranges keep what underflows far below the bounds; NaN fails them)
+    if (a > 0.0f && d > 0.0f && f > 0.0f && least > 1e-20f && most < 1e8f && sum < 1e30f) {
+        const float m1 = ad - bb, m2 = af - cc, m3 = df - ee, det = (t1 + t2) - (t3 + t4 + t5);
+        const float e1 = 0x1p-22f * (ad + bb), e2 = 0x1p-22f * (af + cc), e3 = 0x1p-22f * (df + ee), ed = 0x1p-20f * sum;
+        if (m1 > e1 && m2 > e2 && m3 > e3 && det > ed) return 0;
+        if (m1 < -e1 || m2 < -e2 || m3 < -e3 || det < -ed) return 1;
+    }
+    return asv_m6_negative(M);
+}
+
 __device__ void asv_m6_nearest_psd(const float M[6], float out[6])
 {
     double w[3], V[3][3];
@@ -312,16 +352,27 @@ __device__ __forceinline__ int asv_seed_key(const SegDesc &S, float4 p)
     return (frame * S.H + y) * S.W + x;
 }
 
-// neg[g]: 0 = PSD, 1 = non-PSD (fallbacks run), 2 = memo hit (reseed only),
-// 3 = solved, PSD test pending (k_metric_psd).  Which seed positions:
-// reseed 0 -> pos0 (seed_matrix), 1 -> pos (reseed).
+// neg[g]: 0 = PSD, 1 = non-PSD (fallbacks run), 2 = memo hit (reseed only).
+// Which seed positions: reseed 0 -> pos0 (seed_matrix), 1 -> pos (reseed),
+// 2 -> pos formed here from the centroid sums (asv_reseed).
 __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
 {
     const int lane = threadIdx.x & 31;
     SeedRef r;
     if (!asv_seed_ref(d, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, r)) return;   // warp-uniform
     const SegDesc &S = d.segs[r.si];
-    float4 p = reseed ? d.pos[r.g] : d.pos0[r.g];
+    float4 p;
+    if (reseed == 2) {
+        float q[3], c[3];
+        asv_reseed(d, S, r.i, q, c);                  // every lane the same
+        p = make_float4(q[0], q[1], q[2], (float)r.i);
+        if (lane == 0) {
+            d.pos[r.g] = p;
+            d.slab[r.g] = make_float4(c[0], c[1], c[2], 0.0f);
+        }
+    } else {
+        p = reseed ? d.pos[r.g] : d.pos0[r.g];
+    }
     if (reseed && d.mkey[r.g] == asv_seed_key(S, p)) {
         if (lane == 0) d.neg[r.g] = 2;
         return;
@@ -330,69 +381,52 @@ __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
     int frame = min(max((int)p.z, 0), S.D - 1);   // positions are inside; keep reads in bounds
     float M[6];
     asv_metric_solve_warp(d.fwd + S.vox_off, d.bwd + S.vox_off, S.W, S.H, S.D, fx, fy, frame, M);
-    if (lane < 6) d.Mself[8 * r.g + lane] = M[lane];
-    if (lane == 0) d.neg[r.g] = 3;
-}
-
-// The FP64 PSD tests of the solves, one thread per solve: the warp solves
-// leave them pending so that each 3x3 eigen-decomposition runs on one lane
-// of a full warp instead of on all 32 lanes of the solving warp (GB300's FP64
-// pipe is narrow).  flag 3 (self) / 2 (ring) marks a pending test.
-__global__ void k_metric_psd(AsvDev d)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long nself = d.total_seeds;
-    SeedRef r;
-    if (t < nself) {
-        if (asv_seed_ref(d, (int)t, r) && d.neg[t] == 3) d.neg[t] = asv_m6_negative(d.Mself + 8 * t);
-        return;
+    if (lane == 0) {
+#pragma unroll
+        for (int e = 0; e < 6; e++) d.Mself[8 * r.g + e] = M[e];
+        const int neg = asv_m6_negative_quick(M);
+        d.neg[r.g] = neg;
+        if (neg) d.neglist[atomicAdd(d.negcount, 1)] = r.g;
     }
-    const long long k = t - nself;                       // ring task: seed * ASV_RING + neighbour
-    if (k >= nself * ASV_RING || !asv_seed_ref(d, (int)(k / ASV_RING), r)) return;
-    if (d.ringok[k] == 2) d.ringok[k] = asv_m6_negative(d.Mring + 8 * k) ? 0 : 1;
 }
 
+// a warp per listed seed and ring neighbour
 __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
 {
-    const int lane = threadIdx.x & 31;
-    int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    int g = task / ASV_RING, t = task - g * ASV_RING;
-    SeedRef r;
-    if (!asv_seed_ref(d, g, r)) return;
-    int *ok = d.ringok + ASV_RING * g + t;
-    if (d.neg[g] != 1) { if (lane == 0) *ok = 0; return; }
-    const SegDesc &S = d.segs[r.si];
-    float4 p = reseed ? d.pos[g] : d.pos0[g];
-    float fx = floorf(p.x), fy = floorf(p.y);
-    int frame = min(max((int)p.z, 0), S.D - 1);
-    float nx = fx + (float)c_ringx[t], ny = fy + (float)c_ringy[t];
-    if (!(nx >= 0 && nx < S.W && ny >= 0 && ny < S.H)) { if (lane == 0) *ok = 0; return; }
-    const float2 *fwd = d.fwd + S.vox_off, *bwd = d.bwd + S.vox_off;
-    if (reseed && S.angle_filter &&
-        !asv_angle_ok(fwd, S.W, S.H, S.D, frame, (int)fx, (int)fy, (int)nx, (int)ny)) {
-        if (lane == 0) *ok = 0;
-        return;
+    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+    const int tasks = *d.negcount * ASV_RING;
+    for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += warps) {
+        const int g = d.neglist[task / ASV_RING], t = task % ASV_RING;
+        SeedRef r;
+        asv_seed_ref(d, g, r);
+        int *ok = d.ringok + ASV_RING * g + t;
+        const SegDesc &S = d.segs[r.si];
+        float4 p = reseed ? d.pos[g] : d.pos0[g];
+        float fx = floorf(p.x), fy = floorf(p.y);
+        int frame = min(max((int)p.z, 0), S.D - 1);
+        float nx = fx + (float)c_ringx[t], ny = fy + (float)c_ringy[t];
+        const float2 *fwd = d.fwd + S.vox_off, *bwd = d.bwd + S.vox_off;
+        if (!(nx >= 0 && nx < S.W && ny >= 0 && ny < S.H) ||
+            (reseed && S.angle_filter &&
+             !asv_angle_ok(fwd, S.W, S.H, S.D, frame, (int)fx, (int)fy, (int)nx, (int)ny))) {
+            if (lane == 0) *ok = 0;
+            continue;
+        }
+        float M[6];
+        asv_metric_solve_warp(fwd, bwd, S.W, S.H, S.D, nx, ny, frame, M);
+        if (lane == 0) {
+            float *dst = d.Mring + 8 * (ASV_RING * g + t);
+#pragma unroll
+            for (int e = 0; e < 6; e++) dst[e] = M[e];
+            *ok = asv_m6_negative_quick(M) ? 0 : 1;
+        }
     }
-    float M[6];
-    asv_metric_solve_warp(fwd, bwd, S.W, S.H, S.D, nx, ny, frame, M);
-    float *dst = d.Mring + 8 * (ASV_RING * g + t);
-    if (lane < 6) dst[lane] = M[lane];
-    if (lane == 0) *ok = 2;                              // PSD test pending (k_metric_psd)
 }
 
-// writes M0 (reseed 0) or M (reseed 1, and the memo)
-__global__ void k_metric_combine(AsvDev d, int reseed)
+// the metric of seed g: its own, the mean of a ring's PSD ones, or the nearest
+// PSD matrix
+__device__ __forceinline__ void asv_metric_result(const AsvDev &d, int g, int neg, float res[6])
 {
-    SeedRef r;
-    if (!asv_seed_ref(d, blockIdx.x * blockDim.x + threadIdx.x, r)) return;
-    const int g = r.g;
-    float *out = (reseed ? d.M : d.M0) + 8 * g;
-    const int neg = d.neg[g];
-    if (neg == 2) {
-        for (int e = 0; e < 6; e++) out[e] = d.Mmemo[8 * g + e];
-        return;
-    }
-    float res[6];
     float self[6];
     for (int e = 0; e < 6; e++) self[e] = d.Mself[8 * g + e];
     bool done = false;
@@ -416,20 +450,66 @@ __global__ void k_metric_combine(AsvDev d, int reseed)
         }
     }
     if (!done) asv_m6_nearest_psd(self, res);
-    for (int e = 0; e < 6; e++) out[e] = res[e];
-    if (reseed) {
-        for (int e = 0; e < 6; e++) d.Mmemo[8 * g + e] = res[e];
-        d.mkey[g] = asv_seed_key(d.segs[r.si], d.pos[g]);
-    }
 }
+
+// Writes M0 (reseed 0) or M (reseed 1, and the memo) and empties the list of
+// non-PSD seeds.  draw: also draws the seed for the next flood (labA is all
+// -1) and empties the list of the first pass's voxels; clear: and zeroes the
+// seed slot's centroid sums.
+__global__ void k_metric_combine(AsvDev d, int reseed, bool draw, bool clear)
+{
+    const int g = blockIdx.x * blockDim.x + threadIdx.x;
+    if (g == 0) {
+        *d.negcount = 0;
+        if (draw) *d.tcount = 0;
+    }
+    if (clear && g < d.total_seeds) {
+        ulonglong2 *q = (ulonglong2 *)(d.sums + 8ull * g);
+#pragma unroll
+        for (int k = 0; k < 4; k++) q[k] = make_ulonglong2(0ull, 0ull);
+    }
+    SeedRef r;
+    if (!asv_seed_ref(d, g, r)) return;
+    const SegDesc &S = d.segs[r.si];
+    const float4 p = reseed ? d.pos[g] : d.pos0[g];
+    const int neg = d.neg[g];
+    float res[6];
+    if (neg == 2) {
+        for (int e = 0; e < 6; e++) res[e] = d.Mmemo[8 * g + e];
+    } else {
+        asv_metric_result(d, g, neg, res);
+        if (reseed) {
+            for (int e = 0; e < 6; e++) d.Mmemo[8 * g + e] = res[e];
+            d.mkey[g] = asv_seed_key(S, p);
+        }
+    }
+    float *out = (reseed ? d.M : d.M0) + 8 * g;
+    for (int e = 0; e < 6; e++) out[e] = res[e];
+    if (draw) asv_draw_seed(d, S, g, r.i, p, d.slab[g], res);
+}
+
+static void metric_solves(const AsvDev &d, int reseed, cudaStream_t st)
+{
+    const long long warps = d.total_seeds, ring = warps * ASV_RING;
+    k_metric_self<<<(int)((warps * 32 + 127) / 128), 128, 0, st>>>(d, reseed);
+    const long long blocks = (ring + 3) / 4;
+    k_metric_ring<<<(int)(blocks < 1216 ? blocks : 1216), 128, 0, st>>>(d, reseed);   // 8 blocks per SM at most
+}
+
 
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st)
 {
-    long long warps = d.total_seeds;
-    k_metric_self<<<(int)((warps * 32 + 127) / 128), 128, 0, st>>>(d, reseed);
-    long long rw = (long long)d.total_seeds * ASV_RING;
-    k_metric_psd<<<(int)((warps + 127) / 128), 128, 0, st>>>(d);     // self tests
-    k_metric_ring<<<(int)((rw * 32 + 127) / 128), 128, 0, st>>>(d, reseed);
-    k_metric_psd<<<(int)((warps + rw + 127) / 128), 128, 0, st>>>(d); // ring tests
-    k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, reseed);
+    metric_solves(d, reseed, st);
+    k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, reseed, false, false);
+}
+
+// The next iteration's seeds: positions from the centroid sums (finalize),
+// metrics, draw.  before_draw(arg) is called when what follows needs labA all
+// -1 (the fills of another stream are awaited there).
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st, void (*before_draw)(void *),
+                           void *arg)
+{
+    metric_solves(d, finalize ? 2 : 1, st);
+    before_draw(arg);
+    k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, 1, true, clear_sums);
 }

@@ -4,7 +4,7 @@
 // the order written, so the labels match the CPU restatement bit for bit.
 // Reference files (in dongxiao0401/anisotropic_supervoxel): GPU-AS/shaders/*,
 // GPU-AS/Image.cpp.
-#include "asv_common.cuh"
+#include "asv_seed.cuh"
 
 #include <cuda_fp16.h>
 
@@ -411,19 +411,7 @@ __global__ void k_draw(AsvDev d)
     int si = asv_seed_seg(d, g, i);
     const SegDesc &S = d.segs[si];
     if (i >= S.Kp) return;
-    float4 p = d.pos[g], c = d.slab[g];
-    const float *m = d.M + 8 * g;
-    // table: (-x, -y, -z, -L) (M00, M11, 2M01, 2M12) (2M02, M22, -a, -b),
-    // laid out for asv_jfa_dist's paired operations.  v - s == v + (-s) in
-    // IEEE arithmetic, and doubling is exact, so
-    // (dx*dy)*(2*M01) == ((2*dx)*dy)*M01 (flood.gs:85).
-    d.jtab[3 * g + 0] = make_float4(-p.x, -p.y, -p.z, -c.x);
-    d.jtab[3 * g + 1] = make_float4(m[0], m[3], 2.0f * m[2], 2.0f * m[4]);
-    d.jtab[3 * g + 2] = make_float4(2.0f * m[1], m[5], -c.y, -c.z);
-    if (!(p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f)) return;
-    int x = (int)p.x, y = (int)p.y, z = (int)p.z;
-    if (x >= S.W || y >= S.H || z >= S.D) return;
-    atomicMax(d.labA + S.vox_off + ((long long)z * S.H + y) * S.W + x, i);
+    asv_draw_seed(d, S, g, i, d.pos[g], d.slab[g], d.M + 8 * g);
 }
 
 // ---------------------------------------------------------------------------
@@ -1340,88 +1328,81 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
 }
 
 // ---------------------------------------------------------------------------
-// The first pass of a Lloyd iteration as a scatter from the seeds.  Its input
-// is the drawn seed volume: -1 everywhere but at the seed voxels, each
-// holding the seed that won its voxel.  At step 1 a voxel's candidates are
-// the seeds within its 3x3x3 neighbourhood (clamped to the edges), so instead
-// of every voxel gathering 27 mostly empty labels, each drawn seed visits the
-// up to 27 voxels around it.  The winner rule of the gather (least distance,
-// the first of equal ones in the shader's candidate order) becomes a 64-bit
-// minimum per voxel over keys (distance bits, candidate rank, label):
-// distances are >= +0, so their bits order like their values, and the rank is
-// the seed's first position in the voxel's candidate order (slices z, z-1,
-// z+1; rows y-1..y+1; columns x-1..x+1), which with edge clamping can be an
-// earlier offset than the plain one.  A distance that is not below 1e8 (or
-// NaN) never wins (flood.gs:63, :95-99).  The output volume is filled with
-// -1 first; k_jfa_first_take then hands each touched voxel's key to exactly
-// one thread (atomicExch leaves the key empty for the next iteration), which
-// writes the label.
+// The first pass of a Lloyd iteration from the seeds.  Its input is the drawn
+// seed volume: -1 everywhere but at the seed voxels, each holding the seed that
+// won its voxel.  At step 1 only the up to 27 voxels around a drawn seed see
+// any label, so a thread takes one drawn seed and one of them and gathers that
+// voxel's 27 candidates by the shader's own rule (order and clamping of k_jfa's
+// list form, strict '<' from 1e8, flood.gs:63, :95-99); nearly all are -1, and
+// a candidate is evaluated once per run of equal ids.  Where two seeds reach
+// one voxel each of their threads finds the same winner, and the winner's
+// thread writes it and lists the voxel for the second pass.  (Two kernels
+// before, a 64-bit atomicMin of keys and a take: 5.1 + 5.2 us a pass on the
+// 320x240x85 clip.)  The output volume is filled with -1 first.  stale: the seed
+// table was replaced after the draw, and only records that stand at their
+// seed's position count.
 // ---------------------------------------------------------------------------
 #define ASV_KEY_EMPTY 0xffffffffffffffffull
 
-// first rank, in the order `order` of offsets, of an offset o with
-// clamp(v + o) == s along one axis of length n
-__device__ __forceinline__ int asv_first_rank(int v, int s, int n, const int order[3])
+__global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = t / 27, o = t - g * 27;
+    bool won = false;
+    int si = 0;
+    long long vl = 0;
+    if (g < d.total_seeds) {
+        int i;
+        si = asv_seed_seg(d, g, i);
+        const SegDesc &S = d.segs[si];
+        const float4 p = d.pos[g];
+        const int W = S.W, H = S.H, D = S.D;
+        const int32_t *in = d.labA + S.vox_off;
+        int sx = -1, sy = -1, sz = -1;
+        if (i < S.Kp && p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f) { sx = (int)p.x; sy = (int)p.y; sz = (int)p.z; }   // as the draw
+        const bool inside = sx >= 0 && sx < W && sy < H && sz < D;
+        const int x = sx + (o % 3 - 1), y = sy + ((o / 3) % 3 - 1), z = sz + (o / 9 - 1);
+        if (inside && x >= 0 && x < W && y >= 0 && y < H && z >= 0 && z < D &&
+            in[((long long)sz * H + sy) * W + sx] == i) {                          // the seed won its voxel
+            vl = ((long long)z * H + y) * W + x;
+            const uchar4 c = __ldg(d.lab + S.vox_off + vl);
+            const float2 vxy = make_float2((float)x + 0.5f, (float)y + 0.5f);
+            const float2 vzl = make_float2((float)z + 0.5f, (float)c.x), vab = make_float2((float)c.y, (float)c.z);
+            const int zs[3] = { z, max(z - 1, 0), min(z + 1, D - 1) };
+            const int ys[3] = { max(y - 1, 0), y, min(y + 1, H - 1) };
+            const int xs[3] = { max(x - 1, 0), x, min(x + 1, W - 1) };
+            int32_t l[27];
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-        const int q = min(max(v + order[r], 0), n - 1);
-        if (q == s) return r;
+            for (int k = 0; k < 27; k++)
+                l[k] = in[((long long)zs[k / 9] * H + ys[(k / 3) % 3]) * W + xs[k % 3]];
+            if (stale) {
+#pragma unroll
+                for (int k = 0; k < 27; k++) {
+                    if (l[k] < 0 || l[k] >= S.Kp) { l[k] = -1; continue; }
+                    const float4 q = d.pos[S.seed_off + l[k]];
+                    if ((int)q.x != xs[k % 3] || (int)q.y != ys[(k / 3) % 3] || (int)q.z != zs[k / 9]) l[k] = -1;
+                }
+            }
+            float mind = 100000000.0f;
+            int best = -1, prev = -1;
+#pragma unroll
+            for (int k = 0; k < 27; k++)
+                if (l[k] >= 0 && l[k] != prev) {
+                    prev = l[k];
+                    const float dist = asv_jfa_dist(d.jtab + 3 * S.seed_off, l[k], vxy, vzl, vab, S.ratio[0]);
+                    if (dist < mind) { mind = dist; best = l[k]; }
+                }
+            won = best == i;
+            if (won) d.labB[S.vox_off + vl] = i;
+        }
     }
-    return 3;    // not reached: s lies within one step of v
-}
-
-// thread -> (drawn seed, offset); false when the seed lost its voxel or the
-// voxel lies outside the segment
-__device__ __forceinline__ bool asv_first_target(const AsvDev &d, long long t, int &si, int &i, int &x, int &y,
-                                                 int &z, int &sx, int &sy, int &sz)
-{
-    const int g = (int)(t / 27), o = (int)(t - (long long)g * 27);
-    if (g >= d.total_seeds) return false;
-    si = asv_seed_seg(d, g, i);
-    const SegDesc &S = d.segs[si];
-    if (i >= S.Kp) return false;
-    const float4 p = d.pos[g];
-    if (!(p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f)) return false;     // as k_draw
-    sx = (int)p.x; sy = (int)p.y; sz = (int)p.z;
-    if (sx >= S.W || sy >= S.H || sz >= S.D) return false;
-    if (d.labA[S.vox_off + ((long long)sz * S.H + sy) * S.W + sx] != i) return false;   // lost the draw
-    x = sx + (o % 3 - 1); y = sy + ((o / 3) % 3 - 1); z = sz + (o / 9 - 1);
-    return x >= 0 && x < S.W && y >= 0 && y < S.H && z >= 0 && z < S.D;
-}
-
-__global__ void __launch_bounds__(256) k_jfa_first_scatter(AsvDev d)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int si, i, x, y, z, sx, sy, sz;
-    if (!asv_first_target(d, t, si, i, x, y, z, sx, sy, sz)) return;
-    const SegDesc &S = d.segs[si];
-    const int xy_order[3] = { -1, 0, 1 }, z_order[3] = { 0, -1, 1 };
-    const int rank = asv_first_rank(z, sz, S.D, z_order) * 9 + asv_first_rank(y, sy, S.H, xy_order) * 3 +
-                     asv_first_rank(x, sx, S.W, xy_order);
-    const long long v = ((long long)z * S.H + y) * S.W + x;
-    const uchar4 c = __ldg(d.lab + S.vox_off + v);
-    const float dist = asv_jfa_dist(d.jtab + 3 * S.seed_off, i, make_float2((float)x + 0.5f, (float)y + 0.5f),
-                                    make_float2((float)z + 0.5f, (float)c.x), make_float2((float)c.y, (float)c.z),
-                                    S.ratio[0]);
-    if (!(dist < 100000000.0f)) return;
-    const unsigned long long key = ((unsigned long long)__float_as_uint(dist) << 32) |
-                                   ((unsigned long long)rank << 16) | (unsigned long long)i;
-    atomicMin(d.jkeys + S.vox_off + v, key);
-}
-
-__global__ void __launch_bounds__(256) k_jfa_first_take(AsvDev d)
-{
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    int si, i, x, y, z, sx, sy, sz;
-    if (!asv_first_target(d, t, si, i, x, y, z, sx, sy, sz)) return;
-    const SegDesc &S = d.segs[si];
-    const long long vl = ((long long)z * S.H + y) * S.W + x, v = S.vox_off + vl;
-    const unsigned long long key = atomicExch(d.jkeys + v, ASV_KEY_EMPTY);
-    if (key != ASV_KEY_EMPTY) {
-        d.labB[v] = (int32_t)(key & 0x7fffu);
-        d.tlist[atomicAdd(d.tcount, 1)] = ((unsigned long long)si << 32) | (unsigned long long)vl;
-    }
+    const unsigned m = __ballot_sync(FULL, won);                                   // one addition per warp
+    if (!m) return;
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    if (lane == __ffs(m) - 1) at = atomicAdd(d.tcount, __popc(m));
+    at = __shfl_sync(FULL, at, __ffs(m) - 1);
+    if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = ((unsigned long long)si << 32) | (unsigned long long)vl;
 }
 
 // ---------------------------------------------------------------------------
@@ -1453,48 +1434,91 @@ __device__ __forceinline__ int asv_first_rank_step(int v, int u, int s, int n, c
     return 3;    // not reached: v is one of u's sources
 }
 
+// one voxel of an entry's box: its key into jkeys, or (TAKE) the least key's
+// label out of them
 template <bool TAKE>
-__global__ void __launch_bounds__(256) k_jfa_second(AsvDev d)
+__device__ __forceinline__ void asv_second_voxel(const AsvDev &d, const SegDesc &S, int label, int ux, int uy, int uz,
+                                                 int x, int y, int z, int s)
+{
+    const long long v = S.vox_off + ((long long)z * S.H + y) * S.W + x;
+    if (TAKE) {
+        const unsigned long long key = atomicExch(d.jkeys + v, ASV_KEY_EMPTY);
+        if (key != ASV_KEY_EMPTY) d.labA[v] = (int32_t)(key & 0x7fffu);
+        return;
+    }
+    const int xy_order[3] = { -1, 0, 1 }, z_order[3] = { 0, -1, 1 };
+    const int rank = asv_first_rank_step(z, uz, s, S.D, z_order) * 9 + asv_first_rank_step(y, uy, s, S.H, xy_order) * 3 +
+                     asv_first_rank_step(x, ux, s, S.W, xy_order);
+    const uchar4 c = __ldg(d.lab + v);
+    const float dist = asv_jfa_dist(d.jtab + 3 * S.seed_off, label, make_float2((float)x + 0.5f, (float)y + 0.5f),
+                                    make_float2((float)z + 0.5f, (float)c.x), make_float2((float)c.y, (float)c.z),
+                                    S.ratio[1]);
+    if (!(dist < 100000000.0f)) return;
+    const unsigned long long key = ((unsigned long long)__float_as_uint(dist) << 32) |
+                                   ((unsigned long long)rank << 16) | (unsigned long long)label;
+    atomicMin(d.jkeys + v, key);
+}
+
+// A thread per listed voxel and offset.  Inside the volume the box is one
+// voxel; next to an edge it has s + 1 to (s + 1)^3 (1728 at step 11), and one
+// thread alone made the kernel as long as its largest box (26 to 36 us): boxes
+// of more than one voxel are walked by the whole warp, one after another.
+// undraw: the threads of the scatter also take the drawn seeds out of labA
+// again, so that it is all -1 for the take without a fill (nothing else of
+// this kernel reads labA).
+template <bool TAKE>
+__global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
 {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (!TAKE && undraw && t < d.total_seeds) {
+        int i;
+        const SegDesc &S = d.segs[asv_seed_seg(d, (int)t, i)];
+        const float4 p = d.pos[t];
+        if (i < S.Kp && p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f && (int)p.x < S.W && (int)p.y < S.H && (int)p.z < S.D)
+            d.labA[S.vox_off + ((long long)(int)p.z * S.H + (int)p.y) * S.W + (int)p.x] = -1;
+    }
     const long long e = t / 27;
-    if (e >= *d.tcount) return;
-    const int o = (int)(t - e * 27);
-    const unsigned long long ent = d.tlist[e];
-    const int si = (int)(ent >> 32);
-    const long long ul = (long long)(ent & 0xffffffffull);
-    const SegDesc &S = d.segs[si];
-    const int s = S.steps[1];
-    const int ux = (int)(ul % S.W), uy = (int)((ul / S.W) % S.H), uz = (int)(ul / ((long long)S.W * S.H));
-    int x0, x1, y0, y1, z0, z1;
-    asv_axis_sources(ux, o % 3 - 1, s, S.W, x0, x1);
-    asv_axis_sources(uy, (o / 3) % 3 - 1, s, S.H, y0, y1);
-    asv_axis_sources(uz, o / 9 - 1, s, S.D, z0, z1);
-    if (x0 > x1 || y0 > y1 || z0 > z1) return;
-    const int label = d.labB[S.vox_off + ul];
-    const int xy_order[3] = { -1, 0, 1 }, z_order[3] = { 0, -1, 1 };
-    for (int z = z0; z <= z1; z++)
-        for (int y = y0; y <= y1; y++)
-            for (int x = x0; x <= x1; x++) {
-                const long long v = S.vox_off + ((long long)z * S.H + y) * S.W + x;
-                if (TAKE) {
-                    const unsigned long long key = atomicExch(d.jkeys + v, ASV_KEY_EMPTY);
-                    if (key != ASV_KEY_EMPTY) d.labA[v] = (int32_t)(key & 0x7fffu);
-                    continue;
-                }
-                const int rank = asv_first_rank_step(z, uz, s, S.D, z_order) * 9 +
-                                 asv_first_rank_step(y, uy, s, S.H, xy_order) * 3 +
-                                 asv_first_rank_step(x, ux, s, S.W, xy_order);
-                const uchar4 c = __ldg(d.lab + v);
-                const float dist = asv_jfa_dist(d.jtab + 3 * S.seed_off, label,
-                                                make_float2((float)x + 0.5f, (float)y + 0.5f),
-                                                make_float2((float)z + 0.5f, (float)c.x),
-                                                make_float2((float)c.y, (float)c.z), S.ratio[1]);
-                if (!(dist < 100000000.0f)) continue;
-                const unsigned long long key = ((unsigned long long)__float_as_uint(dist) << 32) |
-                                               ((unsigned long long)rank << 16) | (unsigned long long)label;
-                atomicMin(d.jkeys + v, key);
+    const int count = *d.tcount;
+    int si = 0, ux = 0, uy = 0, uz = 0, label = 0;
+    int x0 = 0, y0 = 0, z0 = 0, nx = 0, ny = 0, nz = 0;
+    if (e < count) {
+        const int o = (int)(t - e * 27);
+        const unsigned long long ent = d.tlist[e];
+        si = (int)(ent >> 32);
+        const int ul = (int)(ent & 0xffffffffull);                 // segments hold < 2^31 voxels
+        const SegDesc &S = d.segs[si];
+        const int s = S.steps[1];
+        const int row = ul / S.W;
+        ux = ul - row * S.W; uz = row / S.H; uy = row - uz * S.H;
+        int x1, y1, z1;
+        asv_axis_sources(ux, o % 3 - 1, s, S.W, x0, x1);
+        asv_axis_sources(uy, (o / 3) % 3 - 1, s, S.H, y0, y1);
+        asv_axis_sources(uz, o / 9 - 1, s, S.D, z0, z1);
+        nx = x1 - x0 + 1; ny = y1 - y0 + 1; nz = z1 - z0 + 1;
+        if (nx <= 0 || ny <= 0 || nz <= 0) nx = 0;
+        else {
+            label = TAKE ? 0 : d.labB[S.vox_off + ul];
+            if (nx * ny * nz == 1) {
+                asv_second_voxel<TAKE>(d, S, label, ux, uy, uz, x0, y0, z0, s);
+                nx = 0;
             }
+        }
+    }
+    unsigned big = __ballot_sync(FULL, nx > 0);
+    const int lane = threadIdx.x & 31;
+    while (big) {
+        const int from = __ffs(big) - 1;
+        big &= big - 1;
+        const int bsi = __shfl_sync(FULL, si, from), bl = __shfl_sync(FULL, label, from);
+        const int bux = __shfl_sync(FULL, ux, from), buy = __shfl_sync(FULL, uy, from), buz = __shfl_sync(FULL, uz, from);
+        const int bx = __shfl_sync(FULL, x0, from), by = __shfl_sync(FULL, y0, from), bz = __shfl_sync(FULL, z0, from);
+        const int bnx = __shfl_sync(FULL, nx, from), bny = __shfl_sync(FULL, ny, from), bnz = __shfl_sync(FULL, nz, from);
+        const SegDesc &S = d.segs[bsi];
+        for (int k = lane; k < bnx * bny * bnz; k += 32) {
+            const int r = k / bnx;
+            asv_second_voxel<TAKE>(d, S, bl, bux, buy, buz, bx + k - r * bnx, by + r % bny, bz + r / bny, S.steps[1]);
+        }
+    }
 }
 
 // a caller's labels outside [0, Kp) become -1, as the passes' own labels are
@@ -1565,25 +1589,6 @@ __global__ void __launch_bounds__(256) k_centroids(AsvDev d)
     }
 }
 
-// ---------------------------------------------------------------------------
-// Reseed (aver_exception.vs:22-81).  Alive seed: position floor(mean)+0.5,
-// colour = mean LAB.  Dead seed: midpoint of the means of slots id-1 and
-// id+1 (id 0 reads texel (W-1, 0); slot Kp is the -1 slot), colour sampled
-// at the new position.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void asv_slot_mean(const unsigned long long *sums, int Kp, int slot,
-                                              float q[3])
-{
-    if (slot < 0 || slot > Kp) { q[0] = q[1] = q[2] = 0.0f; return; }
-    const unsigned long long *s = sums + 8ull * slot;
-    float cnt = __ull2float_rn(s[3]);
-#pragma unroll
-    for (int a = 0; a < 3; a++) {
-        float sf = __ull2float_rn(s[a]) * 0.5f;
-        q[a] = ((int)cnt != 0) ? sf / cnt : sf;
-    }
-}
-
 __global__ void k_finalize(AsvDev d)
 {
     int g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1592,29 +1597,8 @@ __global__ void k_finalize(AsvDev d)
     int si = asv_seed_seg(d, g, id);
     const SegDesc &S = d.segs[si];
     if (id >= S.Kp) return;
-    const unsigned long long *sums = d.sums + 8ull * S.seed_off;
-    const unsigned long long *s = sums + 8ull * id;
     float p[3], c[3];
-    if (s[3] != 0) {
-        float cnt = __ull2float_rn(s[3]);
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            float sf = __ull2float_rn(s[a]) * 0.5f;
-            p[a] = floorf(sf / cnt) + 0.5f;
-            c[a] = __ull2float_rn(s[4 + a]) / cnt;
-        }
-    } else {
-        float q1[3], q2[3];
-        asv_slot_mean(sums, S.Kp, id == 0 ? S.W - 1 : id - 1, q1);
-        asv_slot_mean(sums, S.Kp, id + 1, q2);
-#pragma unroll
-        for (int a = 0; a < 3; a++) p[a] = floorf(0.5f * (q1[a] + q2[a])) + 0.5f;
-        int x = min(max((int)floorf(p[0]), 0), S.W - 1);
-        int y = min(max((int)floorf(p[1]), 0), S.H - 1);
-        int z = min(max((int)floorf(p[2]), 0), S.D - 1);
-        uchar4 l = d.lab[S.vox_off + ((long long)z * S.H + y) * S.W + x];
-        c[0] = l.x; c[1] = l.y; c[2] = l.z;
-    }
+    asv_reseed(d, S, id, p, c);
     d.pos[g] = make_float4(p[0], p[1], p[2], (float)id);
     d.slab[g] = make_float4(c[0], c[1], c[2], 0.0f);
 }
@@ -1979,23 +1963,24 @@ void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_bloc
                                   st>>>(d, pass, in, out);
 }
 
-void asv_launch_jfa_first_scatter(const AsvDev &d, cudaStream_t st)
+// filled: the output volume is all -1 and the list empty already
+void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t st)
 {
-    cudaMemsetAsync(d.labB, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
-    cudaMemsetAsync(d.tcount, 0, sizeof(int), st);
-    const long long threads = 27LL * d.total_seeds;
-    const int blocks = (int)((threads + 255) / 256);
-    k_jfa_first_scatter<<<blocks, 256, 0, st>>>(d);
-    k_jfa_first_take<<<blocks, 256, 0, st>>>(d);
+    if (!filled) {
+        cudaMemsetAsync(d.labB, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
+        cudaMemsetAsync(d.tcount, 0, sizeof(int), st);
+    }
+    k_jfa_first<<<(27 * d.total_seeds + 255) / 256, 256, 0, st>>>(d, stale);
 }
 
-void asv_launch_jfa_second_scatter(const AsvDev &d, cudaStream_t st)
+// undraw: labA holds nothing but the seeds at their current positions
+void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st)
 {
-    cudaMemsetAsync(d.labA, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
+    if (!undraw) cudaMemsetAsync(d.labA, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
     const long long threads = 27LL * 27LL * d.total_seeds;   // tlist holds <= 27 entries per seed
     const int blocks = (int)((threads + 255) / 256);
-    k_jfa_second<false><<<blocks, 256, 0, st>>>(d);
-    k_jfa_second<true><<<blocks, 256, 0, st>>>(d);
+    k_jfa_second<false><<<blocks, 256, 0, st>>>(d, undraw);
+    k_jfa_second<true><<<blocks, 256, 0, st>>>(d, false);
 }
 
 void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
