@@ -345,6 +345,7 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
     size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 4 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 8;
     // each of the ~30 allocations rounds up to 256 bytes
     size_t fixed = 32 * 256 + 256 * 4 + 16;
+    fixed += sizeof(SegDesc);
     size_t per_seg = sizeof(SegDesc) + 3 * 4 + ASV_POST_WORDS * 4;
     return vox * per_vox + seeds * per_seed + cells * 4 + chunks * 4 + fixed + seg.size() * per_seg;
 }
@@ -379,21 +380,51 @@ static int label_depth(int D, double spacing, int step)
 
 static double seed_spacing(long long nvox, int Kp) { return std::cbrt((double)nvox / std::max(Kp, 1)); }
 
-// SegDesc::depth of every pass.  The first gathering pass (the third) sees
-// labels around the seeds only and takes the deepest sub-tiles.  A tile is
-// cut evenly: 30 positions are 15 + 15, not 16 + 14.
+// Footprint slots of all sub-tiles of `depth` positions of a column's D
+// positions cut in tiles of zrun, and 3 for each sub-tile (as in pick_zrun);
+// -1 when a sub-tile has more slots than fit.  A sub-tile has its positions
+// and the two slices next to them, and where a chain ends inside it slices 0
+// and D - 1, unless those are the two.
+static int depth_cost(int D, int zrun, int step, int depth, int most)
+{
+    auto slice = [&](int p) {                              // asv_chain_pos
+        if (step >= D) return p;
+        const int q = D / step, m = D - q * step, big = m * (q + 1);
+        return p < big ? p / (q + 1) + p % (q + 1) * step : m + (p - big) / q + (p - big) % q * step;
+    };
+    int cost = 0;
+    for (int t0 = 0; t0 < D; t0 += zrun)
+        for (int p0 = t0, e = std::min(t0 + zrun, D); p0 < e; p0 += depth) {
+            const int n = std::min(depth, e - p0);
+            bool ends = false;
+            for (int p = p0; p < p0 + n - 1; p++) ends = ends || slice(p) + step >= D;
+            int slots = n + 2;
+            if (ends) slots += (slice(p0) > step) + (slice(p0 + n - 1) + step < D - 1);
+            if (slots > most) return -1;
+            cost += slots + 3;
+        }
+    return cost;
+}
+
+// SegDesc::depth of every pass: of the depths that the labels allow the one
+// of least cost, so that 30 positions are 15 + 15, not 16 + 14, or at step 6
+// three sub-tiles of two whole chains (12 slots each), not four of 8 or 7.  The
+// first gathering pass (the third) sees labels around the seeds only and takes
+// any depth.
 static void set_depths(SegDesc &s)
 {
     const double spacing = seed_spacing(s.nvox, s.Kp);
     for (int p = 0; p < s.npass; p++) {
-        const int step = s.steps[p];
-        const int cap = std::min(asv_jfa_max_depth(step), p == s.npass - 1 ? 15 : 16);   // 15: asv_run_words
-        int d = cap ? std::min(cap, p == 2 ? 16 : label_depth(s.D, spacing, step)) : 0;
-        if (d) {
-            const int z = std::min(s.zrun, s.D), parts = (z + d - 1) / d;
-            d = std::max((z + parts - 1) / parts, 4);
+        const int step = s.steps[p], most = asv_jfa_slots(step);
+        s.depth[p] = 0;
+        if (!most) continue;
+        const int by_labels = p == 2 ? 16 : label_depth(s.D, spacing, step);
+        const int cap = std::min(std::min(by_labels, most - 2), p == s.npass - 1 ? 15 : 16);   // 15: asv_run_words
+        int least = 0;
+        for (int d = cap; d >= 4; d--) {
+            const int c = depth_cost(s.D, s.zrun, step, d, most);
+            if (c >= 0 && (!s.depth[p] || c < least)) { s.depth[p] = d; least = c; }
         }
-        s.depth[p] = d;
     }
 }
 
@@ -486,7 +517,8 @@ asv_status asv_build_layout(asv_ctx *ctx)
     d.nseg = nseg;
     d.total_tiles = tiles; d.total_chunks = chunks; d.total_seeds = seeds;
     SegDesc *segs; int *tp, *cp, *sp;
-    AL(segs, nseg); AL(tp, nseg + 1); AL(cp, nseg + 1); AL(sp, nseg + 1);
+    AL(segs, nseg + 1);                              // (one more: asv_jfa_pass_host's)
+    AL(tp, nseg + 1); AL(cp, nseg + 1); AL(sp, nseg + 1);
     d.segs = segs; d.tile_prefix = tp; d.chunk_prefix = cp; d.seed_prefix = sp;
     AL(d.rgb, (size_t)vox * 3);
     AL(d.lab, (size_t)vox);
@@ -570,20 +602,29 @@ static void do_first_init(asv_ctx *ctx)
     ctx->launches += 2;
 }
 
-// the step of pass p, and whether it forms the centroid sums, where both are
-// the same for every segment that runs the pass (k_jfa's variant for them
-// takes it), else 0
-static int pass_step(const asv_ctx *ctx, int p, int *sums)
+// Pass p of every segment that has it: a launch of k_jfa's variant for each
+// different step (and for the segments whose last pass it is); the first on the
+// context's stream, the others beside it on the side stream, where their blocks
+// fill the SMs that the first leaves at its end.
+static void do_pass(asv_ctx *ctx, int p)
 {
-    int step = 0;
+    int kinds[2 * (ASV_BITS_MAXS + 2)], n = 0;                // step (capped at the list form's), last pass
     for (const SegDesc &s : ctx->sd) {
         if (p >= s.npass) continue;
-        const int last = p == s.npass - 1;
-        if (step && (s.steps[p] != step || last != *sums)) return 0;
-        step = s.steps[p];
-        *sums = last;
+        const int k = 2 * std::min(s.steps[p], ASV_BITS_MAXS + 1) + (p == s.npass - 1);
+        if (std::find(kinds, kinds + n, k) == kinds + n) kinds[n++] = k;
     }
-    return step;
+    if (n > 1) {
+        cudaEventRecord(ctx->side_ev[0], ctx->st);
+        cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0);
+    }
+    for (int i = 0; i < n; i++)
+        asv_launch_jfa(ctx->d, p, kinds[i] / 2, kinds[i] & 1, ctx->jfa_blocks, i ? ctx->side : ctx->st);
+    if (n > 1) {
+        cudaEventRecord(ctx->side_ev[1], ctx->side);
+        cudaStreamWaitEvent(ctx->st, ctx->side_ev[1], 0);
+    }
+    ctx->launches += n;
 }
 
 // the JFA ladder; the last pass of each segment also forms its centroid sums
@@ -602,10 +643,7 @@ static void do_flood(asv_ctx *ctx, int evbase, bool prepared)
             asv_launch_jfa_second_scatter(ctx->d, ctx->undraw, ctx->st);   // from the first pass's sparse labels
             ctx->launches += 2;
         } else {
-            int sums = 0;
-            const int step = pass_step(ctx, p, &sums);
-            asv_launch_jfa(ctx->d, p, step, sums, ctx->jfa_blocks, ctx->st);
-            ctx->launches++;
+            do_pass(ctx, p);
         }
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p + 1);
     }
@@ -1423,7 +1461,17 @@ asv_status asv_jfa_pass_host(asv_ctx *ctx, int step, float ratio, const int32_t 
     ctx->undraw = false;
     int32_t *din = ctx->d.labA + s.vox_off, *dout = ctx->d.labB + s.vox_off;
     CK(cudaMemcpyAsync(din, in, 4 * n, cudaMemcpyHostToDevice, ctx->st));
-    asv_launch_jfa_single(ctx->d, din, s.nvox, s.Kp, dout, step, ratio, ctx->st);
+    // a descriptor of the one pass (not a last one), behind the segments'
+    SegDesc one = s;
+    one.npass = 2;
+    one.steps[0] = step;
+    one.ratio[0] = ratio;
+    one.depth[0] = std::min(16, std::max(asv_jfa_slots(step) - 2, 0));
+    AsvDev d = ctx->d;
+    d.segs = ctx->d.segs + 1;
+    CK(cudaMemcpyAsync((void *)d.segs, &one, sizeof(one), cudaMemcpyHostToDevice, ctx->st));
+    asv_launch_label_clean(din, s.nvox, s.Kp, ctx->st);
+    asv_launch_jfa(d, 0, step, false, ctx->jfa_blocks, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout, 4 * n, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));

@@ -15,7 +15,7 @@
 #define ASV_CHUNK 2048       // voxels per block in the per-voxel kernels
 #define ASV_TILE_X 16        // JFA tile: 16 x 16 columns x SegDesc::zrun chain positions
 #define ASV_TILE_Y 16        // (a warp covers 16 x 2 columns: fewer distinct candidates)
-#define ASV_BITS_MAXS 6      // largest step of a JFA pass's bit-set form
+#define ASV_BITS_MAXS 6      // largest step of a JFA pass's bit-set form (larger ones: list form)
 #define ASV_RING 24          // 8 one-ring + 16 two-ring neighbours of the metric fallback
 #define ASV_POST_WORDS 16    // per-segment post-processing record
 
@@ -120,11 +120,10 @@ void asv_launch_density(const AsvDev &d, cudaStream_t st);
 void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st);
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st);
 void asv_launch_draw(const AsvDev &d, cudaStream_t st);
-void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_blocks, cudaStream_t st);
+void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, cudaStream_t st);
 void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t st);
 void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st);
-void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
-                           cudaStream_t st);
+void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st);
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);
 void asv_launch_post(const AsvDev &d, cudaStream_t st);
@@ -133,4 +132,4 @@ void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cuda
                            void *arg);
 int asv_jfa_grid_blocks(int total_tiles);
 int asv_jfa_resident_blocks();
-int asv_jfa_max_depth(int step);   // chain positions a sub-tile of the step can hold
+int asv_jfa_slots(int step);   // footprint slots a sub-tile of the step can hold, 0: no bit-set form

@@ -691,13 +691,21 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // values read straight from global memory (one position ahead) four blocks
 // fit an SM, three before.  Passes of a 1280x720x30 window (steps 6, 3, 2, 1,
 // 2, 1 + sums) 499, 479, 439, 409, 443, 509 -> 316, 342, 315, 298, 326,
-// 425 us; issue slots 63 -> 67 % used.
+// 425 us.
+//
+// Then the shared-memory data path bound the passes (103 of its cycles for 32
+// voxels of the step-3 pass, 85 % busy): a candidate's fourteen coefficients
+// are fourteen words per lane whatever the load's width, and rows of 24 words
+// let the two rows of a warp collide in eight banks.  Two positions share a
+// candidate's load, a warp walks rows r and r + 2, and runs flush into four
+// copies of the sums: 89 -> 59 million cycles at step 3, passes 289, 291, 273, 262, 282, 325 us.
 //
 // Footprint slices ("slots") of a sub-tile of n chain positions: slot 0 the
 // minus slice of position 0, slots 1..n the centre slices, slot n+1 the plus
-// slice of position n-1, and where a chain ends inside the sub-tile slot
-// n+2 (slice 0, the minus slice of every chain start after the first) and
-// slot n+3 (slice D-1, the clamped plus slice of every chain end).  Along a
+// slice of position n-1, and where a chain ends inside the sub-tile one for
+// slice 0 (the minus slice of every chain start after the first) and one for
+// slice D-1 (the clamped plus slice of every chain end), unless slot 0 or n+1
+// is that slice already, as for a sub-tile of whole chains.  Along a
 // chain the minus slice of a position is the centre of the one before it
 // and its plus slice the centre of the one after it.
 // ---------------------------------------------------------------------------
@@ -710,15 +718,13 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 #define ASV_BITS_OVER 253        // map8: a label past the 32nd (the sub-tile takes the list form)
 #define ASV_ACC_ROW 5            // words per entry of the sub-tile's centroid-sum table (odd: the
                                  // entries' rows start in different shared-memory banks)
-#define ASV_BITS_AREA 43264      // shared bytes of the largest sub-tiles (step 5, 9 positions): four blocks per SM
-#define ASV_JFA_AREA (ASV_BITS_AREA > ASV_JFA_LIST_BYTES ? ASV_BITS_AREA : ASV_JFA_LIST_BYTES)
+#define ASV_BITS_AREA 43264      // shared bytes of the footprint: four blocks per SM
 
 #define ASV_ECO_ROW 5            // float4 per label of the score table (3.5 used; the odd count
                                  // spreads the rows of eight labels over all banks)
 
 struct AsvBitsShared {
     float4 eco[ASV_ECO_ROW * ASV_BITS_MAXT];    // score coefficients per table entry (asv_bits_coefs)
-    unsigned acc[(ASV_BITS_MAXT + 1) * ASV_ACC_ROW];   // centroid sums of the sub-tile per table entry (+ label -1)
     unsigned claim[ASV_BITS_MAXKP / 32];        // labels numbered in this sub-tile (all zero between)
     int4 slot[20];                              // per footprint slot: offset of its slice, slice relative to the
                                                 // sub-tile's middle one (float bits), 2 z + 1 (positions' slots)
@@ -728,7 +734,14 @@ struct AsvBitsShared {
     int tcount;
     unsigned char map8[ASV_BITS_MAXKP + 4];     // number of each claimed label, ASV_BITS_FREE between
 };
-#define ASV_JFA_SMEM (ASV_JFA_AREA + (int)sizeof(AsvBitsShared))
+
+// The summing variant's centroid sums of the sub-tile, behind AsvBitsShared: per
+// table entry (+ label -1) four copies of a row, taken by lanes in turn, so that
+// the flushes of neighbouring columns, which mostly end runs of one label
+// together, do not queue at one address.
+#define ASV_ACC_COPIES 4
+#define ASV_ACC_WORDS ((ASV_BITS_MAXT + 1) * ASV_ACC_COPIES * ASV_ACC_ROW)
+
 
 // The footprint of a slot is kept as rows of 16-byte groups of four entries
 // (quads): its left edge is rounded down to four columns, so that for widths
@@ -740,12 +753,14 @@ template <int S> struct AsvBitsGeo {
     static constexpr int FH = ASV_TILE_Y + 2 * S;
     static constexpr int FP = FW * FH;                                // footprint entries per slot
     static constexpr int QW = FW / 4, QPS = FP / 4;                   // quads per row and per slot
-    // chain positions per sub-tile: as many as the shared area holds, up to 16
-    static constexpr int SUB = S <= 3 ? 16 : (S == 4 ? 14 : (S == 5 ? 9 : 8));
-    static constexpr int NSLOT = SUB + 4;
-    static constexpr int FLAB_BYTES = NSLOT * FP * 4;
-    static_assert(FLAB_BYTES <= ASV_BITS_AREA, "bit-set sub-tile exceeds the shared area");
-    static_assert(NSLOT <= 20, "slotz");
+    // slots the shared area holds, and chain positions per sub-tile, up to 16:
+    // a sub-tile of n positions has n + 2 slots, or up to n + 4 where chains
+    // end inside it
+    static constexpr int NSLOT = ASV_BITS_AREA / (4 * FP) < 20 ? ASV_BITS_AREA / (4 * FP) : 20;
+    static constexpr int SUB = NSLOT - 2 < 16 ? NSLOT - 2 : 16;
+    // shared memory: the footprint (or the list rows), AsvBitsShared, sums
+    static constexpr int AREA = NSLOT * FP * 4 > ASV_JFA_LIST_BYTES ? NSLOT * FP * 4 : ASV_JFA_LIST_BYTES;
+    static constexpr int SMEM = AREA + (int)sizeof(AsvBitsShared);
 };
 
 // Slice of chain position p of the D slices for step S (asv_chain_pos's z).
@@ -1007,10 +1022,13 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     using G = AsvBitsGeo<S>;
     constexpr int FW = G::FW, FP = G::FP;
     int *flab = (int *)smem;                                   // labels, then their bits
-    AsvBitsShared &b = *(AsvBitsShared *)(smem + ASV_JFA_AREA);
+    AsvBitsShared &b = *(AsvBitsShared *)(smem + G::AREA);
+    unsigned *const acc = (unsigned *)(smem + G::SMEM);           // (summing variant)
     const int tid = threadIdx.x, lane = tid & 31;
     const int sl = W * H;
-    const int lx = tid % ASV_TILE_X, ly = tid / ASV_TILE_X;
+    // a warp walks rows r and r + 2 of the tile: with footprint rows of 24
+    // words their reads fall in different banks (rows r and r + 1 shared eight)
+    const int lx = tid % ASV_TILE_X, ly = (tid >> 6) * 4 + ((tid >> 5) & 1) + ((tid >> 3) & 2);
     const int gx = tx0 + lx, gy = ty0 + ly;
     const bool valid = gx < W && gy < H;                       // other lanes run along, store nothing
     const int x = min(gx, W - 1), y = min(gy, H - 1);
@@ -1020,25 +1038,31 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     // the same values, so no barrier is needed before they are read; brk
     // has a bit for each position but the last where a chain ends
     unsigned brk;
+    int nf, zslot = 0, lslot;                                  // slots; those of slice 0 and slice D - 1
     int zc;                                                    // middle slice of the positions
     float wmax;                                                // largest distance from it
     {
         const int z = lane < n ? asv_chain_z<S>(p0 + lane, D) : 0;
         const bool end = lane < n - 1 && z + S >= D;
         brk = __ballot_sync(FULL, end);
+        const int zf = __shfl_sync(FULL, z, 0), zl = __shfl_sync(FULL, z, n - 1);
+        if (zf > S) zslot = n + 2;
+        if (zl + S < D - 1) lslot = zslot ? n + 3 : n + 2;
+        else lslot = n + 1;
+        nf = n + 2 + (brk ? (zslot != 0) + (lslot != n + 1) : 0);
+        if (nf > G::NSLOT) return false;
         const int z0 = __reduce_min_sync(FULL, lane < n ? z : D), z1 = __reduce_max_sync(FULL, z);
         zc = (z0 + z1) >> 1;
         wmax = (float)(z1 - zc);                               // z1 - zc >= zc - z0
         if (lane < n) b.slot[1 + lane] = make_int4(z * sl, __float_as_int((float)(z - zc)), 2 * z + 1, 0);
-        if (lane == 0) {
-            b.slot[0].x = max(z - S, 0) * sl;
-            b.slot[n + 2].x = 0;
+        if (lane == 0) {                                       // (every entry a slice of the volume, used or not)
+            b.slot[0].x = max(zf - S, 0) * sl;
+            b.slot[n + 1].x = min(zl + S, D - 1) * sl;
+            b.slot[n + 2].x = zslot ? 0 : (D - 1) * sl;
             b.slot[n + 3].x = (D - 1) * sl;
         }
-        if (lane == n - 1) b.slot[n + 1].x = (z + S < D ? z + S : D - 1) * sl;
         __syncwarp();
     }
-    const int nf = brk ? n + 4 : n + 2;
 
     // footprint labels (clamp-to-edge), copied asynchronously a quad at a time
     const bool vec = (W & 3) == 0;
@@ -1089,7 +1113,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
         return false;
     }
     if (SUMS)
-        for (int i = tid; i < (ASV_BITS_MAXT + 1) * ASV_ACC_ROW; i += ASV_JFA_THREADS) b.acc[i] = 0u;
+        for (int i = tid; i < ASV_ACC_WORDS; i += ASV_JFA_THREADS) acc[i] = 0u;
     while (pend) {
         int4 *q = (int4 *)(flab + 4 * (tid + ASV_JFA_THREADS * (__ffs(pend) - 1)));
         pend &= pend - 1;
@@ -1118,8 +1142,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     const float2 uv = make_float2((float)lx - 7.5f, (float)ly - 7.5f);
     const float mg0 = b.margin[0], mg1 = b.margin[1];
     const float mgl = b.magic[0], mga = b.magic[1], mgb = b.magic[2];
-    const bool fast = mg0 < 1e30f;
-    const unsigned m_zero = brk ? smask(f0 + (n + 2) * FP) : 0u, m_last = brk ? smask(f0 + (n + 3) * FP) : 0u;
+    const unsigned m_zero = brk ? smask(f0 + zslot * FP) : 0u, m_last = brk ? smask(f0 + lslot * FP) : 0u;
     unsigned mm = smask(f0), mc = smask(f0 + FP);
     // centroid sums (last pass of an iteration): the thread's current run of
     // equal labels along its column, flushed into the sub-tile's table when
@@ -1130,57 +1153,17 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     unsigned run_z = 0u, run_la = 0u, run_bn = 0u;            // L | a << 16, b | count << 16 (16 x 255 < 2^16)
     const unsigned *fn = f0 + 2 * FP;                         // the next slot
     const unsigned *lab32 = (const unsigned *)lab;
-    unsigned ends = brk, c4n = __ldg(lab32 + (b.slot[1].x + col));
-    for (int j = 0; j < n; j++, fn += FP, ends >>= 1) {
-        const int4 at = b.slot[j + 1];
-        const unsigned c4 = c4n;
-        c4n = __ldg(lab32 + (b.slot[j + 2].x + col));         // the next position's (after the last one: unused)
-        const bool end = ends & 1u;                           // the chain ends here and another one starts:
-        const unsigned mx = smask(fn);                        // the next slot is its centre, else this one's plus
-        const unsigned m = mm | mc | (end ? m_last : mx);
-        int bt = 31 - __clz((int)m);                          // the only candidate, or -1
-        bool slow = !fast && m;
-        if (fast && (m & (m - 1))) {
-            const float w = __int_as_float(at.y);
-            const float2 ww = make_float2(w, w);
-            // bytes to floats: 2^23 + byte, minus 2^23 + the middle colour
-            const float fl = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7650)) - mgl;
-            const float fa = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7651)) - mga;
-            const float fb = __uint_as_float(__byte_perm(c4, 0x4b000000u, 0x7652)) - mgb;
-            float best = 3e38f, sec = 3e38f;
-            unsigned rest = m;
-            do {
-                const int t = 31 - __clz((int)rest);
-                rest ^= 1u << t;
-                const float4 *e = b.eco + ASV_ECO_ROW * t;
-                const float4 e0 = e[0], e1 = e[1], e2 = e[2];
-                const float2 e3 = *(const float2 *)(e + 3);
-                float2 g = __ffma2_rn(make_float2(e0.z, e0.w), uv, make_float2(e0.x, e0.y));
-                g = __ffma2_rn(make_float2(e1.x, e1.y), ww, g);
-                g.x = __fmaf_rn(e1.w, uv.y, g.x);
-                float p = __fmaf_rn(__fmaf_rn(e1.z, w, e2.x), w, e2.y);
-                p = __fmaf_rn(g.x, uv.x, p);
-                p = fmaxf(__fmaf_rn(g.y, uv.y, p), e2.z);
-                p = __fmaf_rn(e2.w, fl, p);
-                p = __fmaf_rn(e3.x, fa, p);
-                p = __fmaf_rn(e3.y, fb, p);
-                sec = fminf(sec, fmaxf(best, p));
-                bt = p < best ? t : bt;
-                best = fminf(best, p);
-            } while (rest);
-            const float q = __fmaf_rn(fl, fl, __fmaf_rn(fa, fa, fb * fb));
-            slow = !(sec - best > __fmaf_rn(16.0f * ASV_EPS, sec + best, __fmaf_rn(mg1, q, mg0)));
-        }
-        if (slow) {
-            const unsigned *fm = j > 0 && ((brk >> (j - 1)) & 1u) ? f0 + (n + 2) * FP : fn - 2 * FP;   // minus slice
-            bt = asv_bits_exact<S>(m, fn - FP, fm, end ? f0 + (n + 3) * FP : fn, b, tab, x, y, at.z >> 1, c4, ratio);
-        }
+    unsigned ends = brk, ca = __ldg(lab32 + (b.slot[1].x + col)), cb = __ldg(lab32 + (b.slot[2].x + col));
+    // positions left to the shader's arithmetic: all of them without scores
+    unsigned slow = mg0 < 1e30f ? 0u : (1u << n) - 1u;
+    // a position's label out and, in a summing pass, into the run
+    auto put = [&](int j, const int4 at, unsigned c4, int bt) {
         const int label = bt >= 0 ? b.tlab[bt] : -1;
-        if (valid) out[at.x + col] = label;
-        if (SUMS && valid) {
+        if (valid) out[at.x + col] = label;                   // (a slow position's is replaced below)
+        if (SUMS && valid && !((slow >> j) & 1u)) {
             const int e = bt >= 0 ? bt : ASV_BITS_MAXT;
             if (e != run_e) {
-                if (run_e >= 0) asv_run_flush(b.acc + ASV_ACC_ROW * run_e, run_z, run_la, run_bn, lxy);
+                if (run_e >= 0) asv_run_flush(acc + ASV_ACC_ROW * (ASV_ACC_COPIES * run_e + lane % ASV_ACC_COPIES), run_z, run_la, run_bn, lxy);
                 run_e = e;
                 run_z = run_la = run_bn = 0u;
             }
@@ -1188,35 +1171,102 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
             run_la += __byte_perm(c4, 0u, 0x4140);
             run_bn += __byte_perm(c4, 1u, 0x7472);            // bytes (b, 0, 1, 0)
         }
-        mm = end ? m_zero : mc;
-        mc = mx;
+    };
+    // Two positions at a time: their candidates are mostly the same, so a
+    // label's fourteen coefficients are read once for both.  (What bounds the
+    // passes is the shared-memory data path, 85 % busy with one position at a
+    // time, most of it with coefficients.)
+    for (int j = 0; j < n; j += 2, fn += 2 * FP, ends >>= 2) {
+        const int4 at0 = b.slot[j + 1], at1 = b.slot[j + 2];
+        const unsigned c0 = ca, c1 = cb;
+        ca = __ldg(lab32 + (b.slot[j + 3].x + col));          // the next pair's (past the last one: unused)
+        cb = __ldg(lab32 + (b.slot[j + 4].x + col));
+        const bool end0 = ends & 1u, end1 = ends & 2u;        // the chain ends here and another one starts:
+        const unsigned mx = smask(fn), my = smask(fn + FP);   // the next slot is its centre, else this one's plus
+        const unsigned ma = mm | mc | (end0 ? m_last : mx);
+        const unsigned mb = j + 1 < n ? (end0 ? m_zero : mc) | mx | (end1 ? m_last : my) : 0u;
+        mm = end1 ? m_zero : mx;
+        mc = my;
+        int bta = 31 - __clz((int)ma), btb = 31 - __clz((int)mb);   // the only candidate, or -1
+        const bool twoa = ma & (ma - 1), twob = mb & (mb - 1);
+        unsigned rest = (twoa ? ma : 0u) | (twob ? mb : 0u);
+        if (rest) {
+            const float wa = __int_as_float(at0.y), wb = __int_as_float(at1.y);
+            // bytes to floats: 2^23 + byte, minus 2^23 + the middle colour
+            const float la = __uint_as_float(__byte_perm(c0, 0x4b000000u, 0x7650)) - mgl;
+            const float aa = __uint_as_float(__byte_perm(c0, 0x4b000000u, 0x7651)) - mga;
+            const float ba = __uint_as_float(__byte_perm(c0, 0x4b000000u, 0x7652)) - mgb;
+            const float lb = __uint_as_float(__byte_perm(c1, 0x4b000000u, 0x7650)) - mgl;
+            const float ab = __uint_as_float(__byte_perm(c1, 0x4b000000u, 0x7651)) - mga;
+            const float bb = __uint_as_float(__byte_perm(c1, 0x4b000000u, 0x7652)) - mgb;
+            float besta = 3e38f, seca = 3e38f, bestb = 3e38f, secb = 3e38f;
+            do {
+                const int t = 31 - __clz((int)rest);
+                const unsigned bit = 1u << t;
+                rest ^= bit;
+                const float4 *e = b.eco + ASV_ECO_ROW * t;
+                const float4 e0 = e[0], e1 = e[1], e2 = e[2];
+                const float2 e3 = *(const float2 *)(e + 3);
+                const float2 g = __ffma2_rn(make_float2(e0.z, e0.w), uv, make_float2(e0.x, e0.y));
+                const float k = __fmaf_rn(g.y, uv.y, __fmaf_rn(__fmaf_rn(e1.w, uv.y, g.x), uv.x, e2.y));
+                const float h = __fmaf_rn(e1.y, uv.y, __fmaf_rn(e1.x, uv.x, e2.x));
+                if (ma & bit) {
+                    float p = fmaxf(__fmaf_rn(__fmaf_rn(e1.z, wa, h), wa, k), e2.z);
+                    p = __fmaf_rn(e3.y, ba, __fmaf_rn(e3.x, aa, __fmaf_rn(e2.w, la, p)));
+                    seca = fminf(seca, fmaxf(besta, p));
+                    bta = p < besta ? t : bta;
+                    besta = fminf(besta, p);
+                }
+                if (mb & bit) {
+                    float p = fmaxf(__fmaf_rn(__fmaf_rn(e1.z, wb, h), wb, k), e2.z);
+                    p = __fmaf_rn(e3.y, bb, __fmaf_rn(e3.x, ab, __fmaf_rn(e2.w, lb, p)));
+                    secb = fminf(secb, fmaxf(bestb, p));
+                    btb = p < bestb ? t : btb;
+                    bestb = fminf(bestb, p);
+                }
+            } while (rest);
+            const float qa = __fmaf_rn(la, la, __fmaf_rn(aa, aa, ba * ba)), qb = __fmaf_rn(lb, lb, __fmaf_rn(ab, ab, bb * bb));
+            // (a position whose only candidate also came by keeps it: second stays 3e38)
+            if (twoa && !(seca - besta > __fmaf_rn(16.0f * ASV_EPS, seca + besta, __fmaf_rn(mg1, qa, mg0)))) slow |= 1u << j;
+            if (twob && !(secb - bestb > __fmaf_rn(16.0f * ASV_EPS, secb + bestb, __fmaf_rn(mg1, qb, mg0)))) slow |= 2u << j;
+        }
+        put(j, at0, c0, bta);
+        if (j + 1 < n) put(j + 1, at1, c1, btb);
+    }
+    while (slow && valid) {
+        const int j = __ffs(slow) - 1;
+        slow &= slow - 1;
+        const unsigned *fc = f0 + (j + 1) * FP;
+        const unsigned *fm = j > 0 && ((brk >> (j - 1)) & 1u) ? f0 + zslot * FP : fc - FP;   // minus slice
+        const unsigned *fp = (brk >> j) & 1u ? f0 + lslot * FP : fc + FP;
+        const int4 at = b.slot[j + 1];
+        const unsigned c4 = __ldg(lab32 + (at.x + col));
+        const int bt = asv_bits_exact<S>(smask(fm) | smask(fc) | smask(fp), fc, fm, fp, b, tab, x, y, at.z >> 1, c4, ratio);
+        out[at.x + col] = bt >= 0 ? b.tlab[bt] : -1;
+        if (SUMS)
+            asv_run_flush(acc + ASV_ACC_ROW * ASV_ACC_COPIES * (bt >= 0 ? bt : ASV_BITS_MAXT), (unsigned)at.z, __byte_perm(c4, 0u, 0x4140),
+                          __byte_perm(c4, 1u, 0x7472), lxy);
     }
     if (SUMS) {
-        // the runs left at the end, grouped by entry across the warp (every
-        // lane of the block gets here; lanes without a run join with entry
-        // -1, which adds nothing), so a warp adds each entry once
-        const unsigned grp = __match_any_sync(0xffffffffu, run_e);
-        unsigned w[ASV_ACC_ROW];
-        asv_run_words(w, run_z, run_la, run_bn, lxy);
-#pragma unroll
-        for (int k = 0; k < ASV_ACC_ROW; k++) w[k] = __reduce_add_sync(grp, w[k]);
-        if (run_e >= 0 && lane == __ffs(grp) - 1) {
-#pragma unroll
-            for (int k = 0; k < ASV_ACC_ROW; k++) atomicAdd(b.acc + ASV_ACC_ROW * run_e + k, w[k]);
-        }
+        // the runs left at the end (straight into the copies: grouping a
+        // warp's lanes by entry first took 2 % of the 64x48x12 clip's loop)
+        if (run_e >= 0)
+            asv_run_flush(acc + ASV_ACC_ROW * (ASV_ACC_COPIES * run_e + lane % ASV_ACC_COPIES), run_z, run_la, run_bn, lxy);
         __syncthreads();
         for (int i = tid; i < (T + 1) * 8; i += ASV_JFA_THREADS) {
             const int e = i >> 3, k = i & 7;
             const int ent = e < T ? e : ASV_BITS_MAXT;           // the -1 entry after the T labels
-            const unsigned *a = b.acc + ASV_ACC_ROW * ent;
-            const unsigned cnt = a[1] >> 20;
-            if (k == 7 || !cnt) continue;
-            unsigned v;                                          // 2 x + 1 = 2 (tx0 + column) + 1
-            if (k == 0) v = 2u * (a[0] & 0xffffu) + cnt * (2u * (unsigned)tx0 + 1u);
-            else if (k == 1) v = 2u * (a[0] >> 16) + cnt * (2u * (unsigned)ty0 + 1u);
-            else if (k == 3) v = cnt;
-            else if (k == 4) v = a[1] & 0xfffffu;
-            else v = a[k == 2 ? 2 : k - 2];
+            if (k == 7) continue;
+            unsigned cnt = 0u, v = 0u;
+#pragma unroll
+            for (int c = 0; c < ASV_ACC_COPIES; c++) {
+                const unsigned *a = acc + ASV_ACC_ROW * (ASV_ACC_COPIES * ent + c);
+                cnt += a[1] >> 20;
+                v += k < 2 ? (a[0] >> (16 * k)) & 0xffffu : (k == 4 ? a[1] & 0xfffffu : (k == 3 ? 0u : a[k == 2 ? 2 : k - 2]));
+            }
+            if (!cnt) continue;
+            if (k < 2) v = 2u * v + cnt * (2u * (unsigned)(k ? ty0 : tx0) + 1u);   // 2 x + 1 = 2 (tx0 + column) + 1
+            if (k == 3) v = cnt;
             atomicAdd(sums + 8ull * (slot0 + (ent < ASV_BITS_MAXT ? b.tlab[ent] : Kp)) + k, (unsigned long long)v);
         }
     }
@@ -1224,16 +1274,10 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
     return true;
 }
 
-// Variants of k_jfa: ST is the step of the pass (1 to 6), ASV_JFA_LIST for the
-// larger ones (list form only) or 0 for segments of different steps; SUMS 0
-// or 1, or 2 where the pass is the last one of some segments only.  A variant
-// holds just the code of its pass: against the one kernel for all (now <0,
-// 2>), which keeps the registers of the worst of them, the 240x160x30 clip
-// with its full ladder took 3.96 instead of 4.39 ms, the 640x480x60 one 16.1
-// instead of 16.7.
+// One tile of a pass: bit-set form by sub-tiles (ST the pass's step, 1 to 6),
+// else (ST = ASV_JFA_LIST: larger steps; or for a sub-tile whose footprint
+// holds too many labels) the list form.
 #define ASV_JFA_LIST 7
-// one tile of a pass: bit-set form by sub-tiles where it applies, else (or
-// for a sub-tile whose footprint holds too many labels) the list form
 template <int ST, bool SUMS>
 __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int32_t *__restrict__ out,
                                              const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
@@ -1253,30 +1297,24 @@ __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int
         const int nc = min(n - c0, 32), pc = p0 + c0;
         unsigned todo = 0xffffffffu >> (32 - nc);
         int cap = SUMS ? min(depth, 15) : depth;               // 15: asv_run_words
-        if (Kp > ASV_BITS_MAXKP) cap = 0;
-#define ASV_BITS_CASE(S_)                                                                                    \
-    case S_:                                                                                                 \
-        cap = min(cap, AsvBitsGeo<S_>::SUB);                                                                 \
-        do {                                                                                                 \
-            const int q = __ffs(todo) - 1;                                                                   \
-            const unsigned past = ~(todo >> q);                                                              \
-            const int m = min(cap, past ? __ffs(past) - 1 : 32);                                             \
-            const unsigned bits = (0xffffffffu >> (32 - m)) << q;                                            \
-            todo &= ~bits;                                                                                   \
-            if (!asv_jfa_bits_sub<S_, SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, tx0, ty0, pc + q,   \
-                                            m, ratio, smem))                                                 \
-                fail |= bits;                                                                                \
-        } while (todo);                                                                                      \
-        break;
-        while (ST != ASV_JFA_LIST && cap >= 4 && todo) {
-            unsigned fail = 0u;
-            switch (ST ? ST : step) {
-                ASV_BITS_CASE(1) ASV_BITS_CASE(2) ASV_BITS_CASE(3) ASV_BITS_CASE(4) ASV_BITS_CASE(5) ASV_BITS_CASE(6)
+        if constexpr (ST < ASV_JFA_LIST) {
+            cap = Kp > ASV_BITS_MAXKP ? 0 : min(cap, AsvBitsGeo<ST>::SUB);
+            while (cap >= 4 && todo) {
+                unsigned fail = 0u;
+                do {
+                    const int q = __ffs(todo) - 1;
+                    const unsigned past = ~(todo >> q);
+                    const int m = min(cap, past ? __ffs(past) - 1 : 32);
+                    const unsigned bits = (0xffffffffu >> (32 - m)) << q;
+                    todo &= ~bits;
+                    if (!asv_jfa_bits_sub<ST, SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, tx0, ty0, pc + q, m,
+                                                    ratio, smem))
+                        fail |= bits;
+                } while (todo);
+                todo = fail;
+                cap = (cap + 1) >> 1;
             }
-            todo = fail;
-            cap = (cap + 1) >> 1;
         }
-#undef ASV_BITS_CASE
         while (todo) {                                         // runs of positions left
             const int q = __ffs(todo) - 1;
             const unsigned past = ~(todo >> q);
@@ -1289,9 +1327,8 @@ __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int
     }
 }
 
-__device__ __forceinline__ void asv_jfa_smem_init(unsigned char *smem)
+__device__ __forceinline__ void asv_jfa_smem_init(AsvBitsShared &b)
 {
-    AsvBitsShared &b = *(AsvBitsShared *)(smem + ASV_JFA_AREA);
     for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 32; i += blockDim.x) b.claim[i] = 0u;
     for (int i = threadIdx.x; i < ASV_BITS_MAXKP / 4; i += blockDim.x) ((unsigned *)b.map8)[i] = 0xffffffffu;
     if (threadIdx.x == 0) {
@@ -1301,29 +1338,32 @@ __device__ __forceinline__ void asv_jfa_smem_init(unsigned char *smem)
     __syncthreads();
 }
 
-// tile = ASV_TILE_X x ASV_TILE_Y columns x S.zrun chain positions
-template <int ST, int SUMS>
+// A pass over the tiles (ASV_TILE_X x ASV_TILE_Y columns x S.zrun chain
+// positions) of the segments whose step in this pass is ST (ASV_JFA_LIST: larger
+// than 6) and, with SUMS, whose last pass it is (always of step 1); a pass of
+// segments of different steps is a launch of each.  A variant holds just the
+// code of its pass: against one kernel for all, which kept the registers of the
+// worst, the 240x160x30 clip with its full ladder took 3.96 instead of 4.39 ms,
+// the 640x480x60 one 16.1 instead of 16.7.
+template <int ST, bool SUMS>
 __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
                                                          const int32_t *__restrict__ in,
                                                          int32_t *__restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char asv_jfa_smem[];
-    if (ST != ASV_JFA_LIST) asv_jfa_smem_init(asv_jfa_smem);
+    if constexpr (ST < ASV_JFA_LIST) asv_jfa_smem_init(*(AsvBitsShared *)(asv_jfa_smem + AsvBitsGeo<ST>::AREA));
     for (int t = blockIdx.x; t < d.total_tiles; t += gridDim.x) {
         const int si = asv_find_seg(d.tile_prefix, d.nseg, t);
         const SegDesc &S = d.segs[si];
         if (pass >= S.npass) continue;
+        const int step = S.steps[pass];
+        if (min(step, ASV_JFA_LIST) != ST || (ST == 1 && (pass == S.npass - 1) != SUMS)) continue;
         const int lt = t - d.tile_prefix[si];
         const int rest = asv_quotient(lt, S.inv_tiles_x), tx = lt - rest * S.tiles_x;
         const int tz = asv_quotient(rest, S.inv_tiles_y), ty = rest - tz * S.tiles_y, p0 = tz * S.zrun;
-        if (SUMS == 1 || (SUMS == 2 && pass == S.npass - 1))   // the iteration's labels: sum them
-            asv_jfa_tile<ST, true>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
-                               d.sums, S.seed_off, S.W, S.H, S.D, S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0,
-                               S.zrun, S.depth[pass], S.steps[pass], S.ratio[pass], asv_jfa_smem);
-        else
-            asv_jfa_tile<ST, false>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
-                                nullptr, 0, S.W, S.H, S.D, S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0,
-                                S.zrun, S.depth[pass], S.steps[pass], S.ratio[pass], asv_jfa_smem);
+        asv_jfa_tile<ST, SUMS>(in + S.vox_off, out + S.vox_off, d.lab + S.vox_off, d.jtab + 3 * S.seed_off,
+                               SUMS ? d.sums : nullptr, S.seed_off, S.W, S.H, S.D, S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y,
+                               p0, S.zrun, S.depth[pass], ST < ASV_JFA_LIST ? ST : step, S.ratio[pass], asv_jfa_smem);
     }
 }
 
@@ -1526,25 +1566,6 @@ __global__ void k_label_clean(int32_t *__restrict__ lbl, long long n, int Kp)
 {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v < n && (unsigned)lbl[v] >= (unsigned)Kp) lbl[v] = -1;
-}
-
-// single-segment pass with explicit step and ratio (test entry point)
-__global__ void __launch_bounds__(ASV_JFA_THREADS) k_jfa_single(AsvDev d, const int32_t *__restrict__ in,
-                                                                int32_t *__restrict__ out, int step,
-                                                                float ratio)
-{
-    extern __shared__ __align__(16) unsigned char asv_jfa_smem[];
-    asv_jfa_smem_init(asv_jfa_smem);
-    const SegDesc &S = d.segs[0];
-    const int tiles_z = (S.D + S.zrun - 1) / S.zrun;
-    const int ntiles = S.tiles_x * S.tiles_y * tiles_z;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int tx = t % S.tiles_x, rest = t / S.tiles_x;
-        const int ty = rest % S.tiles_y, p0 = (rest / S.tiles_y) * S.zrun;
-        asv_jfa_tile<0, false>(in, out, d.lab + S.vox_off, d.jtab + 3 * S.seed_off, nullptr, 0, S.W, S.H, S.D,
-                            S.Kp, tx * ASV_TILE_X, ty * ASV_TILE_Y, p0, S.zrun, step <= ASV_BITS_MAXS ? 16 : 0, step, ratio,
-                            asv_jfa_smem);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1894,21 +1915,25 @@ void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st)
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st) { k_first_init<<<seed_blocks(d), 128, 0, st>>>(d); }
 void asv_launch_draw(const AsvDev &d, cudaStream_t st) { k_draw<<<seed_blocks(d), 128, 0, st>>>(d); }
 
-typedef void (*AsvJfaKernel)(AsvDev, int, const int32_t *, int32_t *);
+struct AsvJfaVariant {
+    void (*kernel)(AsvDev, int, const int32_t *, int32_t *);
+    int smem;                                      // dynamic shared memory
+};
 
-// k_jfa's variant for a pass of this step (0: segments of different steps, or
-// of different ladders' lengths at a last pass)
-static AsvJfaKernel asv_jfa_variant(int step, int sums)
+// k_jfa's variant for a pass of this step (last: the pass that also sums)
+static const AsvJfaVariant &asv_jfa_variant(int step, bool last)
 {
-    static const AsvJfaKernel k[ASV_JFA_LIST + 1][2] = {
-        { k_jfa<0, 2>, k_jfa<0, 2> }, { k_jfa<1, 0>, k_jfa<1, 1> }, { k_jfa<2, 0>, k_jfa<2, 1> },
-        { k_jfa<3, 0>, k_jfa<3, 1> }, { k_jfa<4, 0>, k_jfa<4, 1> }, { k_jfa<5, 0>, k_jfa<5, 1> },
-        { k_jfa<6, 0>, k_jfa<6, 1> }, { k_jfa<ASV_JFA_LIST, 0>, k_jfa<ASV_JFA_LIST, 1> } };
-    return k[step < ASV_JFA_LIST ? step : ASV_JFA_LIST][sums];
+    static const AsvJfaVariant v[ASV_JFA_LIST + 1] = {
+        { k_jfa<1, true>, AsvBitsGeo<1>::SMEM + 4 * ASV_ACC_WORDS },
+        { k_jfa<1, false>, AsvBitsGeo<1>::SMEM }, { k_jfa<2, false>, AsvBitsGeo<2>::SMEM },
+        { k_jfa<3, false>, AsvBitsGeo<3>::SMEM }, { k_jfa<4, false>, AsvBitsGeo<4>::SMEM },
+        { k_jfa<5, false>, AsvBitsGeo<5>::SMEM }, { k_jfa<6, false>, AsvBitsGeo<6>::SMEM },
+        { k_jfa<ASV_JFA_LIST, false>, ASV_JFA_LIST_BYTES } };
+    return v[last ? 0 : (step < ASV_JFA_LIST ? step : ASV_JFA_LIST)];
 }
 
-// k_jfa's dynamic shared memory (list rows or bit-set footprint, and the
-// bit-set table) exceeds the 48 KiB default: raised once per device
+// the variants' dynamic shared memory exceeds the 48 KiB default: raised once
+// per device
 static void asv_jfa_attributes()
 {
     static std::mutex mu;
@@ -1917,35 +1942,39 @@ static void asv_jfa_attributes()
     cudaGetDevice(&dev);
     std::lock_guard<std::mutex> lk(mu);
     if (dev >= 0 && dev < 64 && done[dev]) return;
-    for (int st = 0; st < ASV_JFA_LIST; st++)
-        for (int sums = 0; sums < 2; sums++)
-            cudaFuncSetAttribute((const void *)asv_jfa_variant(st, sums), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 ASV_JFA_SMEM);
-    cudaFuncSetAttribute(k_jfa_single, cudaFuncAttributeMaxDynamicSharedMemorySize, ASV_JFA_SMEM);
+    for (int st = 0; st <= ASV_JFA_LIST; st++) {
+        const AsvJfaVariant &v = asv_jfa_variant(st, st == 0);
+        cudaFuncSetAttribute((const void *)v.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v.smem);
+    }
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
 
-// resident k_jfa blocks on the device (persistent grid size); computed once
-// per process (thread-safe static initialisation)
+// resident k_jfa blocks on the device (persistent grid size): the least of
+// the variants', computed once per process (thread-safe static initialisation)
 int asv_jfa_resident_blocks()
 {
     static const int blocks = [] {
-        int dev = 0, sms = 0, per = 0;
+        int dev = 0, sms = 0, least = 0;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         asv_jfa_attributes();
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_jfa<0, 2>, ASV_JFA_THREADS, ASV_JFA_SMEM);
-        const int b = sms * (per > 0 ? per : 1);
+        for (int st = 0; st <= ASV_JFA_LIST; st++) {
+            const AsvJfaVariant &v = asv_jfa_variant(st, st == 0);
+            int per = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, v.kernel, ASV_JFA_THREADS, v.smem);
+            if (per > 0 && (!least || per < least)) least = per;
+        }
+        const int b = sms * (least > 0 ? least : 1);
         return b > 0 ? b : 1024;
     }();
     return blocks;
 }
 
-int asv_jfa_max_depth(int step)
+int asv_jfa_slots(int step)
 {
-    static const int sub[ASV_BITS_MAXS + 1] = { 0, AsvBitsGeo<1>::SUB, AsvBitsGeo<2>::SUB, AsvBitsGeo<3>::SUB,
-                                                AsvBitsGeo<4>::SUB, AsvBitsGeo<5>::SUB, AsvBitsGeo<6>::SUB };
-    return step >= 1 && step <= ASV_BITS_MAXS ? sub[step] : 0;
+    static const int slots[ASV_BITS_MAXS + 1] = { 0, AsvBitsGeo<1>::NSLOT, AsvBitsGeo<2>::NSLOT, AsvBitsGeo<3>::NSLOT,
+                                                  AsvBitsGeo<4>::NSLOT, AsvBitsGeo<5>::NSLOT, AsvBitsGeo<6>::NSLOT };
+    return step >= 1 && step <= ASV_BITS_MAXS ? slots[step] : 0;
 }
 
 int asv_jfa_grid_blocks(int total_tiles)
@@ -1954,13 +1983,13 @@ int asv_jfa_grid_blocks(int total_tiles)
     return total_tiles < blocks ? total_tiles : blocks;
 }
 
-void asv_launch_jfa(const AsvDev &d, int pass, int step, int sums, int grid_blocks, cudaStream_t st)
+void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, cudaStream_t st)
 {
     const int32_t *in = (pass & 1) ? d.labB : d.labA;
     int32_t *out = (pass & 1) ? d.labA : d.labB;
     asv_jfa_attributes();
-    asv_jfa_variant(step, sums)<<<grid_blocks, ASV_JFA_THREADS, step < ASV_JFA_LIST ? ASV_JFA_SMEM : ASV_JFA_LIST_BYTES,
-                                  st>>>(d, pass, in, out);
+    const AsvJfaVariant &v = asv_jfa_variant(step, last);
+    v.kernel<<<grid_blocks, ASV_JFA_THREADS, v.smem, st>>>(d, pass, in, out);
 }
 
 // filled: the output volume is all -1 and the list empty already
@@ -1983,12 +2012,9 @@ void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st
     k_jfa_second<true><<<blocks, 256, 0, st>>>(d, false);
 }
 
-void asv_launch_jfa_single(const AsvDev &d, int32_t *in, long long nvox, int Kp, int32_t *out, int step, float ratio,
-                           cudaStream_t st)
+void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st)
 {
-    asv_jfa_attributes();
-    k_label_clean<<<(unsigned)((nvox + 255) / 256), 256, 0, st>>>(in, nvox, Kp);
-    k_jfa_single<<<asv_jfa_grid_blocks(d.total_tiles), 256, ASV_JFA_SMEM, st>>>(d, in, out, step, ratio);
+    k_label_clean<<<(unsigned)((nvox + 255) / 256), 256, 0, st>>>(labels, nvox, Kp);
 }
 
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st) { k_centroids<<<d.total_chunks, 256, 0, st>>>(d); }
