@@ -130,7 +130,8 @@ __device__ __forceinline__ void fl_pair(int p, int D, int &src, int &dst)
 // the per-pixel products A^T A (g11, g12, g22) and A^T db (h1, h2) at pixel
 // (x, y) of the frame with the current flow (dx, dy), from the expansions
 // sA/sB of the source frame and dA/dB of the destination frame; zero when
-// x + d falls outside the frame
+// x + d falls outside the frame.  THIN: the frame may be one pixel wide or high.
+template <bool THIN>
 __device__ __forceinline__ void fl_matrix(const float4 *__restrict__ sA, const float *__restrict__ sB,
                                           const float4 *__restrict__ dA, const float *__restrict__ dB, int W,
                                           int H, int x, int y, float dx, float dy, float o[5])
@@ -140,14 +141,14 @@ __device__ __forceinline__ void fl_matrix(const float4 *__restrict__ sA, const f
     // a select, so a thread's evaluations overlap their loads
     const float qx = (float)x + dx, qy = (float)y + dy;
     const bool inside = qx >= 0.f && qy >= 0.f && qx <= (float)(W - 1) && qy <= (float)(H - 1);
-    const int x0 = min(max((int)qx, 0), W - 2 < 0 ? 0 : W - 2), y0 = min(max((int)qy, 0), H - 2 < 0 ? 0 : H - 2);
-    const int x1 = min(x0 + 1, W - 1), y1 = min(y0 + 1, H - 1);
+    const int x0 = min(max((int)qx, 0), THIN ? max(W - 2, 0) : W - 2), y0 = min(max((int)qy, 0), THIN ? max(H - 2, 0) : H - 2);
+    const int right = THIN && W < 2 ? 0 : 1, below = THIN && H < 2 ? 0 : W;   // to the samples at x0 + 1, y0 + 1
     const float fx = qx - (float)x0, fy = qy - (float)y0;
     const float w00 = (1.f - fx) * (1.f - fy), w01 = fx * (1.f - fy), w10 = (1.f - fx) * fy, w11 = fx * fy;
     const int s = y * W + x;                                   // frames hold < 2^31 pixels
-    const int i00 = y0 * W + x0, i01 = y0 * W + x1, i10 = y1 * W + x0, i11 = y1 * W + x1;
-    const float4 t00 = __ldg(dA + i00), t01 = __ldg(dA + i01), t10 = __ldg(dA + i10), t11 = __ldg(dA + i11);
-    const float u00 = __ldg(dB + i00), u01 = __ldg(dB + i01), u10 = __ldg(dB + i10), u11 = __ldg(dB + i11);
+    const int i0 = y0 * W + x0, i1 = i0 + below;
+    const float4 t00 = __ldg(dA + i0), t01 = __ldg(dA + i0 + right), t10 = __ldg(dA + i1), t11 = __ldg(dA + i1 + right);
+    const float u00 = __ldg(dB + i0), u01 = __ldg(dB + i0 + right), u10 = __ldg(dB + i1), u11 = __ldg(dB + i1 + right);
     const float4 sa = __ldg(sA + s);
     const float sb = __ldg(sB + s);
     float q[5];
@@ -168,144 +169,244 @@ __device__ __forceinline__ void fl_matrix(const float4 *__restrict__ sA, const f
     o[4] = inside ? a12 * db1 + a22 * db2 : 0.f;
 }
 
-// One iteration for a TW x TH tile of one frame pair: the five matrix planes
-// of the tile and its 6-pixel halo are computed from the flow `fin` straight
-// into shared memory (zero outside the frame), summed over the 13x13 window
-// -- rows along x, then the row sums along y, both in ascending index order,
-// so the sums equal those of separate x and y passes -- and each pixel's 2x2
-// system is solved into `fout`.  fin and fout are separate buffers: halo
-// pixels read flow that neighbouring tiles overwrite.
-template <int TW, int TH, int NT>
-__global__ void __launch_bounds__(NT) k_fl_iter(const float4 *__restrict__ polyA, const float *__restrict__ polyB,
-                                                const float *__restrict__ fin, float *__restrict__ fout, int W,
-                                                int H, int D, int P)
+// One iteration for a strip of FL_TW columns and `rows` rows of one frame pair.
+// The block goes down the strip eight rows at a time: it computes the five
+// matrix planes of the next rows and their 6-pixel halo in x from the flow
+// `fin` (zero outside the frame), sums them over 13 columns into a ring of 20
+// rows, and sums the ring over 13 rows for eight finished ones, whose 2x2
+// systems it solves into `fout`.  Both sums run in ascending index order, so
+// they equal those of separate x and y passes.  fin and fout are separate
+// buffers: halo pixels read flow that neighbouring strips overwrite.
+//
+// The iterations are bound by instruction issue and the shared-memory data path
+// (68 % each with a tile of 64 x 32 per block: 1.63 matrices per pixel, 632
+// instructions).  Going down a strip leaves the halo in x and twelve rows per
+// strip, 1.2 to 1.3 matrices per pixel; the sums of two planes are two-wide
+// additions (sums only: no product feeds them); four windows share a thread's
+// sixteen loads in both directions.  At 640x480x16, level 0, 240 -> 178 us an
+// iteration.
+//
+// Shared memory: S[5][8][FL_SP], where a column c lies at c + c / 4: the threads
+// of a warp, two rows of sixteen windows four columns apart, then read sixteen
+// banks five apart and, the row pitch being 16 modulo 32, the other sixteen.
+// T[5][20][FL_TW], the ring: row y of the strip is at (y + 6) mod 20.
+#define FL_TW 64
+#define FL_NT 128
+#define FL_RS 8                              // rows per step
+#define FL_RING (FL_RS + 2 * FL_BOX)
+#define FL_RW (FL_TW + 2 * FL_BOX)
+#define FL_PX ((FL_RS * FL_RW + FL_NT - 1) / FL_NT)   // matrices per thread and step
+#define FL_SP 112
+#define FL_SMEM (4 * 5 * (FL_RS * FL_SP + FL_RING * FL_TW))
+
+template <bool THIN>
+__global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__ polyA, const float *__restrict__ polyB,
+                                                   const float *__restrict__ fin, float *__restrict__ fout, int W,
+                                                   int H, int D, int P, int rows)
 {
-    constexpr int RPT = TH / (NT / 32);              // output rows per thread
-    static_assert(TW % 32 == 0 && RPT >= 1 && RPT * (NT / 32) == TH, "tile shape");
-    extern __shared__ float fl_sm[];
-    constexpr int RW = TW + 2 * FL_BOX, RH = TH + 2 * FL_BOX, SP = RW + 1, TP = TW + 1;
-    float *S = fl_sm;                                  // [5][RH][SP]
-    float *T = fl_sm + 5 * RH * SP;                    // [RH][TP]
+    extern __shared__ __align__(16) float fl_sm[];
+    float *S = fl_sm, *T = fl_sm + 5 * FL_RS * FL_SP;
     const long long fr = (long long)W * H, mplane = fr * P;
-    const int tiles_x = (W + TW - 1) / TW, tiles_y = (H + TH - 1) / TH;
+    const int strips = (W + FL_TW - 1) / FL_TW, chunks = (H + rows - 1) / rows;
     // blocks take the pairs as z -> z+1, z+1 -> z, z+1 -> z+2, ...: the two
     // pairs of a frame pair read the same two expansions while both are in L2
-    const int j = blockIdx.x / (tiles_x * tiles_y);
+    const int j = blockIdx.x / (strips * chunks);
     const int pr = (j & 1) ? D - 1 + (j >> 1) : (j >> 1);
-    const int rem = blockIdx.x - j * tiles_x * tiles_y;
-    const int x0 = (rem % tiles_x) * TW, y0 = (rem / tiles_x) * TH;
+    const int rem = blockIdx.x - j * strips * chunks;
+    const int x0 = (rem % strips) * FL_TW, yb = (rem / strips) * rows, ye = min(yb + rows, H);
     int src, dst;
     fl_pair(pr, D, src, dst);
     const float4 *sA = polyA + fr * src, *dA = polyA + fr * dst;
     const float *sB = polyB + fr * src, *dB = polyB + fr * dst;
     const float *fx_in = fin + fr * pr, *fy_in = fin + mplane + fr * pr;
-    for (int i0 = threadIdx.x; i0 < RW * RH; i0 += 2 * NT) {     // two pixels per trip
-        int cell[2];
-        bool keep[2];
-        float o[2][5];
+    const int t = threadIdx.x;
+
+    // a thread's pixels of a step: the same columns and rows of S every time.
+    // Their flow is loaded a step ahead (before the vertical sums), so that a
+    // step waits for the samples only, two or three pixels' at a time.
+    int cx[FL_PX], pr_[FL_PX];                                           // column in the frame; row of S and place in it
+    unsigned keepx = 0u;
+    float fx[FL_PX], fy[FL_PX];
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-            const int i = i0 + u * NT;
-            cell[u] = i < RW * RH ? i : 0;
-            const int r = cell[u] / RW, q = cell[u] - r * RW;
-            const int gy = y0 - FL_BOX + r, gx = x0 - FL_BOX + q;
-            keep[u] = gx >= 0 && gx < W && gy >= 0 && gy < H;       // zero outside the frame
-            const int cx = min(max(gx, 0), W - 1), cy = min(max(gy, 0), H - 1);
-            const int e = cy * W + cx;
-            fl_matrix(sA, sB, dA, dB, W, H, cx, cy, __ldg(fx_in + e), __ldg(fy_in + e), o[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < 2; u++) {
-            if (i0 + u * NT >= RW * RH) continue;
-            const int r = cell[u] / RW, q = cell[u] - r * RW;
-#pragma unroll
-            for (int c = 0; c < 5; c++) S[(c * RH + r) * SP + q] = keep[u] ? o[u][c] : 0.f;
-        }
+    for (int k = 0; k < FL_PX; k++) {
+        const int i = min(t + k * FL_NT, FL_RS * FL_RW - 1), r = i / FL_RW, q = i - r * FL_RW, gx = x0 - FL_BOX + q;
+        cx[k] = min(max(gx, 0), W - 1);
+        if (gx >= 0 && gx < W) keepx |= 1u << k;                         // zero outside the frame
+        pr_[k] = t + k * FL_NT < FL_RS * FL_RW ? (r << 16) | (r * FL_SP + q + (q >> 2)) : -1;
     }
-    __syncthreads();
-    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;            // 32 x NT/32 threads
-    float acc[TW / 32][RPT][5];
-    // window sums several at a time from registers: a thread loads the
-    // values of adjacent windows once (horizontal: four windows, one column
-    // group per warp with lanes on rows, so with the odd row pitches a
-    // warp's loads and stores fall in distinct banks; vertical: RPT rows)
+    auto load_flow = [&](int y) {
 #pragma unroll
-    for (int c = 0; c < 5; c++) {
-        const float *Sc = S + c * RH * SP;
-        for (int g = threadIdx.x / 32; g < TW / 4; g += NT / 32)
-            for (int r = threadIdx.x % 32; r < RH; r += 32) {
-                const int q = 4 * g;
-                float w[16];
+        for (int k = 0; k < FL_PX; k++) {
+            const int e = min(max(y + (pr_[k] >> 16), 0), H - 1) * W + cx[k];
+            fx[k] = __ldg(fx_in + e);
+            fy[k] = __ldg(fy_in + e);
+        }
+    };
+
+    // matrices of rows y .. y + n - 1 (their flow loaded) into S, then their
+    // window sums along x into the ring from row `slot`
+    auto add_rows = [&](int y, int n, int slot) {
 #pragma unroll
-                for (int k = 0; k < 16; k++) w[k] = Sc[r * SP + q + k];
+        for (int k0 = 0; k0 < FL_PX; k0 += 3) {
+            float o[3][5];
+#pragma unroll
+            for (int u = 0; u < 3 && k0 + u < FL_PX; u++) {
+                const int k = k0 + u;
+                fl_matrix<THIN>(sA, sB, dA, dB, W, H, cx[k], min(max(y + (pr_[k] >> 16), 0), H - 1), fx[k], fy[k], o[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 3 && k0 + u < FL_PX; u++) {
+                const int k = k0 + u, gy = y + (pr_[k] >> 16);
+                if (pr_[k] < 0) continue;
+                const bool keep = (keepx >> k) & 1u && gy >= 0 && gy < H;
+#pragma unroll
+                for (int c = 0; c < 5; c++) S[c * FL_RS * FL_SP + (pr_[k] & 0xffff)] = keep ? o[u][c] : 0.f;
+            }
+        }
+        __syncthreads();
+        const int r = t >> 4, q = t & 15;                                // row, window group (four windows)
+        if (r < n) {
+            const float *Sr = S + r * FL_SP + 5 * q;
+            int d = slot + r;
+            d = d >= FL_RING ? d - FL_RING : d;
+            float4 *Td = (float4 *)(T + d * FL_TW) + q;
+#pragma unroll
+            for (int c = 0; c < 4; c += 2) {
+                float2 w[16];
+#pragma unroll
+                for (int k = 0; k < 16; k++)
+                    w[k] = make_float2(Sr[c * FL_RS * FL_SP + k + (k >> 2)], Sr[(c + 1) * FL_RS * FL_SP + k + (k >> 2)]);
+                float2 v[4];
 #pragma unroll
                 for (int m = 0; m < 4; m++) {
-                    float v = 0.f;
+                    v[m] = make_float2(0.f, 0.f);
 #pragma unroll
-                    for (int k = 0; k <= 2 * FL_BOX; k++) v += w[m + k];
-                    T[r * TP + q + m] = v;
+                    for (int k = 0; k <= 2 * FL_BOX; k++) v[m] = __fadd2_rn(v[m], w[m + k]);
                 }
+                Td[c * FL_RING * FL_TW / 4] = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+                Td[(c + 1) * FL_RING * FL_TW / 4] = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
             }
-        __syncthreads();
+            float w[16], v[4];
 #pragma unroll
-        for (int a = 0; a < TW / 32; a++) {
-            const int q = tx + 32 * a;
-            float w[RPT + 2 * FL_BOX];
+            for (int k = 0; k < 16; k++) w[k] = Sr[4 * FL_RS * FL_SP + k + (k >> 2)];
 #pragma unroll
-            for (int k = 0; k < RPT + 2 * FL_BOX; k++) w[k] = T[(RPT * ty + k) * TP + q];
+            for (int m = 0; m < 4; m++) {
+                v[m] = 0.f;
 #pragma unroll
-            for (int j = 0; j < RPT; j++) {
-                float v = 0.f;
-#pragma unroll
-                for (int k = 0; k <= 2 * FL_BOX; k++) v += w[j + k];
-                acc[a][j][c] = v;
+                for (int k = 0; k <= 2 * FL_BOX; k++) v[m] += w[m + k];
             }
+            Td[4 * FL_RING * FL_TW / 4] = make_float4(v[0], v[1], v[2], v[3]);
         }
         __syncthreads();
-    }
+    };
+
+    load_flow(yb - FL_BOX);
+    add_rows(yb - FL_BOX, FL_RS, 0);                                     // the first twelve rows
+    load_flow(yb - FL_BOX + FL_RS);
+    add_rows(yb - FL_BOX + FL_RS, 2 * FL_BOX - FL_RS, FL_RS);
+    load_flow(yb + FL_BOX);
+    int slot = 2 * FL_BOX;                                               // ring row of the next rows
+    const int col = t & (FL_TW - 1), h = t / FL_TW;                      // column, half of the eight rows
+    for (int y = yb; y < ye; y += FL_RS) {
+        add_rows(y + FL_BOX, FL_RS, slot);
+        slot += FL_RS;
+        slot = slot >= FL_RING ? slot - FL_RING : slot;                  // now the ring row of y - 6
+        load_flow(y + FL_RS + FL_BOX);                                   // (clamped into the frame past the strip)
+        const float *g[4];                                               // ring rows of y - 6 + 4 h + 0, 4, 8, 12
 #pragma unroll
-    for (int a = 0; a < TW / 32; a++)
+        for (int k = 0; k < 4; k++) {
+            int d = slot + 4 * (h + k);
+            d = d >= FL_RING ? d - FL_RING : d;
+            g[k] = T + d * FL_TW + col;
+        }
+        float acc[5][4];
 #pragma unroll
-        for (int j = 0; j < RPT; j++) {
-            const int x = x0 + tx + 32 * a, y = y0 + RPT * ty + j;
-            if (x >= W || y >= H) continue;
-            const float g11 = acc[a][j][0], g12 = acc[a][j][1], g22 = acc[a][j][2];
-            const float h1 = acc[a][j][3], h2 = acc[a][j][4];
+        for (int c = 0; c < 4; c += 2) {
+            float2 w[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const float *e = g[k >> 2] + (k & 3) * FL_TW;
+                w[k] = make_float2(e[c * FL_RING * FL_TW], e[(c + 1) * FL_RING * FL_TW]);
+            }
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int k = 0; k <= 2 * FL_BOX; k++) v = __fadd2_rn(v, w[m + k]);
+                acc[c][m] = v.x;
+                acc[c + 1][m] = v.y;
+            }
+        }
+        {
+            float w[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) w[k] = g[k >> 2][4 * FL_RING * FL_TW + (k & 3) * FL_TW];
+#pragma unroll
+            for (int m = 0; m < 4; m++) {
+                float v = 0.f;
+#pragma unroll
+                for (int k = 0; k <= 2 * FL_BOX; k++) v += w[m + k];
+                acc[4][m] = v;
+            }
+        }
+        const int x = x0 + col;
+#pragma unroll
+        for (int m = 0; m < 4; m++) {
+            const int yy = y + 4 * h + m;
+            if (x >= W || yy >= ye) continue;
+            const float g11 = acc[0][m], g12 = acc[1][m], g22 = acc[2][m], h1 = acc[3][m], h2 = acc[4][m];
             const float idet = 1.f / (g11 * g22 - g12 * g12 + 1e-3f);
-            const long long e = fr * pr + (long long)y * W + x;
+            const long long e = fr * pr + (long long)yy * W + x;
             fout[e] = (g22 * h1 - g12 * h2) * idet;
             fout[mplane + e] = (g11 * h2 - g12 * h1) * idet;
         }
+    }
 }
 
-#define FL_TW 64
-#define FL_TH 32
-#define FL_NT 512
-static constexpr size_t fl_iter_smem(int tw, int th)
+// Rows of a strip per block: a multiple of the eight of a step such that the
+// blocks' rounds on the GPU take least, a block costing its rows, the twelve
+// before them and about as much as four more to start
+static int fl_rows(int W, int H, int P, int resident)
 {
-    return sizeof(float) * (size_t)(5 * (th + 2 * FL_BOX) * (tw + 2 * FL_BOX + 1) + (th + 2 * FL_BOX) * (tw + 1));
+    const long long columns = (long long)((W + FL_TW - 1) / FL_TW) * P;
+    int best = FL_RS;
+    long long least = 0;
+    for (int r = FL_RS; r <= ((H + FL_RS - 1) / FL_RS) * FL_RS; r += FL_RS) {
+        const long long blocks = columns * ((H + r - 1) / r);
+        const long long cost = (blocks + resident - 1) / resident * (r + 2 * FL_BOX + 4);
+        if (!least || cost < least) { least = cost; best = r; }
+    }
+    return best;
 }
 
-// flow of level k from level k+1: bilinear, scaled by the size ratio
-__global__ void k_fl_up(const float *__restrict__ coarse, int Wc, int Hc, float *__restrict__ fine, int W, int H,
-                        int P)
+// flow of level k from level k+1: bilinear, scaled by the size ratio; a block
+// per 256 columns, eight rows and pair (one thread per pixel of a flat index,
+// with its 64-bit divisions: 68 us for the 640x480 level of 30 pairs, 39 us now)
+#define FL_UP_ROWS 8
+__global__ void __launch_bounds__(FL_T) k_fl_up(const float *__restrict__ coarse, int Wc, int Hc, float *__restrict__ fine,
+                                                int W, int H, int P)
 {
-    const long long fr = (long long)W * H, mplane = fr * P, cfr = (long long)Wc * Hc, cplane = cfr * P;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= mplane) return;
-    const int pr = (int)(t / fr);
-    const int pix = (int)(t - pr * fr), y = pix / W, x = pix - y * W;
+    const int x = blockIdx.x * FL_T + threadIdx.x, pr = blockIdx.z;
+    if (x >= W) return;
+    const long long mplane = (long long)W * H * P, cplane = (long long)Wc * Hc * P;
+    const float *F = coarse + (long long)Wc * Hc * pr;
+    float *out = fine + (long long)W * H * pr + x;
     const float sx = (float)Wc / (float)W, sy = (float)Hc / (float)H;
     const float cx = fminf(fmaxf(((float)x + 0.5f) * sx - 0.5f, 0.f), (float)(Wc - 1));
-    const float cy = fminf(fmaxf(((float)y + 0.5f) * sy - 0.5f, 0.f), (float)(Hc - 1));
-    const int x0 = (int)cx, y0 = (int)cy, x1 = min(x0 + 1, Wc - 1), y1 = min(y0 + 1, Hc - 1);
-    const float fx = cx - (float)x0, fy = cy - (float)y0;
-    const long long b = cfr * pr;
-    for (int c = 0; c < 2; c++) {
-        const float *F = coarse + c * cplane + b;
-        const float v = (1.f - fx) * (1.f - fy) * F[(long long)y0 * Wc + x0] + fx * (1.f - fy) * F[(long long)y0 * Wc + x1] +
-                        (1.f - fx) * fy * F[(long long)y1 * Wc + x0] + fx * fy * F[(long long)y1 * Wc + x1];
-        fine[c * mplane + t] = v / (c == 0 ? sx : sy);
+    const int x0 = (int)cx, x1 = min(x0 + 1, Wc - 1);
+    const float fx = cx - (float)x0;
+    const int ye = min((int)(blockIdx.y + 1) * FL_UP_ROWS, H);
+    for (int y = blockIdx.y * FL_UP_ROWS; y < ye; y++) {
+        const float cy = fminf(fmaxf(((float)y + 0.5f) * sy - 0.5f, 0.f), (float)(Hc - 1));
+        const int y0 = (int)cy, y1 = min(y0 + 1, Hc - 1);
+        const float fy = cy - (float)y0;
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float *G = F + c * cplane;
+            const float v = (1.f - fx) * (1.f - fy) * G[y0 * Wc + x0] + fx * (1.f - fy) * G[y0 * Wc + x1] +
+                            (1.f - fx) * fy * G[y1 * Wc + x0] + fx * fy * G[y1 * Wc + x1];
+            out[c * mplane + y * W] = v / (c == 0 ? sx : sy);
+        }
     }
 }
 
@@ -441,9 +542,9 @@ int asv_launch_flow(const uint8_t *rgb, int W, int H, int D, float2 *fwd, float2
     }
     const size_t fr0 = (size_t)W * H;
     float *alt = fl_carve(p, fr0 * P * 2);
-    const size_t smem = fl_iter_smem(FL_TW, FL_TH);
-    if (cudaFuncSetAttribute(k_fl_iter<FL_TW, FL_TH, FL_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    int dev = 0, sms = 1, per = 1;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fl_iter<false>, FL_NT, FL_SMEM) != cudaSuccess)
         return -1;
 
     k_fl_gray<<<fl_blocks((long long)fr0 * D), FL_T, 0, st>>>(rgb, img[0], (long long)fr0 * D);
@@ -459,12 +560,18 @@ int asv_launch_flow(const uint8_t *rgb, int W, int H, int D, float2 *fwd, float2
         const int w = Ws[k], h = Hs[k];
         const long long mplane = (long long)w * h * P;
         if (k == L - 1) cudaMemsetAsync(flow[k], 0, sizeof(float) * mplane * 2, st);
-        else k_fl_up<<<fl_blocks(mplane), FL_T, 0, st>>>(flow[k + 1], Ws[k + 1], Hs[k + 1], flow[k], w, h, P);
-        const unsigned tiles = (unsigned)(((w + FL_TW - 1) / FL_TW) * ((h + FL_TH - 1) / FL_TH) * P);
+        else
+            k_fl_up<<<dim3((w + FL_T - 1) / FL_T, (h + FL_UP_ROWS - 1) / FL_UP_ROWS, P), FL_T, 0, st>>>(
+                flow[k + 1], Ws[k + 1], Hs[k + 1], flow[k], w, h, P);
+        const int rows = fl_rows(w, h, P, sms * (per > 0 ? per : 1));
+        const unsigned blocks = (unsigned)((w + FL_TW - 1) / FL_TW) * ((h + rows - 1) / rows) * P;
         for (int it = 0; it < 10; it++) {                 // even count: the result ends in flow[k]
             const float *fin = (it & 1) ? alt : flow[k];
             float *fout = (it & 1) ? flow[k] : alt;
-            k_fl_iter<FL_TW, FL_TH, FL_NT><<<tiles, FL_NT, smem, st>>>(polyA[k], polyB[k], fin, fout, w, h, D, P);
+            if (w > 1 && h > 1)
+                k_fl_iter<false><<<blocks, FL_NT, FL_SMEM, st>>>(polyA[k], polyB[k], fin, fout, w, h, D, P, rows);
+            else
+                k_fl_iter<true><<<blocks, FL_NT, FL_SMEM, st>>>(polyA[k], polyB[k], fin, fout, w, h, D, P, rows);
         }
     }
     k_fl_store<<<fl_blocks((long long)fr0 * D), FL_T, 0, st>>>(flow[0], W, H, D, fwd, bwd, keep_first_bwd);
