@@ -216,12 +216,19 @@ struct asv_ctx {
     // connectivity enforcement scratch (asv_enforce_connectivity*), grown on demand
     void *cc = nullptr;
     size_t cc_bytes = 0;
+    // evaluation scratch (asv_evaluate): volumes, counts; grown on demand, kept up
+    // to EV_KEEP bytes, given back when another allocation of the context fails
+    void *evs[2] = { nullptr, nullptr };
+    size_t evs_bytes[2] = { 0, 0 };
     // optical-flow scratch (asv_compute_flow), grown on demand
     void *fl = nullptr;
     size_t fl_bytes = 0;
 };
 
-size_t asv::ctx_bytes(const asv_ctx *c) { return c ? c->bytes + c->cc_bytes + c->fl_bytes : 0; }
+size_t asv::ctx_bytes(const asv_ctx *c)
+{
+    return c ? c->bytes + c->cc_bytes + c->fl_bytes + c->evs_bytes[0] + c->evs_bytes[1] : 0;
+}
 
 void asv::set_stream(asv_ctx *c, cudaStream_t st)
 {
@@ -263,11 +270,29 @@ static int jfa_blocks_for(const asv_ctx *ctx, int tiles)
 // other contexts sharing the GPU (the server's slots) keep running.  The
 // context's stream changes only after a synchronize (asv::set_stream), so a
 // buffer is always allocated, used and freed in stream order.
-static cudaError_t ctx_malloc(asv_ctx *ctx, void **p, size_t b) { return cudaMallocAsync(p, b, ctx->st); }
-
 static void ctx_free(asv_ctx *ctx, void *p)
 {
     if (p) cudaFreeAsync(p, ctx->st);
+}
+
+static void free_eval(asv_ctx *ctx)
+{
+    for (int k = 0; k < 2; k++) {
+        ctx_free(ctx, ctx->evs[k]);
+        ctx->evs[k] = nullptr;
+        ctx->evs_bytes[k] = 0;
+    }
+}
+
+static cudaError_t ctx_malloc(asv_ctx *ctx, void **p, size_t b)
+{
+    cudaError_t e = cudaMallocAsync(p, b, ctx->st);
+    if (e != cudaSuccess && (ctx->evs[0] || ctx->evs[1])) {    // the evaluation's scratch is only kept for speed
+        cudaGetLastError();
+        free_eval(ctx);
+        e = cudaMallocAsync(p, b, ctx->st);
+    }
+    return e;
 }
 
 static void free_layout(asv_ctx *ctx)
@@ -727,20 +752,30 @@ static asv_status read_post(asv_ctx *ctx)
 // ---------------------------------------------------------------------------
 // C ABI
 // ---------------------------------------------------------------------------
-// device buffers of one evaluation, stream-ordered on the context's stream
-// and freed on return
-struct EvalBuffers {
-    asv_ctx *ctx;
-    std::vector<void *> p;
-    explicit EvalBuffers(asv_ctx *c) : ctx(c) {}
-    ~EvalBuffers() { for (void *q : p) ctx_free(ctx, q); }
-    template <typename T> cudaError_t get(T **out, size_t n)
-    {
-        void *q = nullptr;
-        cudaError_t e = ctx_malloc(ctx, &q, std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) { p.push_back(q); *out = (T *)q; }
-        return e;
+// The evaluation's scratch of at least b bytes, kept by the context: the pool
+// gives its memory back at a synchronize, and taking it anew cost 0.32 ms of a
+// call on a 320x240x85 volume
+#define EV_KEEP (256ull << 20)
+static cudaError_t eval_scratch(asv_ctx *ctx, int k, size_t b)
+{
+    if (ctx->evs_bytes[k] >= b) return cudaSuccess;
+    ctx_free(ctx, ctx->evs[k]);
+    ctx->evs[k] = nullptr;
+    ctx->evs_bytes[k] = 0;
+    void *p = nullptr;
+    cudaError_t e = cudaMallocAsync(&p, b, ctx->st);
+    if (e != cudaSuccess && k == 0 && ctx->evs[1]) {   // the counts of the call before may go
+        cudaGetLastError();
+        free_eval(ctx);
+        e = cudaMallocAsync(&p, b, ctx->st);
     }
+    if (e == cudaSuccess) { ctx->evs[k] = p; ctx->evs_bytes[k] = b; }
+    return e;
+}
+
+struct EvalRelease {                                   // large scratch goes back at the end of the call
+    asv_ctx *ctx;
+    ~EvalRelease() { if (ctx->evs_bytes[0] + ctx->evs_bytes[1] > EV_KEEP) free_eval(ctx); }
 };
 
 extern "C" {
@@ -806,6 +841,7 @@ asv_status asv_destroy(asv_ctx *ctx)
     free_layout(ctx);
     ctx_free(ctx, ctx->cc);
     ctx_free(ctx, ctx->fl);
+    free_eval(ctx);
     cudaStreamSynchronize(ctx->st);
     for (auto e : ctx->ev) cudaEventDestroy(e);
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
@@ -1226,40 +1262,50 @@ asv_status asv_evaluate(asv_ctx *ctx, const int32_t *labels, const int32_t *trut
     cudaSetDevice(ctx->cfg.device);
     const long long n = (long long)W * H * D;
     cudaStream_t st = ctx->st;
-    EvalBuffers b(ctx);
-    int32_t *lab, *gt;
-    int *meta;
-    if (b.get(&lab, n) != cudaSuccess || b.get(&gt, n) != cudaSuccess || b.get(&meta, 4) != cudaSuccess) {
+    EvalRelease release{ ctx };
+    const size_t vol = (sizeof(int32_t) * (size_t)n + 255) & ~(size_t)255, words = asv_eval_sbound_words(W, H, D);
+    if (eval_scratch(ctx, 0, 2 * vol + 256 + 4 * words) != cudaSuccess) {
         cudaGetLastError();
         return fail(ctx, ASV_ERR_OOM, "cudaMallocAsync: evaluation buffers");
     }
-    CK(cudaMemcpyAsync(lab, labels, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(gt, truth, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st));
+    int32_t *lab = (int32_t *)ctx->evs[0], *gt = (int32_t *)((char *)ctx->evs[0] + vol);
+    int *meta = (int *)((char *)ctx->evs[0] + 2 * vol);
+    unsigned *sb = (unsigned *)((char *)ctx->evs[0] + 2 * vol + 256);
+    // the truth is copied beside the labels and their boundary flags
+    CK(cudaEventRecord(ctx->side_ev[0], st));
+    CK(cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
+    cudaError_t ce = cudaMemcpyAsync(lab, labels, sizeof(int32_t) * n, cudaMemcpyHostToDevice, st);
+    int le = asv_launch_eval_sbound(lab, W, H, D, sb, st);
+    if (ce == cudaSuccess) ce = cudaMemcpyAsync(gt, truth, sizeof(int32_t) * n, cudaMemcpyHostToDevice, ctx->side);
+    cudaEventRecord(ctx->side_ev[1], ctx->side);       // joined whatever failed: the buffers outlive the copy
+    cudaStreamWaitEvent(st, ctx->side_ev[1], 0);
+    CK(ce);
     int hm[3];
-    if (asv_launch_eval_range(lab, gt, n, meta, st) != 0) return cuda_fail(ctx, cudaGetLastError(), "eval range");
+    if (le == 0) le = asv_launch_eval_range_init(meta, st);
+    if (le == 0) le = asv_launch_eval_range(lab, gt, n, meta, st);
+    if (le != 0) return cuda_fail(ctx, cudaGetLastError(), "eval range");
     CK(cudaMemcpyAsync(hm, meta, sizeof(hm), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     if (hm[2]) return fail(ctx, ASV_ERR_BAD_ARG, "labels must lie in [-1, 32767) and truth ids in [0, 4096)");
     const int rows = hm[0] + 2, NG = hm[1] + 1;
-    unsigned *cnt;
-    int *zmin, *zmax;
-    uint8_t *sb;
-    unsigned long long *tot;
-    if (b.get(&cnt, (size_t)rows * NG) != cudaSuccess || b.get(&zmin, rows) != cudaSuccess ||
-        b.get(&zmax, rows) != cudaSuccess || b.get(&sb, n) != cudaSuccess || b.get(&tot, 2) != cudaSuccess) {
+    // totals, frame ranges and counts, in one block and one copy
+    const size_t o_z0 = 16, o_z1 = o_z0 + 4 * (size_t)rows, o_cnt = o_z1 + 4 * (size_t)rows;
+    const size_t total = o_cnt + sizeof(unsigned) * (size_t)rows * NG;
+    if (eval_scratch(ctx, 1, total) != cudaSuccess) {
         cudaGetLastError();
         return fail(ctx, ASV_ERR_OOM, "cudaMallocAsync: evaluation counts");
     }
-    if (asv_launch_eval(lab, gt, W, H, D, rows, NG, cnt, zmin, zmax, sb, tot, st) != 0)
+    char *q = (char *)ctx->evs[1];
+    if (asv_launch_eval(lab, gt, W, H, D, rows, NG, (unsigned *)(q + o_cnt), (int *)(q + o_z0), (int *)(q + o_z1), sb,
+                        (unsigned long long *)q, st) != 0)
         return cuda_fail(ctx, cudaGetLastError(), "evaluation kernels");
-    std::vector<unsigned> c((size_t)rows * NG);
-    std::vector<int> z0(rows), z1(rows);
-    unsigned long long t[2];
-    CK(cudaMemcpyAsync(c.data(), cnt, sizeof(unsigned) * c.size(), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(z0.data(), zmin, sizeof(int) * rows, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(z1.data(), zmax, sizeof(int) * rows, cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(t, tot, sizeof(t), cudaMemcpyDeviceToHost, st));
+    std::vector<unsigned long long> host((total + 7) / 8);
+    CK(cudaMemcpyAsync(host.data(), q, total, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
+    const unsigned long long *t = host.data();
+    const char *hb = (const char *)host.data();
+    const int *z0 = (const int *)(hb + o_z0), *z1 = (const int *)(hb + o_z1);
+    const unsigned *c = (const unsigned *)(hb + o_cnt);
     // sizes, argmax assignment, then the measures (sums in truth-id order)
     std::vector<long long> ssz(rows, 0), gsz(NG, 0), cover(NG, 0), under(NG, 0);
     std::vector<int> arg(rows, -1);
