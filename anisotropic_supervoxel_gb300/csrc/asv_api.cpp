@@ -153,7 +153,7 @@ struct asv_ctx {
     bool have_rgb = false, have_flow = false, have_pos0 = false, have_M0 = false, have_lab = false;
     bool seeded = false, ran = false;
     bool drawn = false;          // labA holds a fresh seed draw: the first pass may scatter
-    bool undraw = false;         // ... and nothing else: the second pass may take the seeds out instead of a fill
+    bool undraw = false;         // ... and nothing else: the first pass need not check the seeds' places
     // fills of the label volumes run beside the (latency-bound) metric solves
     // of the next seeds, on a stream of their own between two events
     cudaStream_t side = nullptr;
@@ -551,10 +551,9 @@ asv_status asv_build_layout(asv_ctx *ctx)
     AL(d.bwd, (size_t)vox);
     AL(d.labA, (size_t)vox);
     AL(d.labB, (size_t)vox);
-    AL(d.jkeys, (size_t)vox);
+    AL(d.drawn, (size_t)vox);
     AL(d.tlist, (size_t)seeds * 27);
     AL(d.tcount, 1);
-    CK(cudaMemsetAsync(d.jkeys, 0xff, sizeof(unsigned long long) * (size_t)vox, ctx->st));
     AL(d.pos0, seeds); AL(d.M0, (size_t)seeds * 8);
     AL(d.pos, seeds); AL(d.slab, seeds); AL(d.M, (size_t)seeds * 8);
     AL(d.jtab, (size_t)seeds * 3);
@@ -618,11 +617,23 @@ static asv_status ensure_events(asv_ctx *ctx, size_t n)
     return ASV_OK;
 }
 
+static size_t label_bytes(const asv_ctx *ctx) { return sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK; }
+
+// Outside the Lloyd loop the seeds are drawn into labA, which other calls may
+// change before the flood; the loop has a volume for them, so that the second
+// pass finds labA filled.
+static AsvDev step_dev(const asv_ctx *ctx)
+{
+    AsvDev d = ctx->d;
+    d.drawn = d.labA;
+    return d;
+}
+
 static void do_first_init(asv_ctx *ctx)
 {
     asv_launch_first_init(ctx->d, ctx->st);
-    cudaMemsetAsync(ctx->d.labA, 0xff, sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK, ctx->st);
-    asv_launch_draw(ctx->d, ctx->st);
+    cudaMemsetAsync(ctx->d.labA, 0xff, label_bytes(ctx), ctx->st);
+    asv_launch_draw(step_dev(ctx), ctx->st);
     ctx->drawn = ctx->undraw = true;
     ctx->launches += 2;
 }
@@ -653,20 +664,21 @@ static void do_pass(asv_ctx *ctx, int p)
 }
 
 // the JFA ladder; the last pass of each segment also forms its centroid sums
-// (prepared: the next seeds left labB at -1, the sums at zero and the first
-// pass's list empty)
-static void do_flood(asv_ctx *ctx, int evbase, bool prepared)
+// (loop: the seeds stand in d.drawn alone, the label volumes are -1, the sums
+// zero and the first pass's list empty)
+static void do_flood(asv_ctx *ctx, int evbase, bool loop)
 {
-    if (!prepared)
+    if (!loop)
         cudaMemsetAsync(ctx->d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)ctx->d.total_seeds, ctx->st);
     for (int p = 0; p < ctx->maxpass; p++) {
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p);
-        if (p == 0 && ctx->drawn) {
-            asv_launch_jfa_first(ctx->d, prepared, !ctx->undraw, ctx->st);   // step 1 from the drawn seeds
+        if (p == 0 && (loop || ctx->drawn)) {
+            asv_launch_jfa_first(loop ? ctx->d : step_dev(ctx), loop, !loop && !ctx->undraw, ctx->st);   // step 1 from the drawn seeds
             ctx->launches++;
-        } else if (p == 1 && ctx->drawn) {
-            asv_launch_jfa_second_scatter(ctx->d, ctx->undraw, ctx->st);   // from the first pass's sparse labels
-            ctx->launches += 2;
+        } else if (p == 1 && (loop || ctx->drawn)) {
+            if (!loop) cudaMemsetAsync(ctx->d.labA, 0xff, label_bytes(ctx), ctx->st);
+            asv_launch_jfa_second_scatter(ctx->d, loop, ctx->st);   // from the first pass's sparse labels
+            ctx->launches++;
         } else {
             do_pass(ctx, p);
         }
@@ -689,21 +701,50 @@ static void do_sums_from_labels(asv_ctx *ctx)
     ctx->launches++;
 }
 
-// The metric at the new seed positions and the redraw.  loop: inside the
-// Lloyd loop, where the positions are formed here too (k_finalize otherwise)
-// and the next flood finds labB filled, the sums zeroed and its list empty.
-static void do_next_seeds(asv_ctx *ctx, bool loop)
+// The metric at the new seed positions and the redraw
+static void do_next_seeds(asv_ctx *ctx)
 {
-    const size_t bytes = sizeof(int32_t) * (size_t)ctx->d.total_chunks * ASV_CHUNK;
-    cudaEventRecord(ctx->side_ev[0], ctx->st);
-    cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0);
-    cudaMemsetAsync(ctx->d.labA, 0xff, bytes, ctx->side);
-    if (loop) cudaMemsetAsync(ctx->d.labB, 0xff, bytes, ctx->side);
-    cudaEventRecord(ctx->side_ev[1], ctx->side);
-    asv_launch_next_seeds(ctx->d, loop, loop, ctx->st,
-                          [](void *c) { cudaStreamWaitEvent(((asv_ctx *)c)->st, ((asv_ctx *)c)->side_ev[1], 0); }, ctx);
+    cudaMemsetAsync(ctx->d.labA, 0xff, label_bytes(ctx), ctx->st);
+    asv_launch_next_seeds(step_dev(ctx), false, false, ctx->st);
     ctx->drawn = ctx->undraw = true;
     ctx->launches += 3;       // two metric kernels, the combination with the draw
+}
+
+// The loop's fills of the label volumes, beside the seeds' kernels, which are
+// latency-bound: between the two events of the side stream.  first: of the first
+// iteration, with the sums, the list and the drawn seeds' volume (the kernels of
+// an iteration leave those ready for the next one).
+static void loop_fills(asv_ctx *ctx, bool first)
+{
+    const AsvDev &d = ctx->d;
+    const size_t bytes = label_bytes(ctx);
+    cudaEventRecord(ctx->side_ev[0], ctx->st);
+    cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0);
+    if (first) {
+        cudaMemsetAsync(d.drawn, 0xff, bytes, ctx->side);
+        cudaMemsetAsync(d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)d.total_seeds, ctx->side);
+        cudaMemsetAsync(d.tcount, 0, sizeof(int), ctx->side);
+    }
+    cudaMemsetAsync(d.labB, 0xff, bytes, ctx->side);
+    cudaMemsetAsync(d.labA, 0xff, bytes, ctx->side);
+    cudaEventRecord(ctx->side_ev[1], ctx->side);
+}
+
+// The loop's seeds of iteration it, drawn into d.drawn: the initial ones, or
+// from the centroid sums with the metric at their positions
+static void loop_seeds(asv_ctx *ctx, int it)
+{
+    loop_fills(ctx, it == 1);
+    if (it == 1) {
+        asv_launch_first_init(ctx->d, ctx->st);
+        cudaStreamWaitEvent(ctx->st, ctx->side_ev[1], 0);
+        asv_launch_draw(ctx->d, ctx->st);
+        ctx->launches += 2;
+    } else {
+        asv_launch_next_seeds(ctx->d, true, true, ctx->st);
+        cudaStreamWaitEvent(ctx->st, ctx->side_ev[1], 0);
+        ctx->launches += 3;   // two metric kernels, the combination with the draw
+    }
 }
 
 static void do_post(asv_ctx *ctx)
@@ -718,10 +759,9 @@ static void enqueue_lloyd(asv_ctx *ctx, bool instrument)
 {
     const int I = ctx->cfg.lloyd_iters;
     const int per_it = 2 * ctx->maxpass;
-    do_first_init(ctx);
     for (int it = 1; it <= I; it++) {
-        if (it > 1) do_next_seeds(ctx, true);
-        do_flood(ctx, instrument ? (it - 1) * per_it : -1, it > 1);
+        loop_seeds(ctx, it);
+        do_flood(ctx, instrument ? (it - 1) * per_it : -1, true);
     }
     do_post(ctx);
 }
@@ -1045,7 +1085,7 @@ asv_status asv_ld_next_seeds_matrix(asv_ctx *ctx, int lloyd_iter)
     if (!ctx) return ASV_ERR_BAD_ARG;
     (void)lloyd_iter;
     if (!ctx->seeded) return fail(ctx, ASV_ERR_STATE, "no seeds drawn: call asv_ld_first_init first");
-    do_next_seeds(ctx, false);
+    do_next_seeds(ctx);
     CK(cudaGetLastError());
     return ASV_OK;
 }
@@ -1435,7 +1475,7 @@ asv_status asv_set_seeds(asv_ctx *ctx, const float *in, int Kp)
     CK(cudaMemcpyAsync(ctx->d.slab + off, c.data(), sizeof(float4) * Kp, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemcpyAsync(ctx->d.M + 8 * (size_t)off, m.data(), sizeof(float) * 8 * Kp, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaMemsetAsync(ctx->d.mkey + off, 0xff, sizeof(int) * Kp, ctx->st));   // drop the reseed memo
-    asv_launch_draw(ctx->d, ctx->st);   // packs the JFA table (the label write is ignored here)
+    asv_launch_draw(step_dev(ctx), ctx->st);   // packs the JFA table (the label write is ignored here)
     ctx->undraw = false;                // (but the seeds drawn before may stand elsewhere)
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->st));

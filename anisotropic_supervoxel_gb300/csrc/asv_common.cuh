@@ -88,7 +88,7 @@ struct AsvDev {
     uchar4 *lab;                 // L, a, b, 0
     float2 *fwd, *bwd;
     int32_t *labA, *labB;
-    unsigned long long *jkeys;   // first-pass scatter keys, one per voxel, all ~0 between passes
+    int32_t *drawn;              // the drawn seeds at their voxels, else -1 (loop: all -1 between its draws; else labA)
     unsigned long long *tlist;   // voxels labelled by the first pass: (segment << 32) | voxel, 27 per seed
     int *tcount;                 // entries of tlist
     float4 *pos0;                // initial seeds (density placement)
@@ -128,8 +128,7 @@ void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);
 void asv_launch_post(const AsvDev &d, cudaStream_t st);
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st);
-void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st, void (*before_draw)(void *),
-                           void *arg);
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st);
 int asv_jfa_grid_blocks(int total_tiles);
 int asv_jfa_resident_blocks();
 int asv_jfa_slots(int step);   // footprint slots a sub-tile of the step can hold, 0: no bit-set form

@@ -453,8 +453,8 @@ __device__ __forceinline__ void asv_metric_result(const AsvDev &d, int g, int ne
 }
 
 // Writes M0 (reseed 0) or M (reseed 1, and the memo) and empties the list of
-// non-PSD seeds.  draw: also draws the seed for the next flood (labA is all
-// -1) and empties the list of the first pass's voxels; clear: and zeroes the
+// non-PSD seeds.  draw: also draws the seed for the next flood (d.drawn is
+// all -1) and empties the list of the first pass's voxels; clear: and zeroes the
 // seed slot's centroid sums.
 __global__ void k_metric_combine(AsvDev d, int reseed, bool draw, bool clear)
 {
@@ -504,12 +504,9 @@ void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st)
 }
 
 // The next iteration's seeds: positions from the centroid sums (finalize),
-// metrics, draw.  before_draw(arg) is called when what follows needs labA all
-// -1 (the fills of another stream are awaited there).
-void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st, void (*before_draw)(void *),
-                           void *arg)
+// metrics, draw
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st)
 {
     metric_solves(d, finalize ? 2 : 1, st);
-    before_draw(arg);
     k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, 1, true, clear_sums);
 }

@@ -69,7 +69,7 @@ __device__ __forceinline__ void asv_draw_seed(const AsvDev &d, const SegDesc &S,
     if (!(p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f)) return;
     int x = (int)p.x, y = (int)p.y, z = (int)p.z;
     if (x >= S.W || y >= S.H || z >= S.D) return;
-    atomicMax(d.labA + S.vox_off + ((long long)z * S.H + y) * S.W + x, i);
+    atomicMax(d.drawn + S.vox_off + ((long long)z * S.H + y) * S.W + x, i);
 }
 
 #endif

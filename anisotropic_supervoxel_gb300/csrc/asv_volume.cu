@@ -1382,7 +1382,6 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
 // table was replaced after the draw, and only records that stand at their
 // seed's position count.
 // ---------------------------------------------------------------------------
-#define ASV_KEY_EMPTY 0xffffffffffffffffull
 
 __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 {
@@ -1397,7 +1396,7 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
         const SegDesc &S = d.segs[si];
         const float4 p = d.pos[g];
         const int W = S.W, H = S.H, D = S.D;
-        const int32_t *in = d.labA + S.vox_off;
+        const int32_t *in = d.drawn + S.vox_off;
         int sx = -1, sy = -1, sz = -1;
         if (i < S.Kp && p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f) { sx = (int)p.x; sy = (int)p.y; sz = (int)p.z; }   // as the draw
         const bool inside = sx >= 0 && sx < W && sy < H && sz < D;
@@ -1446,12 +1445,20 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 }
 
 // ---------------------------------------------------------------------------
-// The second pass (step s = steps[1]) as a scatter too: its input, the first
+// The second pass (step s = steps[1]) as a scatter: its input, the first
 // pass's output, is labelled only at the voxels listed in tlist.  A voxel v
 // sees the label at u through offset o when clamp(v + o*s) == u along every
 // axis; per axis those v form a range (one voxel inside the volume, up to
 // s + 1 next to an edge, where several offsets clamp onto u).  Each (u, o)
-// thread visits that box; ranks and keys as in the first pass.
+// thread visits that box and puts its label into the output, all -1 before, by
+// compare-and-swap.  Where a label stands already the two are compared by the
+// gather's rule: the least distance, and of equal ones the label met first in
+// the shader's order.  Blocks hold one offset of neighbouring entries, whose
+// voxels adjoin (an entry's 27 offsets side by side: 36 us a pass on the
+// 320x240x85 clip, so 25).  Before, 64-bit keys of distance, rank and label by
+// atomicMin and a kernel to take the labels out, 8 bytes more a voxel: 15
+// iterations of that clip took 9.22 ms, now 8.98, 4 of a 64x48x12 one 0.326, now
+// 0.302.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void asv_axis_sources(int u, int o, int s, int n, int &lo, int &hi)
 {
@@ -1465,71 +1472,72 @@ __device__ __forceinline__ void asv_axis_sources(int u, int o, int s, int n, int
     hi = min(hi, n - 1);                      // empty when lo > hi
 }
 
-// first rank, in the order `order`, of an offset o with clamp(v + o*s) == u
-__device__ __forceinline__ int asv_first_rank_step(int v, int u, int s, int n, const int order[3])
+// whether voxel (x, y, z) meets label a before label b among its candidates, in the
+// shader's order (slices z, z-s, z+s; rows and columns from - to +, clamped)
+__device__ __forceinline__ bool asv_met_before(const int32_t *__restrict__ in, int W, int H, int D, int x, int y, int z,
+                                               int s, int a, int b)
 {
+    const int xs[3] = { max(x - s, 0), x, min(x + s, W - 1) }, ys[3] = { max(y - s, 0), y, min(y + s, H - 1) };
+    const int zs[3] = { z, max(z - s, 0), min(z + s, D - 1) };
+    unsigned ma = 0, mb = 0;
 #pragma unroll
-    for (int r = 0; r < 3; r++)
-        if (min(max(v + order[r] * s, 0), n - 1) == u) return r;
-    return 3;    // not reached: v is one of u's sources
+    for (int k = 0; k < 27; k++) {
+        const int l = in[((long long)zs[k / 9] * H + ys[(k / 3) % 3]) * W + xs[k % 3]];
+        ma |= l == a ? 1u << k : 0u;
+        mb |= l == b ? 1u << k : 0u;
+    }
+    return __ffs(ma) < __ffs(mb);       // both are among them
 }
 
-// one voxel of an entry's box: its key into jkeys, or (TAKE) the least key's
-// label out of them
-template <bool TAKE>
-__device__ __forceinline__ void asv_second_voxel(const AsvDev &d, const SegDesc &S, int label, int ux, int uy, int uz,
-                                                 int x, int y, int z, int s)
+// label's claim on one voxel of an entry's box
+__device__ __forceinline__ void asv_second_voxel(const AsvDev &d, const SegDesc &S, int label, int x, int y, int z, int s)
 {
     const long long v = S.vox_off + ((long long)z * S.H + y) * S.W + x;
-    if (TAKE) {
-        const unsigned long long key = atomicExch(d.jkeys + v, ASV_KEY_EMPTY);
-        if (key != ASV_KEY_EMPTY) d.labA[v] = (int32_t)(key & 0x7fffu);
-        return;
-    }
-    const int xy_order[3] = { -1, 0, 1 }, z_order[3] = { 0, -1, 1 };
-    const int rank = asv_first_rank_step(z, uz, s, S.D, z_order) * 9 + asv_first_rank_step(y, uy, s, S.H, xy_order) * 3 +
-                     asv_first_rank_step(x, ux, s, S.W, xy_order);
     const uchar4 c = __ldg(d.lab + v);
-    const float dist = asv_jfa_dist(d.jtab + 3 * S.seed_off, label, make_float2((float)x + 0.5f, (float)y + 0.5f),
-                                    make_float2((float)z + 0.5f, (float)c.x), make_float2((float)c.y, (float)c.z),
-                                    S.ratio[1]);
+    const float2 vxy = make_float2((float)x + 0.5f, (float)y + 0.5f), vzl = make_float2((float)z + 0.5f, (float)c.x);
+    const float2 vab = make_float2((float)c.y, (float)c.z);
+    const float4 *tab = d.jtab + 3 * S.seed_off;
+    const float dist = asv_jfa_dist(tab, label, vxy, vzl, vab, S.ratio[1]);
     if (!(dist < 100000000.0f)) return;
-    const unsigned long long key = ((unsigned long long)__float_as_uint(dist) << 32) |
-                                   ((unsigned long long)rank << 16) | (unsigned long long)label;
-    atomicMin(d.jkeys + v, key);
+    int old = -1;
+    for (;;) {                          // the voxel's label only gets better: at most its 27 candidates
+        const int was = atomicCAS(d.labA + v, old, label);
+        if (was == old || was == label) return;
+        old = was;
+        const float od = asv_jfa_dist(tab, old, vxy, vzl, vab, S.ratio[1]);
+        if (od < dist) return;
+        if (od == dist && asv_met_before(d.labB + S.vox_off, S.W, S.H, S.D, x, y, z, s, old, label)) return;
+    }
 }
 
 // A thread per listed voxel and offset.  Inside the volume the box is one
 // voxel; next to an edge it has s + 1 to (s + 1)^3 (1728 at step 11), and one
 // thread alone made the kernel as long as its largest box (26 to 36 us): boxes
 // of more than one voxel are walked by the whole warp, one after another.
-// undraw: the threads of the scatter also take the drawn seeds out of labA
-// again, so that it is all -1 for the take without a fill (nothing else of
-// this kernel reads labA).
-template <bool TAKE>
+// undraw: the threads also take the drawn seeds out of their volume again, so
+// that it is all -1 for the next draw without a fill (the first pass has read it).
 __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (!TAKE && undraw && t < d.total_seeds) {
+    const unsigned group = blockIdx.x / 27;
+    const int o = (int)(blockIdx.x - 27 * group);              // one offset per block: neighbouring entries' targets
+    const long long e = (long long)group * 256 + threadIdx.x, t = (long long)blockIdx.x * 256 + threadIdx.x;   // adjoin
+    if (undraw && t < d.total_seeds) {
         int i;
         const SegDesc &S = d.segs[asv_seed_seg(d, (int)t, i)];
         const float4 p = d.pos[t];
         if (i < S.Kp && p.x >= 0.0f && p.y >= 0.0f && p.z >= 0.0f && (int)p.x < S.W && (int)p.y < S.H && (int)p.z < S.D)
-            d.labA[S.vox_off + ((long long)(int)p.z * S.H + (int)p.y) * S.W + (int)p.x] = -1;
+            d.drawn[S.vox_off + ((long long)(int)p.z * S.H + (int)p.y) * S.W + (int)p.x] = -1;
     }
-    const long long e = t / 27;
-    const int count = *d.tcount;
-    int si = 0, ux = 0, uy = 0, uz = 0, label = 0;
+    int si = 0, label = 0;
     int x0 = 0, y0 = 0, z0 = 0, nx = 0, ny = 0, nz = 0;
-    if (e < count) {
-        const int o = (int)(t - e * 27);
+    if (e < *d.tcount) {
         const unsigned long long ent = d.tlist[e];
         si = (int)(ent >> 32);
         const int ul = (int)(ent & 0xffffffffull);                 // segments hold < 2^31 voxels
         const SegDesc &S = d.segs[si];
         const int s = S.steps[1];
         const int row = ul / S.W;
-        ux = ul - row * S.W; uz = row / S.H; uy = row - uz * S.H;
+        const int ux = ul - row * S.W, uz = row / S.H, uy = row - uz * S.H;
         int x1, y1, z1;
         asv_axis_sources(ux, o % 3 - 1, s, S.W, x0, x1);
         asv_axis_sources(uy, (o / 3) % 3 - 1, s, S.H, y0, y1);
@@ -1537,9 +1545,9 @@ __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
         nx = x1 - x0 + 1; ny = y1 - y0 + 1; nz = z1 - z0 + 1;
         if (nx <= 0 || ny <= 0 || nz <= 0) nx = 0;
         else {
-            label = TAKE ? 0 : d.labB[S.vox_off + ul];
+            label = d.labB[S.vox_off + ul];
             if (nx * ny * nz == 1) {
-                asv_second_voxel<TAKE>(d, S, label, ux, uy, uz, x0, y0, z0, s);
+                asv_second_voxel(d, S, label, x0, y0, z0, s);
                 nx = 0;
             }
         }
@@ -1550,13 +1558,12 @@ __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
         const int from = __ffs(big) - 1;
         big &= big - 1;
         const int bsi = __shfl_sync(FULL, si, from), bl = __shfl_sync(FULL, label, from);
-        const int bux = __shfl_sync(FULL, ux, from), buy = __shfl_sync(FULL, uy, from), buz = __shfl_sync(FULL, uz, from);
         const int bx = __shfl_sync(FULL, x0, from), by = __shfl_sync(FULL, y0, from), bz = __shfl_sync(FULL, z0, from);
         const int bnx = __shfl_sync(FULL, nx, from), bny = __shfl_sync(FULL, ny, from), bnz = __shfl_sync(FULL, nz, from);
         const SegDesc &S = d.segs[bsi];
         for (int k = lane; k < bnx * bny * bnz; k += 32) {
             const int r = k / bnx;
-            asv_second_voxel<TAKE>(d, S, bl, bux, buy, buz, bx + k - r * bnx, by + r % bny, bz + r / bny, S.steps[1]);
+            asv_second_voxel(d, S, bl, bx + k - r * bnx, by + r % bny, bz + r / bny, S.steps[1]);
         }
     }
 }
@@ -2002,14 +2009,12 @@ void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t
     k_jfa_first<<<(27 * d.total_seeds + 255) / 256, 256, 0, st>>>(d, stale);
 }
 
-// undraw: labA holds nothing but the seeds at their current positions
+// into labA, which is all -1.  undraw: d.drawn holds nothing but the seeds at
+// their current positions, and becomes all -1 again
 void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st)
 {
-    if (!undraw) cudaMemsetAsync(d.labA, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
-    const long long threads = 27LL * 27LL * d.total_seeds;   // tlist holds <= 27 entries per seed
-    const int blocks = (int)((threads + 255) / 256);
-    k_jfa_second<false><<<blocks, 256, 0, st>>>(d, undraw);
-    k_jfa_second<true><<<blocks, 256, 0, st>>>(d, false);
+    const unsigned blocks = 27u * (unsigned)((27LL * d.total_seeds + 255) / 256);   // tlist holds <= 27 entries per seed
+    k_jfa_second<<<blocks, 256, 0, st>>>(d, undraw);
 }
 
 void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st)
