@@ -13,20 +13,25 @@
 // the PSD metrics of the 1-ring, then 2-ring neighbours, then to the nearest
 // PSD matrix.
 //
-// One warp per solve: lane i holds row i of the system; column dot products
-// are butterfly sums over the lanes (asv_lane_sum), which leave the same bits
-// on every lane, so all lanes apply the same rotations.
-// Launches: k_metric_self (a warp per seed: in a reseed first the seed's new
-// position, then its solve and PSD test; the non-PSD seeds are listed),
-// k_metric_ring (a warp per listed seed and neighbour) and k_metric_combine (a
-// thread per seed: the fallbacks, and the seed's draw where the next flood
-// follows).  A reseed solve is skipped when the seed's voxel is the one of its
-// previous reseed solve in this Lloyd run: the metric is a function of that
-// voxel and the flow only, so the stored result is the solve's result.
-// The chain is latency-bound (a few warps per SM, at most some sixty rotations
-// one after another), so its launches count: seven kernels before, with the
-// position, the PSD tests (twice) and the draw on their own and a ring warp
-// for every seed, took about 80 us of a Lloyd iteration on the 320x240x85 clip.
+// Sixteen lanes per solve: two per column of the system, with its even and odd
+// rows.  A sweep's rotations of different columns don't touch each other, and the
+// pair (p, q) only needs the pairs of p and q before it in the cyclic order, all
+// of which have a smaller p + q (6 more per sweep): so the pairs of equal p + q
+// modulo 6 rotate together, the last ones of a sweep beside the first of the next,
+// in 6 steps a sweep instead of 15, with the same bits.  In step c column i meets
+// column c - i (modulo 6): both fetch the other, form the same sums and angle, and
+// update themselves.
+// Launches: k_metric_self (in a reseed first the seed's new position, then its
+// solve and PSD test; the non-PSD seeds are listed), k_metric_ring (a solve per
+// listed seed and neighbour) and k_metric_combine (a thread per seed: the
+// fallbacks, and the seed's draw where the next flood follows).  A reseed solve is
+// skipped when the seed's voxel is the one of its previous reseed solve in this
+// Lloyd run: the metric is a function of that voxel and the flow only, so the
+// stored result is the solve's result.
+// The chain is latency-bound (a few warps per SM, up to some sixty rotations of
+// two square roots and three divisions): a warp per solve, a row per lane and one
+// pair after the other took 33 us for the seeds of the 320x240x85 clip and 54 us
+// for the rings of one with computed flow, now 19 and 35 us.
 // Compiled with -fmad=false.
 #include "asv_seed.cuh"
 
@@ -35,17 +40,25 @@
 #define SVD_SWEEPS 30
 #define FULL 0xffffffffu
 
-// Sum of a per-lane value over the warp as a butterfly: at each level a lane
-// adds its partner's partial sum (lane ^ 16, 8, 4, 2, 1) to its own.  Both
-// partners add the same two operands and IEEE addition commutes, so every
-// lane ends with the same bits: slot i takes t[i] + t[i + off] for
-// off = 16, 8, 4, 2, 1 over the 32 slots (rows 0..m-1, then +0), the order
-// the oracle restates.  Lanes at or beyond m hold +0 (their rows are zero).
-__device__ __forceinline__ float asv_lane_sum(float v)
+#define SVD_ROWS 9                  // rows of a lane: h, h + 2, ... of its column (h = lane & 1)
+
+// Sum over the 32 row slots (rows 0..17, then +0) of products t, of which this lane
+// holds slots h + 2k: slot i takes t[i] + t[i + off] for off = 16, 8, 4, 2, 1, the
+// order the oracle restates; the last addition is the neighbour lane's (IEEE
+// addition commutes, so both end with the same bits).
+__device__ __forceinline__ float asv_row_sum(const float t[SVD_ROWS])
 {
+    const float a0 = (t[0] + t[8]) + t[4], a1 = t[1] + t[5], a2 = t[2] + t[6], a3 = t[3] + t[7];
+    const float c = (a0 + a2) + (a1 + a3);
+    return c + __shfl_xor_sync(FULL, c, 1);
+}
+
+__device__ __forceinline__ float asv_row_dot(const float a[SVD_ROWS], const float b[SVD_ROWS])
+{
+    float t[SVD_ROWS];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v = v + __shfl_xor_sync(FULL, v, off);
-    return v;
+    for (int k = 0; k < SVD_ROWS; k++) t[k] = a[k] * b[k];
+    return asv_row_sum(t);
 }
 
 // |ga| <= FLT_EPSILON * sqrtf(q), the rotation test, mostly without the square
@@ -61,58 +74,63 @@ __device__ __forceinline__ bool asv_orthogonal(float ga, float q)
     return fabsf(ga) <= FLT_EPSILON * sqrtf(q);
 }
 
-// min-norm least squares in FP32; u = this lane's row (zero beyond m),
-// bl = its rhs.  Returns x[0..5] on every lane.
-__device__ void asv_lsq_minnorm_warp(int m, float u[6], float bl, float x[6])
+// Min-norm least squares in FP32 of m rows, two solves per warp.  Lane 2i + h of
+// a half: u = rows h, h + 2, ... of column i (zero beyond m, and for i = 6, 7), bl =
+// the right-hand side of those rows.  Returns x[0..5] on every lane.
+__device__ void asv_lsq_minnorm(int m, float u[SVD_ROWS], const float bl[SVD_ROWS], float x[6])
 {
-    const int lane = threadIdx.x & 31;
-    float v[6];
+    const int lane = threadIdx.x & 31, base = lane & 17, i = (lane >> 1) & 7;   // base: the half's lane of column 0, this h
+    float v[3];                                                // rows h, h + 2, h + 4 of column i of V
 #pragma unroll
-    for (int c = 0; c < 6; c++) v[c] = lane == c ? 1.0f : 0.0f;   // lane r < 6 holds row r of V
-    for (int sw = 0; sw < SVD_SWEEPS; sw++) {
-        int rot = 0;
+    for (int k = 0; k < 3; k++) v[k] = i == (lane & 1) + 2 * k ? 1.0f : 0.0f;
+    for (int sw = 0; sw <= SVD_SWEEPS; sw++) {                 // the last sweep's last pairs come in one more
+        bool any = false;
+        for (int c = 1; c <= 6; c++) {
+            int j = c - i;
+            j = j < 0 ? j + 6 : j;
+            if (i > 5) j = i;
+            const int src = base + 2 * j;
+            float o[SVD_ROWS], vo[3];
 #pragma unroll
-        for (int p = 0; p < 5; p++)
+            for (int k = 0; k < SVD_ROWS; k++) o[k] = __shfl_sync(FULL, u[k], src);
 #pragma unroll
-            for (int q = p + 1; q < 6; q++) {
-                const float al = asv_lane_sum(u[p] * u[p]);
-                const float be = asv_lane_sum(u[q] * u[q]);
-                const float ga = asv_lane_sum(u[p] * u[q]);
-                if (ga == 0.0f) continue;
-                if (asv_orthogonal(ga, al * be)) continue;
-                float zeta = (be - al) / (2.0f * ga);
-                float t = 1.0f / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
-                if (zeta < 0.0f) t = -t;
-                float c = 1.0f / sqrtf(1.0f + t * t);
-                float s = c * t;
-                float up = u[p], uq = u[q];
-                u[p] = c * up - s * uq;
-                u[q] = s * up + c * uq;
-                float vp = v[p], vq = v[q];
-                v[p] = c * vp - s * vq;
-                v[q] = s * vp + c * vq;
-                rot++;
-            }
-        if (!rot) break;
+            for (int k = 0; k < 3; k++) vo[k] = __shfl_sync(FULL, v[k], src);
+            const float own = asv_row_dot(u, u), ga = asv_row_dot(u, o);
+            const float other = __shfl_sync(FULL, own, src);
+            const bool now = i + j == c ? sw < SVD_SWEEPS : sw > 0;   // of this sweep, else of the one before
+            const bool rot = i != j && now && ga != 0.0f && !asv_orthogonal(ga, own * other);
+            any |= rot;
+            if (!rot) continue;
+            const bool first = i < j;                          // this column is p, the other q
+            const float zeta = ((first ? other : own) - (first ? own : other)) / (2.0f * ga);
+            float t = 1.0f / (fabsf(zeta) + sqrtf(1.0f + zeta * zeta));
+            if (zeta < 0.0f) t = -t;
+            const float cs = 1.0f / sqrtf(1.0f + t * t), sn = first ? -(cs * t) : cs * t;
+#pragma unroll
+            for (int k = 0; k < SVD_ROWS; k++) u[k] = cs * u[k] + sn * o[k];
+#pragma unroll
+            for (int k = 0; k < 3; k++) v[k] = cs * v[k] + sn * vo[k];
+        }
+        if (!__any_sync(FULL, any) && sw > 0) break;
     }
-    float sig[6], smax = 0.0f;
+    const float sig = sqrtf(asv_row_dot(u, u));
+    float smax = sig > 0.0f ? sig : 0.0f;
 #pragma unroll
-    for (int j = 0; j < 6; j++) {
-        sig[j] = sqrtf(asv_lane_sum(u[j] * u[j]));
-        if (sig[j] > smax) smax = sig[j];
-    }
+    for (int o = 2; o < 16; o <<= 1) smax = fmaxf(smax, __shfl_xor_sync(FULL, smax, o));
     float thr = smax * ((float)(m < 6 ? m : 6) * FLT_EPSILON);
     if (thr < FLT_MIN) thr = FLT_MIN;
-    float xr = 0.0f;   // lane r < 6 accumulates x[r]
+    const float ub = asv_row_dot(u, bl);
+    const bool keep = sig >= thr;
+    const float coef = (ub / sig) / sig;
+    float xr[3] = { 0.0f, 0.0f, 0.0f };                        // x[h], x[h + 2], x[h + 4]
 #pragma unroll
-    for (int j = 0; j < 6; j++) {
-        if (!(sig[j] >= thr)) continue;
-        float ub = asv_lane_sum(u[j] * bl);
-        float coef = (ub / sig[j]) / sig[j];
-        xr = xr + v[j] * coef;
+    for (int k = 0; k < 3; k++) {
+        const float term = keep ? v[k] * coef : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 6; j++) xr[k] = xr[k] + __shfl_sync(FULL, term, base + 2 * j);
     }
 #pragma unroll
-    for (int r = 0; r < 6; r++) x[r] = __shfl_sync(FULL, xr, r);
+    for (int r = 0; r < 6; r++) x[r] = __shfl_sync(FULL, xr[r >> 1], (lane & 16) + (r & 1));
 }
 
 // symmetric 3x3 eigen-decomposition, cyclic Jacobi
@@ -253,57 +271,59 @@ __device__ __forceinline__ float asv_round_half_up(float f)
     return (f - r >= 0.5f ? r + 1.0f : r) + 0.0f;
 }
 
-// matrix_slover (GPU-AS/Image.cpp:874-1009) for one warp; M valid on every
-// lane (its PSD test, :997-1006, is k_metric_psd).  Rows are numbered in the
+// matrix_slover (GPU-AS/Image.cpp:874-1009) by sixteen lanes; M valid on every
+// lane (its PSD test, :997-1006, is the caller's).  Rows are numbered in the
 // reference's order (neighbour y outer, x inner; forward row, then backward).
-__device__ void asv_metric_solve_warp(const float2 *__restrict__ fwd, const float2 *__restrict__ bwd,
-                                      int W, int H, int D, float sx, float sy, int frame, float M[6])
+// Both halves of a warp call it; with active false one has no rows.
+__device__ void asv_metric_solve(bool active, const float2 *__restrict__ fwd, const float2 *__restrict__ bwd, int W,
+                                 int H, int D, float sx, float sy, int frame, float M[6])
 {
-    const int lane = threadIdx.x & 31;
-    // rows: each in-bounds neighbour in order gives a forward row (unless
-    // the last frame) then a backward row (unless the first frame); lane r
-    // finds its row's neighbour and direction, so all flow reads issue at once
+    const int h = threadIdx.x & 1, col = (threadIdx.x >> 1) & 7;
+    // rows: each in-bounds neighbour in order gives a forward row (unless the last
+    // frame) then a backward row (unless the first frame): with both, this lane's
+    // rows are all forward or all backward ones, with one, every other neighbour's
     const bool hf = frame != D - 1, hb = frame != 0;     // D >= 2: at least one
-    const int per = (int)hf + (int)hb;
+    const bool both = hf && hb;
     unsigned inb = 0;
 #pragma unroll
     for (int k = 0; k < 9; k++) {
         const int nx = (int)sx + (k % 3 - 1), ny = (int)sy + (k / 3 - 1);
         if (nx >= 0 && nx < W && ny >= 0 && ny < H) inb |= 1u << k;
     }
-    const int m = per * __popc(inb);
-    float u[6] = { 0, 0, 0, 0, 0, 0 }, bl = 0.0f;
-    if (lane < m) {
-        const int j = per == 2 ? lane >> 1 : lane;
-        const bool back = per == 2 ? (lane & 1) != 0 : hb;
-        unsigned rest = inb;
-        for (int k = 0; k < j; k++) rest &= rest - 1;    // drop the j lower neighbours
-        const int id_b = __ffs(rest) - 1;
-        const int ox = id_b % 3 - 1, oy = id_b / 3 - 1;
-        const long long o = ((long long)frame * H + ((int)sy + oy)) * W + ((int)sx + ox);
-        const float2 f = __ldg((back ? bwd : fwd) + o);
-        if (!back) {
-            float dx = (float)ox + asv_round_half_up(f.x);
-            float dy = (float)oy + asv_round_half_up(f.y);
-            u[0] = dx * dx; u[1] = 2.0f * dx * dy;
-            u[2] = 2.0f * dx; u[3] = dy * dy;
-            u[4] = 2.0f * dy; u[5] = 1.0f;
-        } else {
-            float dx = asv_round_half_up(f.x) + (float)ox;
-            float dy = asv_round_half_up(f.y) + (float)oy;
-            u[0] = dx * dx; u[1] = 2.0f * dx * dy;
-            u[2] = -2.0f * dx; u[3] = dy * dy;
-            u[4] = -2.0f * dy; u[5] = 1.0f;
-        }
-        bl = (float)(ox * ox + oy * oy + 1);             // expected_b of :884: 3 2 3 / 2 1 2 / 3 2 3
+    if (!active) inb = 0;
+    const int m = (both ? 2 : 1) * __popc(inb);
+    const bool back = both ? h != 0 : hb;
+    const float2 *flow = back ? bwd : fwd;
+    unsigned rest = inb;
+    if (!both && h) rest &= rest - 1;
+    float u[SVD_ROWS], bl[SVD_ROWS];
+    float2 f[SVD_ROWS];
+    int at[SVD_ROWS];
+#pragma unroll
+    for (int k = 0; k < SVD_ROWS; k++) {
+        at[k] = __ffs(rest) - 1;
+        rest &= rest - 1;
+        if (!both) rest &= rest - 1;
+        f[k] = make_float2(0.0f, 0.0f);
+        if (at[k] >= 0)
+            f[k] = __ldg(flow + ((long long)frame * H + ((int)sy + at[k] / 3 - 1)) * W + ((int)sx + at[k] % 3 - 1));
     }
-    float x[6];
-    if (m == 0) {
-        for (int k = 0; k < 6; k++) x[k] = 0.0f;
-    } else {
-        asv_lsq_minnorm_warp(m, u, bl, x);
+#pragma unroll
+    for (int k = 0; k < SVD_ROWS; k++) {
+        const int ox = at[k] % 3 - 1, oy = at[k] / 3 - 1;
+        const float dx = asv_round_half_up(f[k].x) + (float)ox, dy = asv_round_half_up(f[k].y) + (float)oy;
+        const float sgn = back ? -2.0f : 2.0f;
+        float r = 0.0f;
+        if (col == 0) r = dx * dx;
+        if (col == 1) r = 2.0f * dx * dy;
+        if (col == 2) r = sgn * dx;
+        if (col == 3) r = dy * dy;
+        if (col == 4) r = sgn * dy;
+        if (col == 5) r = 1.0f;
+        u[k] = at[k] >= 0 ? r : 0.0f;
+        bl[k] = at[k] >= 0 ? (float)(ox * ox + oy * oy + 1) : 0.0f;   // expected_b of :884: 3 2 3 / 2 1 2 / 3 2 3
     }
-    for (int k = 0; k < 6; k++) M[k] = x[k];
+    asv_lsq_minnorm(m, u, bl, M);
 }
 
 // plain reseed flow-angle filter (GPU-AS/Image.cpp:1406-1409): accept iff
@@ -357,31 +377,35 @@ __device__ __forceinline__ int asv_seed_key(const SegDesc &S, float4 p)
 // 2 -> pos formed here from the centroid sums (asv_reseed).
 __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
 {
-    const int lane = threadIdx.x & 31;
+    const bool writer = (threadIdx.x & 15) == 0;
     SeedRef r;
-    if (!asv_seed_ref(d, (blockIdx.x * blockDim.x + threadIdx.x) >> 5, r)) return;   // warp-uniform
-    const SegDesc &S = d.segs[r.si];
-    float4 p;
-    if (reseed == 2) {
-        float q[3], c[3];
-        asv_reseed(d, S, r.i, q, c);                  // every lane the same
-        p = make_float4(q[0], q[1], q[2], (float)r.i);
-        if (lane == 0) {
-            d.pos[r.g] = p;
-            d.slab[r.g] = make_float4(c[0], c[1], c[2], 0.0f);
+    bool active = asv_seed_ref(d, (blockIdx.x * blockDim.x + threadIdx.x) >> 4, r);
+    if (!__any_sync(FULL, active)) return;
+    const SegDesc &S = d.segs[active ? r.si : 0];
+    float4 p = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (active) {
+        if (reseed == 2) {
+            float q[3], c[3];
+            asv_reseed(d, S, r.i, q, c);              // every lane of the half the same
+            p = make_float4(q[0], q[1], q[2], (float)r.i);
+            if (writer) {
+                d.pos[r.g] = p;
+                d.slab[r.g] = make_float4(c[0], c[1], c[2], 0.0f);
+            }
+        } else {
+            p = reseed ? d.pos[r.g] : d.pos0[r.g];
         }
-    } else {
-        p = reseed ? d.pos[r.g] : d.pos0[r.g];
+        if (reseed && d.mkey[r.g] == asv_seed_key(S, p)) {
+            if (writer) d.neg[r.g] = 2;
+            active = false;
+        }
     }
-    if (reseed && d.mkey[r.g] == asv_seed_key(S, p)) {
-        if (lane == 0) d.neg[r.g] = 2;
-        return;
-    }
+    if (!__any_sync(FULL, active)) return;
     float fx = floorf(p.x), fy = floorf(p.y);
     int frame = min(max((int)p.z, 0), S.D - 1);   // positions are inside; keep reads in bounds
     float M[6];
-    asv_metric_solve_warp(d.fwd + S.vox_off, d.bwd + S.vox_off, S.W, S.H, S.D, fx, fy, frame, M);
-    if (lane == 0) {
+    asv_metric_solve(active, d.fwd + S.vox_off, d.bwd + S.vox_off, S.W, S.H, S.D, fx, fy, frame, M);
+    if (active && writer) {
 #pragma unroll
         for (int e = 0; e < 6; e++) d.Mself[8 * r.g + e] = M[e];
         const int neg = asv_m6_negative_quick(M);
@@ -390,13 +414,15 @@ __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
     }
 }
 
-// a warp per listed seed and ring neighbour
+// a solve per listed seed and ring neighbour
 __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
 {
-    const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
-    const int tasks = *d.negcount * ASV_RING;
-    for (int task = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; task < tasks; task += warps) {
-        const int g = d.neglist[task / ASV_RING], t = task % ASV_RING;
+    const bool writer = (threadIdx.x & 15) == 0;
+    const int step = (gridDim.x * blockDim.x) >> 4, tasks = *d.negcount * ASV_RING;
+    for (int task0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; task0 < tasks; task0 += step) {
+        const int task = task0 + ((threadIdx.x >> 4) & 1);     // of this half
+        bool active = task < tasks;
+        const int g = d.neglist[active ? task / ASV_RING : 0], t = active ? task % ASV_RING : 0;
         SeedRef r;
         asv_seed_ref(d, g, r);
         int *ok = d.ringok + ASV_RING * g + t;
@@ -406,15 +432,16 @@ __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
         int frame = min(max((int)p.z, 0), S.D - 1);
         float nx = fx + (float)c_ringx[t], ny = fy + (float)c_ringy[t];
         const float2 *fwd = d.fwd + S.vox_off, *bwd = d.bwd + S.vox_off;
-        if (!(nx >= 0 && nx < S.W && ny >= 0 && ny < S.H) ||
-            (reseed && S.angle_filter &&
-             !asv_angle_ok(fwd, S.W, S.H, S.D, frame, (int)fx, (int)fy, (int)nx, (int)ny))) {
-            if (lane == 0) *ok = 0;
-            continue;
+        if (active && (!(nx >= 0 && nx < S.W && ny >= 0 && ny < S.H) ||
+                       (reseed && S.angle_filter &&
+                        !asv_angle_ok(fwd, S.W, S.H, S.D, frame, (int)fx, (int)fy, (int)nx, (int)ny)))) {
+            if (writer) *ok = 0;
+            active = false;
         }
+        if (!__any_sync(FULL, active)) continue;
         float M[6];
-        asv_metric_solve_warp(fwd, bwd, S.W, S.H, S.D, nx, ny, frame, M);
-        if (lane == 0) {
+        asv_metric_solve(active, fwd, bwd, S.W, S.H, S.D, nx, ny, frame, M);
+        if (active && writer) {
             float *dst = d.Mring + 8 * (ASV_RING * g + t);
 #pragma unroll
             for (int e = 0; e < 6; e++) dst[e] = M[e];
@@ -490,9 +517,9 @@ __global__ void k_metric_combine(AsvDev d, int reseed, bool draw, bool clear)
 
 static void metric_solves(const AsvDev &d, int reseed, cudaStream_t st)
 {
-    const long long warps = d.total_seeds, ring = warps * ASV_RING;
-    k_metric_self<<<(int)((warps * 32 + 127) / 128), 128, 0, st>>>(d, reseed);
-    const long long blocks = (ring + 3) / 4;
+    const long long solves = d.total_seeds, ring = solves * ASV_RING;             // 8 per block
+    k_metric_self<<<(int)((solves + 7) / 8), 128, 0, st>>>(d, reseed);
+    const long long blocks = (ring + 7) / 8;
     k_metric_ring<<<(int)(blocks < 1216 ? blocks : 1216), 128, 0, st>>>(d, reseed);   // 8 blocks per SM at most
 }
 
