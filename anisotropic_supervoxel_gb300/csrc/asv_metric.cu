@@ -461,17 +461,30 @@ __device__ __forceinline__ void asv_metric_result(const AsvDev &d, int g, int ne
         for (int e = 0; e < 6; e++) res[e] = self[e];
         done = true;
     }
-    for (int ring = 0; ring < 2 && !done; ring++) {
-        int t0 = ring == 0 ? 0 : 8, t1 = ring == 0 ? 8 : ASV_RING;
-        float sum[6] = { 0, 0, 0, 0, 0, 0 };
-        int n = 0;
-        for (int t = t0; t < t1; t++) {
-            if (!d.ringok[ASV_RING * g + t]) continue;
-            const float *m = d.Mring + 8 * (ASV_RING * g + t);
-            n++;
-            for (int e = 0; e < 6; e++) sum[e] = sum[e] + m[e];
-        }
-        if (n > 0) {
+    // eight neighbours at a time (the 1-ring, then the 2-ring's halves): their
+    // flags in two loads, their matrices side by side, summed in order
+    float sum[6] = { 0, 0, 0, 0, 0, 0 };
+    int n = 0;
+    for (int t0 = 0; t0 < ASV_RING && !done; t0 += 8) {
+        const int4 *fl = (const int4 *)(d.ringok + ASV_RING * g + t0);
+        const int4 f0 = fl[0], f1 = fl[1];
+        const int ok[8] = { f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w };
+        float m[8][6];
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+            if (ok[t]) {
+                const float *q = d.Mring + 8 * (ASV_RING * g + t0 + t);
+                const float4 a = *(const float4 *)q;
+                const float2 b = *(const float2 *)(q + 4);
+                m[t][0] = a.x; m[t][1] = a.y; m[t][2] = a.z; m[t][3] = a.w; m[t][4] = b.x; m[t][5] = b.y;
+            }
+#pragma unroll
+        for (int t = 0; t < 8; t++)
+            if (ok[t]) {
+                n++;
+                for (int e = 0; e < 6; e++) sum[e] = sum[e] + m[t][e];
+            }
+        if (t0 != 8 && n > 0) {                      // a whole ring
             for (int e = 0; e < 6; e++) res[e] = sum[e] / (float)n;
             done = true;
         }
