@@ -89,7 +89,7 @@ struct AsvDev {
     float2 *fwd, *bwd;
     int32_t *labA, *labB;
     int32_t *drawn;              // the drawn seeds at their voxels, else -1 (loop: all -1 between its draws; else labA)
-    unsigned long long *tlist;   // voxels labelled by the first pass: (segment << 32) | voxel, 27 per seed
+    int4 *tlist;                 // voxels labelled by the first pass: (segment, voxel, label, -), 27 per seed
     int *tcount;                 // entries of tlist
     float4 *pos0;                // initial seeds (density placement)
     float *M0;                   // initial metric, 8 floats / seed

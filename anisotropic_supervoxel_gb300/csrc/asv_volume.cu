@@ -1388,7 +1388,7 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int g = t / 27, o = t - g * 27;
     bool won = false;
-    int si = 0;
+    int si = 0, label = 0;
     long long vl = 0;
     if (g < d.total_seeds) {
         int i;
@@ -1432,6 +1432,7 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
                     if (dist < mind) { mind = dist; best = l[k]; }
                 }
             won = best == i;
+            label = i;
             if (won) d.labB[S.vox_off + vl] = i;
         }
     }
@@ -1441,7 +1442,7 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
     int at = 0;
     if (lane == __ffs(m) - 1) at = atomicAdd(d.tcount, __popc(m));
     at = __shfl_sync(FULL, at, __ffs(m) - 1);
-    if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = ((unsigned long long)si << 32) | (unsigned long long)vl;
+    if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = make_int4(si, (int)vl, label, 0);   // segments hold < 2^31 voxels
 }
 
 // ---------------------------------------------------------------------------
@@ -1455,10 +1456,11 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 // gather's rule: the least distance, and of equal ones the label met first in
 // the shader's order.  Blocks hold one offset of neighbouring entries, whose
 // voxels adjoin (an entry's 27 offsets side by side: 36 us a pass on the
-// 320x240x85 clip, so 25).  Before, 64-bit keys of distance, rank and label by
-// atomicMin and a kernel to take the labels out, 8 bytes more a voxel: 15
-// iterations of that clip took 9.22 ms, now 8.98, 4 of a 64x48x12 one 0.326, now
-// 0.302.
+// 320x240x85 clip, so 25; with the registers held to 64, four blocks per SM
+// instead of three, and the label in the list 22).  Before, 64-bit keys of
+// distance, rank and label by atomicMin and a kernel to take the labels out, 8
+// bytes more a voxel: 15 iterations of that clip took 9.22 ms, so 8.95, 4 of a
+// 64x48x12 one 0.326, so 0.302.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void asv_axis_sources(int u, int o, int s, int n, int &lo, int &hi)
 {
@@ -1477,14 +1479,18 @@ __device__ __forceinline__ void asv_axis_sources(int u, int o, int s, int n, int
 __device__ __forceinline__ bool asv_met_before(const int32_t *__restrict__ in, int W, int H, int D, int x, int y, int z,
                                                int s, int a, int b)
 {
-    const int xs[3] = { max(x - s, 0), x, min(x + s, W - 1) }, ys[3] = { max(y - s, 0), y, min(y + s, H - 1) };
-    const int zs[3] = { z, max(z - s, 0), min(z + s, D - 1) };
     unsigned ma = 0, mb = 0;
-#pragma unroll
-    for (int k = 0; k < 27; k++) {
-        const int l = in[((long long)zs[k / 9] * H + ys[(k / 3) % 3]) * W + xs[k % 3]];
-        ma |= l == a ? 1u << k : 0u;
-        mb |= l == b ? 1u << k : 0u;
+#pragma unroll 1
+    for (int i = 0; i < 3; i++) {
+        const int zz = i == 0 ? z : (i == 1 ? max(z - s, 0) : min(z + s, D - 1));
+#pragma unroll 1
+        for (int j = 0; j < 3; j++) {
+            const int yy = j == 0 ? max(y - s, 0) : (j == 1 ? y : min(y + s, H - 1)), k = 9 * i + 3 * j;
+            const int32_t *row = in + ((long long)zz * H + yy) * W;
+            const int l0 = row[max(x - s, 0)], l1 = row[x], l2 = row[min(x + s, W - 1)];
+            ma |= (l0 == a ? 1u << k : 0u) | (l1 == a ? 2u << k : 0u) | (l2 == a ? 4u << k : 0u);
+            mb |= (l0 == b ? 1u << k : 0u) | (l1 == b ? 2u << k : 0u) | (l2 == b ? 4u << k : 0u);
+        }
     }
     return __ffs(ma) < __ffs(mb);       // both are among them
 }
@@ -1516,7 +1522,7 @@ __device__ __forceinline__ void asv_second_voxel(const AsvDev &d, const SegDesc 
 // of more than one voxel are walked by the whole warp, one after another.
 // undraw: the threads also take the drawn seeds out of their volume again, so
 // that it is all -1 for the next draw without a fill (the first pass has read it).
-__global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
+__global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
 {
     const unsigned group = blockIdx.x / 27;
     const int o = (int)(blockIdx.x - 27 * group);              // one offset per block: neighbouring entries' targets
@@ -1530,10 +1536,10 @@ __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
     }
     int si = 0, label = 0;
     int x0 = 0, y0 = 0, z0 = 0, nx = 0, ny = 0, nz = 0;
+    const int4 ent = e < 27LL * d.total_seeds ? d.tlist[e] : make_int4(0, 0, 0, 0);   // asked for beside their number
     if (e < *d.tcount) {
-        const unsigned long long ent = d.tlist[e];
-        si = (int)(ent >> 32);
-        const int ul = (int)(ent & 0xffffffffull);                 // segments hold < 2^31 voxels
+        si = ent.x;
+        const int ul = ent.y;
         const SegDesc &S = d.segs[si];
         const int s = S.steps[1];
         const int row = ul / S.W;
@@ -1545,7 +1551,7 @@ __global__ void __launch_bounds__(256) k_jfa_second(AsvDev d, bool undraw)
         nx = x1 - x0 + 1; ny = y1 - y0 + 1; nz = z1 - z0 + 1;
         if (nx <= 0 || ny <= 0 || nz <= 0) nx = 0;
         else {
-            label = d.labB[S.vox_off + ul];
+            label = ent.z;
             if (nx * ny * nz == 1) {
                 asv_second_voxel(d, S, label, x0, y0, z0, s);
                 nx = 0;
