@@ -363,11 +363,11 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
         seeds += (size_t)((s.Kp + 64 + 31) / 32) * 32;
         cells += s.W + s.H + s.D + 2 * s.g.wNum;
     }
-    // rgb 3 + lab 4 + fwd/bwd 16 + two label buffers 8 + first-pass keys 8
-    size_t per_vox = 3 + 4 + 8 + 8 + 4 + 4 + 8;
+    // rgb 3 + lab 4 + fwd/bwd 16 + two label buffers 8 + drawn seeds 4
+    size_t per_vox = 3 + 4 + 8 + 8 + 4 + 4 + 4;
     // float4 pos0/pos/slab/grid, 8-float M0/M/Mself/Mmemo, jtab 3 float4, 8 u64
     // sums, int neg/mkey/rank/neglist, u64 dacc, the metric ring
-    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 4 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 8;
+    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 4 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 16;
     // each of the ~30 allocations rounds up to 256 bytes
     size_t fixed = 32 * 256 + 256 * 4 + 16;
     fixed += sizeof(SegDesc);
