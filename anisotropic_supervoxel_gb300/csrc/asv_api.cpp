@@ -431,22 +431,27 @@ static int depth_cost(int D, int zrun, int step, int depth, int most)
     return cost;
 }
 
+// The most chain positions of a sub-tile in pass p; below 4: list form.  The
+// first gathering pass (the third) sees labels around the seeds only and takes
+// any depth; 15 in the last: asv_run_words.
+static int most_depth(int D, double spacing, const int *steps, int npass, int p)
+{
+    const int step = steps[p], most = asv_jfa_slots(step);
+    if (!most) return 0;
+    return std::min(std::min(p == 2 ? 16 : label_depth(D, spacing, step), most - 2), p == npass - 1 ? 15 : 16);
+}
+
 // SegDesc::depth of every pass: of the depths that the labels allow the one
 // of least cost, so that 30 positions are 15 + 15, not 16 + 14, or at step 6
-// three sub-tiles of two whole chains (12 slots each), not four of 8 or 7.  The
-// first gathering pass (the third) sees labels around the seeds only and takes
-// any depth.
+// three sub-tiles of two whole chains (12 slots each), not four of 8 or 7.
 static void set_depths(SegDesc &s)
 {
     const double spacing = seed_spacing(s.nvox, s.Kp);
     for (int p = 0; p < s.npass; p++) {
         const int step = s.steps[p], most = asv_jfa_slots(step);
         s.depth[p] = 0;
-        if (!most) continue;
-        const int by_labels = p == 2 ? 16 : label_depth(s.D, spacing, step);
-        const int cap = std::min(std::min(by_labels, most - 2), p == s.npass - 1 ? 15 : 16);   // 15: asv_run_words
         int least = 0;
-        for (int d = cap; d >= 4; d--) {
+        for (int d = most_depth(s.D, spacing, s.steps, s.npass, p); d >= 4; d--) {
             const int c = depth_cost(s.D, s.zrun, step, d, most);
             if (c >= 0 && (!s.depth[p] || c < least)) { s.depth[p] = d; least = c; }
         }
@@ -454,21 +459,24 @@ static void set_depths(SegDesc &s)
 }
 
 // JFA tile depth for a set of segments: the configured one, else the one of
-// least estimated time.  A tile of z positions costs about z + 3 per sub-tile
-// (staging, numbering and barriers weigh like three positions).  The resident
-// blocks, four per SM, take the tiles in rounds; fewer tiles than that on an
-// SM run at 0.41, 0.69 and 0.85 of its full rate (one, two and three blocks),
-// which behind a full round costs a bit less, as the blocks do not end
-// together.  Fitted on clips of 160x120x40 to 1280x720x30 at every depth: the
-// choice is within 2 % of the best one, where the deepest of 32, 16 and 8 that
-// gave every block four tiles was up to 8 % off (320x240x85: depth 8 4.50 ms
-// for six iterations, 15 4.34; 641x360x30: depth 8 4.80, 15 4.46).
+// least estimated time over the gathering passes.  A tile of z positions costs z
+// + 1.55 per sub-tile (staging, numbering, barriers) + 0.36, or 1.8 z + 0.36 in
+// list form.
+// The resident blocks, four per SM, take the tiles in rounds; fewer tiles than
+// that on an SM run at 0.57, 0.83 and 0.92 of its full rate (one, two and three
+// blocks), which behind full rounds matters the less the more of those there
+// are, as the blocks do not end together; a quarter tile more for the last ones.
+// Fitted on 18 clips of 64x48x12 to 1280x720x30 with 60 to 10000 seeds at up to
+// 15 depths each: the choice is within 2 % of the best one on all of them.  (With
+// 3 per sub-tile, from the depths of steps 1 and 2 alone, and 0.41, 0.69 and
+// 0.85 it was up to 6.6 % off: 1280x720x30 with 10000 seeds, six iterations,
+// depth 5 27.1 ms, 30 25.4; 640x480x60, ten iterations, 15 13.45, 30 13.17.)
 static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
 {
     if (ctx->cfg.jfa_zrun > 0) return std::min(ctx->cfg.jfa_zrun, 256);
     const int per_sm = 4;
     const long long sms = std::max(1, asv_jfa_resident_blocks() / per_sm);
-    static const double rate[4] = { 1.0, 0.41, 0.69, 0.85 };
+    static const double rate[4] = { 1.0, 0.57, 0.83, 0.92 };
     int best = 4;
     double least = 0.0;
     for (int z = 1; z <= 32; z++) {
@@ -479,12 +487,17 @@ static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
             const int ze = even_depth(h.D, z), nz = (h.D + ze - 1) / ze;
             tiles += col * nz;
             const double sp = seed_spacing((long long)h.W * h.H * h.D, h.Kp);
-            const int d1 = label_depth(h.D, sp, 1), d2 = label_depth(h.D, sp, 2), d = std::max((d1 + d2) / 2, 4);
-            work += (double)col * (h.D + 3.0 * nz * ((ze + d - 1) / d));
+            for (int p = 2; p < h.npass; p++) {
+                const int d = most_depth(h.D, sp, h.steps, h.npass, p);
+                work += (double)col * ((d < 4 ? 1.8 * h.D : h.D + 1.55 * nz * ((ze + d - 1) / d)) + 0.36 * nz);
+            }
         }
         const long long m = (tiles + sms - 1) / sms, q = m / per_sm, k = m % per_sm;
-        double rounds = (double)(per_sm * q);
-        if (k) rounds += q ? 0.6 * k / rate[k] + 0.4 * k : k / rate[k];
+        double rounds = (double)(per_sm * q) + 0.24;
+        if (k) {
+            const double mix = q ? std::min(0.36 / q, 1.0) : 1.0;
+            rounds += mix * k / rate[k] + (1.0 - mix) * k;
+        }
         const double cost = work / tiles * rounds;
         if (least == 0.0 || cost < least) { best = z; least = cost; }
     }
