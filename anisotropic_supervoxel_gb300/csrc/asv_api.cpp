@@ -386,19 +386,24 @@ static int even_depth(int D, int z)
 // that its labels fit the 32 of its masks, 0: list form.  The footprint's box
 // (16 + 2 AL columns, AL the step rounded up to four, by 16 + 2 step rows by
 // (depth + 2) step slices) crosses about prod(1 + side / spacing) seeds'
-// cells; real ones are less regular, so up to 14 of the estimate are taken
-// without loss (measured at spacings 9 to 23: at spacing 18 and step 2 a loop
-// of six iterations took 4.81 ms with depth 8, estimate 10, 5.05 with 16,
-// estimate 15), and up to 24 at the least depth, which still beats the list
-// form there (spacing 9, step 1: 5.56 against 5.78 ms; step 2, estimate 28:
-// 5.67 against 5.63).
-static int label_depth(int D, double spacing, int step)
+// cells; real ones are less regular, so up to 18 of the estimate are taken
+// (measured at spacings 12 to 26 at all depths: at spacing 16 and step 2 six
+// iterations on 480x270x50 took 3.10 ms with depth 8, estimate 13, 3.04 with 16,
+// estimate 18; at 12.8 and step 2 on 427x239x61 4.37 with 4, estimate 14, 4.32
+// with 7, estimate 18, 4.41 with 16, estimate 28), 14 for steps above 3 (a full
+// ladder's step 4 at spacing 18: depth 4, estimate 13, 2.054 ms, 8, estimate 15,
+// 2.085), and up to 24 at the least depth, which still beats the list form there
+// (spacing 9, step 1: 5.56 against 5.78 ms; step 2, estimate 28: 5.67 against
+// 5.63).  The first gathering pass sees labels around the seeds only: 27 (spacing
+// 12.8, step 3: depth 8, estimate 26, 4.28 ms, 16, estimate 41, 4.37; spacing 16,
+// step 4: 16, estimate 25, 3.10, 8 3.17).
+static int label_depth(int D, double spacing, int step, bool sparse)
 {
     const int al = (step + 3) & ~3;
     const double xy = (1.0 + (16 + 2 * al) / spacing) * (1.0 + (16 + 2 * step) / spacing);
-    for (int c : { 16, 8, 4 }) {
+    for (int c = 16; c >= 4; c--) {
         const double labels = xy * (1.0 + std::min(D, (c + 2) * step) / spacing);
-        if (labels <= 14.0 || (c == 4 && labels <= 24.0)) return c;
+        if (labels <= (sparse ? 27.0 : c == 4 ? 24.0 : step > 3 ? 14.0 : 18.0)) return c;
     }
     return 0;
 }
@@ -406,10 +411,10 @@ static int label_depth(int D, double spacing, int step)
 static double seed_spacing(long long nvox, int Kp) { return std::cbrt((double)nvox / std::max(Kp, 1)); }
 
 // Footprint slots of all sub-tiles of `depth` positions of a column's D
-// positions cut in tiles of zrun, and 3 for each sub-tile (as in pick_zrun);
-// -1 when a sub-tile has more slots than fit.  A sub-tile has its positions
-// and the two slices next to them, and where a chain ends inside it slices 0
-// and D - 1, unless those are the two.
+// positions cut in tiles of zrun, and 3 for each sub-tile, in quarters, and one
+// for an odd sub-tile (positions go two at a time); -1 when a sub-tile has more
+// slots than fit.  A sub-tile has its positions and the two slices next to them,
+// and where a chain ends inside it slices 0 and D - 1, unless those are the two.
 static int depth_cost(int D, int zrun, int step, int depth, int most)
 {
     auto slice = [&](int p) {                              // asv_chain_pos
@@ -426,23 +431,23 @@ static int depth_cost(int D, int zrun, int step, int depth, int most)
             int slots = n + 2;
             if (ends) slots += (slice(p0) > step) + (slice(p0 + n - 1) + step < D - 1);
             if (slots > most) return -1;
-            cost += slots + 3;
+            cost += 4 * (slots + 3) + (n & 1);
         }
     return cost;
 }
 
-// The most chain positions of a sub-tile in pass p; below 4: list form.  The
-// first gathering pass (the third) sees labels around the seeds only and takes
-// any depth; 15 in the last: asv_run_words.
+// The most chain positions of a sub-tile in pass p; below 4: list form.  15 in
+// the last pass: asv_run_words.
 static int most_depth(int D, double spacing, const int *steps, int npass, int p)
 {
     const int step = steps[p], most = asv_jfa_slots(step);
     if (!most) return 0;
-    return std::min(std::min(p == 2 ? 16 : label_depth(D, spacing, step), most - 2), p == npass - 1 ? 15 : 16);
+    return std::min(std::min(label_depth(D, spacing, step, p == 2), most - 2), p == npass - 1 ? 15 : 16);
 }
 
 // SegDesc::depth of every pass: of the depths that the labels allow the one
-// of least cost, so that 30 positions are 15 + 15, not 16 + 14, or at step 6
+// of least cost (the smallest of equal ones, as a sub-tile that overflows goes on
+// with half the depth), so that 30 positions are 15 + 15, not 16 + 14, or at step 6
 // three sub-tiles of two whole chains (12 slots each), not four of 8 or 7.
 static void set_depths(SegDesc &s)
 {
@@ -453,7 +458,7 @@ static void set_depths(SegDesc &s)
         int least = 0;
         for (int d = most_depth(s.D, spacing, s.steps, s.npass, p); d >= 4; d--) {
             const int c = depth_cost(s.D, s.zrun, step, d, most);
-            if (c >= 0 && (!s.depth[p] || c < least)) { s.depth[p] = d; least = c; }
+            if (c >= 0 && (!s.depth[p] || c <= least)) { s.depth[p] = d; least = c; }
         }
     }
 }
