@@ -660,7 +660,9 @@ static void do_first_init(asv_ctx *ctx)
 // different step (and for the segments whose last pass it is); the first on the
 // context's stream, the others beside it on the side stream, where their blocks
 // fill the SMs that the first leaves at its end.
-static void do_pass(asv_ctx *ctx, int p)
+// follow: the operation before on the context's stream is a kernel; returns whether
+// it is now.
+static bool do_pass(asv_ctx *ctx, int p, bool follow)
 {
     int kinds[2 * (ASV_BITS_MAXS + 2)], n = 0;                // step (capped at the list form's), last pass
     for (const SegDesc &s : ctx->sd) {
@@ -673,19 +675,22 @@ static void do_pass(asv_ctx *ctx, int p)
         cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0);
     }
     for (int i = 0; i < n; i++)
-        asv_launch_jfa(ctx->d, p, kinds[i] / 2, kinds[i] & 1, ctx->jfa_blocks, i ? ctx->side : ctx->st);
+        asv_launch_jfa(ctx->d, p, kinds[i] / 2, kinds[i] & 1, ctx->jfa_blocks, follow && n == 1,
+                       i ? ctx->side : ctx->st);
     if (n > 1) {
         cudaEventRecord(ctx->side_ev[1], ctx->side);
         cudaStreamWaitEvent(ctx->st, ctx->side_ev[1], 0);
     }
     ctx->launches += n;
+    return n == 1;
 }
 
 // the JFA ladder; the last pass of each segment also forms its centroid sums
 // (loop: the seeds stand in d.drawn alone, the label volumes are -1, the sums
 // zero and the first pass's list empty)
-static void do_flood(asv_ctx *ctx, int evbase, bool loop)
+static bool do_flood(asv_ctx *ctx, int evbase, bool loop)
 {
+    bool follow = false;                                      // as do_pass's
     if (!loop)
         cudaMemsetAsync(ctx->d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)ctx->d.total_seeds, ctx->st);
     for (int p = 0; p < ctx->maxpass; p++) {
@@ -693,16 +698,19 @@ static void do_flood(asv_ctx *ctx, int evbase, bool loop)
         if (p == 0 && (loop || ctx->drawn)) {
             asv_launch_jfa_first(loop ? ctx->d : step_dev(ctx), loop, !loop && !ctx->undraw, ctx->st);   // step 1 from the drawn seeds
             ctx->launches++;
+            follow = true;
         } else if (p == 1 && (loop || ctx->drawn)) {
             if (!loop) cudaMemsetAsync(ctx->d.labA, 0xff, label_bytes(ctx), ctx->st);
             asv_launch_jfa_second_scatter(ctx->d, loop, ctx->st);   // from the first pass's sparse labels
             ctx->launches++;
+            follow = true;
         } else {
-            do_pass(ctx, p);
+            follow = do_pass(ctx, p, follow);
         }
         if (evbase >= 0) rec_begin(ctx, evbase + 2 * p + 1);
     }
     ctx->drawn = ctx->undraw = false;
+    return follow;
 }
 
 // the reseed of centroids_next_seeds (the sums came with the flood)
@@ -723,7 +731,7 @@ static void do_sums_from_labels(asv_ctx *ctx)
 static void do_next_seeds(asv_ctx *ctx)
 {
     cudaMemsetAsync(ctx->d.labA, 0xff, label_bytes(ctx), ctx->st);
-    asv_launch_next_seeds(step_dev(ctx), false, false, ctx->st);
+    asv_launch_next_seeds(step_dev(ctx), false, false, false, ctx->st);
     ctx->drawn = ctx->undraw = true;
     ctx->launches += 3;       // two metric kernels, the combination with the draw
 }
@@ -750,7 +758,7 @@ static void loop_fills(asv_ctx *ctx, bool first)
 
 // The loop's seeds of iteration it, drawn into d.drawn: the initial ones, or
 // from the centroid sums with the metric at their positions
-static void loop_seeds(asv_ctx *ctx, int it)
+static void loop_seeds(asv_ctx *ctx, int it, bool follow)
 {
     loop_fills(ctx, it == 1);
     if (it == 1) {
@@ -759,7 +767,7 @@ static void loop_seeds(asv_ctx *ctx, int it)
         asv_launch_draw(ctx->d, ctx->st);
         ctx->launches += 2;
     } else {
-        asv_launch_next_seeds(ctx->d, true, true, ctx->st);
+        asv_launch_next_seeds(ctx->d, true, true, follow, ctx->st);
         cudaStreamWaitEvent(ctx->st, ctx->side_ev[1], 0);
         ctx->launches += 3;   // two metric kernels, the combination with the draw
     }
@@ -777,9 +785,10 @@ static void enqueue_lloyd(asv_ctx *ctx, bool instrument)
 {
     const int I = ctx->cfg.lloyd_iters;
     const int per_it = 2 * ctx->maxpass;
+    bool follow = false;
     for (int it = 1; it <= I; it++) {
-        loop_seeds(ctx, it);
-        do_flood(ctx, instrument ? (it - 1) * per_it : -1, true);
+        loop_seeds(ctx, it, follow);
+        follow = do_flood(ctx, instrument ? (it - 1) * per_it : -1, true);
     }
     do_post(ctx);
 }
@@ -1575,7 +1584,7 @@ asv_status asv_jfa_pass_host(asv_ctx *ctx, int step, float ratio, const int32_t 
     d.segs = ctx->d.segs + 1;
     CK(cudaMemcpyAsync((void *)d.segs, &one, sizeof(one), cudaMemcpyHostToDevice, ctx->st));
     asv_launch_label_clean(din, s.nvox, s.Kp, ctx->st);
-    asv_launch_jfa(d, 0, step, false, ctx->jfa_blocks, ctx->st);
+    asv_launch_jfa(d, 0, step, false, ctx->jfa_blocks, false, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout, 4 * n, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));

@@ -120,7 +120,8 @@ void asv_launch_density(const AsvDev &d, cudaStream_t st);
 void asv_launch_density_adjust(const AsvDev &d, cudaStream_t st);
 void asv_launch_first_init(const AsvDev &d, cudaStream_t st);
 void asv_launch_draw(const AsvDev &d, cudaStream_t st);
-void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, cudaStream_t st);
+// (follow: the operation before on st is a kernel, see asv_launch_follow)
+void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, bool follow, cudaStream_t st);
 void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t st);
 void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st);
 void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st);
@@ -128,7 +129,7 @@ void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);
 void asv_launch_post(const AsvDev &d, cudaStream_t st);
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st);
-void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st);
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, bool follow, cudaStream_t st);
 int asv_jfa_grid_blocks(int total_tiles);
 int asv_jfa_resident_blocks();
 int asv_jfa_slots(int step);   // footprint slots a sub-tile of the step can hold, 0: no bit-set form

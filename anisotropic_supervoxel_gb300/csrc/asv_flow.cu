@@ -23,6 +23,7 @@
 //   3. the flow is upsampled to the next finer level.
 // The grey frames use the integer RGB -> grey of ITU-R BT.601 with 14-bit
 // fixed-point weights (4899, 9617, 1868).
+#include "asv_follow.cuh"
 #include "asv_flow.cuh"
 
 #include <math.h>
@@ -38,6 +39,7 @@ __constant__ float c_fl_ginv[5][6];           // rows b1, b2, a11, a22, 2*a12 of
 // ---------------------------------------------------------------------------
 __global__ void k_fl_gray(const uint8_t *__restrict__ rgb, float *__restrict__ out, long long n)
 {
+    asv_follow();
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= n) return;
     const uint8_t *p = rgb + 3 * v;
@@ -48,6 +50,7 @@ __global__ void k_fl_gray(const uint8_t *__restrict__ rgb, float *__restrict__ o
 __global__ void k_fl_down(const float *__restrict__ in, int Wi, int Hi, float *__restrict__ out, int Wo,
                           int Ho, int D)
 {
+    asv_follow();
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long fo = (long long)Wo * Ho;
     if (t >= fo * D) return;
@@ -67,6 +70,7 @@ __global__ void k_fl_down(const float *__restrict__ in, int Wi, int Hi, float *_
 // horizontal moments: h_p(x, y) = sum_u t^p g(u) f(x + u, y), p = 0, 1, 2
 __global__ void k_fl_poly_h(const float *__restrict__ img, int W, int H, int D, float *__restrict__ h)
 {
+    asv_follow();
     const long long plane = (long long)W * H * D;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= plane) return;
@@ -90,6 +94,7 @@ __global__ void k_fl_poly_h(const float *__restrict__ img, int W, int H, int D, 
 __global__ void k_fl_poly_v(const float *__restrict__ h, int W, int H, int D, float4 *__restrict__ polyA,
                             float *__restrict__ polyB)
 {
+    asv_follow();
     const long long plane = (long long)W * H * D;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= plane) return;
@@ -204,6 +209,7 @@ __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__
                                                    const float *__restrict__ fin, float *__restrict__ fout, int W,
                                                    int H, int D, int P, int rows)
 {
+    asv_follow();
     extern __shared__ __align__(16) float fl_sm[];
     float *S = fl_sm, *T = fl_sm + 5 * FL_RS * FL_SP;
     const long long fr = (long long)W * H, mplane = fr * P;
@@ -386,6 +392,7 @@ static int fl_rows(int W, int H, int P, int resident)
 __global__ void __launch_bounds__(FL_T) k_fl_up(const float *__restrict__ coarse, int Wc, int Hc, float *__restrict__ fine,
                                                 int W, int H, int P)
 {
+    asv_follow();
     const int x = blockIdx.x * FL_T + threadIdx.x, pr = blockIdx.z;
     if (x >= W) return;
     const long long mplane = (long long)W * H * P, cplane = (long long)Wc * Hc * P;
@@ -414,6 +421,7 @@ __global__ void __launch_bounds__(FL_T) k_fl_up(const float *__restrict__ coarse
 __global__ void k_fl_store(const float *__restrict__ flow, int W, int H, int D, float2 *__restrict__ fwd,
                            float2 *__restrict__ bwd, int keep_first_bwd)
 {
+    asv_follow();
     const long long fr = (long long)W * H, vox = fr * D, mplane = fr * 2 * (D - 1);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= vox) return;
@@ -549,31 +557,29 @@ int asv_launch_flow(const uint8_t *rgb, int W, int H, int D, float2 *fwd, float2
 
     k_fl_gray<<<fl_blocks((long long)fr0 * D), FL_T, 0, st>>>(rgb, img[0], (long long)fr0 * D);
     for (int k = 1; k < L; k++)
-        k_fl_down<<<fl_blocks((long long)Ws[k] * Hs[k] * D), FL_T, 0, st>>>(img[k - 1], Ws[k - 1], Hs[k - 1], img[k],
-                                                                          Ws[k], Hs[k], D);
+        asv_launch_follow(true, k_fl_down, fl_blocks((long long)Ws[k] * Hs[k] * D), FL_T, 0, st, img[k - 1], Ws[k - 1],
+                          Hs[k - 1], img[k], Ws[k], Hs[k], D);
     for (int k = 0; k < L; k++) {
         const long long n = (long long)Ws[k] * Hs[k] * D;
-        k_fl_poly_h<<<fl_blocks(n), FL_T, 0, st>>>(img[k], Ws[k], Hs[k], D, hm[k]);
-        k_fl_poly_v<<<fl_blocks(n), FL_T, 0, st>>>(hm[k], Ws[k], Hs[k], D, polyA[k], polyB[k]);
+        asv_launch_follow(true, k_fl_poly_h, fl_blocks(n), FL_T, 0, st, img[k], Ws[k], Hs[k], D, hm[k]);
+        asv_launch_follow(true, k_fl_poly_v, fl_blocks(n), FL_T, 0, st, hm[k], Ws[k], Hs[k], D, polyA[k], polyB[k]);
     }
     for (int k = L - 1; k >= 0; k--) {
         const int w = Ws[k], h = Hs[k];
         const long long mplane = (long long)w * h * P;
         if (k == L - 1) cudaMemsetAsync(flow[k], 0, sizeof(float) * mplane * 2, st);
         else
-            k_fl_up<<<dim3((w + FL_T - 1) / FL_T, (h + FL_UP_ROWS - 1) / FL_UP_ROWS, P), FL_T, 0, st>>>(
-                flow[k + 1], Ws[k + 1], Hs[k + 1], flow[k], w, h, P);
+            asv_launch_follow(true, k_fl_up, dim3((w + FL_T - 1) / FL_T, (h + FL_UP_ROWS - 1) / FL_UP_ROWS, P), FL_T, 0, st,
+                              flow[k + 1], Ws[k + 1], Hs[k + 1], flow[k], w, h, P);
         const int rows = fl_rows(w, h, P, sms * (per > 0 ? per : 1));
         const unsigned blocks = (unsigned)((w + FL_TW - 1) / FL_TW) * ((h + rows - 1) / rows) * P;
         for (int it = 0; it < 10; it++) {                 // even count: the result ends in flow[k]
             const float *fin = (it & 1) ? alt : flow[k];
             float *fout = (it & 1) ? flow[k] : alt;
-            if (w > 1 && h > 1)
-                k_fl_iter<false><<<blocks, FL_NT, FL_SMEM, st>>>(polyA[k], polyB[k], fin, fout, w, h, D, P, rows);
-            else
-                k_fl_iter<true><<<blocks, FL_NT, FL_SMEM, st>>>(polyA[k], polyB[k], fin, fout, w, h, D, P, rows);
+            asv_launch_follow(it > 0 || k < L - 1, w > 1 && h > 1 ? k_fl_iter<false> : k_fl_iter<true>, blocks, FL_NT, FL_SMEM,
+                              st, polyA[k], polyB[k], fin, fout, w, h, D, P, rows);
         }
     }
-    k_fl_store<<<fl_blocks((long long)fr0 * D), FL_T, 0, st>>>(flow[0], W, H, D, fwd, bwd, keep_first_bwd);
+    asv_launch_follow(true, k_fl_store, fl_blocks((long long)fr0 * D), FL_T, 0, st, flow[0], W, H, D, fwd, bwd, keep_first_bwd);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -33,6 +33,7 @@
 // pair after the other took 33 us for the seeds of the 320x240x85 clip and 54 us
 // for the rings of one with computed flow, now 19 and 35 us.
 // Compiled with -fmad=false.
+#include "asv_follow.cuh"
 #include "asv_seed.cuh"
 
 #include <float.h>
@@ -377,6 +378,7 @@ __device__ __forceinline__ int asv_seed_key(const SegDesc &S, float4 p)
 // 2 -> pos formed here from the centroid sums (asv_reseed).
 __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
 {
+    asv_follow();
     const bool writer = (threadIdx.x & 15) == 0;
     SeedRef r;
     bool active = asv_seed_ref(d, (blockIdx.x * blockDim.x + threadIdx.x) >> 4, r);
@@ -417,6 +419,7 @@ __global__ void __launch_bounds__(128) k_metric_self(AsvDev d, int reseed)
 // a solve per listed seed and ring neighbour
 __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
 {
+    asv_follow();
     const bool writer = (threadIdx.x & 15) == 0;
     const int step = (gridDim.x * blockDim.x) >> 4, tasks = *d.negcount * ASV_RING;
     for (int task0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; task0 < tasks; task0 += step) {
@@ -498,6 +501,7 @@ __device__ __forceinline__ void asv_metric_result(const AsvDev &d, int g, int ne
 // seed slot's centroid sums.
 __global__ void k_metric_combine(AsvDev d, int reseed, bool draw, bool clear)
 {
+    asv_follow();
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g == 0) {
         *d.negcount = 0;
@@ -528,25 +532,25 @@ __global__ void k_metric_combine(AsvDev d, int reseed, bool draw, bool clear)
     if (draw) asv_draw_seed(d, S, g, r.i, p, d.slab[g], res);
 }
 
-static void metric_solves(const AsvDev &d, int reseed, cudaStream_t st)
+static void metric_solves(const AsvDev &d, int reseed, bool follow, cudaStream_t st)
 {
     const long long solves = d.total_seeds, ring = solves * ASV_RING;             // 8 per block
-    k_metric_self<<<(int)((solves + 7) / 8), 128, 0, st>>>(d, reseed);
+    asv_launch_follow(follow, k_metric_self, (unsigned)((solves + 7) / 8), 128, 0, st, d, reseed);
     const long long blocks = (ring + 7) / 8;
-    k_metric_ring<<<(int)(blocks < 1216 ? blocks : 1216), 128, 0, st>>>(d, reseed);   // 8 blocks per SM at most
+    asv_launch_follow(true, k_metric_ring, (unsigned)(blocks < 1216 ? blocks : 1216), 128, 0, st, d, reseed);   // 8 blocks per SM at most
 }
 
 
 void asv_launch_metric(const AsvDev &d, int reseed, cudaStream_t st)
 {
-    metric_solves(d, reseed, st);
-    k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, reseed, false, false);
+    metric_solves(d, reseed, false, st);
+    asv_launch_follow(true, k_metric_combine, (d.total_seeds + 63) / 64, 64, 0, st, d, reseed, false, false);
 }
 
 // The next iteration's seeds: positions from the centroid sums (finalize),
 // metrics, draw
-void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, cudaStream_t st)
+void asv_launch_next_seeds(const AsvDev &d, bool finalize, bool clear_sums, bool follow, cudaStream_t st)
 {
-    metric_solves(d, finalize ? 2 : 1, st);
-    k_metric_combine<<<(d.total_seeds + 63) / 64, 64, 0, st>>>(d, 1, true, clear_sums);
+    metric_solves(d, finalize ? 2 : 1, follow, st);
+    asv_launch_follow(true, k_metric_combine, (d.total_seeds + 63) / 64, 64, 0, st, d, 1, true, clear_sums);
 }

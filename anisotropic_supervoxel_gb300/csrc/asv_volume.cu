@@ -4,6 +4,7 @@
 // the order written, so the labels match the CPU restatement bit for bit.
 // Reference files (in dongxiao0401/anisotropic_supervoxel): GPU-AS/shaders/*,
 // GPU-AS/Image.cpp.
+#include "asv_follow.cuh"
 #include "asv_seed.cuh"
 
 #include <cuda_fp16.h>
@@ -1370,6 +1371,8 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
 {
     extern __shared__ __align__(16) unsigned char asv_jfa_smem[];
     if constexpr (ST < ASV_JFA_LIST) asv_jfa_smem_init(*(AsvBitsShared *)(asv_jfa_smem + AsvBitsGeo<ST>::AREA));
+    if constexpr (SUMS) asv_follow();                         // (the seeds' kernels have few blocks)
+    else asv_follow_wait();
     for (int t = blockIdx.x; t < d.total_tiles; t += gridDim.x) {
         const int si = asv_find_seg(d.tile_prefix, d.nseg, t);
         const SegDesc &S = d.segs[si];
@@ -1403,6 +1406,7 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
 
 __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 {
+    asv_follow();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int g = t / 27, o = t - g * 27;
     bool won = false;
@@ -1542,6 +1546,7 @@ __device__ __forceinline__ void asv_second_voxel(const AsvDev &d, const SegDesc 
 // that it is all -1 for the next draw without a fill (the first pass has read it).
 __global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
 {
+    asv_follow_wait();
     const unsigned group = blockIdx.x / 27;
     const int o = (int)(blockIdx.x - 27 * group);              // one offset per block: neighbouring entries' targets
     const long long e = (long long)group * 256 + threadIdx.x, t = (long long)blockIdx.x * 256 + threadIdx.x;   // adjoin
@@ -1665,6 +1670,7 @@ __global__ void k_finalize(AsvDev d)
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(1024) k_post_stats(AsvDev d)
 {
+    asv_follow();
     const int si = blockIdx.x;
     const SegDesc &S = d.segs[si];
     const int Kp = S.Kp;
@@ -1753,6 +1759,7 @@ __device__ __forceinline__ bool asv_needs_scan(const int *rec)
 
 __global__ void __launch_bounds__(256) k_post_chunk_max(AsvDev d)
 {
+    asv_follow();
     int si = asv_find_seg(d.chunk_prefix, d.nseg, blockIdx.x);
     const SegDesc &S = d.segs[si];
     const int *rec = d.post + si * ASV_POST_WORDS;
@@ -1780,6 +1787,7 @@ __global__ void __launch_bounds__(256) k_post_chunk_max(AsvDev d)
 // exclusive max-scan of the chunk maxima within each segment (1 block / segment)
 __global__ void __launch_bounds__(1024) k_post_prefix(AsvDev d)
 {
+    asv_follow();
     int si = blockIdx.x;
     const int *rec = d.post + si * ASV_POST_WORDS;
     if (!asv_needs_scan(rec)) return;
@@ -1824,6 +1832,7 @@ __global__ void __launch_bounds__(1024) k_post_prefix(AsvDev d)
 // us, now 47.)
 __global__ void __launch_bounds__(256) k_post_apply(AsvDev d)
 {
+    asv_follow();
     constexpr int PER = ASV_CHUNK / 256, NONE = -2;
     __shared__ int wlast[8];                                // label of the warp's last source, NONE without
     const int si = asv_find_seg(d.chunk_prefix, d.nseg, blockIdx.x);
@@ -2016,13 +2025,13 @@ int asv_jfa_grid_blocks(int total_tiles)
     return total_tiles < blocks ? total_tiles : blocks;
 }
 
-void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, cudaStream_t st)
+void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, bool follow, cudaStream_t st)
 {
     const int32_t *in = (pass & 1) ? d.labB : d.labA;
     int32_t *out = (pass & 1) ? d.labA : d.labB;
     asv_jfa_attributes();
     const AsvJfaVariant &v = asv_jfa_variant(step, last);
-    v.kernel<<<grid_blocks, ASV_JFA_THREADS, v.smem, st>>>(d, pass, in, out);
+    asv_launch_follow(follow, v.kernel, grid_blocks, ASV_JFA_THREADS, v.smem, st, d, pass, in, out);
 }
 
 // filled: the output volume is all -1 and the list empty already
@@ -2040,7 +2049,7 @@ void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t
 void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st)
 {
     const unsigned blocks = 27u * (unsigned)((27LL * d.total_seeds + 255) / 256);   // tlist holds <= 27 entries per seed
-    k_jfa_second<<<blocks, 256, 0, st>>>(d, undraw);
+    asv_launch_follow(undraw, k_jfa_second, blocks, 256, 0, st, d, undraw);      // (undraw: behind the first pass)
 }
 
 void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st)
@@ -2054,7 +2063,7 @@ void asv_launch_finalize(const AsvDev &d, cudaStream_t st) { k_finalize<<<seed_b
 void asv_launch_post(const AsvDev &d, cudaStream_t st)
 {
     k_post_stats<<<d.nseg, 1024, 0, st>>>(d);
-    k_post_chunk_max<<<d.total_chunks, 256, 0, st>>>(d);
-    k_post_prefix<<<d.nseg, 1024, 0, st>>>(d);
-    k_post_apply<<<d.total_chunks, 256, 0, st>>>(d);
+    asv_launch_follow(true, k_post_chunk_max, d.total_chunks, 256, 0, st, d);
+    asv_launch_follow(true, k_post_prefix, d.nseg, 1024, 0, st, d);
+    asv_launch_follow(true, k_post_apply, d.total_chunks, 256, 0, st, d);
 }
