@@ -36,6 +36,8 @@
 // Compiled with -fmad=false (integer work only).
 #include "asv_connect.cuh"
 
+#include "asv_follow.cuh"
+
 #define CC_CHUNK 2048
 #define CC_THREADS 256
 #define CC_TZ 8                     // a tile: 32 x 8 (the block's warps) x CC_TZ voxels
@@ -173,6 +175,7 @@ struct CcTile {
 __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restrict__ lab, int *par, int *cnt, int W,
                                                         int H, int D, int tx, int ty, int *err)
 {
+    asv_follow();
     __shared__ int sl[CC_TILE], sp[CC_TILE], sc[CC_TILE];      // sc: the queue, then the sizes
     __shared__ int nq;
     if (threadIdx.x == 0) nq = 0;
@@ -231,6 +234,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restric
 __global__ void __launch_bounds__(CC_THREADS) k_cc_union(const int32_t *__restrict__ lab, int *par, int W, int H, int D,
                                                          int tx, int ty, int *err)
 {
+    asv_follow();
     constexpr unsigned PREV = 0x1ffu << 9, NORTH = 7u | (7u << 9), SOUTH = 7u << 15, WEST = 0x9249u, EAST = WEST << 2;
     constexpr int NW = CC_THREADS / 32, ROWS = NW + 2 * (CC_TZ - 1), TASKS = ROWS + 2 * NW * CC_TZ / 32;
     __shared__ int queue[CC_TILE], nq;
@@ -274,6 +278,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_union(const int32_t *__restri
 // roots, and only thread v writes par[v].
 __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *par, int *cnt, int n, int *chunk, int *err)
 {
+    asv_follow();
     constexpr int IT = CC_CHUNK / CC_THREADS;
     __shared__ int tot;
     if (threadIdx.x == 0) tot = 0;
@@ -314,6 +319,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *par, int *cnt, i
 // count: m = ceil(*count / CC_SEGS) instead
 __global__ void __launch_bounds__(1024) k_cc_prefix(int *chunk, int m, const int *count, int *total)
 {
+    asv_follow();
     __shared__ int part[32];
     __shared__ int carry;
     if (count) m = *count > CC_MAX_R ? 0 : (*count + CC_SEGS - 1) / CC_SEGS;
@@ -354,6 +360,7 @@ __global__ void __launch_bounds__(1024) k_cc_prefix(int *chunk, int m, const int
 __global__ void __launch_bounds__(CC_THREADS) k_cc_compact(const int *__restrict__ par, int *cnt_cid,
                                                            const int *__restrict__ chunk, int n, int *rvox, int *rsize)
 {
+    asv_follow();
     constexpr int IT = CC_CHUNK / CC_THREADS, NW = CC_THREADS / 32;
     __shared__ int sum[IT * NW];                               // roots per iteration and warp, then their prefix
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -384,6 +391,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_compact(const int *__restrict
 // kept segments per group of CC_SEGS, for the rank scan
 __global__ void __launch_bounds__(CC_SEGS) k_cc_kept_count(const int *__restrict__ rsize, const int *R, int minsz, int *chunk)
 {
+    asv_follow();
     const int r = *R > CC_MAX_R ? 0 : *R;
     for (int g = blockIdx.x; (long long)g * CC_SEGS < r; g += gridDim.x) {
         const int j = g * CC_SEGS + threadIdx.x;
@@ -399,6 +407,7 @@ __global__ void __launch_bounds__(CC_SEGS) k_cc_nodes(const int *__restrict__ pa
                                                       const int *__restrict__ chunk, const int *R, int minsz, int W,
                                                       int H, int D, int *node)
 {
+    asv_follow();
     __shared__ int wsum[CC_SEGS / 32];
     const int r = *R > CC_MAX_R ? 0 : *R, lane = threadIdx.x & 31, w = threadIdx.x >> 5, sl = W * H;
     for (int g = blockIdx.x; (long long)g * CC_SEGS < r; g += gridDim.x) {
@@ -439,6 +448,7 @@ __global__ void __launch_bounds__(CC_SEGS) k_cc_nodes(const int *__restrict__ pa
 // every node; most end in the first.
 __global__ void __launch_bounds__(CC_THREADS) k_cc_jump(int *node, const int *R)
 {
+    asv_follow();
     const int r = *R > CC_MAX_R ? 0 : *R;
     const unsigned step = gridDim.x * CC_THREADS;
     for (unsigned t = blockIdx.x * CC_THREADS + threadIdx.x; t < 2u * (unsigned)r; t += step) {
@@ -452,6 +462,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_jump(int *node, const int *R)
 __global__ void __launch_bounds__(CC_THREADS) k_cc_output(const int *__restrict__ par, const int *__restrict__ cid,
                                                           const int *__restrict__ node, int n, const int *R, int32_t *out)
 {
+    asv_follow();
     if (*R > CC_MAX_R) return;
     const long long base = (long long)blockIdx.x * (4 * CC_THREADS) + threadIdx.x;
 #pragma unroll
@@ -491,19 +502,20 @@ int asv_launch_connect(const int32_t *lab, int W, int H, int D, int supsz, int32
     const unsigned tiles = (unsigned)tx * ty * ((D + CC_TZ - 1) / CC_TZ);
     int *R = meta, *err = meta + 1, *num = meta + 2;
     cudaMemsetAsync(meta, 0, 16, st);
-    k_cc_tile<<<tiles, CC_THREADS, 0, st>>>(lab, par, cid, W, H, D, tx, ty, err);
-    k_cc_union<<<tiles, CC_THREADS, 0, st>>>(lab, par, W, H, D, tx, ty, err);
-    k_cc_flatten<<<(unsigned)chunks, CC_THREADS, 0, st>>>(par, cid, ni, chunk, err);
-    k_cc_prefix<<<1, 1024, 0, st>>>(chunk, (int)chunks, nullptr, R);
-    k_cc_compact<<<(unsigned)chunks, CC_THREADS, 0, st>>>(par, cid, chunk, ni, rvox, rsize);
+    asv_launch_follow(false, k_cc_tile, tiles, CC_THREADS, 0, st, lab, par, cid, W, H, D, tx, ty, err);
+    asv_launch_follow(true, k_cc_union, tiles, CC_THREADS, 0, st, lab, par, W, H, D, tx, ty, err);
+    asv_launch_follow(true, k_cc_flatten, (unsigned)chunks, CC_THREADS, 0, st, par, cid, ni, chunk, err);
+    asv_launch_follow(true, k_cc_prefix, 1, 1024, 0, st, chunk, (int)chunks, nullptr, R);
+    asv_launch_follow(true, k_cc_compact, (unsigned)chunks, CC_THREADS, 0, st, par, cid, chunk, ni, rvox, rsize);
     // the segments' kernels: enough threads for a few segments per chunk, any
     // number by grid strides
     const unsigned groups = (unsigned)(chunks < 1216 ? chunks : 1216);
-    k_cc_kept_count<<<groups, CC_SEGS, 0, st>>>(rsize, R, minsz, kept);
-    k_cc_prefix<<<1, 1024, 0, st>>>(kept, 0, R, num);
-    k_cc_nodes<<<groups, CC_SEGS, 0, st>>>(par, cid, rvox, rsize, kept, R, minsz, W, H, D, node);
-    for (int k = 0; k < CC_ROUNDS; k++) k_cc_jump<<<groups, CC_THREADS, 0, st>>>(node, R);
-    k_cc_output<<<(unsigned)((n + 4 * CC_THREADS - 1) / (4 * CC_THREADS)), CC_THREADS, 0, st>>>(par, cid, node, ni, R, out);
+    asv_launch_follow(true, k_cc_kept_count, groups, CC_SEGS, 0, st, rsize, R, minsz, kept);
+    asv_launch_follow(true, k_cc_prefix, 1, 1024, 0, st, kept, 0, R, num);
+    asv_launch_follow(true, k_cc_nodes, groups, CC_SEGS, 0, st, par, cid, rvox, rsize, kept, R, minsz, W, H, D, node);
+    for (int k = 0; k < CC_ROUNDS; k++) asv_launch_follow(true, k_cc_jump, groups, CC_THREADS, 0, st, node, R);
+    asv_launch_follow(true, k_cc_output, (unsigned)((n + 4 * CC_THREADS - 1) / (4 * CC_THREADS)), CC_THREADS, 0, st, par, cid,
+                      node, ni, R, out);
     int got[3] = { 0, 0, 0 };
     cudaMemcpyAsync(got, meta, sizeof(got), cudaMemcpyDeviceToHost, st);
     if (cudaStreamSynchronize(st) != cudaSuccess) return -1;

@@ -22,6 +22,7 @@
 // and forward-fill label -1.  A label outside [-1, Kp) (which the JFA never
 // writes) is read as -1 by every stage: counted in the -1 slot and filled.
 #include "asv.h"
+#include "asv_follow.cuh"
 #include "asv_tally.cuh"
 
 #include <cuda_runtime.h>
@@ -87,6 +88,7 @@ static __device__ __forceinline__ bool na_scan_needed(const int *rec)
 // volume, this one 27 us).
 __global__ void __launch_bounds__(256) k_na_count(NaScratch s, const int32_t *__restrict__ raw, int n, int Kp)
 {
+    asv_follow();
     __shared__ Tally t;
     __shared__ unsigned last[NA_GROUP][2];
     tally_clear(t);
@@ -133,6 +135,7 @@ __global__ void __launch_bounds__(256) k_na_count(NaScratch s, const int32_t *__
 // source in the chunks before it (voxel + 1): one block
 __global__ void __launch_bounds__(1024) k_na_scan(NaScratch s, const int32_t *__restrict__ raw, int Kp, int nchunks)
 {
+    asv_follow();
     __shared__ int warp_tot[32];
     __shared__ int carry;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -212,6 +215,7 @@ template <bool VEC>
 __global__ void __launch_bounds__(256) k_na_apply(NaScratch s, const int32_t *__restrict__ raw,
                                                   int32_t *__restrict__ out, int n, int Kp)
 {
+    asv_follow();
     constexpr int PER = NA_CHUNK / 256;
     __shared__ int wlast[8];                                // label of the warp's last source, NONE without
     const int *rec = s.rec;
@@ -331,9 +335,9 @@ extern "C" asv_status asv_check_dead_seeds_noalloc(const int32_t *d_raw, int32_t
         return ASV_ERR_CUDA;
     }
     k_na_count<<<(nchunks + NA_GROUP - 1) / NA_GROUP, 256, 0, st>>>(s, d_raw, (int)n, Kp);
-    k_na_scan<<<1, 1024, 0, st>>>(s, d_raw, Kp, nchunks);
-    if (((r0 | o0) & 15) == 0) k_na_apply<true><<<nchunks, 256, 0, st>>>(s, d_raw, d_out, (int)n, Kp);
-    else k_na_apply<false><<<nchunks, 256, 0, st>>>(s, d_raw, d_out, (int)n, Kp);
+    asv_launch_follow(true, k_na_scan, 1, 1024, 0, st, s, d_raw, Kp, nchunks);
+    asv_launch_follow(true, ((r0 | o0) & 15) == 0 ? k_na_apply<true> : k_na_apply<false>, nchunks, 256, 0, st, s, d_raw, d_out,
+                      (int)n, Kp);
     if (cudaGetLastError() != cudaSuccess) return ASV_ERR_CUDA;
     return ASV_OK;
 }
