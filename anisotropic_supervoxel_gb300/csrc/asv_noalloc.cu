@@ -30,7 +30,7 @@
 #include <mutex>
 
 #define NA_CHUNK 2048
-#define NA_GROUP 4                  // chunks per block of the count
+#define NA_GROUP 2                  // chunks per block of the count (1: 38.2 us a call on 320x240x85, 2: 36.8, 4: 38.0)
 #define NA_FULL 0xffffffffu
 #define NA_MAX_VOXELS (1LL << 25)
 #define NA_MAX_SEEDS 32767
