@@ -163,7 +163,7 @@ def fp32_rate(ops_per_voxel, nvox, launch_s):
     if ops_per_voxel is None or not launch_s:
         return None
     return {"ops_per_voxel_ncu": ops_per_voxel, "tops": ops_per_voxel * nvox / launch_s / 1e12,
-            "what": "executed FP32 operations (ncu sass counts, no FMA executes) per voxel of the "
+            "what": "executed FP32 operations (ncu sass counts, a fused one as two) per voxel of the "
                     "captured passes x voxels / average gather-pass time"}
 
 

@@ -225,7 +225,8 @@ asv_status asv_enforce_connectivity_labels(asv_ctx *ctx, const int32_t *labels, 
  *                        truth segment) with a supervoxel boundary voxel in
  *                        their 3x3x3 neighbourhood, over all of them
  *   mean_duration        mean over labels >= 0 of last - first frame + 1
- * Label -1 counts as one more supervoxel in the other measures.  labels: D*H*W int32 in
+ * Label -1 counts as one more supervoxel in the other measures.  The context
+ * holds up to 256 MiB of device scratch after the first call.  labels: D*H*W int32 in
  * [-1, 32767); truth: D*H*W int32 in [0, 4096); both host arrays. */
 typedef struct asv_eval {
     double undersegmentation;
