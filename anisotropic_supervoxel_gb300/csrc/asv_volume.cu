@@ -670,6 +670,70 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
     }
 }
 
+// The same for steps above the bit-set form's, whose chains have few positions
+// (one at steps of D and more): the lists of slice 0 and of the last slice, where
+// chains start and end, are made once per run, in two more rows, instead of up to
+// two of three lists of every voxel (the 240x160x30 clip with its full ladder:
+// steps 64 to 8, ten iterations 3.30 ms, so 3.16).  Small steps, whose crowded
+// sub-tiles come here too, lose by it (the 64x48x12 clip 0.250 ms, so 0.256).
+__device__ __forceinline__ void asv_jfa_run_far(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+                                                const uchar4 *__restrict__ lab, const float4 *__restrict__ tab, int W,
+                                                int H, int D, int Kp, int x, int y, int p0, int n, int step,
+                                                float ratio, asv_list_t *__restrict__ lists, bool valid)
+{
+    const int sl = W * H;                       // segments hold < 2^31 voxels
+    const int xs[3] = { max(x - step, 0), x, min(x + step, W - 1) };
+    const int ys[3] = { max(y - step, 0) * W, y * W, min(y + step, H - 1) * W };
+    const int col = y * W + x;
+    const float vx = (float)x + 0.5f, vy = (float)y + 0.5f;
+    const int row = ASV_SLICE_MAX * ASV_JFA_THREADS;
+    int r, j, len;
+    asv_chain_pos(p0, D, step, r, j, len);
+    int z = r + j * step;
+    // list rows: 0 to 2 the chain's slices in turn, 3 and 4 the merge's, 5 and 6
+    // slice 0 and slice D - 1, where chains start and end
+    int rm, rc = 0, nm, n0 = -1, nl = -1;       // minus and centre rows
+    auto first = [&]() {
+        if (n0 < 0) n0 = asv_slice_list(in, 0, xs, ys, Kp, lists + 5 * row);
+        rm = 5;
+        nm = n0;
+    };
+    if (z > step) {
+        rm = 2;
+        nm = asv_slice_list(in, (z - step) * sl, xs, ys, Kp, lists + rm * row);
+    } else first();
+    int nc = asv_slice_list(in, z * sl, xs, ys, Kp, lists + rc * row);
+    while (true) {
+        const bool more = z + step < D;         // the chain goes on
+        int rp = 6, np;
+        if (more) {
+            rp = rc == 2 ? 0 : rc + 1;
+            np = asv_slice_list(in, (z + step) * sl, xs, ys, Kp, lists + rp * row);
+        } else {
+            if (nl < 0) nl = asv_slice_list(in, (D - 1) * sl, xs, ys, Kp, lists + 6 * row);
+            np = nl;
+        }
+        const uchar4 c = __ldg(lab + z * sl + col);
+        const int nx = asv_merge_lists(lists + rc * row, nc, lists + rm * row, nm, lists + rp * row, np,
+                                       lists + 3 * row);
+        const int32_t best = asv_jfa_eval(lists + rc * row, nc, lists + 3 * row, nx, tab, c, vx, vy,
+                                          (float)z + 0.5f, ratio);
+        if (valid) out[z * sl + col] = best;
+        if (--n == 0) break;
+        if (more) {                             // next voxel of the chain: rotate the rows
+            z += step;
+            rm = rc;
+            nm = nc;
+            rc = rp;
+            nc = np;
+        } else {                                // next residue: a new chain
+            z = z - (z / step) * step + 1;
+            first();
+            nc = asv_slice_list(in, z * sl, xs, ys, Kp, lists + rc * row);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Bit-set form of a JFA pass (steps 1..ASV_BITS_MAXS).
 //
@@ -729,6 +793,7 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // and its plus slice the centre of the one after it.
 // ---------------------------------------------------------------------------
 #define ASV_JFA_LIST_BYTES (5 * ASV_SLICE_MAX * ASV_JFA_THREADS * (int)sizeof(asv_list_t))
+#define ASV_JFA_FAR_BYTES (7 * ASV_SLICE_MAX * ASV_JFA_THREADS * (int)sizeof(asv_list_t))   // asv_jfa_run_far's
 #define ASV_BITS_MAXT 32         // labels per sub-tile footprint (one 32-bit mask)
 #define ASV_BITS_MAXKP 8192      // segment seed counts up to this use the bit-set form
 #define ASV_BITS_TLCAP 256       // claimed labels remembered for the reset
@@ -1339,8 +1404,12 @@ __device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int
             const unsigned past = ~(todo >> q);
             const int m = past ? __ffs(past) - 1 : 32;
             todo &= ~((0xffffffffu >> (32 - m)) << q);
-            asv_jfa_run<SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, min(gx, W - 1), min(gy, H - 1), pc + q, m,
-                              step, ratio, (asv_list_t *)smem + threadIdx.x, valid);
+            if constexpr (ST == ASV_JFA_LIST)
+                asv_jfa_run_far(in, out, lab, tab, W, H, D, Kp, min(gx, W - 1), min(gy, H - 1), pc + q, m, step, ratio,
+                                (asv_list_t *)smem + threadIdx.x, valid);
+            else
+                asv_jfa_run<SUMS>(in, out, lab, tab, sums, slot0, W, H, D, Kp, min(gx, W - 1), min(gy, H - 1), pc + q, m,
+                                  step, ratio, (asv_list_t *)smem + threadIdx.x, valid);
             __syncthreads();                                   // the list rows alias the footprint
         }
     }
@@ -1970,7 +2039,7 @@ static const AsvJfaVariant &asv_jfa_variant(int step, bool last)
         { k_jfa<1, false>, AsvBitsGeo<1>::SMEM }, { k_jfa<2, false>, AsvBitsGeo<2>::SMEM },
         { k_jfa<3, false>, AsvBitsGeo<3>::SMEM }, { k_jfa<4, false>, AsvBitsGeo<4>::SMEM },
         { k_jfa<5, false>, AsvBitsGeo<5>::SMEM }, { k_jfa<6, false>, AsvBitsGeo<6>::SMEM },
-        { k_jfa<ASV_JFA_LIST, false>, ASV_JFA_LIST_BYTES } };
+        { k_jfa<ASV_JFA_LIST, false>, ASV_JFA_FAR_BYTES } };
     return v[last ? 0 : (step < ASV_JFA_LIST ? step : ASV_JFA_LIST)];
 }
 
