@@ -85,7 +85,7 @@ static __device__ __forceinline__ bool na_scan_needed(const int *rec)
 // Neighbouring voxels mostly share a label: a warp adds each run once, found by
 // one ballot, to the block's table (grouping all equal lanes into the global
 // counts, and a second kernel for the sources, took 72 + 19 us on a 320x240x85
-// volume, this one 27 us).
+// volume, this one 20 us).
 __global__ void __launch_bounds__(256) k_na_count(NaScratch s, const int32_t *__restrict__ raw, int n, int Kp)
 {
     asv_follow();
@@ -99,11 +99,16 @@ __global__ void __launch_bounds__(256) k_na_count(NaScratch s, const int32_t *__
         const int v0 = (blockIdx.x * NA_GROUP + c) * NA_CHUNK;
         if (v0 >= n) break;
         unsigned any = 0u, other = 0u;                         // place + 1 of the last source of each rule
+        int all[NA_CHUNK / 256];                               // asked for together, before the table's accesses
 #pragma unroll
         for (int i = 0; i < NA_CHUNK / 256; i++) {
-            const int k = i * 256 + threadIdx.x, v = v0 + k;
+            const int v = v0 + i * 256 + threadIdx.x;
+            all[i] = v < n ? na_label(raw, v, Kp) : -2;
+        }
+#pragma unroll
+        for (int i = 0; i < NA_CHUNK / 256; i++) {
+            const int k = i * 256 + threadIdx.x, v = v0 + k, l = all[i];
             const bool in = v < n;
-            const int l = in ? na_label(raw, v, Kp) : -2;
             const int before = __shfl_up_sync(NA_FULL, l, 1);
             const unsigned starts = __ballot_sync(NA_FULL, lane == 0 || before != l);
             if (in && ((starts >> lane) & 1u)) {
