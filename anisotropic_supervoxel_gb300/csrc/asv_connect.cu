@@ -200,15 +200,34 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restric
         const int q = b % 9;
         cc_union_tile(sp, i - (b >= 9 ? CC_THREADS : 0) + (q / 3 - 1) * 32 + q % 3 - 1, i, err);
     };
-    if (in)
-        for (int k = 0; k < CC_TZ && t.z + k < D; k++) {
-            const int i = k * CC_THREADS + threadIdx.x;
-            const unsigned m = cc_links(sl[i], t.lane > 0, t.lane < 31 && t.x < W - 1, t.w > 0,
-                                        t.w < CC_THREADS / 32 - 1 && t.y < H - 1, k > 0, [&](int dx, int dy, int dz) {
-                                            return sl[i + dx + dy * 32 + dz * CC_THREADS];
-                                        });
-            cc_put(sc, &nq, m & ~(1u << 3), i, join);
+    if (in) {
+        // cc_links in the tile without its branches: nine labels a slice, of which
+        // the next slice's voxel sees eight again
+        const bool hw = t.lane > 0, he = t.lane < 31 && t.x < W - 1, hn = t.w > 0;
+        const bool hs = t.w < CC_THREADS / 32 - 1 && t.y < H - 1;
+        const int ow = hw ? -1 : 0, oe = he ? 1 : 0, on = hn ? -32 : 0, os = hs ? 32 : 0;   // missing: itself, not counted
+        int pw = 0, pe = 0, pn = 0, ps = 0, pnw = 0, pne = 0, psw = 0, pse = 0;
+#pragma unroll
+        for (int k = 0; k < CC_TZ; k++) {
+            if (t.z + k >= D) break;
+            const int i = k * CC_THREADS + threadIdx.x, l = sl[i];
+            const int w = sl[i + ow], e = sl[i + oe], n = sl[i + on], s = sl[i + os];
+            const int nw = sl[i + on + ow], ne = sl[i + on + oe], sw = sl[i + os + ow], se = sl[i + os + oe];
+            const bool bw = hw && w == l, bn = hn && n == l, bnw = hw && hn && nw == l;
+            unsigned m = (bn ? (bw && bnw ? 0u : 1u << 1) : (bnw && !bw ? 1u << 0 : 0u)) |
+                         (!bn && hn && he && ne == l && e != l ? 1u << 2 : 0u);
+            if (k > 0) {
+                const bool qn = hn && pn == l, qs = hs && ps == l, qw = hw && pw == l, qe = he && pe == l;
+                const bool qnw = hn && hw && pnw == l, qsw = hs && hw && psw == l;
+                m |= (qn ? (bw && qnw ? 0u : 1u << 10) : (qnw && !qw ? 1u << 9 : 0u)) |
+                     (qs ? (bw && qsw ? 0u : 1u << 16) : (qsw && !qw ? 1u << 15 : 0u));
+                if (!qn && !qs) m |= (qw ? 1u << 12 : 0u) | (qe ? 1u << 14 : 0u);
+                if (he && !qe) m |= (!qn && hn && pne == l ? 1u << 11 : 0u) | (!qs && hs && pse == l ? 1u << 17 : 0u);
+            }
+            cc_put(sc, &nq, m, i, join);
+            pw = w; pe = e; pn = n; ps = s; pnw = nw; pne = ne; psw = sw; pse = se;
         }
+    }
     __syncthreads();
     cc_make(sc, nq, join);
     __syncthreads();

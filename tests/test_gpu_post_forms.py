@@ -43,3 +43,36 @@ def test_noalloc_edges(asv, orc, shape, offset):
         got = dst.cpu().numpy()
         assert np.array_equal(got[offset:offset + n].reshape(shape), want)
         assert (np.delete(got, np.arange(offset, offset + n)) == -9).all()
+
+
+def test_noalloc_under_capture(asv, orc):
+    torch = pytest.importorskip("torch")
+    lib, shape, kp = asv.load(), (4, 64, 40), 20
+    D, H, W = shape
+    rng = np.random.default_rng(8)
+    raws = []
+    for dead in (0, 2, 5):
+        raw = _blocky(rng, shape, kp - dead)
+        raw[rng.random(shape) < 0.1] = -1
+        raws.append(raw)
+    src = torch.from_numpy(raws[0]).cuda()
+    dst = torch.empty_like(src)
+
+    def call():
+        return lib.asv_check_dead_seeds_noalloc(src.data_ptr(), dst.data_ptr(), W, H, D, kp,
+                                                torch.cuda.current_stream().cuda_stream)
+
+    assert call() == 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        st = call()
+    assert st == 0
+    for raw in raws:
+        src.copy_(torch.from_numpy(raw))
+        graph.replay()
+        torch.cuda.synchronize()
+        counts = np.zeros((kp + 1, 7), np.int64)
+        counts[:, 3] = np.bincount(np.where(raw < 0, kp, raw).ravel(), minlength=kp + 1)
+        want, _ = orc.postprocess(raw, counts, kp)
+        assert np.array_equal(dst.cpu().numpy(), want)
