@@ -31,7 +31,7 @@
 // imply (cc_links), all kinds in one loop, so that the lanes' walks run side by
 // side.  On the 320x240x85 clip's labels: 12 links per voxel, one after the
 // other, 543 us; a root walk and an atomic per voxel 113 us, segments numbered by
-// few blocks 91 us, 18 jumping rounds 60 us; now 105 us in the tiles
+// few blocks 91 us, 18 jumping rounds 60 us; now 95 us in the tiles
 // and 58 between them, 28, 12 and 17 us.
 // Compiled with -fmad=false (integer work only).
 #include "asv_connect.cuh"
@@ -137,24 +137,26 @@ __device__ __forceinline__ unsigned cc_links(int l, bool hw, bool he, bool hn, b
 
 // A block's links, put down first and then made by all its threads: a few voxels
 // in a warp have links, and each link is a chain of dependent accesses.  An entry:
-// the voxel's place in the tile and the link's bit; those that find no room are
-// made at once by fn(place, bit).
-template <class F>
-__device__ __forceinline__ void cc_put(int *queue, int *count, unsigned m, int i, F fn)
+// the voxel's place in the tile and its links' bits, so a tile's voxels have room.
+// By whole warps, m = 0 without links.
+__device__ __forceinline__ void cc_put(unsigned *queue, int *count, unsigned m, int i)
 {
-    if (!m) return;
-    int at = atomicAdd(count, __popc(m));
-    for (; m; m &= m - 1, at++) {
-        const int b = __ffs(m) - 1;
-        if (at < CC_TILE) queue[at] = (i << 5) | b;
-        else fn(i, b);
-    }
+    const unsigned some = __ballot_sync(0xffffffffu, m != 0u);
+    if (!some) return;
+    const int lane = threadIdx.x & 31, lead = __ffs(some) - 1;
+    int at = 0;
+    if (lane == lead) at = atomicAdd(count, __popc(some));
+    at = __shfl_sync(0xffffffffu, at, lead) + __popc(some & ((1u << lane) - 1u));
+    if (m) queue[at] = ((unsigned)i << 18) | m;
 }
 
 template <class F>
-__device__ __forceinline__ void cc_make(const int *queue, int count, F fn)
+__device__ __forceinline__ void cc_make(const unsigned *queue, int count, F fn)
 {
-    for (int j = threadIdx.x; j < min(count, CC_TILE); j += CC_THREADS) fn(queue[j] >> 5, queue[j] & 31);
+    for (int j = threadIdx.x; j < count; j += CC_THREADS) {
+        const unsigned e = queue[j];
+        for (unsigned m = e & 0x3ffffu; m; m &= m - 1) fn((int)(e >> 18), __ffs(m) - 1);
+    }
 }
 
 struct CcTile {
@@ -200,11 +202,11 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restric
         const int q = b % 9;
         cc_union_tile(sp, i - (b >= 9 ? CC_THREADS : 0) + (q / 3 - 1) * 32 + q % 3 - 1, i, err);
     };
-    if (in) {
+    if (t.y < H) {
         // cc_links in the tile without its branches: nine labels a slice, of which
         // the next slice's voxel sees eight again
-        const bool hw = t.lane > 0, he = t.lane < 31 && t.x < W - 1, hn = t.w > 0;
-        const bool hs = t.w < CC_THREADS / 32 - 1 && t.y < H - 1;
+        const bool hw = in && t.lane > 0, he = t.lane < 31 && t.x < W - 1, hn = in && t.w > 0;
+        const bool hs = in && t.w < CC_THREADS / 32 - 1 && t.y < H - 1;
         const int ow = hw ? -1 : 0, oe = he ? 1 : 0, on = hn ? -32 : 0, os = hs ? 32 : 0;   // missing: itself, not counted
         int pw = 0, pe = 0, pn = 0, ps = 0, pnw = 0, pne = 0, psw = 0, pse = 0;
 #pragma unroll
@@ -224,12 +226,12 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restric
                 if (!qn && !qs) m |= (qw ? 1u << 12 : 0u) | (qe ? 1u << 14 : 0u);
                 if (he && !qe) m |= (!qn && hn && pne == l ? 1u << 11 : 0u) | (!qs && hs && pse == l ? 1u << 17 : 0u);
             }
-            cc_put(sc, &nq, m, i, join);
+            cc_put((unsigned *)sc, &nq, m, i);
             pw = w; pe = e; pn = n; ps = s; pnw = nw; pne = ne; psw = sw; pse = se;
         }
     }
     __syncthreads();
-    cc_make(sc, nq, join);
+    cc_make((const unsigned *)sc, nq, join);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < CC_TZ; k++) sc[k * CC_THREADS + threadIdx.x] = 0;
@@ -256,7 +258,8 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_union(const int32_t *__restri
     asv_follow();
     constexpr unsigned PREV = 0x1ffu << 9, NORTH = 7u | (7u << 9), SOUTH = 7u << 15, WEST = 0x9249u, EAST = WEST << 2;
     constexpr int NW = CC_THREADS / 32, ROWS = NW + 2 * (CC_TZ - 1), TASKS = ROWS + 2 * NW * CC_TZ / 32;
-    __shared__ int queue[CC_TILE], nq;
+    __shared__ unsigned queue[CC_TILE];
+    __shared__ int nq;
     if (threadIdx.x == 0) nq = 0;
     __syncthreads();
     const CcTile t(tx, ty);
@@ -286,10 +289,16 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_union(const int32_t *__restri
             m = cross & cc_links(__ldg(p), x > 0, x < W - 1, y > 0, y < H - 1, z > 0,
                                  [&](int dx, int dy, int dz) { return __ldg(p + dx + dy * W + dz * fr); });
         }
-        cc_put(queue, &nq, m, k * CC_THREADS + r * 32 + lane, join);
+        // an entry per link: two in a row by one thread wait twice as long here
+        const int i = k * CC_THREADS + r * 32 + lane;
+        int at = m ? atomicAdd(&nq, __popc(m)) : 0;
+        for (; m; m &= m - 1, at++) {
+            if (at < CC_TILE) queue[at] = ((unsigned)i << 18) | (m & (0u - m));
+            else join(i, __ffs(m) - 1);
+        }
     }
     __syncthreads();
-    cc_make(queue, nq, join);
+    cc_make(queue, min(nq, CC_TILE), join);
 }
 
 // par[v] = root, the tiles' component sizes added up at the roots, roots per
