@@ -146,31 +146,38 @@ __global__ void __launch_bounds__(1024) k_na_scan(NaScratch s, const int32_t *__
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
-    for (int b0 = 0; b0 < Kp; b0 += blockDim.x) {
-        int i = b0 + threadIdx.x;
-        int alive = (i < Kp && s.counts[i] >= 1) ? 1 : 0;
-        unsigned bal = __ballot_sync(NA_FULL, alive);
-        int pre = __popc(bal & ((1u << lane) - 1u));
-        if (lane == 0) warp_tot[w] = __popc(bal);
+    // four seeds a thread (the counts and the sources end on multiples of four)
+    for (int b0 = 0; b0 < Kp; b0 += 4096) {
+        const int i0 = b0 + 4 * threadIdx.x;
+        unsigned alive = 0u;
+        if (i0 < Kp) {
+            const uint4 q = *(const uint4 *)(s.counts + i0);
+            alive = (q.x ? 1u : 0u) | (q.y ? 2u : 0u) | (q.z ? 4u : 0u) | (q.w ? 8u : 0u);
+            if (Kp - i0 < 4) alive &= (1u << (Kp - i0)) - 1u;
+        }
+        int incl = __popc(alive);
+        for (int o = 1; o < 32; o <<= 1) { const int q = __shfl_up_sync(NA_FULL, incl, o); if (lane >= o) incl += q; }
+        if (lane == 31) warp_tot[w] = incl;
         __syncthreads();
         if (threadIdx.x < 32) {
-            int v = warp_tot[threadIdx.x];
-            int incl = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                int m = __shfl_up_sync(NA_FULL, incl, o);
-                if (threadIdx.x >= o) incl += m;
+            int ix = warp_tot[threadIdx.x];
+            for (int o = 1; o < 32; o <<= 1) { const int q = __shfl_up_sync(NA_FULL, ix, o); if (threadIdx.x >= o) ix += q; }
+            warp_tot[threadIdx.x] = ix;
+        }
+        __syncthreads();
+        const int before = carry + (w > 0 ? warp_tot[w - 1] : 0) + incl - __popc(alive);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const int i = i0 + k, live_before = before + __popc(alive & ((1u << k) - 1u));
+            const bool live = (alive >> k) & 1u;
+            if (i < Kp) {
+                s.rank[i] = live ? live_before : -1;
+                const int dead_before = i - live_before;        // the first four dead seeds, in order
+                if (!live && dead_before < 4) s.rec[R_DEAD0 + dead_before] = i;
             }
-            warp_tot[threadIdx.x] = incl - v;
         }
         __syncthreads();
-        if (i < Kp) {
-            const int live_before = carry + warp_tot[w] + pre;
-            s.rank[i] = alive ? live_before : -1;
-            const int dead_before = i - live_before;        // the first four dead seeds, in order
-            if (!alive && dead_before < 4) s.rec[R_DEAD0 + dead_before] = i;
-        }
-        __syncthreads();
-        if (threadIdx.x == blockDim.x - 1) carry += warp_tot[w] + pre + alive;
+        if (threadIdx.x == 0) carry += warp_tot[31];
         __syncthreads();
     }
     const int dead = Kp - carry;
@@ -187,10 +194,19 @@ __global__ void __launch_bounds__(1024) k_na_scan(NaScratch s, const int32_t *__
     __syncthreads();
     if (!na_scan_needed(s.rec)) return;
     const int half = s.rec[R_MODE] == 2 ? 16 : 0;
-    for (int b0 = 0; b0 < nchunks; b0 += blockDim.x) {
-        const int c = b0 + threadIdx.x;
-        const int place = c < nchunks ? (s.scan[c] >> half) & 0xffff : 0;
-        int incl = place ? c * NA_CHUNK + place : 0;
+    for (int b0 = 0; b0 < nchunks; b0 += 4096) {
+        const int c0 = b0 + 4 * threadIdx.x;
+        int v[4] = { 0, 0, 0, 0 };                             // voxel + 1 of the chunk's last source
+        if (c0 < nchunks) {
+            const int4 q = *(const int4 *)(s.scan + c0);
+            const int p[4] = { q.x, q.y, q.z, q.w };
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int place = c0 + k < nchunks ? (p[k] >> half) & 0xffff : 0;
+                v[k] = place ? (c0 + k) * NA_CHUNK + place : 0;
+            }
+        }
+        int incl = max(max(v[0], v[1]), max(v[2], v[3]));
         for (int o = 1; o < 32; o <<= 1) { int q = __shfl_up_sync(NA_FULL, incl, o); if (lane >= o && q > incl) incl = q; }
         if (lane == 31) warp_tot[w] = incl;
         __syncthreads();
@@ -202,10 +218,14 @@ __global__ void __launch_bounds__(1024) k_na_scan(NaScratch s, const int32_t *__
         __syncthreads();
         int ew = __shfl_up_sync(NA_FULL, incl, 1);
         if (lane == 0) ew = 0;
-        const int ex = max(max(carry, w > 0 ? warp_tot[w - 1] : 0), ew), tot = max(carry, warp_tot[31]);
+        int ex = max(max(carry, w > 0 ? warp_tot[w - 1] : 0), ew);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (c0 + k < nchunks) s.scan[c0 + k] = ex;
+            ex = max(ex, v[k]);
+        }
         __syncthreads();
-        if (c < nchunks) s.scan[c] = ex;
-        if (threadIdx.x == 0) carry = tot;
+        if (threadIdx.x == 0) carry = max(carry, warp_tot[31]);
         __syncthreads();
     }
 }

@@ -76,3 +76,24 @@ def test_noalloc_under_capture(asv, orc):
         counts[:, 3] = np.bincount(np.where(raw < 0, kp, raw).ravel(), minlength=kp + 1)
         want, _ = orc.postprocess(raw, counts, kp)
         assert np.array_equal(dst.cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("kp,dead", [(4095, (0, 4094)), (4096, (3, 4095)), (4098, (4095, 4096)), (9000, (1, 4096, 8191, 8192, 8999)),
+                                     (4100, (4096, 4097, 4098, 4099))])
+def test_noalloc_scan_rounds(asv, orc, kp, dead):
+    """Ranks and chunk carries over several rounds of 4096, sources rounds apart."""
+    torch = pytest.importorskip("torch")
+    lib, W, H, D = asv.load(), 2048, 1, 4099
+    n = W * H * D
+    alive = np.setdiff1d(np.arange(kp), dead).astype(np.int32)
+    raw = alive[(np.arange(n) // 3) % len(alive)].reshape(D, H, W)
+    raw[5:4097] = -1                                # chunks without a source across a round's end
+    raw[4097, 0, 9:] = -1
+    counts = np.zeros((kp + 1, 7), np.int64)
+    counts[:, 3] = np.bincount(np.where(raw < 0, kp, raw).ravel(), minlength=kp + 1)
+    want, _ = orc.postprocess(raw, counts, kp)
+    src = torch.from_numpy(raw).cuda()
+    dst = torch.empty_like(src)
+    assert lib.asv_check_dead_seeds_noalloc(src.data_ptr(), dst.data_ptr(), W, H, D, kp,
+                                            torch.cuda.current_stream().cuda_stream) == 0
+    assert np.array_equal(dst.cpu().numpy(), want)
