@@ -112,18 +112,30 @@ __global__ void __launch_bounds__(EV_T) k_ev_sbound(const int32_t *__restrict__ 
     }
 }
 
-// flags of 32 voxels of row y, those of their neighbours along x and z included
-__device__ __forceinline__ unsigned ev_around(const unsigned *__restrict__ sb, int tx, int H, int D, int xt, int y, int z)
-{
-    const int lane = threadIdx.x & 31, zz = z + lane - 1;
-    unsigned m = 0;
-    if (lane < 3 && zz >= 0 && zz < D && y >= 0 && y < H) {
-        const unsigned *p = sb + ((size_t)zz * H + y) * tx + xt;
-        const unsigned w = __ldg(p);
-        m = w | (w << 1) | (w >> 1) | (xt > 0 ? __ldg(p - 1) >> 31 : 0u) | (xt < tx - 1 ? __ldg(p + 1) << 31 : 0u);
+// Flags of 32 voxels of one row after the other, those of their neighbours along x
+// and z included: lanes 0 to 2 each go down one slice's words
+struct EvFlags {
+    const unsigned *p;
+    int tx;
+    bool mine, left, right;
+
+    __device__ __forceinline__ EvFlags(const unsigned *sb, int tx_, int H, int D, int xt, int y, int z)
+    {
+        const int zz = z + (int)(threadIdx.x & 31) - 1;
+        tx = tx_;
+        mine = (threadIdx.x & 31) < 3 && zz >= 0 && zz < D;
+        left = mine && xt > 0;
+        right = mine && xt < tx - 1;
+        p = sb + ((long long)zz * H + y) * tx + xt;
     }
-    return __reduce_or_sync(0xffffffffu, m);
-}
+    __device__ __forceinline__ unsigned step(bool there)       // the next row (outside the volume: none)
+    {
+        const unsigned w = mine && there ? __ldg(p) : 0u, a = left && there ? __ldg(p - 1) : 0u;
+        const unsigned c = right && there ? __ldg(p + 1) : 0u;
+        p += tx;
+        return __reduce_or_sync(0xffffffffu, w | __funnelshift_l(a, w, 1) | __funnelshift_r(w, c, 1));
+    }
+};
 
 // hands out c voxels of (supervoxel, truth) key in frame z; the frame range goes
 // out where it widens the one read
@@ -160,12 +172,13 @@ __global__ void __launch_bounds__(EV_T) k_ev_counts(const int32_t *__restrict__ 
     if (y0 < H) {
         EvRows row(gt, W, H, D, x, y0, z);
         const int32_t *pl = lab + (size_t)z * W * H + (size_t)y0 * W + x;
-        unsigned above = ev_around(sb, tx, H, D, xt, y0 - 1, z), here = ev_around(sb, tx, H, D, xt, y0, z);
+        EvFlags flags(sb, tx, H, D, xt, y0 - 1, z);
+        unsigned above = flags.step(y0 > 0), here = flags.step(true);
 #pragma unroll
         for (int k = 0; k < EV_ROWS; k++) {
             if (y0 + k >= H) break;
             const int s = row.in ? __ldg(pl + (size_t)k * W) + 1 : 0;
-            const unsigned below = ev_around(sb, tx, H, D, xt, y0 + k + 1, z);
+            const unsigned below = flags.step(y0 + k + 1 < H);
             int g;
             const bool b = row.step(y0 + k < H - 1, &g);
             const int key = row.in ? s * NG + g : -1;
