@@ -155,7 +155,7 @@ __device__ __forceinline__ void ev_out(int key, unsigned c, int z, int NG, unsig
 // frame in shared memory, a run of a row at a time, and keeps the rows' values
 // and flags while it goes down them.  (Equal lanes of a warp grouped into three
 // global updates, and nine rows of a byte volume per boundary voxel: 135 + 100 us
-// on a 320x240x85 volume, now 73 us.)
+// on a 320x240x85 volume, now 71 us.)
 __global__ void __launch_bounds__(EV_T) k_ev_counts(const int32_t *__restrict__ lab, const int32_t *__restrict__ gt,
                                                     int W, int H, int D, int tx, int ty, int NG,
                                                     unsigned *__restrict__ cnt, int *__restrict__ zmin,
