@@ -208,7 +208,8 @@ struct asv_ctx {
     // (seed counts, segment descriptor) is read from device memory
     cudaGraphExec_t sgexec = nullptr;
     AsvDev skey{};
-    int skey_blocks = -1, skey_passes = -1, skey_iters = -1, sg_launches = 0;
+    int skey_blocks = -1, skey_iters = -1, sg_launches = 0;
+    std::vector<int> skey_kinds;                   // k_jfa's variant of every pass (jfa_kind)
     // copy stream of asv_stream_feed and its events (created on first use):
     // fed_ev[k] = slot k's upload done, used_ev[k] = slot k read by its push
     cudaStream_t cp = nullptr;
@@ -657,6 +658,14 @@ static void do_first_init(asv_ctx *ctx)
     ctx->launches += 2;
 }
 
+// k_jfa's variant for pass p of a segment: its step (capped at the list form's),
+// and whether it is the last pass.  The host chooses it, so a captured graph is
+// good for segments with the same variants only.
+static int jfa_kind(const SegDesc &s, int p)
+{
+    return 2 * std::min(s.steps[p], ASV_BITS_MAXS + 1) + (p == s.npass - 1);
+}
+
 // Pass p of every segment that has it: a launch of k_jfa's variant for each
 // different step (and for the segments whose last pass it is); the first on the
 // context's stream, the others beside it on the side stream, where their blocks
@@ -665,10 +674,10 @@ static void do_first_init(asv_ctx *ctx)
 // it is now.
 static bool do_pass(asv_ctx *ctx, int p, bool follow)
 {
-    int kinds[2 * (ASV_BITS_MAXS + 2)], n = 0;                // step (capped at the list form's), last pass
+    int kinds[2 * (ASV_BITS_MAXS + 2)], n = 0;
     for (const SegDesc &s : ctx->sd) {
         if (p >= s.npass) continue;
-        const int k = 2 * std::min(s.steps[p], ASV_BITS_MAXS + 1) + (p == s.npass - 1);
+        const int k = jfa_kind(s, p);
         if (std::find(kinds, kinds + n, k) == kinds + n) kinds[n++] = k;
     }
     if (n > 1) {
@@ -2069,8 +2078,10 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
     asv_launch_metric(d, 0, st);
     ctx->launches += 3;
     if (ctx->cfg.use_graph && !ctx->cfg.instrument) {
+        std::vector<int> kinds(sd.npass);                          // (also the number of passes)
+        for (int p = 0; p < sd.npass; p++) kinds[p] = jfa_kind(sd, p);
         const bool same = ctx->sgexec && std::memcmp(&ctx->skey, &d, sizeof(AsvDev)) == 0 &&
-                          ctx->skey_blocks == ctx->jfa_blocks && ctx->skey_passes == ctx->maxpass &&
+                          ctx->skey_blocks == ctx->jfa_blocks && ctx->skey_kinds == kinds &&
                           ctx->skey_iters == ctx->cfg.lloyd_iters;
         if (!same) {
             if (ctx->sgexec) { cudaGraphExecDestroy(ctx->sgexec); ctx->sgexec = nullptr; }
@@ -2085,7 +2096,7 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
             if (e != cudaSuccess) { ctx->sgexec = nullptr; return cuda_fail(ctx, e, "cudaGraphInstantiate"); }
             std::memcpy(&ctx->skey, &d, sizeof(AsvDev));
             ctx->skey_blocks = ctx->jfa_blocks;
-            ctx->skey_passes = ctx->maxpass;
+            ctx->skey_kinds = kinds;
             ctx->skey_iters = ctx->cfg.lloyd_iters;
             ctx->sg_launches = ctx->launches - before;
         } else {
