@@ -973,7 +973,9 @@ __device__ __forceinline__ void asv_bits_reset(AsvBitsShared &b, int T)
 // Any closer voxel is evaluated in the shader's order (asv_bits_exact), so
 // the labels are the shader's in every case.  A label whose A or colour is
 // not finite or so large that a distance might reach 1e8 gives an infinite
-// margin: that sub-tile takes no scores.
+// margin: that sub-tile takes no scores.  So does a negative ratio (a caller's own
+// pass): the shader clamps the form before it is multiplied, and max(ratio * form, 0)
+// is that only for ratios of zero and more.
 // ---------------------------------------------------------------------------
 #define ASV_EPS 5.9604645e-8f    // 2^-24
 
@@ -1009,7 +1011,7 @@ __device__ __forceinline__ void asv_bits_coefs(AsvBitsShared &b, int T, float ox
     const float A = fabsf(a00) * X * X + fabsf(a01) * X * Y + fabsf(a02) * X * Z + fabsf(a11) * Y * Y +
                     fabsf(a12) * Y * Z + fabsf(a22) * Z * Z;
     const float smax = fmaxf(fmaxf(fabsf(s[0]), fabsf(s[1])), fabsf(s[2]));
-    const bool ok = A < 1e7f && smax < 1000.0f && s[0] == s[0] && s[1] == s[1] && s[2] == s[2];   // false for NaN
+    const bool ok = ratio >= 0.0f && A < 1e7f && smax < 1000.0f && s[0] == s[0] && s[1] == s[1] && s[2] == s[2];   // false for NaN
     const float mg = ok ? 72.0f * ASV_EPS * A + 32.0f * ASV_EPS * c0 + 1e-30f : __int_as_float(0x7f800000);
     const unsigned top = __reduce_max_sync(FULL, on ? __float_as_uint(mg) : 0u);     // non-negative floats
     const unsigned stop = __reduce_max_sync(FULL, on && ok ? __float_as_uint(smax) : 0u);
