@@ -1592,9 +1592,8 @@ asv_status asv_jfa_pass_host(asv_ctx *ctx, int step, float ratio, const int32_t 
     one.depth[0] = std::min(16, std::max(asv_jfa_slots(step) - 2, 0));
     AsvDev d = ctx->d;
     d.segs = ctx->d.segs + 1;
-    CK(cudaMemcpyAsync((void *)d.segs, &one, sizeof(one), cudaMemcpyHostToDevice, ctx->st));
-    asv_launch_label_clean(din, s.nvox, s.Kp, ctx->st);
-    asv_launch_jfa(d, 0, step, false, ctx->jfa_blocks, false, ctx->st);
+    asv_launch_pass_prepare(din, one, ctx->d.segs, (SegDesc *)d.segs, ctx->st);
+    asv_launch_jfa(d, 0, step, false, ctx->jfa_blocks, true, ctx->st);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out, dout, 4 * n, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));

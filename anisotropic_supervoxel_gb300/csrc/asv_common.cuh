@@ -124,7 +124,8 @@ void asv_launch_draw(const AsvDev &d, cudaStream_t st);
 void asv_launch_jfa(const AsvDev &d, int pass, int step, bool last, int grid_blocks, bool follow, cudaStream_t st);
 void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t st);
 void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st);
-void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st);
+// (seg, out: on the device)
+void asv_launch_pass_prepare(int32_t *labels, const SegDesc &one, const SegDesc *seg, SegDesc *out, cudaStream_t st);
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st);
 void asv_launch_finalize(const AsvDev &d, cudaStream_t st);
 void asv_launch_post(const AsvDev &d, cudaStream_t st);

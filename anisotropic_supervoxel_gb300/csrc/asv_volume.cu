@@ -9,6 +9,7 @@
 
 #include <cuda_fp16.h>
 
+#include <cstddef>
 #include <mutex>
 
 #define FULL 0xffffffffu
@@ -1668,11 +1669,17 @@ __global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
     }
 }
 
-// a caller's labels outside [0, Kp) become -1, as the passes' own labels are
-__global__ void k_label_clean(int32_t *__restrict__ lbl, long long n, int Kp)
+// Before a single pass over a caller's labels: those outside [0, Kp) become -1, as
+// the passes' own are, and the pass's descriptor goes to *out.  Kp is the segment's
+// on the device, where a streaming window's seeds are counted (k_stream_compose).
+__global__ void k_pass_prepare(int32_t *lbl, const __grid_constant__ SegDesc one, const SegDesc *seg, SegDesc *out)
 {
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (v < n && (unsigned)lbl[v] >= (unsigned)Kp) lbl[v] = -1;
+    const int Kp = seg->Kp;
+    if (v < one.nvox && (unsigned)lbl[v] >= (unsigned)Kp) lbl[v] = -1;
+    if (blockIdx.x) return;
+    for (int i = threadIdx.x; i < (int)(sizeof(SegDesc) / 4); i += blockDim.x)
+        ((int *)out)[i] = i == (int)(offsetof(SegDesc, Kp) / 4) ? Kp : ((const int *)&one)[i];
 }
 
 // ---------------------------------------------------------------------------
@@ -2123,9 +2130,9 @@ void asv_launch_jfa_second_scatter(const AsvDev &d, bool undraw, cudaStream_t st
     asv_launch_follow(undraw, k_jfa_second, blocks, 256, 0, st, d, undraw);      // (undraw: behind the first pass)
 }
 
-void asv_launch_label_clean(int32_t *labels, long long nvox, int Kp, cudaStream_t st)
+void asv_launch_pass_prepare(int32_t *labels, const SegDesc &one, const SegDesc *seg, SegDesc *out, cudaStream_t st)
 {
-    k_label_clean<<<(unsigned)((nvox + 255) / 256), 256, 0, st>>>(labels, nvox, Kp);
+    k_pass_prepare<<<(unsigned)((one.nvox + 255) / 256), 256, 0, st>>>(labels, one, seg, out);
 }
 
 void asv_launch_centroids(const AsvDev &d, cudaStream_t st) { k_centroids<<<d.total_chunks, 256, 0, st>>>(d); }
