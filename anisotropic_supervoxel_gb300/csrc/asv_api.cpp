@@ -726,7 +726,10 @@ static bool do_flood(asv_ctx *ctx, int evbase, bool loop)
 // the reseed of centroids_next_seeds (the sums came with the flood)
 static void do_centroids(asv_ctx *ctx, bool reseed)
 {
-    if (reseed) { asv_launch_finalize(ctx->d, ctx->st); ctx->launches++; }
+    if (!reseed) return;
+    asv_launch_finalize(ctx->d, ctx->st);
+    ctx->launches++;
+    ctx->undraw = false;      // the seeds move away from where they were drawn
 }
 
 // per-label sums of the labels in the final buffers (caller-supplied labels)
