@@ -1194,6 +1194,7 @@ asv_status asv_run_lloyd(asv_ctx *ctx)
         CK(cudaGetLastError());
         ctx->stats.launches = ctx->launches;
     }
+    ctx->drawn = ctx->undraw = false;      // (a replayed graph leaves the flags as they are)
     ctx->seeded = true;
     ctx->ran = true;
     return ASV_OK;
@@ -2126,6 +2127,7 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
     m.next++;
     m.fed_next = std::max(m.fed_next, m.next);
     ctx->have_rgb = ctx->have_flow = ctx->have_pos0 = ctx->have_M0 = ctx->have_lab = true;
+    ctx->drawn = ctx->undraw = false;                      // (a replayed graph leaves the flags as they are)
     ctx->seeded = ctx->ran = true;
     auto &f = m.flight[m.nflight++];
     f.block = b;

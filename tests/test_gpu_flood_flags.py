@@ -50,3 +50,18 @@ def test_seeds_moved_after_their_draw(asv, orc, K):
         img.flood(2)
         img.check_dead_seeds()
         assert mismatch(img.raw_labels(), _flood(orc, img, drawn, vol)) == 0
+
+
+def test_flood_after_a_replayed_loop(asv, orc):
+    """A draw before the loop's second run, which replays the captured graph, is
+    not the flood's: it gathers from the labels that the loop left."""
+    W, H, D = 48, 40, 16
+    with _image(asv, W, H, D, 40) as img:
+        img.run_lloyd()
+        img.Ld_first_init()
+        img.run_lloyd()
+        vol = img.raw_labels() if img.info().passes % 2 == 0 else img.labels()
+        want = _flood(orc, img, img.seeds(), vol)
+        img.flood(1)
+        img.check_dead_seeds()
+        assert mismatch(img.raw_labels(), want) == 0
