@@ -361,7 +361,7 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
         long long n = (long long)s.W * s.H * s.D;
         vox += (size_t)((n + ASV_CHUNK - 1) / ASV_CHUNK) * ASV_CHUNK;
         chunks += (size_t)((n + ASV_CHUNK - 1) / ASV_CHUNK);
-        seeds += (size_t)((s.Kp + 64 + 31) / 32) * 32;
+        seeds += (size_t)asv_seed_slots(s.Kp);
         cells += s.W + s.H + s.D + 2 * s.g.wNum;
     }
     // rgb 3 + lab 4 + fwd/bwd 16 + two label buffers 8 + drawn seeds 4
@@ -553,7 +553,7 @@ asv_status asv_build_layout(asv_ctx *ctx)
         vox += (long long)nchunk * ASV_CHUNK;
         chunks += nchunk;
         tiles += s.tiles_x * s.tiles_y * ((h.D + s.zrun - 1) / s.zrun);
-        seeds += ((h.Kp + 64 + 31) / 32) * 32;
+        seeds += asv_seed_slots(h.Kp);
         cells += h.W + h.H + h.D + 2 * h.g.wNum;
         ctx->maxpass = std::max(ctx->maxpass, h.npass);
     }
@@ -762,7 +762,7 @@ static void loop_fills(asv_ctx *ctx, bool first)
     if (first) {
         cudaMemsetAsync(d.drawn, 0xff, bytes, ctx->side);
         cudaMemsetAsync(d.sums, 0, sizeof(unsigned long long) * 8 * (size_t)d.total_seeds, ctx->side);
-        cudaMemsetAsync(d.tcount, 0, sizeof(int), ctx->side);
+        cudaMemsetAsync(d.tcount, 0, sizeof(*d.tcount), ctx->side);
     }
     cudaMemsetAsync(d.labB, 0xff, bytes, ctx->side);
     cudaMemsetAsync(d.labA, 0xff, bytes, ctx->side);
@@ -1632,7 +1632,7 @@ asv_status asv_synchronize(asv_ctx *ctx)
 static asv_status batch_segments(asv_ctx *ctx, int n, const int *W, const int *H, const int *D,
                                  const int *K, std::vector<SegHost> *v)
 {
-    if (n < 1 || n > 4096 || !W || !H || !D || !K) return fail(ctx, ASV_ERR_BAD_ARG, "bad batch description");
+    if (n < 1 || n > ASV_MAX_CLIPS || !W || !H || !D || !K) return fail(ctx, ASV_ERR_BAD_ARG, "bad batch description");
     v->clear();
     for (int i = 0; i < n; i++) {
         SegHost h;

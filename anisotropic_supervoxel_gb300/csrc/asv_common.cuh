@@ -46,6 +46,25 @@ enum {
 };
 
 #ifdef __CUDACC__
+#define ASV_HD __host__ __device__ __forceinline__
+#else
+#define ASV_HD inline
+#endif
+
+// A batch has up to ASV_MAX_CLIPS clips of up to 32767 seeds, each in a run of
+// slots rounded up, 134 million in all: 27 or ASV_RING of something per seed
+// pass 2^31 and stay below 2^32, bytes and words of them pass that too.
+#define ASV_MAX_CLIPS 4096
+ASV_HD int asv_seed_slots(int Kp) { return ((Kp + 64 + 31) / 32) * 32; }
+
+// blocks of 256 for a thread per seed slot and voxel around it; solves of the rings
+ASV_HD unsigned asv_first_blocks(int slots) { return (27u * (unsigned)slots + 255u) / 256u; }
+ASV_HD unsigned asv_ring_tasks(int slots) { return (unsigned)ASV_RING * (unsigned)slots; }
+
+// place of ring neighbour t of seed slot g (of Mring's rows of 8 floats, of ringok)
+ASV_HD size_t asv_ring_at(int g, int t) { return (size_t)ASV_RING * g + t; }
+
+#ifdef __CUDACC__
 // n / d for n < 2^24, d <= 256, from inv = ceil(2^32 / d) (0 for d = 1): inv * d
 // exceeds 2^32 by less than d, so the product's error stays below 1 / d.
 __device__ __forceinline__ int asv_quotient(int n, unsigned inv)
@@ -90,7 +109,7 @@ struct AsvDev {
     int32_t *labA, *labB;
     int32_t *drawn;              // the drawn seeds at their voxels, else -1 (loop: all -1 between its draws; else labA)
     int4 *tlist;                 // voxels labelled by the first pass: (segment, voxel, label, -), 27 per seed
-    int *tcount;                 // entries of tlist
+    unsigned *tcount;            // entries of tlist
     float4 *pos0;                // initial seeds (density placement)
     float *M0;                   // initial metric, 8 floats / seed
     float4 *pos, *slab;          // working seeds

@@ -421,14 +421,14 @@ __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
 {
     asv_follow();
     const bool writer = (threadIdx.x & 15) == 0;
-    const int step = (gridDim.x * blockDim.x) >> 4, tasks = *d.negcount * ASV_RING;
-    for (int task0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; task0 < tasks; task0 += step) {
-        const int task = task0 + ((threadIdx.x >> 4) & 1);     // of this half
+    const unsigned step = (gridDim.x * blockDim.x) >> 4, tasks = asv_ring_tasks(*d.negcount);
+    for (unsigned task0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; task0 < tasks; task0 += step) {
+        const unsigned task = task0 + ((threadIdx.x >> 4) & 1);   // of this half
         bool active = task < tasks;
-        const int g = d.neglist[active ? task / ASV_RING : 0], t = active ? task % ASV_RING : 0;
+        const int g = d.neglist[active ? task / ASV_RING : 0], t = active ? (int)(task % ASV_RING) : 0;
         SeedRef r;
         asv_seed_ref(d, g, r);
-        int *ok = d.ringok + ASV_RING * g + t;
+        int *ok = d.ringok + asv_ring_at(g, t);
         const SegDesc &S = d.segs[r.si];
         float4 p = reseed ? d.pos[g] : d.pos0[g];
         float fx = floorf(p.x), fy = floorf(p.y);
@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(128) k_metric_ring(AsvDev d, int reseed)
         float M[6];
         asv_metric_solve(active, fwd, bwd, S.W, S.H, S.D, nx, ny, frame, M);
         if (active && writer) {
-            float *dst = d.Mring + 8 * (ASV_RING * g + t);
+            float *dst = d.Mring + 8 * asv_ring_at(g, t);
 #pragma unroll
             for (int e = 0; e < 6; e++) dst[e] = M[e];
             *ok = asv_m6_negative_quick(M) ? 0 : 1;
@@ -469,14 +469,14 @@ __device__ __forceinline__ void asv_metric_result(const AsvDev &d, int g, int ne
     float sum[6] = { 0, 0, 0, 0, 0, 0 };
     int n = 0;
     for (int t0 = 0; t0 < ASV_RING && !done; t0 += 8) {
-        const int4 *fl = (const int4 *)(d.ringok + ASV_RING * g + t0);
+        const int4 *fl = (const int4 *)(d.ringok + asv_ring_at(g, t0));
         const int4 f0 = fl[0], f1 = fl[1];
         const int ok[8] = { f0.x, f0.y, f0.z, f0.w, f1.x, f1.y, f1.z, f1.w };
         float m[8][6];
 #pragma unroll
         for (int t = 0; t < 8; t++)
             if (ok[t]) {
-                const float *q = d.Mring + 8 * (ASV_RING * g + t0 + t);
+                const float *q = d.Mring + 8 * asv_ring_at(g, t0 + t);
                 const float4 a = *(const float4 *)q;
                 const float2 b = *(const float2 *)(q + 4);
                 m[t][0] = a.x; m[t][1] = a.y; m[t][2] = a.z; m[t][3] = a.w; m[t][4] = b.x; m[t][5] = b.y;

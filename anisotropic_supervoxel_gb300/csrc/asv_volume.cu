@@ -1479,8 +1479,8 @@ __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
 __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
 {
     asv_follow();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int g = t / 27, o = t - g * 27;
+    const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int g = (int)(t / 27u), o = (int)(t - 27u * (unsigned)g);
     bool won = false;
     int si = 0, label = 0;
     long long vl = 0;
@@ -1533,8 +1533,8 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
     const unsigned m = __ballot_sync(FULL, won);                                   // one addition per warp
     if (!m) return;
     const int lane = threadIdx.x & 31;
-    int at = 0;
-    if (lane == __ffs(m) - 1) at = atomicAdd(d.tcount, __popc(m));
+    unsigned at = 0;
+    if (lane == __ffs(m) - 1) at = atomicAdd(d.tcount, (unsigned)__popc(m));
     at = __shfl_sync(FULL, at, __ffs(m) - 1);
     if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = make_int4(si, (int)vl, label, 0);   // segments hold < 2^31 voxels
 }
@@ -2117,9 +2117,9 @@ void asv_launch_jfa_first(const AsvDev &d, bool filled, bool stale, cudaStream_t
 {
     if (!filled) {
         cudaMemsetAsync(d.labB, 0xff, sizeof(int32_t) * (size_t)d.total_chunks * ASV_CHUNK, st);
-        cudaMemsetAsync(d.tcount, 0, sizeof(int), st);
+        cudaMemsetAsync(d.tcount, 0, sizeof(*d.tcount), st);
     }
-    k_jfa_first<<<(27 * d.total_seeds + 255) / 256, 256, 0, st>>>(d, stale);
+    k_jfa_first<<<asv_first_blocks(d.total_seeds), 256, 0, st>>>(d, stale);
 }
 
 // into labA, which is all -1.  undraw: d.drawn holds nothing but the seeds at
