@@ -51,6 +51,9 @@ enum {
 #define ASV_HD inline
 #endif
 
+// tiles of `size` along n >= 1 voxels, for any int n
+ASV_HD int asv_tiles_along(int n, int size) { return (n - 1) / size + 1; }
+
 // A batch has up to ASV_MAX_CLIPS clips of up to 32767 seeds, each in a run of
 // slots rounded up, 134 million in all: 27 or ASV_RING of something per seed
 // pass 2^31 and stay below 2^32, bytes and words of them pass that too.

@@ -36,6 +36,7 @@
 // Compiled with -fmad=false (integer work only).
 #include "asv_connect.cuh"
 
+#include "asv_common.cuh"
 #include "asv_follow.cuh"
 
 #define CC_CHUNK 2048
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_tile(const int32_t *__restric
     const CcTile t(tx, ty);
     const bool in = t.x < W && t.y < H;
     const int g0 = (t.z * H + t.y - t.w) * W + t.x - t.lane;   // the tile's first voxel
-    const int gv = (t.z * H + t.y) * W + t.x, fr = W * H;
+    const int gv = (int)(((unsigned)t.z * H + t.y) * W + t.x), fr = W * H;   // (lanes outside wrap, and use it not)
     unsigned len[CC_TZ];                                       // of the run that starts here, else 0
 #pragma unroll
     for (int k = 0; k < CC_TZ; k++) {
@@ -526,8 +527,8 @@ int asv_launch_connect(const int32_t *lab, int W, int H, int D, int supsz, int32
     int *par = carve(p, n), *cid = carve(p, n), *rvox = carve(p, n), *rsize = carve(p, n);
     int *node = carve(p, 2 * n), *chunk = carve(p, chunks + 1), *kept = carve(p, n / CC_SEGS + 1), *meta = carve(p, 4);
     const int minsz = supsz / 4, ni = (int)n;
-    const int tx = (W + 31) / 32, ty = (H + CC_THREADS / 32 - 1) / (CC_THREADS / 32);
-    const unsigned tiles = (unsigned)tx * ty * ((D + CC_TZ - 1) / CC_TZ);
+    const int tx = asv_tiles_along(W, 32), ty = asv_tiles_along(H, CC_THREADS / 32);
+    const unsigned tiles = (unsigned)tx * ty * asv_tiles_along(D, CC_TZ);
     int *R = meta, *err = meta + 1, *num = meta + 2;
     cudaMemsetAsync(meta, 0, 16, st);
     asv_launch_follow(false, k_cc_tile, tiles, CC_THREADS, 0, st, lab, par, cid, W, H, D, tx, ty, err);

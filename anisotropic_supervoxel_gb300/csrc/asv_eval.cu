@@ -11,6 +11,7 @@
 // turns the counts into the measures.
 #include "asv_eval.cuh"
 
+#include "asv_common.cuh"
 #include "asv_tally.cuh"
 
 #define EV_T 256                    // = TALLY_SLOTS
@@ -217,8 +218,8 @@ __global__ void __launch_bounds__(EV_T) k_ev_counts(const int32_t *__restrict__ 
     }
 }
 
-static int ev_tx(int W) { return (W + 31) / 32; }
-static int ev_ty(int H) { return (H + EV_T / 32 * EV_ROWS - 1) / (EV_T / 32 * EV_ROWS); }
+static int ev_tx(int W) { return asv_tiles_along(W, 32); }
+static int ev_ty(int H) { return asv_tiles_along(H, EV_T / 32 * EV_ROWS); }
 
 size_t asv_eval_sbound_words(int W, int H, int D) { return (size_t)ev_tx(W) * H * D; }
 
