@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(1024) k_cc_prefix(int *chunk, int m, const int
 // compact ids of the roots in raster order: rvox[id] = root voxel,
 // rsize[id] = its size, cid[root] = id (cid overwrites the size array)
 __global__ void __launch_bounds__(CC_THREADS) k_cc_compact(const int *__restrict__ par, int *cnt_cid,
-                                                           const int *__restrict__ chunk, int n, int *rvox, int *rsize)
+                                                           const int *chunk, int n, int *rvox, int *rsize)
 {
     asv_follow();
     constexpr int IT = CC_CHUNK / CC_THREADS, NW = CC_THREADS / 32;
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_compact(const int *__restrict
 }
 
 // kept segments per group of CC_SEGS, for the rank scan
-__global__ void __launch_bounds__(CC_SEGS) k_cc_kept_count(const int *__restrict__ rsize, const int *R, int minsz, int *chunk)
+__global__ void __launch_bounds__(CC_SEGS) k_cc_kept_count(const int *rsize, const int *R, int minsz, int *chunk)
 {
     asv_follow();
     const int r = *R > CC_MAX_R ? 0 : *R;
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(CC_SEGS) k_cc_kept_count(const int *__restrict
 // >= 0 pointer to a node (F_j = j, A_j = R + j), < 0 final value -1 - v.
 __global__ void __launch_bounds__(CC_SEGS) k_cc_nodes(const int *__restrict__ par, const int *__restrict__ cid,
                                                       const int *__restrict__ rvox, const int *__restrict__ rsize,
-                                                      const int *__restrict__ chunk, const int *R, int minsz, int W,
+                                                      const int *chunk, const int *R, int minsz, int W,
                                                       int H, int D, int *node)
 {
     asv_follow();
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_jump(int *node, const int *R)
 }
 
 __global__ void __launch_bounds__(CC_THREADS) k_cc_output(const int *__restrict__ par, const int *__restrict__ cid,
-                                                          const int *__restrict__ node, int n, const int *R, int32_t *out)
+                                                          const int *node, int n, const int *R, int32_t *out)
 {
     asv_follow();
     if (*R > CC_MAX_R) return;

@@ -47,7 +47,7 @@ __global__ void k_fl_gray(const uint8_t *__restrict__ rgb, float *__restrict__ o
 }
 
 // 5x5 binomial blur ([1 4 6 4 1]^2 / 256, clamp to edge) and decimation by 2
-__global__ void k_fl_down(const float *__restrict__ in, int Wi, int Hi, float *__restrict__ out, int Wo,
+__global__ void k_fl_down(const float *in, int Wi, int Hi, float *__restrict__ out, int Wo,
                           int Ho, int D)
 {
     asv_follow();
@@ -68,7 +68,7 @@ __global__ void k_fl_down(const float *__restrict__ in, int Wi, int Hi, float *_
 }
 
 // horizontal moments: h_p(x, y) = sum_u t^p g(u) f(x + u, y), p = 0, 1, 2
-__global__ void k_fl_poly_h(const float *__restrict__ img, int W, int H, int D, float *__restrict__ h)
+__global__ void k_fl_poly_h(const float *img, int W, int H, int D, float *__restrict__ h)
 {
     asv_follow();
     const long long plane = (long long)W * H * D;
@@ -91,7 +91,7 @@ __global__ void k_fl_poly_h(const float *__restrict__ img, int W, int H, int D, 
 
 // vertical moments and the fit: per pixel (b1, b2, a11, a22) in polyA and
 // a12 in polyB, so a bilinear tap of the expansion is two loads
-__global__ void k_fl_poly_v(const float *__restrict__ h, int W, int H, int D, float4 *__restrict__ polyA,
+__global__ void k_fl_poly_v(const float *h, int W, int H, int D, float4 *__restrict__ polyA,
                             float *__restrict__ polyB)
 {
     asv_follow();
@@ -206,7 +206,7 @@ __device__ __forceinline__ void fl_matrix(const float4 *__restrict__ sA, const f
 
 template <bool THIN>
 __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__ polyA, const float *__restrict__ polyB,
-                                                   const float *__restrict__ fin, float *__restrict__ fout, int W,
+                                                   const float *fin, float *__restrict__ fout, int W,
                                                    int H, int D, int P, int rows)
 {
     asv_follow();
@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__
 #pragma unroll
         for (int k = 0; k < FL_PX; k++) {
             const int e = min(max(y + (pr_[k] >> 16), 0), H - 1) * W + cx[k];
-            fx[k] = __ldg(fx_in + e);
-            fy[k] = __ldg(fy_in + e);
+            fx[k] = fx_in[e];
+            fy[k] = fy_in[e];
         }
     };
 
@@ -389,7 +389,7 @@ static int fl_rows(int W, int H, int P, int resident)
 // per 256 columns, eight rows and pair (one thread per pixel of a flat index,
 // with its 64-bit divisions: 68 us for the 640x480 level of 30 pairs, 39 us now)
 #define FL_UP_ROWS 8
-__global__ void __launch_bounds__(FL_T) k_fl_up(const float *__restrict__ coarse, int Wc, int Hc, float *__restrict__ fine,
+__global__ void __launch_bounds__(FL_T) k_fl_up(const float *coarse, int Wc, int Hc, float *__restrict__ fine,
                                                 int W, int H, int P)
 {
     asv_follow();
@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(FL_T) k_fl_up(const float *__restrict__ coarse
 }
 
 // level-0 flow of the pairs into the clip's interleaved fwd / bwd volumes
-__global__ void k_fl_store(const float *__restrict__ flow, int W, int H, int D, float2 *__restrict__ fwd,
+__global__ void k_fl_store(const float *flow, int W, int H, int D, float2 *__restrict__ fwd,
                            float2 *__restrict__ bwd, int keep_first_bwd)
 {
     asv_follow();

@@ -8,7 +8,10 @@
 // visible.  Each block calls it, also one without work: the next kernel relies on
 // this one's end to know that those before have ended.  It lets the next kernel
 // start only after its own wait, so at most two kernels of a chain are on the GPU
-// at once.
+// at once.  What the kernel before writes is not read-only while this one runs:
+// it is read by plain or L2 loads behind asv_follow, through pointers that are not
+// const __restrict__ (__ldg, or a load that the compiler makes one, may be moved
+// ahead of the wait).
 // The passes of the flood let the next kernel start at their end only: blocks that
 // start beside the last ones of a pass crowd on the SMs that are free first, which
 // then have more tiles (1280x720x30, ten iterations: 20.0 ms so, 19.33 with the

@@ -474,14 +474,14 @@ __device__ __forceinline__ void asv_chain_pos(int p, int D, int step, int &r, in
 // equals one of the labels before it (compares against the loaded labels,
 // all in registers, so nothing is shifted or stored to dedup).  Writes the
 // list (stride ASV_JFA_THREADS), returns its length.
-__device__ __forceinline__ int asv_slice_list(const int32_t *__restrict__ in, int zoff, const int xs[3],
+__device__ __forceinline__ int asv_slice_list(const int32_t *in, int zoff, const int xs[3],
                                               const int ys[3], int Kp, asv_list_t *__restrict__ lst)
 {
     int32_t c[9];
 #pragma unroll
     for (int oy = 0; oy < 3; oy++)
 #pragma unroll
-        for (int ox = 0; ox < 3; ox++) c[oy * 3 + ox] = __ldg(in + zoff + ys[oy] + xs[ox]);
+        for (int ox = 0; ox < 3; ox++) c[oy * 3 + ox] = in[zoff + ys[oy] + xs[ox]];
     int n = 0;
 #pragma unroll
     for (int k = 0; k < 9; k++) {
@@ -628,7 +628,7 @@ __device__ __forceinline__ void asv_accumulate(unsigned long long *__restrict__ 
 // the segment runs the same loop on the clamped column (valid = false) and
 // stores nothing, so the lanes of a warp stay in the same tile.
 template <bool SUMS>
-__device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+__device__ __forceinline__ void asv_jfa_run(const int32_t *in, int32_t *__restrict__ out,
                                             const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
                                             unsigned long long *__restrict__ sums, int slot0, int W, int H, int D,
                                             int Kp, int x, int y, int p0, int n, int step,
@@ -677,7 +677,7 @@ __device__ __forceinline__ void asv_jfa_run(const int32_t *__restrict__ in, int3
 // two of three lists of every voxel (the 240x160x30 clip with its full ladder:
 // steps 64 to 8, ten iterations 3.30 ms, so 3.16).  Small steps, whose crowded
 // sub-tiles come here too, lose by it (the 64x48x12 clip 0.250 ms, so 0.256).
-__device__ __forceinline__ void asv_jfa_run_far(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+__device__ __forceinline__ void asv_jfa_run_far(const int32_t *in, int32_t *__restrict__ out,
                                                 const uchar4 *__restrict__ lab, const float4 *__restrict__ tab, int W,
                                                 int H, int D, int Kp, int x, int y, int p0, int n, int step,
                                                 float ratio, asv_list_t *__restrict__ lists, bool valid)
@@ -1101,7 +1101,7 @@ __device__ __forceinline__ void asv_run_flush(unsigned *__restrict__ a, unsigned
 // (nothing written) when its footprint holds more than 32 labels.  Called
 // by the whole block.
 template <int S, bool SUMS>
-__device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+__device__ bool asv_jfa_bits_sub(const int32_t *in, int32_t *__restrict__ out,
                                  const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
                                  unsigned long long *__restrict__ sums, int slot0, int W, int H, int D, int Kp,
                                  int tx0, int ty0, int p0, int n, float ratio, unsigned char *smem)
@@ -1366,7 +1366,7 @@ __device__ bool asv_jfa_bits_sub(const int32_t *__restrict__ in, int32_t *__rest
 // holds too many labels) the list form.
 #define ASV_JFA_LIST 7
 template <int ST, bool SUMS>
-__device__ __forceinline__ void asv_jfa_tile(const int32_t *__restrict__ in, int32_t *__restrict__ out,
+__device__ __forceinline__ void asv_jfa_tile(const int32_t *in, int32_t *__restrict__ out,
                                              const uchar4 *__restrict__ lab, const float4 *__restrict__ tab,
                                              unsigned long long *__restrict__ sums, int slot0, int W, int H, int D,
                                              int Kp, int tx0, int ty0, int p0, int zrun, int depth, int step,
@@ -1438,7 +1438,7 @@ __device__ __forceinline__ void asv_jfa_smem_init(AsvBitsShared &b)
 // the 640x480x60 one 16.1 instead of 16.7.
 template <int ST, bool SUMS>
 __global__ void __launch_bounds__(ASV_JFA_THREADS, 4) k_jfa(AsvDev d, int pass,
-                                                         const int32_t *__restrict__ in,
+                                                         const int32_t *in,
                                                          int32_t *__restrict__ out)
 {
     extern __shared__ __align__(16) unsigned char asv_jfa_smem[];
@@ -1570,7 +1570,7 @@ __device__ __forceinline__ void asv_axis_sources(int u, int o, int s, int n, int
 
 // whether voxel (x, y, z) meets label a before label b among its candidates, in the
 // shader's order (slices z, z-s, z+s; rows and columns from - to +, clamped)
-__device__ __forceinline__ bool asv_met_before(const int32_t *__restrict__ in, int W, int H, int D, int x, int y, int z,
+__device__ __forceinline__ bool asv_met_before(const int32_t *in, int W, int H, int D, int x, int y, int z,
                                                int s, int a, int b)
 {
     unsigned ma = 0, mb = 0;
