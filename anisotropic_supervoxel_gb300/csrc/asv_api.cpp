@@ -853,9 +853,17 @@ static cudaError_t eval_scratch(asv_ctx *ctx, int k, size_t b)
     return e;
 }
 
-struct EvalRelease {                                   // large scratch goes back at the end of the call
+struct EvalRelease {                                   // the end of the call, whichever way it returns
     asv_ctx *ctx;
-    ~EvalRelease() { if (ctx->evs_bytes[0] + ctx->evs_bytes[1] > EV_KEEP) free_eval(ctx); }
+    bool done = false;
+    ~EvalRelease()
+    {
+        if (!done) {                                   // copies from the caller's arrays may be under way
+            cudaStreamSynchronize(ctx->side);
+            cudaStreamSynchronize(ctx->st);
+        }
+        if (ctx->evs_bytes[0] + ctx->evs_bytes[1] > EV_KEEP) free_eval(ctx);   // large scratch goes back
+    }
 };
 
 extern "C" {
@@ -1426,6 +1434,7 @@ asv_status asv_evaluate(asv_ctx *ctx, const int32_t *labels, const int32_t *trut
     out->truth_segments = ng;
     out->truth_boundary = (long long)t[0];
     out->recalled = (long long)t[1];
+    release.done = true;
     return ASV_OK;
 }
 
