@@ -155,8 +155,10 @@ struct asv_ctx {
     bool drawn = false;          // labA holds a fresh seed draw: the first pass may scatter
     bool undraw = false;         // ... and nothing else: the first pass need not check the seeds' places
     // fills of the label volumes run beside the (latency-bound) metric solves
-    // of the next seeds, on a stream of their own between two events
+    // of the next seeds, on a stream of their own between two events.  It has the
+    // priority of the context's stream: its work stands in that one's way
     cudaStream_t side = nullptr;
+    std::vector<std::pair<int, cudaStream_t>> sides;   // a side stream per priority met (set_stream)
     cudaEvent_t side_ev[2] = { nullptr, nullptr };
     int post_host[ASV_POST_WORDS];
     // graph
@@ -231,13 +233,34 @@ size_t asv::ctx_bytes(const asv_ctx *c)
     return c ? c->bytes + c->cc_bytes + c->fl_bytes + c->evs_bytes[0] + c->evs_bytes[1] : 0;
 }
 
+// The side stream of the context's stream's priority; false when none can be made
+static bool pick_side(asv_ctx *c)
+{
+    int prio = 0;
+    if (cudaStreamGetPriority(c->st, &prio) != cudaSuccess) return false;
+    for (auto &s : c->sides)
+        if (s.first == prio) { c->side = s.second; return true; }
+    cudaStream_t s = nullptr;
+    if (cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, prio) != cudaSuccess) return false;
+    c->sides.emplace_back(prio, s);
+    c->side = s;
+    return true;
+}
+
+int asv::side_priority(const asv_ctx *c)
+{
+    int prio = 0;
+    return cudaStreamGetPriority(c->side, &prio) == cudaSuccess ? prio : 1;   // priorities are 0 or less
+}
+
 void asv::set_stream(asv_ctx *c, cudaStream_t st)
 {
     if (!c || c->st == st) return;
-    cudaStreamSynchronize(c->st);
+    cudaStreamSynchronize(c->st);                    // (the side stream's work is joined to it)
     if (c->own_st) cudaStreamDestroy(c->st);
     c->st = st;
     c->own_st = false;
+    if (!pick_side(c)) cudaGetLastError();           // the one before serves as well, if later
 }
 
 static asv_status fail(asv_ctx *c, asv_status s, const std::string &m)
@@ -914,7 +937,7 @@ asv_status asv_create(const asv_config *cfg, asv_ctx **out)
         if (cudaStreamCreateWithFlags(&ctx->st, cudaStreamNonBlocking) != cudaSuccess) { delete ctx; return ASV_ERR_CUDA; }
         ctx->own_st = true;
     }
-    bool ok = cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) == cudaSuccess;
+    bool ok = pick_side(ctx);
     for (cudaEvent_t &e : ctx->side_ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) { asv_destroy(ctx); cudaGetLastError(); return ASV_ERR_CUDA; }
     *out = ctx;
@@ -935,7 +958,7 @@ asv_status asv_destroy(asv_ctx *ctx)
     if (ctx->hpin) cudaFreeHost(ctx->hpin);
     for (auto e : ctx->sev) if (e) cudaEventDestroy(e);
     for (auto e : ctx->side_ev) if (e) cudaEventDestroy(e);
-    if (ctx->side) cudaStreamDestroy(ctx->side);
+    for (auto &s : ctx->sides) cudaStreamDestroy(s.second);
     if (ctx->cp) {
         cudaStreamDestroy(ctx->cp);
         for (int k = 0; k < 2; k++) { cudaEventDestroy(ctx->fed_ev[k]); cudaEventDestroy(ctx->used_ev[k]); }
