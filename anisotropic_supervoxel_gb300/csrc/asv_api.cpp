@@ -501,9 +501,8 @@ static void set_depths(SegDesc &s)
 // 3 per sub-tile, from the depths of steps 1 and 2 alone, and 0.41, 0.69 and
 // 0.85 it was up to 6.6 % off: 1280x720x30 with 10000 seeds, six iterations,
 // depth 5 27.1 ms, 30 25.4; 640x480x60, ten iterations, 15 13.45, 30 13.17.)
-static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
+static int estimate_zrun(const std::vector<SegHost> &seg)
 {
-    if (ctx->cfg.jfa_zrun > 0) return std::min(ctx->cfg.jfa_zrun, 256);
     const int per_sm = 4;
     const long long sms = std::max(1, asv_jfa_resident_blocks() / per_sm);
     static const double rate[4] = { 1.0, 0.57, 0.83, 0.92 };
@@ -532,6 +531,23 @@ static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
         if (least == 0.0 || cost < least) { best = z; least = cost; }
     }
     return best;
+}
+
+static int pick_zrun(const asv_ctx *ctx, const std::vector<SegHost> &seg)
+{
+    return ctx->cfg.jfa_zrun > 0 ? std::min(ctx->cfg.jfa_zrun, 256) : estimate_zrun(seg);
+}
+
+// The tile depths that asv_autotune times: the estimate, which may be any of 1 to
+// 32 (10 for the 240x160x30 clip), then the four it chooses from.  Returns their
+// number.
+int asv::autotune_depths(int estimate, int depths[5])
+{
+    int n = 0;
+    depths[n++] = estimate;
+    for (int z : { 4, 8, 16, 32 })
+        if (z != estimate) depths[n++] = z;
+    return n;
 }
 
 static void set_tiles(SegDesc &s)
@@ -1267,8 +1283,11 @@ asv_status asv_autotune(asv_ctx *ctx, int *zrun_out)
     s = ensure_events(ctx, 2);
     if (s != ASV_OK) return s;
     int best = 0;
-    float best_ms = 0.f;
-    for (int z : { 4, 8, 16, 32 }) {
+    float best_ms = 0.f, estimate_ms = 0.f;
+    int depths[5];
+    const int n = autotune_depths(estimate_zrun(ctx->seg), depths);
+    for (int i = 0; i < n; i++) {
+        const int z = depths[i];
         if ((s = set_zrun(ctx, z)) != ASV_OK) return s;
         enqueue_lloyd(ctx, false);                        // warm-up at this depth
         CK(cudaEventRecord(ctx->ev[0], ctx->st));
@@ -1278,10 +1297,12 @@ asv_status asv_autotune(asv_ctx *ctx, int *zrun_out)
         CK(cudaEventSynchronize(ctx->ev[1]));
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]));
-        if (!best || ms < best_ms) { best = z; best_ms = ms; }
+        if (i == 0) estimate_ms = ms;
+        if ((z == 4 || z == 8 || z == 16 || z == 32) && (!best || ms < best_ms)) { best = z; best_ms = ms; }
     }
-    if ((s = set_zrun(ctx, best)) != ASV_OK) return s;
-    ctx->cfg.jfa_zrun = best;                             // later layouts keep it
+    const bool estimate = estimate_ms < best_ms;
+    if ((s = set_zrun(ctx, estimate ? depths[0] : best)) != ASV_OK) return s;
+    ctx->cfg.jfa_zrun = estimate ? 0 : best;              // later layouts: their own estimate, or this depth
     enqueue_lloyd(ctx, false);                            // labels of the final depth (identical)
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->st));

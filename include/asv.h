@@ -180,8 +180,9 @@ asv_status asv_run_lloyd(asv_ctx *ctx);
 /* No counterpart in the reference.  Times the whole Lloyd loop at JFA tile
  * depths 4, 8, 16 and 32 (the voxels of a column one block walks along a
  * step's chains: deeper shares more slice work, shallower fills the GPU
- * better), keeps the fastest for this context (also for its later layouts)
- * and returns it in *zrun (may be NULL).  Needs a context ready for
+ * better) and returns the fastest of them in *zrun (may be NULL).  This
+ * context keeps it, also for its later layouts, unless the loop is faster at
+ * the depth estimated from the clip sizes, which it then keeps.  Needs a context ready for
  * asv_run_lloyd (clip or batch, not streaming); leaves the labels of a
  * complete run, which do not depend on the depth. */
 asv_status asv_autotune(asv_ctx *ctx, int *zrun);
