@@ -14,10 +14,12 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace asv {
@@ -434,30 +436,44 @@ static int label_depth(int D, double spacing, int step, bool sparse)
 
 static double seed_spacing(long long nvox, int Kp) { return std::cbrt((double)nvox / std::max(Kp, 1)); }
 
+// Slice and chain of every chain position of D slices (asv_chain_pos)
+static void chain_table(int D, int step, std::vector<int> &slice, std::vector<int> &chain)
+{
+    slice.clear();
+    chain.clear();
+    for (int r = 0; r < std::min(step, D); r++)
+        for (int z = r; z < D; z += step) { slice.push_back(z); chain.push_back(r); }
+}
+
 // Footprint slots of all sub-tiles of `depth` positions of a column's D
 // positions cut in tiles of zrun, and 3 for each sub-tile, in quarters, and one
 // for an odd sub-tile (positions go two at a time); -1 when a sub-tile has more
-// slots than fit.  A sub-tile has its positions and the two slices next to them,
-// and where a chain ends inside it slices 0 and D - 1, unless those are the two.
-static int depth_cost(int D, int zrun, int step, int depth, int most)
+// slots than fit, or the cost passes `limit`.  A sub-tile has its positions and
+// the two slices next to them, and where a chain ends inside it slices 0 and D -
+// 1, unless those are the two.  (From the table: a batch of 1500 clips of 32x32x32
+// spent 15.0 ms on its layout with quotients for every position, 6.7 without the
+// depths.)
+static int depth_cost(const std::vector<int> &slice, const std::vector<int> &chain, int zrun, int step, int depth, int most,
+                      int limit)
 {
-    auto slice = [&](int p) {                              // asv_chain_pos
-        if (step >= D) return p;
-        const int q = D / step, m = D - q * step, big = m * (q + 1);
-        return p < big ? p / (q + 1) + p % (q + 1) * step : m + (p - big) / q + (p - big) % q * step;
-    };
+    const int D = (int)slice.size();
     int cost = 0;
     for (int t0 = 0; t0 < D; t0 += zrun)
         for (int p0 = t0, e = std::min(t0 + zrun, D); p0 < e; p0 += depth) {
-            const int n = std::min(depth, e - p0);
-            bool ends = false;
-            for (int p = p0; p < p0 + n - 1; p++) ends = ends || slice(p) + step >= D;
+            const int n = std::min(depth, e - p0), last = p0 + n - 1;
             int slots = n + 2;
-            if (ends) slots += (slice(p0) > step) + (slice(p0 + n - 1) + step < D - 1);
-            if (slots > most) return -1;
+            if (chain[p0] != chain[last]) slots += (slice[p0] > step) + (slice[last] + step < D - 1);
             cost += 4 * (slots + 3) + (n & 1);
+            if (slots > most || cost > limit) return -1;
         }
     return cost;
+}
+
+int asv::sub_tile_cost(int D, int zrun, int step, int depth, int most)
+{
+    std::vector<int> slice, chain;
+    chain_table(D, step, slice, chain);
+    return depth_cost(slice, chain, zrun, step, depth, most, INT_MAX);
 }
 
 // The most chain positions of a sub-tile in pass p; below 4: list form.  15 in
@@ -473,16 +489,24 @@ static int most_depth(int D, double spacing, const int *steps, int npass, int p)
 // of least cost (the smallest of equal ones, as a sub-tile that overflows goes on
 // with half the depth), so that 30 positions are 15 + 15, not 16 + 14, or at step 6
 // three sub-tiles of two whole chains (12 slots each), not four of 8 or 7.
-static void set_depths(SegDesc &s)
+// before: the segment before, which has them already, or NULL.
+static void set_depths(SegDesc &s, const SegDesc *before)
 {
+    if (before && before->D == s.D && before->zrun == s.zrun && before->nvox == s.nvox && before->Kp == s.Kp &&
+        before->npass == s.npass && std::equal(s.steps, s.steps + s.npass, before->steps)) {
+        std::copy(before->depth, before->depth + s.npass, s.depth);
+        return;
+    }
     const double spacing = seed_spacing(s.nvox, s.Kp);
+    std::vector<int> slice, chain;
     for (int p = 0; p < s.npass; p++) {
         const int step = s.steps[p], most = asv_jfa_slots(step);
         s.depth[p] = 0;
-        int least = 0;
-        for (int d = most_depth(s.D, spacing, s.steps, s.npass, p); d >= 4; d--) {
-            const int c = depth_cost(s.D, s.zrun, step, d, most);
-            if (c >= 0 && (!s.depth[p] || c <= least)) { s.depth[p] = d; least = c; }
+        int d = most_depth(s.D, spacing, s.steps, s.npass, p), least = INT_MAX;
+        if (d >= 4) chain_table(s.D, step, slice, chain);
+        for (; d >= 4; d--) {
+            const int c = depth_cost(slice, chain, s.zrun, step, d, most, least);
+            if (c >= 0) { s.depth[p] = d; least = c; }
         }
     }
 }
@@ -506,20 +530,29 @@ static int estimate_zrun(const std::vector<SegHost> &seg)
     const int per_sm = 4;
     const long long sms = std::max(1, asv_jfa_resident_blocks() / per_sm);
     static const double rate[4] = { 1.0, 0.57, 0.83, 0.92 };
+    // columns of tiles, slices and the gathering passes' most positions per
+    // sub-tile, of runs of equal segments
+    struct Run { int W, H, D, Kp; long long columns; std::vector<int> most; };
+    std::vector<Run> runs;
+    for (const SegHost &h : seg) {
+        const long long columns = (long long)((h.W + ASV_TILE_X - 1) / ASV_TILE_X) * ((h.H + ASV_TILE_Y - 1) / ASV_TILE_Y);
+        if (runs.empty() || runs.back().W != h.W || runs.back().H != h.H || runs.back().D != h.D || runs.back().Kp != h.Kp) {
+            runs.push_back({ h.W, h.H, h.D, h.Kp, 0, {} });
+            const double sp = seed_spacing((long long)h.W * h.H * h.D, h.Kp);
+            for (int p = 2; p < h.npass; p++) runs.back().most.push_back(most_depth(h.D, sp, h.steps, h.npass, p));
+        }
+        runs.back().columns += columns;
+    }
     int best = 4;
     double least = 0.0;
     for (int z = 1; z <= 32; z++) {
         long long tiles = 0;
         double work = 0.0;
-        for (const SegHost &h : seg) {
-            const long long col = (long long)((h.W + ASV_TILE_X - 1) / ASV_TILE_X) * ((h.H + ASV_TILE_Y - 1) / ASV_TILE_Y);
-            const int ze = even_depth(h.D, z), nz = (h.D + ze - 1) / ze;
-            tiles += col * nz;
-            const double sp = seed_spacing((long long)h.W * h.H * h.D, h.Kp);
-            for (int p = 2; p < h.npass; p++) {
-                const int d = most_depth(h.D, sp, h.steps, h.npass, p);
-                work += (double)col * ((d < 4 ? 1.8 * h.D : h.D + 1.55 * nz * ((ze + d - 1) / d)) + 0.36 * nz);
-            }
+        for (const Run &r : runs) {
+            const int ze = even_depth(r.D, z), nz = (r.D + ze - 1) / ze;
+            tiles += r.columns * nz;
+            for (int d : r.most)
+                work += (double)r.columns * ((d < 4 ? 1.8 * r.D : r.D + 1.55 * nz * ((ze + d - 1) / d)) + 0.36 * nz);
         }
         const long long m = (tiles + sms - 1) / sms, q = m / per_sm, k = m % per_sm;
         double rounds = (double)(per_sm * q) + 0.24;
@@ -585,7 +618,7 @@ asv_status asv_build_layout(asv_ctx *ctx)
         s.wNum = h.g.wNum; s.hNum = h.g.hNum; s.dNum = h.g.dNum;
         s.cell_off = cells;
         s.final_buf = h.npass & 1;
-        set_depths(s);
+        set_depths(s, i ? &ctx->sd[i - 1] : nullptr);
         h.vox_off = vox; h.seed_off = seeds;
         tile_p[i] = tiles; chunk_p[i] = chunks; seed_p[i] = seeds;
         int nchunk = (int)((n + ASV_CHUNK - 1) / ASV_CHUNK);
@@ -1257,7 +1290,7 @@ static asv_status set_zrun(asv_ctx *ctx, int z)
     for (int i = 0; i < nseg; i++) {
         SegDesc &sd = ctx->sd[i];
         sd.zrun = even_depth(sd.D, z);
-        set_depths(sd);
+        set_depths(sd, i ? &ctx->sd[i - 1] : nullptr);
         tp[i] = tiles;
         tiles += sd.tiles_x * sd.tiles_y * ((sd.D + sd.zrun - 1) / sd.zrun);
     }
@@ -2087,7 +2120,7 @@ static asv_status stream_enqueue(asv_ctx *ctx, bool fed, const uint8_t *rgb, con
     sd.wNum = h.g.wNum; sd.hNum = h.g.hNum; sd.dNum = h.g.dNum;
     sd.cell_off = 0;
     sd.final_buf = h.npass & 1;
-    set_depths(sd);
+    set_depths(sd, nullptr);
     sd.lab_from = (long long)z0 * WH;
     const int tiles = sd.tiles_x * sd.tiles_y * ((Db + sd.zrun - 1) / sd.zrun);
     const int chunks = (int)((sd.nvox + ASV_CHUNK - 1) / ASV_CHUNK);

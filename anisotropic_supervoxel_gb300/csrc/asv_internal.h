@@ -31,6 +31,7 @@ int grid_seeds(int W, int H, int D, int K, int middlebury, GridInfo *g, std::vec
 size_t ctx_bytes(const asv_ctx *ctx);   // device bytes a context holds
 void set_stream(asv_ctx *ctx, cudaStream_t st);   // later work of ctx runs on st (caller-owned)
 int autotune_depths(int estimate, int depths[5]);
+int sub_tile_cost(int D, int zrun, int step, int depth, int most);
 int side_priority(const asv_ctx *ctx);  // of the stream beside it, on which the label fills run
 void cell_tables(int W, int H, int D, const GridInfo &g, const std::vector<float> &grid,
                  std::vector<int> *cells);
