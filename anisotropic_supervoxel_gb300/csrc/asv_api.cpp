@@ -392,8 +392,8 @@ size_t asv_layout_bytes(const std::vector<SegHost> &seg)
     // rgb 3 + lab 4 + fwd/bwd 16 + two label buffers 8 + drawn seeds 4
     size_t per_vox = 3 + 4 + 8 + 8 + 4 + 4 + 4;
     // float4 pos0/pos/slab/grid, 8-float M0/M/Mself/Mmemo, jtab 3 float4, 8 u64
-    // sums, int neg/mkey/rank/neglist, u64 dacc, the metric ring
-    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 4 * 4 + 8 + ASV_RING * (32 + 4) + 27 * 16;
+    // sums, int neg/mkey/rank, u64 dacc, the metric ring, the first pass's list
+    size_t per_seed = 4 * 16 + 4 * 32 + 3 * 16 + 8 * 8 + 3 * 4 + 8 + ASV_RING * (32 + 4) + 27 * sizeof(asv_entry_t);
     // each of the ~30 allocations rounds up to 256 bytes
     size_t fixed = 32 * 256 + 256 * 4 + 16;
     fixed += sizeof(SegDesc);
@@ -653,13 +653,14 @@ asv_status asv_build_layout(asv_ctx *ctx)
     AL(d.Mself, (size_t)seeds * 8); AL(d.neg, seeds);
     AL(d.Mmemo, (size_t)seeds * 8); AL(d.mkey, seeds);
     AL(d.Mring, (size_t)seeds * ASV_RING * 8); AL(d.ringok, (size_t)seeds * ASV_RING);
-    AL(d.neglist, seeds); AL(d.negcount, 1);
+    AL(d.negcount, 1);
     CK(cudaMemsetAsync(d.negcount, 0, sizeof(int), ctx->st));
     AL(d.grid, seeds);
     AL(d.dacc, seeds);
     AL(d.cells, std::max(cells, 1));
     AL(d.post, (size_t)nseg * ASV_POST_WORDS);
     AL(d.rank, seeds);
+    d.neglist = d.rank;          // ranks stand in the post-processing only, the list within the metric solves
     AL(d.scan, std::max(chunks, 1));
     AL(d.srgb, 256);
     AL(d.err, 4);

@@ -64,6 +64,17 @@ ASV_HD int asv_seed_slots(int Kp) { return ((Kp + 64 + 31) / 32) * 32; }
 ASV_HD unsigned asv_first_blocks(int slots) { return (27u * (unsigned)slots + 255u) / 256u; }
 ASV_HD unsigned asv_ring_tasks(int slots) { return (unsigned)ASV_RING * (unsigned)slots; }
 
+// an entry of AsvDev::tlist: a voxel of a clip (fewer than 2^31) and its label
+// (below 32768), in 58 bits
+typedef unsigned long long asv_entry_t;
+ASV_HD asv_entry_t asv_entry(int seg, int voxel, int label)
+{
+    return ((asv_entry_t)(unsigned)seg << 46) | ((asv_entry_t)(unsigned)voxel << 15) | (unsigned)label;
+}
+ASV_HD int asv_entry_seg(asv_entry_t e) { return (int)(e >> 46); }
+ASV_HD int asv_entry_voxel(asv_entry_t e) { return (int)((unsigned)(e >> 15) & 0x7fffffffu); }
+ASV_HD int asv_entry_label(asv_entry_t e) { return (int)((unsigned)e & 0x7fffu); }
+
 // place of ring neighbour t of seed slot g (of Mring's rows of 8 floats, of ringok)
 ASV_HD size_t asv_ring_at(int g, int t) { return (size_t)ASV_RING * g + t; }
 
@@ -111,7 +122,7 @@ struct AsvDev {
     float2 *fwd, *bwd;
     int32_t *labA, *labB;
     int32_t *drawn;              // the drawn seeds at their voxels, else -1 (loop: all -1 between its draws; else labA)
-    int4 *tlist;                 // voxels labelled by the first pass: (segment, voxel, label, -), 27 per seed
+    asv_entry_t *tlist;          // voxels labelled by the first pass, 27 per seed
     unsigned *tcount;            // entries of tlist
     float4 *pos0;                // initial seeds (density placement)
     float *M0;                   // initial metric, 8 floats / seed
@@ -122,7 +133,7 @@ struct AsvDev {
     float *Mself; int *neg;      // metric scratch
     float *Mmemo; int *mkey;     // reseed memo: metric of the voxel key of the last solve
     float *Mring; int *ringok;
-    int *neglist, *negcount;     // seeds whose own metric is not PSD (empty between solves)
+    int *neglist, *negcount;     // seeds whose own metric is not PSD (empty between solves; the list in rank's place)
     float4 *grid;                // grid seeds
     unsigned long long *dacc;    // density accumulators (2^-24 units)
     int *cells;                  // cell tables

@@ -1536,7 +1536,7 @@ __global__ void __launch_bounds__(256) k_jfa_first(AsvDev d, bool stale)
     unsigned at = 0;
     if (lane == __ffs(m) - 1) at = atomicAdd(d.tcount, (unsigned)__popc(m));
     at = __shfl_sync(FULL, at, __ffs(m) - 1);
-    if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = make_int4(si, (int)vl, label, 0);   // segments hold < 2^31 voxels
+    if (won) d.tlist[at + __popc(m & ((1u << lane) - 1u))] = asv_entry(si, (int)vl, label);
 }
 
 // ---------------------------------------------------------------------------
@@ -1631,10 +1631,10 @@ __global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
     }
     int si = 0, label = 0;
     int x0 = 0, y0 = 0, z0 = 0, nx = 0, ny = 0, nz = 0;
-    const int4 ent = e < 27LL * d.total_seeds ? d.tlist[e] : make_int4(0, 0, 0, 0);   // asked for beside their number
+    const asv_entry_t ent = e < 27LL * d.total_seeds ? d.tlist[e] : 0ull;             // asked for beside their number
     if (e < *d.tcount) {
-        si = ent.x;
-        const int ul = ent.y;
+        si = asv_entry_seg(ent);
+        const int ul = asv_entry_voxel(ent);
         const SegDesc &S = d.segs[si];
         const int s = S.steps[1];
         const int row = ul / S.W;
@@ -1646,7 +1646,7 @@ __global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
         nx = x1 - x0 + 1; ny = y1 - y0 + 1; nz = z1 - z0 + 1;
         if (nx <= 0 || ny <= 0 || nz <= 0) nx = 0;
         else {
-            label = ent.z;
+            label = asv_entry_label(ent);
             if (nx * ny * nz == 1) {
                 asv_second_voxel(d, S, label, x0, y0, z0, s);
                 nx = 0;
