@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_output(const int *__restrict_
 size_t asv_connect_scratch_bytes(long long n)
 {
     const long long chunks = (n + CC_CHUNK - 1) / CC_CHUNK;
-    // par, cid/size, rvox, rsize, node (2 per segment), chunk sums (+1), kept per group, R, error word, labels
-    return (size_t)(4 * n * 6 + 4 * (chunks + 2) + 4 * (n / CC_SEGS + 2) + 256 * 9);
+    // par, cid/size, rvox, rsize, node (2 per segment), chunk sums (+1), R, error word, labels
+    return (size_t)(4 * n * 6 + 4 * (chunks + 2) + 256 * 8);
 }
 
 static int *carve(unsigned char *&p, long long count)
@@ -525,7 +525,8 @@ int asv_launch_connect(const int32_t *lab, int W, int H, int D, int supsz, int32
     const long long chunks = (n + CC_CHUNK - 1) / CC_CHUNK;
     unsigned char *p = (unsigned char *)scratch;
     int *par = carve(p, n), *cid = carve(p, n), *rvox = carve(p, n), *rsize = carve(p, n);
-    int *node = carve(p, 2 * n), *chunk = carve(p, chunks + 1), *kept = carve(p, n / CC_SEGS + 1), *meta = carve(p, 4);
+    int *node = carve(p, 2 * n), *chunk = carve(p, chunks + 1), *meta = carve(p, 4);
+    int *kept = out;                                     // kept per group: read before k_cc_output writes there
     const int minsz = supsz / 4, ni = (int)n;
     const int tx = asv_tiles_along(W, 32), ty = asv_tiles_along(H, CC_THREADS / 32);
     const unsigned tiles = (unsigned)tx * ty * asv_tiles_along(D, CC_TZ);
