@@ -43,6 +43,7 @@
 #define CC_THREADS 256
 #define CC_TZ 8                     // a tile: 32 x 8 (the block's warps) x CC_TZ voxels
 #define CC_TILE (CC_THREADS * CC_TZ)
+#define CC_SPARSE 64                // voxels per tile up to which the volume goes without tiles
 #define CC_SEGS 128                 // segments per group of the rank scan
 #define CC_HOPS 256
 #define CC_ROUNDS 4
@@ -302,9 +303,46 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_union(const int32_t *__restri
     cc_make(queue, min(nq, CC_TILE), join);
 }
 
+// The same two steps for volumes whose tiles would be nearly empty (lines, columns
+// of a few voxels): the runs of equal label along x within a warp, then each
+// voxel's links in global memory.  At 64 voxels per tile of 2048 the faster one:
+// 131072x2x4 147 us a call, tiles 329; 262144x2x2 192, 567; at 128, 1024x1024x2 with
+// noisy labels, 1266 against 634.
+__global__ void __launch_bounds__(CC_THREADS) k_cc_runs(const int32_t *__restrict__ lab, int *par, int *cnt, int W, int n)
+{
+    asv_follow();
+    const unsigned v = blockIdx.x * CC_THREADS + threadIdx.x, lane = threadIdx.x & 31;
+    const bool in = v < (unsigned)n;
+    const int l = in ? __ldg(lab + v) : 0, before = __shfl_up_sync(0xffffffffu, l, 1);
+    const unsigned starts = __ballot_sync(0xffffffffu, lane == 0 || !in || l != before || v % (unsigned)W == 0);
+    if (!in) return;
+    const unsigned next = lane < 31 ? starts & (0xfffffffeu << lane) : 0u;
+    par[v] = (int)(v - lane + 31 - __clz((int)(starts & (0xffffffffu >> (31 - lane)))));
+    cnt[v] = (starts >> lane) & 1u ? (int)((next ? __ffs(next) - 1 : 32) - lane) : 0;
+}
+
+__global__ void __launch_bounds__(CC_THREADS) k_cc_link(const int32_t *__restrict__ lab, int *par, int W, int H, int D,
+                                                        int n, int *err)
+{
+    asv_follow();
+    const unsigned u = blockIdx.x * CC_THREADS + threadIdx.x;
+    if (u >= (unsigned)n) return;
+    const int v = (int)u, fr = W * H, row = v / W, x = v - row * W, z = row / H, y = row - z * H;
+    const int32_t *p = lab + v;
+    unsigned m = cc_links(__ldg(p), x > 0, x < W - 1, y > 0, y < H - 1, z > 0,
+                          [&](int dx, int dy, int dz) { return __ldg(p + dx + dy * W + dz * fr); });
+    if (threadIdx.x & 31) m &= ~(1u << 3);                     // W: of the same run
+    for (; m; m &= m - 1) {
+        const int b = __ffs(m) - 1, q = b % 9;
+        cc_union(par, v - (b >= 9 ? fr : 0) + (q / 3 - 1) * W + q % 3 - 1, v, err);
+    }
+}
+
 // par[v] = root, the tiles' component sizes added up at the roots, roots per
 // chunk of CC_CHUNK voxels.  No links change any more, so walks end at the true
-// roots, and only thread v writes par[v].
+// roots, and only thread v writes par[v].  SPARSE: sizes are of runs, so most
+// voxels of a warp add to one root, and do it once.
+template <bool SPARSE>
 __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *par, int *cnt, int n, int *chunk, int *err)
 {
     asv_follow();
@@ -330,13 +368,16 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *par, int *cnt, i
 #pragma unroll
     for (int k = 0; k < IT; k++) {
         const int v = v0 + k * CC_THREADS;
-        if (v >= n) continue;
-        if (r[k] == v) roots++;
-        else {
-            const int c = cnt[v];                              // of a tile's component: no one else's to change
-            if (c) atomicAdd(cnt + r[k], c);
-            par[v] = r[k];
+        const bool child = v < n && r[k] != v;
+        roots += v < n && !child;
+        int c = child ? cnt[v] : 0;                            // of a tile's component: no one else's to change
+        if (SPARSE) {
+            const unsigned peers = __match_any_sync(0xffffffffu, child ? r[k] : -1);
+            c = __reduce_add_sync(peers, c);
+            if ((int)(threadIdx.x & 31) != __ffs(peers) - 1) c = 0;
         }
+        if (c) atomicAdd(cnt + r[k], c);
+        if (child) par[v] = r[k];
     }
     roots = __reduce_add_sync(0xffffffffu, roots);
     if ((threadIdx.x & 31) == 0 && roots) atomicAdd(&tot, roots);
@@ -521,6 +562,10 @@ static int *carve(unsigned char *&p, long long count)
 int asv_launch_connect(const int32_t *lab, int W, int H, int D, int supsz, int32_t *out, void *scratch,
                        cudaStream_t st, int *host_R, int *host_num)
 {
+    // One voxel wide: its rows as the rows along x of a volume one row high, the same
+    // voxels in the same order with the same neighbours, that the tiles' lanes fill
+    // (1024x1024x1: 169 us a call, 457 with a voxel per tile row).
+    if (W == 1) { W = H; H = 1; }
     const long long n = (long long)W * H * D;
     const long long chunks = (n + CC_CHUNK - 1) / CC_CHUNK;
     unsigned char *p = (unsigned char *)scratch;
@@ -532,9 +577,16 @@ int asv_launch_connect(const int32_t *lab, int W, int H, int D, int supsz, int32
     const unsigned tiles = (unsigned)tx * ty * asv_tiles_along(D, CC_TZ);
     int *R = meta, *err = meta + 1, *num = meta + 2;
     cudaMemsetAsync(meta, 0, 16, st);
-    asv_launch_follow(false, k_cc_tile, tiles, CC_THREADS, 0, st, lab, par, cid, W, H, D, tx, ty, err);
-    asv_launch_follow(true, k_cc_union, tiles, CC_THREADS, 0, st, lab, par, W, H, D, tx, ty, err);
-    asv_launch_follow(true, k_cc_flatten, (unsigned)chunks, CC_THREADS, 0, st, par, cid, ni, chunk, err);
+    const bool sparse = n <= (long long)CC_SPARSE * tiles;
+    if (sparse) {
+        const unsigned blocks = (unsigned)((n + CC_THREADS - 1) / CC_THREADS);
+        asv_launch_follow(false, k_cc_runs, blocks, CC_THREADS, 0, st, lab, par, cid, W, ni);
+        asv_launch_follow(true, k_cc_link, blocks, CC_THREADS, 0, st, lab, par, W, H, D, ni, err);
+    } else {
+        asv_launch_follow(false, k_cc_tile, tiles, CC_THREADS, 0, st, lab, par, cid, W, H, D, tx, ty, err);
+        asv_launch_follow(true, k_cc_union, tiles, CC_THREADS, 0, st, lab, par, W, H, D, tx, ty, err);
+    }
+    asv_launch_follow(true, sparse ? k_cc_flatten<true> : k_cc_flatten<false>, (unsigned)chunks, CC_THREADS, 0, st, par, cid, ni, chunk, err);
     asv_launch_follow(true, k_cc_prefix, 1, 1024, 0, st, chunk, (int)chunks, nullptr, R);
     asv_launch_follow(true, k_cc_compact, (unsigned)chunks, CC_THREADS, 0, st, par, cid, chunk, ni, rvox, rsize);
     // the segments' kernels: enough threads for a few segments per chunk, any

@@ -15,7 +15,7 @@ CHAINS = {
         "k_fl_up": {"coarse": ["F", "G"]}, "k_fl_iter": {"fin": ["fx_in", "fy_in"]}, "k_fl_store": {"flow": []},
     },
     "asv_connect.cu": {
-        "k_cc_tile": {}, "k_cc_union": {"par": []}, "k_cc_flatten": {"par": [], "cnt": []},
+        "k_cc_tile": {}, "k_cc_union": {"par": []}, "k_cc_runs": {}, "k_cc_link": {"par": []}, "k_cc_flatten": {"par": [], "cnt": []},
         "k_cc_prefix": {"chunk": [], "count": []}, "k_cc_compact": {"chunk": []}, "k_cc_kept_count": {"rsize": []},
         "k_cc_nodes": {"chunk": []}, "k_cc_jump": {"node": []}, "k_cc_output": {"node": []},
     },
