@@ -354,7 +354,7 @@ __global__ void __launch_bounds__(CC_THREADS) k_cc_flatten(int *par, int *cnt, i
     const int v0 = blockIdx.x * CC_CHUNK + threadIdx.x;        // at most 2^31 - 1, as v0 + k * CC_THREADS
     int r[IT];
 #pragma unroll
-    for (int k = 0; k < IT; k++) r[k] = v0 + k * CC_THREADS < n ? __ldcg(par + v0 + k * CC_THREADS) : -1;
+    for (int k = 0; k < IT; k++) r[k] = v0 + k * CC_THREADS < n ? par[v0 + k * CC_THREADS] : -1;
     bool walk = true;
     for (int it = 0; walk && it < CC_SPIN_LIMIT; it++) {       // the eight walks side by side
         walk = false;

@@ -230,22 +230,23 @@ __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__
     // a thread's pixels of a step: the same columns and rows of S every time.
     // Their flow is loaded a step ahead (before the vertical sums), so that a
     // step waits for the samples only, two or three pixels' at a time.
-    int cx[FL_PX], pr_[FL_PX];                                           // column in the frame; row of S and place in it
+    unsigned px[FL_PX];                                                  // column in the frame, row (3 bits) and place
     unsigned keepx = 0u;
     float fx[FL_PX], fy[FL_PX];
 #pragma unroll
     for (int k = 0; k < FL_PX; k++) {
         const int i = min(t + k * FL_NT, FL_RS * FL_RW - 1), r = i / FL_RW, q = i - r * FL_RW, gx = x0 - FL_BOX + q;
-        cx[k] = min(max(gx, 0), W - 1);
         if (gx >= 0 && gx < W) keepx |= 1u << k;                         // zero outside the frame
-        pr_[k] = t + k * FL_NT < FL_RS * FL_RW ? (r << 16) | (r * FL_SP + q + (q >> 2)) : -1;
+        px[k] = ((unsigned)min(max(gx, 0), W - 1) << 13) | (r << 10) | (r * FL_SP + q + (q >> 2));   // (10 bits) in S
     }
+    auto col_of = [&](int k) { return (int)(px[k] >> 13); };
+    auto row_of = [&](int k) { return (int)(px[k] >> 10) & (FL_RS - 1); };
     auto load_flow = [&](int y) {
 #pragma unroll
         for (int k = 0; k < FL_PX; k++) {
-            const int e = min(max(y + (pr_[k] >> 16), 0), H - 1) * W + cx[k];
-            fx[k] = fx_in[e];
-            fy[k] = fy_in[e];
+            const int e = min(max(y + row_of(k), 0), H - 1) * W + col_of(k);
+            fx[k] = asv_load_behind(fx_in + e);
+            fy[k] = asv_load_behind(fy_in + e);
         }
     };
 
@@ -258,15 +259,15 @@ __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__
 #pragma unroll
             for (int u = 0; u < 3 && k0 + u < FL_PX; u++) {
                 const int k = k0 + u;
-                fl_matrix<THIN>(sA, sB, dA, dB, W, H, cx[k], min(max(y + (pr_[k] >> 16), 0), H - 1), fx[k], fy[k], o[u]);
+                fl_matrix<THIN>(sA, sB, dA, dB, W, H, col_of(k), min(max(y + row_of(k), 0), H - 1), fx[k], fy[k], o[u]);
             }
 #pragma unroll
             for (int u = 0; u < 3 && k0 + u < FL_PX; u++) {
-                const int k = k0 + u, gy = y + (pr_[k] >> 16);
-                if (pr_[k] < 0) continue;
+                const int k = k0 + u, gy = y + row_of(k);
+                if (t + k * FL_NT >= FL_RS * FL_RW) continue;
                 const bool keep = (keepx >> k) & 1u && gy >= 0 && gy < H;
 #pragma unroll
-                for (int c = 0; c < 5; c++) S[c * FL_RS * FL_SP + (pr_[k] & 0xffff)] = keep ? o[u][c] : 0.f;
+                for (int c = 0; c < 5; c++) S[c * FL_RS * FL_SP + (px[k] & 1023u)] = keep ? o[u][c] : 0.f;
             }
         }
         __syncthreads();

@@ -481,7 +481,7 @@ __device__ __forceinline__ int asv_slice_list(const int32_t *in, int zoff, const
 #pragma unroll
     for (int oy = 0; oy < 3; oy++)
 #pragma unroll
-        for (int ox = 0; ox < 3; ox++) c[oy * 3 + ox] = in[zoff + ys[oy] + xs[ox]];
+        for (int ox = 0; ox < 3; ox++) c[oy * 3 + ox] = asv_load_behind(in + zoff + ys[oy] + xs[ox]);
     int n = 0;
 #pragma unroll
     for (int k = 0; k < 9; k++) {
