@@ -372,10 +372,14 @@ __global__ void __launch_bounds__(FL_NT, 5) k_fl_iter(const float4 *__restrict__
 
 // Rows of a strip per block: a multiple of the eight of a step such that the
 // blocks' rounds on the GPU take least, a block costing its rows, the twelve
-// before them and about as much as four more to start
-static int fl_rows(int W, int H, int P, int resident)
+// before them and about as much as four more to start.  Frames of up to three steps
+// go in one strip where that gives every other SM two blocks, which fill it: a
+// second strip would do the twelve rows again beside them (500x17x20: 228 us in
+// two, 163 in one; 200x20x30 180 and 164; 64x17x40, half a block per SM, 104 and 139).
+static int fl_rows(int W, int H, int P, int sms, int resident)
 {
     const long long columns = (long long)((W + FL_TW - 1) / FL_TW) * P;
+    if (H <= 3 * FL_RS && 2 * columns >= 3 * sms) return (H + FL_RS - 1) / FL_RS * FL_RS;
     int best = FL_RS;
     long long least = 0;
     for (int r = FL_RS; r <= ((H + FL_RS - 1) / FL_RS) * FL_RS; r += FL_RS) {
@@ -572,7 +576,7 @@ int asv_launch_flow(const uint8_t *rgb, int W, int H, int D, float2 *fwd, float2
         else
             asv_launch_follow(true, k_fl_up, dim3((w + FL_T - 1) / FL_T, (h + FL_UP_ROWS - 1) / FL_UP_ROWS, P), FL_T, 0, st,
                               flow[k + 1], Ws[k + 1], Hs[k + 1], flow[k], w, h, P);
-        const int rows = fl_rows(w, h, P, sms * (per > 0 ? per : 1));
+        const int rows = fl_rows(w, h, P, sms, sms * (per > 0 ? per : 1));
         const unsigned blocks = (unsigned)((w + FL_TW - 1) / FL_TW) * ((h + rows - 1) / rows) * P;
         for (int it = 0; it < 10; it++) {                 // even count: the result ends in flow[k]
             const float *fin = (it & 1) ? alt : flow[k];
