@@ -1674,6 +1674,7 @@ __global__ void __launch_bounds__(256, 4) k_jfa_second(AsvDev d, bool undraw)
 // on the device, where a streaming window's seeds are counted (k_stream_compose).
 __global__ void k_pass_prepare(int32_t *lbl, const __grid_constant__ SegDesc one, const SegDesc *seg, SegDesc *out)
 {
+    asv_follow();                                             // (the pass may start beside it)
     const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int Kp = seg->Kp;
     if (v < one.nvox && (unsigned)lbl[v] >= (unsigned)Kp) lbl[v] = -1;

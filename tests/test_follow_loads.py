@@ -20,7 +20,7 @@ CHAINS = {
         "k_cc_nodes": {"chunk": []}, "k_cc_jump": {"node": []}, "k_cc_output": {"node": []},
     },
     "asv_volume.cu": {
-        "k_jfa": {"in": []}, "k_jfa_first": {}, "k_jfa_second": {}, "k_post_stats": {}, "k_post_chunk_max": {},
+        "k_pass_prepare": {}, "k_jfa": {"in": []}, "k_jfa_first": {}, "k_jfa_second": {}, "k_post_stats": {}, "k_post_chunk_max": {},
         "k_post_prefix": {}, "k_post_apply": {},
     },
     "asv_metric.cu": {"k_metric_self": {}, "k_metric_ring": {}, "k_metric_combine": {}},
