@@ -29,11 +29,12 @@
 // that cross tiles are made in global memory, between sets of known size.  Of its
 // 12 earlier neighbours a voxel links only those that the links of others don't
 // imply (cc_links), all kinds in one loop, so that the lanes' walks run side by
-// side.  On the 320x240x85 clip's labels: 12 links per voxel, one after the
+// side.  Volumes whose tiles would be nearly empty are linked voxel by voxel in
+// global memory.  On the 320x240x85 clip's labels: 12 links per voxel, one after the
 // other, 543 us; a root walk and an atomic per voxel 113 us, segments numbered by
 // few blocks 91 us, 18 jumping rounds 60 us; now 95 us in the tiles
 // and 58 between them, 28, 12 and 17 us.
-// Compiled with -fmad=false (integer work only).
+// Integer work only: compiled without -fmad=false.
 #include "asv_connect.cuh"
 
 #include "asv_common.cuh"

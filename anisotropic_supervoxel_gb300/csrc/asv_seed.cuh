@@ -59,7 +59,7 @@ __device__ __forceinline__ void asv_reseed(const AsvDev &d, const SegDesc &S, in
 __device__ __forceinline__ void asv_draw_seed(const AsvDev &d, const SegDesc &S, int g, int i, float4 p, float4 c,
                                               const float *m)
 {
-    // table: (-x, -y, -z, -L) (M00, M11, 2M01, 2M12) (2M02, M22, -a, -b),
+    // table: (-x, -y, -z, -L) (M00, M11, 2M02, 2M12) (2M01, M22, -a, -b),
     // laid out for asv_jfa_dist's paired operations.  v - s == v + (-s) in
     // IEEE arithmetic, and doubling is exact, so
     // (dx*dy)*(2*M01) == ((2*dx)*dy)*M01 (flood.gs:85).

@@ -745,10 +745,10 @@ __device__ __forceinline__ void asv_jfa_run_far(const int32_t *in, int32_t *__re
 // sub-tile (16 x 16 columns x up to 16 chain positions of the tile) holds
 // few distinct labels in its whole footprint (the sub-tile grown by `step`
 // on every side; on the benchmarked clips mostly under 32).  So the block
-// copies the footprint and the sub-tile's LAB values into shared memory
-// with asynchronous copies (one memory latency per sub-tile), numbers the
-// footprint's distinct labels 0..T-1 (T <= 32, else the sub-tile takes the
-// list form) and turns every footprint entry into its label's bit.  A
+// copies the footprint into shared memory with asynchronous copies (one
+// memory latency per sub-tile), numbers the footprint's distinct labels
+// 0..T-1 (T <= 32; a sub-tile with more is cut in half, and takes the list form
+// below four positions) and turns every footprint entry into its label's bit.  A
 // voxel's candidate mask is the OR of the 9 bits of each of its three
 // slices (the plus slice's mask becomes the next position's centre mask);
 // a voxel with one candidate takes it, the others take the least score of

@@ -507,7 +507,7 @@ def run_batch16(args):
           {"workload": "batch16_uneven", "clips": len(dims),
            "voxels": sum(W * H * D for W, H, D, _ in dims), "K_total": sum(d[3] for d in dims),
            "lloyd_iters": I, "variant": "plain", "parallelism": "replicas1",
-           "jfa_zrun": zrun, "tiles": "autotuned (asv_autotune over depths 4/8/16/32)",
+           "jfa_zrun": zrun, "tiles": "autotuned (asv_autotune: the estimated depth, or the best of 4/8/16/32 as given)",
            "l2": "flushed before every step (512 MiB write)"},
           {"e2e": {"value": vox_it * args.steps / e2e_s / 1e6, "unit": UNIT,
                    "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},

@@ -182,9 +182,10 @@ asv_status asv_run_lloyd(asv_ctx *ctx);
  * step's chains: deeper shares more slice work, shallower fills the GPU
  * better) and returns the fastest of them in *zrun (may be NULL).  This
  * context keeps it, also for its later layouts, unless the loop is faster at
- * the depth estimated from the clip sizes, which it then keeps.  Needs a context ready for
- * asv_run_lloyd (clip or batch, not streaming); leaves the labels of a
- * complete run, which do not depend on the depth. */
+ * the depth estimated from the clip sizes, which it then keeps (and its later
+ * layouts their own).  Needs a context ready for asv_run_lloyd (clip or batch,
+ * not streaming); leaves the labels of a complete run, which do not depend on
+ * the depth. */
 asv_status asv_autotune(asv_ctx *ctx, int *zrun);
 
 /* Convenience: init_gpu + upload_flow + initialization + seed_matrix +
