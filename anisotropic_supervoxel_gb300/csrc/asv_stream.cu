@@ -163,5 +163,14 @@ cudaError_t asv_copy_d2d(void *dst, const void *src, size_t bytes, cudaStream_t 
         k_copy16<<<(unsigned)(want < cap ? want : cap), 256, 0, st>>>((const uint4 *)src, (uint4 *)dst, n);
         return cudaGetLastError();
     }
+    if (!apart && a < b) {
+        // a shift by less than its length (windows of fewer than 20 frames): in
+        // pieces that are apart, each behind the ones whose place it takes
+        for (size_t o = 0, step = b - a; o < bytes; o += step) {
+            const cudaError_t e = asv_copy_d2d((char *)dst + o, (const char *)src + o, bytes - o < step ? bytes - o : step, st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st);
 }
